@@ -155,10 +155,10 @@ struct orctm_handle {
   double rtol = 1e-10;
   int maxit = 5000;
   double* b = nullptr;
-  double *xs = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr, *p1 = nullptr, *q = nullptr;
-  double *d = nullptr, *rw = nullptr;
-  float *r32b = nullptr, *r32 = nullptr, *z32 = nullptr, *p32a = nullptr, *p32b = nullptr,
-        *q32 = nullptr, *d32 = nullptr;
+  double *xs = nullptr, *r = nullptr;  // solution and outer residual
+  RbGeo R{};                           // red-black view of the columns
+  RbVectors<double> v64{};             // vectors of the reduced system, per precision
+  RbVectors<float> v32{};
   SolverState* S = nullptr;
   SolverState* S_tune = nullptr;  // scratch scalars for the autotuner
   SolverState* S_tune0 = nullptr; // their initial value
@@ -696,16 +696,31 @@ int setup(orctm_handle* h, const orctm_desc* d) {
   }
   if ((st = h->dev_alloc(&h->zo, n2))) return st;
 
-  // pivots of the preconditioner (the operator is constant: factorise once)
+  // red-black tables and pivots (the operator is constant: factorise once)
   {
-    double* d64;
-    float* d32;
-    if ((st = h->dev_alloc(&d64, (size_t)L.n3())) || (st = h->dev_alloc(&d32, (size_t)L.n3())))
+    RbGeo& R = h->R;
+    R.ie = IE; R.je = JE; R.ke = KE;
+    R.P2 = L.P / 2;
+    R.plane2 = L.plane / 2;
+    R.M = (IE - 1) / 2 + 1;
+    R.zwn = P.zwn;
+    R.izn = P.izn;
+    ORCTM_CUDA_OK(cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, h->device));
+    const size_t n2h = (size_t)R.plane2, n3h = (size_t)L.n3() / 2;
+    for (RbColour& c : R.col)
+      if ((st = h->dev_alloc(&c.kk, n2h)) || (st = h->dev_alloc(&c.we, n2h)) ||
+          (st = h->dev_alloc(&c.ns, n2h)) || (st = h->dev_alloc(&c.zw, n2h)) ||
+          (st = h->dev_alloc(&c.iz, n2h)))
+        return st;
+    double* r64;
+    float *r32, *b32;
+    if ((st = h->dev_alloc(&r64, n3h)) || (st = h->dev_alloc(&r32, n3h)) ||
+        (st = h->dev_alloc(&b32, n3h)))
       return st;
-    P.dinv64 = d64;
-    P.dinv32 = d32;
-    ORCTM_CUDA_OK(pcg_prepare_device());
-    launch_factor(G, P, d64, d32, h->stream);
+    R.dr64 = r64;
+    R.dr32 = r32;
+    R.db32 = b32;
+    launch_rb_setup(G, P, R, r64, r32, b32, h->stream);
     ORCTM_CUDA_OK(cudaGetLastError());
   }
   // solver scalars
@@ -715,7 +730,6 @@ int setup(orctm_handle* h, const orctm_desc* d) {
   if (!(h->hS = pinned_state_get())) return h->fail(ORCTM_E_NOMEM, "pinned host memory exhausted");
   std::memset(h->hS, 0, sizeof(SolverState));
   h->hS->max_blocks = maxb;
-  h->hS->rows = G.L.je - 2;
   h->hS->partials = h->partials;
   ORCTM_CUDA_OK(cudaMemcpyAsync(h->S, h->hS, sizeof(SolverState), cudaMemcpyHostToDevice, h->stream));
   ORCTM_CUDA_OK(cudaEventCreate(&h->ev0));
@@ -726,25 +740,21 @@ int setup(orctm_handle* h, const orctm_desc* d) {
   return ORCTM_OK;
 }
 
+template <typename T>
+int alloc_rb(orctm_handle* h, RbVectors<T>& v) {
+  const size_t n = (size_t)h->L.n3() / 2;  // zero-filled: values outside the unknowns stay 0
+  int st;
+  for (T** p : {&v.x, &v.r, &v.z, &v.p, &v.q, &v.u, &v.ub})
+    if (!*p && (st = h->dev_alloc(p, n))) return st;
+  return ORCTM_OK;
+}
+
 int ensure_solver_buffers(orctm_handle* h) {
   int st;
   const size_t n = (size_t)h->L.n3();
-  if (!h->b) {
-    if ((st = h->dev_alloc(&h->b, n)) || (st = h->dev_alloc(&h->xs, n)) ||
-        (st = h->dev_alloc(&h->r, n)) || (st = h->dev_alloc(&h->z, n)) ||
-        (st = h->dev_alloc(&h->p0, n)) || (st = h->dev_alloc(&h->p1, n)) ||
-        (st = h->dev_alloc(&h->q, n)) || (st = h->dev_alloc(&h->d, n)) ||
-        (st = h->dev_alloc(&h->rw, n)))
-      return st;
-  }
-  if (h->solver_mode == ORCTM_SOLVER_FP32_REFINED && !h->r32) {
-    if ((st = h->dev_alloc(&h->r32b, n)) || (st = h->dev_alloc(&h->r32, n)) ||
-        (st = h->dev_alloc(&h->z32, n)) || (st = h->dev_alloc(&h->p32a, n)) ||
-        (st = h->dev_alloc(&h->p32b, n)) || (st = h->dev_alloc(&h->q32, n)) ||
-        (st = h->dev_alloc(&h->d32, n)))
-      return st;
-  }
-  return ORCTM_OK;
+  for (double** p : {&h->b, &h->xs, &h->r})
+    if (!*p && (st = h->dev_alloc(p, n))) return st;
+  return h->solver_mode == ORCTM_SOLVER_FP32_REFINED ? alloc_rb(h, h->v32) : alloc_rb(h, h->v64);
 }
 
 int read_state(orctm_handle* h) {
@@ -753,18 +763,30 @@ int read_state(orctm_handle* h) {
   return ORCTM_OK;
 }
 
-// Eight PCG iterations (stencil + column kernel each) are captured once per
-// precision into a CUDA graph and replayed between convergence checks: the
-// vectors, the solver scalars and the kernel variants of a handle are fixed,
-// and after an even number of iterations the two p buffers are back in their
-// starting roles, so every chunk from iteration 8 on issues the same launches.
-// The graph is rebuilt when the variants change; with profiling on, the
-// launches go one by one (they are bracketed by events).
-constexpr int kPcgChunk = 8;
+// A chunk of PCG iterations (three kernels each) is captured once per
+// precision into the body of a graph's conditional while node: the vectors,
+// the solver scalars and the launch shapes of a handle are fixed.  The graph
+// is rebuilt when the shapes change; with profiling on, the launches go one
+// by one (they are bracketed by events).
+constexpr int kPcgChunk = 4;
 
-template <typename T, typename TX>
-int pcg_loop_graph(orctm_handle* h, const T* b, TX* x, T* r, T* z, T* pa, T* pb, T* q,
-                   cudaGraphExec_t* out) {
+template <typename T>
+RbVectors<T>& rb_vectors(orctm_handle* h);
+template <>
+RbVectors<double>& rb_vectors<double>(orctm_handle* h) { return h->v64; }
+template <>
+RbVectors<float>& rb_vectors<float>(orctm_handle* h) { return h->v32; }
+
+template <typename T>
+void pcg_iteration(orctm_handle* h, int cv, int sv) {
+  const RbVectors<T>& v = rb_vectors<T>(h);
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, cv, h->stream));
+  PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, sv, h->stream));
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, cv, h->stream));
+}
+
+template <typename T>
+int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
   const int pr = sizeof(T) == 4;
   const int cv = h->col_var[pr], sv = h->spmv_var[pr];
   if (h->pcg_graph[pr] && h->pcg_graph_key[pr][0] == cv && h->pcg_graph_key[pr][1] == sv) {
@@ -800,20 +822,14 @@ int pcg_loop_graph(orctm_handle* h, const T* b, TX* x, T* r, T* z, T* pa, T* pb,
     cudaGraphDestroy(g);
     return cuda_status(e);
   }
-  cudaError_t e0 = cudaSuccess;
-  T *pc = pa, *pn = pb;
-  for (int k = 0; k < kPcgChunk; ++k) {
-    if (e0 == cudaSuccess) e0 = launch_pcg_spmv<T>(h->G, h->P, h->S, z, pc, pn, q, 0, sv, h->stream);
-    launch_pcg_col<T, TX>(h->G, h->P, h->S, 2, b, x, r, pn, q, z, cv, h->stream);
-    std::swap(pc, pn);
-  }
+  for (int k = 0; k < kPcgChunk; ++k) pcg_iteration<T>(h, cv, sv);
   launch_pcg_continue(hc, h->S, kPcgChunk, h->stream);
   const cudaError_t e1 = cudaStreamEndCapture(h->stream, &body);
   // launches are counted from the iterations the solve reports, not here
   add_launches(-(long long)(launch_count() - before));
-  if (e0 != cudaSuccess || e1 != cudaSuccess) {
+  if (e1 != cudaSuccess) {
     cudaGraphDestroy(g);
-    return cuda_status(e0 != cudaSuccess ? e0 : e1);
+    return cuda_status(e1);
   }
   cudaGraphExec_t ex = nullptr;
   const cudaError_t e2 = cudaGraphInstantiate(&ex, g, 0ULL);
@@ -826,75 +842,61 @@ int pcg_loop_graph(orctm_handle* h, const T* b, TX* x, T* r, T* z, T* pa, T* pb,
   return ORCTM_OK;
 }
 
-template <typename T, typename TX>
-int pcg_loop(orctm_handle* h, int init_mode, const T* b, TX* x, T* r, T* z, T* pa, T* pb, T* q,
-             int maxit, int* iters, int* conv) {
-  const Geo& G = h->G;
+// One correction: A d = r (h->r) to the relative residual S->tol, added to h->xs.
+template <typename T>
+int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   const int pr = sizeof(T) == 4;
   const int cv = h->col_var[pr], sv = h->spmv_var[pr];
-  launch_pcg_col<T, TX>(G, h->P, h->S, init_mode, b, x, r, nullptr, nullptr, z, cv, h->stream);
+  const RbVectors<T>& v = rb_vectors<T>(h);
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_before<T>(h->R, h->S, h->r, v, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
-  int it = 0;
-  T *pc = pa, *pn = pb;
-  // the first chunk one by one (its first stencil launch forms p = z), then,
-  // unless profiling, the device-side loop: chunks of kPcgChunk iterations
-  // replayed by a conditional while node until the solve converges or another
-  // chunk would pass maxit; no host round trip in between.  The p buffers are
-  // back in their roles after every (even) chunk.
-  while (it < maxit) {
-    if (it > 0 && it % kPcgChunk == 0 && it + kPcgChunk <= maxit && !h->prof) {
-      cudaGraphExec_t ex;
-      int st;
-      if ((st = pcg_loop_graph<T, TX>(h, b, x, r, z, pa, pb, q, &ex))) return st;
-      launch_set_limit(h->S, maxit, h->stream);
-      ORCTM_CUDA_OK(cudaGraphLaunch(ex, h->stream));
-      ORCTM_CUDA_OK(cudaGetLastError());
+  int st;
+  // the loop on the device: chunks of kPcgChunk iterations replayed by a
+  // conditional while node until the solve converges or another chunk would
+  // pass maxit, with no host round trip in between; the iterations left before
+  // maxit, and all of them while profiling, one by one
+  int it = 0, conv = 0;
+  if (!h->prof && maxit >= kPcgChunk) {
+    cudaGraphExec_t ex;
+    if ((st = pcg_loop_graph<T>(h, &ex))) return st;
+    launch_set_limit(h->S, maxit, h->stream);
+    ORCTM_CUDA_OK(cudaGraphLaunch(ex, h->stream));
+    if ((st = read_state(h))) return st;
+    // every body run launches the whole chunk and the condition kernel; after
+    // convergence the chunk's remaining kernels return at once
+    it = h->hS->iter;
+    conv = h->hS->converged;
+    add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * (3 * kPcgChunk + 1));
+  }
+  while (!conv && it < maxit) {
+    pcg_iteration<T>(h, cv, sv);
+    ORCTM_CUDA_OK(cudaGetLastError());  // a rejected launch is reported at once
+    if (++it % kPcgChunk == 0 || it == maxit) {
       if ((st = read_state(h))) return st;
-      // every body run launches the whole chunk and the condition kernel;
-      // after convergence the chunk's remaining kernels return at once
-      const int done = h->hS->iter;
-      add_launches((long long)((done - it + kPcgChunk - 1) / kPcgChunk) * (2 * kPcgChunk + 1));
-      if (h->hS->converged) break;
-      // not converged: the loop stopped because one more chunk would pass
-      // maxit, after whole chunks, so the p buffers are in their roles
-      it = done;
-      continue;
-    } else {
-      PROF(h, ORCTM_PROF_PCG_SPMV,
-           ORCTM_CUDA_OK(launch_pcg_spmv<T>(G, h->P, h->S, z, pc, pn, q, it == 0, sv, h->stream)));
-      PROF(h, ORCTM_PROF_PCG_COL, (launch_pcg_col<T, TX>(G, h->P, h->S, 2, b, x, r, pn, q, z, cv, h->stream)));
-      ORCTM_CUDA_OK(cudaGetLastError());  // a rejected launch is reported at once
-      std::swap(pc, pn);
-      ++it;
-    }
-    if (it % kPcgChunk == 0 || it == maxit) {
-      int st;
-      ORCTM_CUDA_OK(cudaGetLastError());
-      if ((st = read_state(h))) return st;
-      if (h->hS->converged) break;
+      conv = h->hS->converged;
     }
   }
-  int st;
-  if ((st = read_state(h))) return st;
   *iters = h->hS->iter;
-  *conv = h->hS->converged;
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_after<T>(h->R, h->S, v, h->xs, h->stream));
+  ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
 }
 
-// Autotuner.  Times every usable variant of the column kernel and of the
-// stencil kernel on this handle's grid in precision T and keeps the fastest
-// (two untimed launches, then three timed with CUDA events).  It runs before
+// Autotuner.  Times every launch shape of the column kernel and of the stencil
+// kernel on this handle's grid in precision T and keeps the fastest
+// (one untimed launch, then two timed with CUDA events).  It runs before
 // the first solve of the precision, on solver vectors that the solve writes
-// before it reads them (x is zeroed before every inner solve), with scratch
-// solver scalars.  The variants compute bit-identical results (the dot
-// products are summed in a fixed order), so the choice changes only speed.
+// before it reads them, with scratch solver scalars.  The shapes compute
+// bit-identical results (the dot products are summed tile by tile in a fixed
+// order), so the choice changes only speed.
 // Choices are cached per grid size and precision for later handles.
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune_cache;
 
 template <typename T>
-int autotune(orctm_handle* h, T* x, T* r, T* z, T* pa, T* pb, T* q) {
+int autotune(orctm_handle* h) {
   const Geo& G = h->G;
+  const RbVectors<T>& v = rb_vectors<T>(h);
   const int pr = sizeof(T) == 4;
   const auto key = std::make_tuple(G.L.ie, G.L.je, G.L.ke, pr);
   {
@@ -912,7 +914,9 @@ int autotune(orctm_handle* h, T* x, T* r, T* z, T* pa, T* pb, T* q) {
     SolverState s0 = *h->hS;
     s0.converged = 0;
     s0.alpha = 0.0;
+    s0.alpha_prev = 0.0;
     s0.beta = 0.0;
+    s0.iter = 1;
     s0.rho = 1.0;
     s0.bb = 1.0;
     s0.tol = 0.0;
@@ -922,13 +926,13 @@ int autotune(orctm_handle* h, T* x, T* r, T* z, T* pa, T* pb, T* q) {
   }
   auto timed = [&](auto launch, float* best_ms) -> int {
     float tot = 0.f;
-    for (int rep = 0; rep < 5; ++rep) {
+    for (int rep = 0; rep < 3; ++rep) {
       ORCTM_CUDA_OK(cudaMemcpyAsync(h->S_tune, h->S_tune0, sizeof(SolverState),
                                     cudaMemcpyDeviceToDevice, h->stream));
-      if (rep >= 2) ORCTM_CUDA_OK(cudaEventRecord(h->ev0, h->stream));
+      if (rep >= 1) ORCTM_CUDA_OK(cudaEventRecord(h->ev0, h->stream));
       launch();
       ORCTM_CUDA_OK(cudaGetLastError());
-      if (rep >= 2) {
+      if (rep >= 1) {
         ORCTM_CUDA_OK(cudaEventRecord(h->ev1, h->stream));
         ORCTM_CUDA_OK(cudaEventSynchronize(h->ev1));
         float ms = 0.f;
@@ -941,23 +945,15 @@ int autotune(orctm_handle* h, T* x, T* r, T* z, T* pa, T* pb, T* q) {
   };
   int st, best_c = 0, best_s = 0;
   float bc = 1e30f, bs = 1e30f;
-  for (int v = 0; v < pcg_col_variants(); ++v) {
-    if (!pcg_col_variant_ok<T>(G, v)) continue;
+  for (int c = 0; c < pcg_col_variants(); ++c) {
     float ms;
-    if ((st = timed([&] { launch_pcg_col<T, T>(G, h->P, h->S_tune, 2, nullptr, x, r, pa, q, z, v,
-                                               h->stream); }, &ms)))
-      return st;
-    if (ms < bc) { bc = ms; best_c = v; }
+    if ((st = timed([&] { launch_rb_col<T>(h->R, h->S_tune, v, c, h->stream); }, &ms))) return st;
+    if (ms < bc) { bc = ms; best_c = c; }
   }
-  for (int v = 0; v < pcg_spmv_variants(); ++v) {
-    if (!pcg_spmv_variant_ok(v)) continue;
+  for (int c = 0; c < pcg_spmv_variants(); ++c) {
     float ms;
-    cudaError_t le = cudaSuccess;
-    if ((st = timed([&] { le = launch_pcg_spmv<T>(G, h->P, h->S_tune, z, pa, pb, q, 0, v, h->stream); },
-                    &ms)))
-      return st;
-    if (le != cudaSuccess) continue;
-    if (ms < bs) { bs = ms; best_s = v; }
+    if ((st = timed([&] { launch_rb_black<T>(h->R, h->S_tune, v, c, h->stream); }, &ms))) return st;
+    if (ms < bs) { bs = ms; best_s = c; }
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -976,16 +972,7 @@ int ensure_tuned(orctm_handle* h, bool f32) {
     h->spmv_var[pr] = h->force_spmv;
     return ORCTM_OK;
   }
-  if (f32) return autotune<float>(h, h->d32, h->r32, h->z32, h->p32a, h->p32b, h->q32);
-  return autotune<double>(h, h->d, h->rw, h->z, h->p0, h->p1, h->q);
-}
-
-// converged = 4: a bounded wait inside a kernel (a TMA stage that never
-// arrived) gave up; the solve stops and reports it as a device error.
-int check_device_wait(orctm_handle* h, int conv) {
-  if (conv != 4) return ORCTM_OK;
-  h->err = "a device-side wait for a staged copy timed out in the Poisson stencil kernel";
-  return ORCTM_E_CUDA;
+  return f32 ? autotune<float>(h) : autotune<double>(h);
 }
 
 // Solves A x = b (b in h->b, x in h->xs holding the warm start) by iterative
@@ -1003,7 +990,7 @@ int poisson_solve(orctm_handle* h, orctm_solve_stats* stats) {
   int total = 0, outer = 0;
   double prev = 1e300, rel = 0.0;
   for (;; ++outer) {
-    launch_solver_reset(h->S, h->rtol, 0, h->stream);
+    launch_solver_reset(h->S, h->rtol, h->stream);
     PROF(h, ORCTM_PROF_RESID, launch_resid(G, h->P, h->S, h->b, h->xs, h->r, h->stream));
     ORCTM_CUDA_OK(cudaGetLastError());
     if ((st = read_state(h))) return st;
@@ -1020,26 +1007,11 @@ int poisson_solve(orctm_handle* h, orctm_solve_stats* stats) {
     prev = rel;
     double inner = 0.3 * h->rtol / rel;
     inner = std::min(0.5, std::max(inner, f32 ? 2e-5 : 1e-13));
-    int its = 0, conv = 0;
-    if (f32) {
-      launch_scale_to_f32(G, h->r, h->S, h->r32b, h->stream);
-      ORCTM_CUDA_OK(cudaMemsetAsync(h->d32, 0, sizeof(float) * n3, h->stream));
-      launch_solver_reset(h->S, inner, 0, h->stream);
-      if ((st = pcg_loop<float, float>(h, 1, h->r32b, h->d32, h->r32, h->z32, h->p32a, h->p32b,
-                                       h->q32, h->maxit - total, &its, &conv)))
-        return st;
-      if ((st = check_device_wait(h, conv))) return st;
-      launch_axpy_f32(G, h->d32, h->S, h->xs, h->stream);
-    } else {
-      ORCTM_CUDA_OK(cudaMemsetAsync(h->d, 0, sizeof(double) * n3, h->stream));
-      launch_solver_reset(h->S, inner, 0, h->stream);
-      if ((st = pcg_loop<double, double>(h, 1, h->r, h->d, h->rw, h->z, h->p0, h->p1, h->q,
-                                         h->maxit - total, &its, &conv)))
-        return st;
-      if ((st = check_device_wait(h, conv))) return st;
-      launch_axpy_f64(G, h->d, h->xs, h->stream);
-    }
-    ORCTM_CUDA_OK(cudaGetLastError());
+    int its = 0;
+    launch_solver_reset(h->S, inner, h->stream);
+    if ((st = f32 ? pcg_loop<float>(h, h->maxit - total, &its)
+                  : pcg_loop<double>(h, h->maxit - total, &its)))
+      return st;
     total += its;
   }
   ORCTM_CUDA_OK(cudaEventRecord(h->ev1, h->stream));
@@ -2693,14 +2665,15 @@ int orctm_estimate_device_bytes(const orctm_desc* d, int solver, unsigned long l
   const double plane = P * (d->je + 1), n3 = plane * (d->ke + 1);
   // 3D buffers: 12 state fields and the tracers, the routine temporaries of
   // the field pool (at most max(8, 2 ntracers + 2), the advection of all
-  // tracers at once, plus the step's initial transports held for it), 9
-  // FP64 solver vectors, the FP64 + FP32 pivots, and 7
-  // FP32 vectors for the refined solver
+  // tracers at once, plus the step's initial transports held for it), 3
+  // FP64 solver vectors, the pivots, and 7 half-length vectors of the
+  // reduced system (in FP64, and for the refined solver in FP32 too: a handle
+  // that has solved in both forms holds both)
   const double tmp = std::max(8.0, 2.0 * d->ntracers + 2.0) + 3.0;  // + the held transports
-  const double f3 = 12.0 + d->ntracers + tmp + 9.0 + 1.5 +
-                    (solver == ORCTM_SOLVER_FP32_REFINED ? 3.5 : 0.0);
+  const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 1.0 +
+                    (solver == ORCTM_SOLVER_FP32_REFINED ? 5.25 : 3.5);
   // 2D tables (compressed columns, metrics, biharmonic and Poisson factors)
-  const double f2 = 96.0;
+  const double f2 = 102.0;
   // every array carries two guard zones of about one plane
   const double guard = 2.0 * (plane + 2.0 * P + 64.0);
   *bytes = (unsigned long long)((f3 * (n3 + guard) + f2 * (plane + guard) + 16.0 * guard) * 8.0) +

@@ -14,19 +14,41 @@ struct PoissonGeo {
   const double *zpa, *zpb, *zpc;               // ZP at levels kb-1, kb, kb+1 (2D)
   const double *zwn, *zpn;                     // ZW(K), K=1..KE+1 and ZP(K), K=1..KE elsewhere
   const double *iza, *izb, *izc, *izn;         // 1/ZP = (1/ZW(K) + 1/ZW(K+1))/2, same selection
-  const double* dinv64;                        // pivots 1/d'(K) of the column tridiagonal of B (3D)
-  const float* dinv32;                         // the same rounded to FP32
+};
+
+// Red-black view of the Poisson columns (poisson.cu): column (i, j) is red when
+// i + j is even; column m = i / 2 of row j in a compact layout of pitch P/2.
+// 2D data of one colour's columns:
+struct RbColour {
+  unsigned long long* kk;     // wet levels: own, west, east, north, south, 10 bits each
+  double2 *we, *ns;           // XU(I-1) XP, XU(I) XP ; YV(J-1) YP, YV(J) YP
+  double2 *zw, *iz;           // ZW at levels kb, kb+1 ; 1/ZP at levels kb-1, kb
+};
+struct RbGeo {
+  int ie, je, ke;
+  int P2, plane2;             // P / 2, P / 2 * JN
+  int M;                      // columns m = 0..M-1 hold every unknown of a row
+  int sms;                    // multiprocessors of the device
+  RbColour col[2];            // red, black
+  const double *zwn, *izn;
+  const double* dr64;         // red pivots 1/d'(K) of the column tridiagonal of B
+  const float *dr32, *db32;   // the same rounded to FP32; the black pivots
+};
+// Vectors of the reduced system (compact layout)
+template <typename T>
+struct RbVectors {
+  T *x, *r, *z, *p, *q;       // black
+  T *u, *ub;                  // red: D_r^-1 C p ; D_r^-1 b
 };
 
 // Device-resident scalars of one Krylov solve.
 struct SolverState {
-  double rho, beta, alpha, pq, rr, bb, tol, res_rr, res_bb;
-  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown, 4 a stage wait timed out
+  double rho, beta, alpha, alpha_prev, pq, rr, bb, tol, res_rr, res_bb;
+  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown
   int iter;
   int limit;      // iteration limit of the device-side loop (orctm handle's maxit)
   unsigned ticket;
-  int rows;          // JE - 2: rows of unknowns, the reduction's row count
-  int max_blocks;    // partial sums per quantity: 32-column chunks x rows
+  int max_blocks;    // partial sums per quantity: the most tiles of a kernel
   double* partials;  // [4 * max_blocks]
 };
 
@@ -170,35 +192,31 @@ void launch_nh_rhs(const Geo& G, const double* uoo, const double* uoo1, const do
                    const double* voe1, const double* wno, const double* wno1, const double* zo,
                    double* b, cudaStream_t st);
 // poisson.cu
-void launch_factor(const Geo& G, const PoissonGeo& P, double* dinv64, float* dinv32,
-                   cudaStream_t st);
+// fills the red-black tables and pivots (once per handle)
+void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, double* dr64, float* dr32,
+                     float* db32, cudaStream_t st);
 size_t solver_max_blocks(const Geo& G);
-template <typename T, typename TX>
-void launch_pcg_col(const Geo& G, const PoissonGeo& P, SolverState* S, int mode, const T* b, TX* x,
-                    T* r, const T* p, const T* q, T* z, int variant, cudaStream_t st);
+// the reduced system's set-up (r, z and the scalars from b, the full-layout
+// right-hand side), the three kernels of an iteration, and the correction's
+// addition to x (full layout).  The FP32 form scales b by 1/||b||_2.
 template <typename T>
-cudaError_t launch_pcg_spmv(const Geo& G, const PoissonGeo& P, SolverState* S, const T* z,
-                            const T* pold, T* pnew, T* q, int first, int variant,
-                            cudaStream_t st);
-// kernel variants the autotuner chooses between (a variant a grid cannot use
-// falls back to variant 0)
+void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbVectors<T>& v,
+                      cudaStream_t st);
+template <typename T>
+void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+template <typename T>
+void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+template <typename T>
+void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+template <typename T>
+void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x, cudaStream_t st);
+// launch shapes the autotuner chooses between (column kernels, stencil kernel)
 int pcg_col_variants();
-// raises the shared-memory opt-in of the column-kernel variants on the
-// current device (called once per handle at creation)
-cudaError_t pcg_prepare_device();
-template <typename T>
-bool pcg_col_variant_ok(const Geo& G, int variant);
 int pcg_spmv_variants();
-bool pcg_spmv_variant_ok(int variant);
 // r = b - A x in double-double, and x := 0 on land rows (their solution)
 void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const double* b, double* x,
                   double* r, cudaStream_t st);
-void launch_axpy_f64(const Geo& G, const double* d, double* x, cudaStream_t st);
-void launch_scale_to_f32(const Geo& G, const double* r, const SolverState* S, float* r32,
-                         cudaStream_t st);
-void launch_axpy_f32(const Geo& G, const float* d, const SolverState* S, double* x,
-                     cudaStream_t st);
-void launch_solver_reset(SolverState* S, double tol, int keep_bb, cudaStream_t st);
+void launch_solver_reset(SolverState* S, double tol, cudaStream_t st);
 // device-side PCG loop: the limit of iterations, and the kernel that ends a
 // while-node body (keep looping while not converged and a further chunk of
 // `chunk` iterations stays within the limit)

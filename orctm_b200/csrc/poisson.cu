@@ -2,12 +2,9 @@
 // (petsc_solve_3D / ComputeRHS / compute_matrix, mo_petsc.f90:211-397,
 // 543-782).
 //
-// The operator is never assembled.  Each thread owns one water column and
-// loads the column's 2D data once (the neighbours' wet-level counts, which
-// decide the land/Neumann/Dirichlet cases, the products of the reciprocal
-// metrics XU, XP, YV, YP, and the column's bottom values of ZW, ZP, 1/ZP);
-// the per-level coefficients of compute_matrix then follow from 1D tables.
-// The matrix costs no HBM traffic.
+// The operator is never assembled: the wet-level counts of a column and its
+// four neighbours, the reciprocal metrics and 1D vertical tables give every
+// entry of compute_matrix, so the matrix costs next to no HBM traffic.
 //
 // The solve is iterative refinement: the outer residual r = b - A x is
 // accumulated in double-double (error-free FMA products) against the exact
@@ -15,23 +12,48 @@
 // preconditioned conjugate gradients (FP64, or FP32 for the refined form) on
 // the row-scaled operator B = diag(1/ZP) A, whose vertical couplings become
 // the symmetric ZW(K) and whose remaining asymmetry is confined to horizontal
-// couplings at partial bottom cells.  The preconditioner is the exact
-// column-tridiagonal (line) solve of B; its pivots are constant and are
-// factorised once at set-up.  A thread applies it to its own column: the
-// forward sweep leaves y' in the output vector (L2-resident) and the
-// backward sweep overwrites it with z.
+// couplings at partial bottom cells.
 //
-// Dot products are reduced deterministically: every block writes a partial
-// sum and the last block to finish (atomic ticket) adds the partials in
-// block order and updates the solver scalars on the device, so an iteration
-// needs no host round trip.  A device flag marks convergence; kernels of an
-// already converged solve return at once.
+// Red-black reduction.  Columns are coloured by i + j: the horizontal
+// couplings C of B join columns of opposite colour only, and what is left, D,
+// is one tridiagonal per column.  Eliminating the red columns leaves
+//     S = D_b - C_br D_r^-1 C_rb        on the black ones,
+// and conjugate gradients on S preconditioned with D_b take half the
+// iterations that they take on B preconditioned with D (the two have the same
+// spectrum up to lambda -> lambda (2 - lambda)), with vectors of half the
+// length.  One iteration is three kernels:
+//     red     u = D_r^-1 C_rb z + beta u        (u = D_r^-1 C_rb p)
+//     black   x += alpha p ; p = z + beta p ; q = D_b p - C_br u ; p.q
+//     column  r -= alpha q ; z = D_b^-1 r ; r.z, r.r
+// which move 14 half-length vectors and the pivots: 62 bytes per cell
+// in FP64, against 91 for an iteration of the unreduced solver before (and
+// twice as many iterations).  Red unknowns are formed from the black ones
+// before and after the iterations.
+//
+// Vectors are stored compactly per colour: column (i, j) at m = i / 2, so both
+// colours use offset m + P/2 (j + JN l).  The in-row neighbours of column
+// (m, j) are (m - 1 + s, j) and (m + s, j) of the other colour, s = 0 or 1 by
+// the parity of the row; north and south are (m, j -+ 1).
+//
+// A column is shared by G lanes of a warp, each with LC consecutive levels in
+// registers (a warp holds 32/G columns: 32-byte segments of a level's row).
+// The tridiagonal recurrences run level by level inside a lane and as a scan
+// of affine maps across the column's lanes, so the whole column is loaded at
+// once and nothing is spilled.  A thread that marches down a column alone
+// waits a memory latency every few levels: 27 us against 5 per launch on the
+// 512 x 1 x 60 slice, and 0.62 of the copy bandwidth on 1024 x 1024 x 80.
+//
+// Dot products are reduced deterministically: every tile writes a partial sum
+// and the last block to finish (atomic ticket) adds the partials in tile
+// order and updates the solver scalars on the device, so an iteration
+// needs no host round trip, and totals do not depend on the launch shape.  A
+// device flag marks convergence; kernels of an already converged solve return
+// at once.
 #include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
 #include "ops.h"
-#include "tma.cuh"
 
 namespace orctm {
 
@@ -40,9 +62,6 @@ namespace {
 #define AT(a, i, j, K) (a)[G.L.at((i), (j), (K)-1)]
 
 inline dim3 grid2(int nx, int ny, dim3 b) { return dim3((nx + b.x - 1) / b.x, (ny + b.y - 1) / b.y, 1); }
-inline dim3 grid3(int nx, int ny, int nz, dim3 b) {
-  return dim3((nx + b.x - 1) / b.x, (ny + b.y - 1) / b.y, nz);
-}
 
 // ------------------------------------------------------- coefficients ----
 struct Coef {
@@ -152,859 +171,513 @@ __device__ __forceinline__ Coef row(const ColC& c, const PoissonGeo& P, int K, i
   return r;
 }
 
-// vertical entries only (the preconditioner's tridiagonal)
-template <bool SCALED>
-__device__ __forceinline__ double down_of(const ColC& c, const PoissonGeo& P, int K, int KE) {
-  if (K > c.kb || K == KE || K + 1 > c.kb) return 0.0;
-  const double zw1 = zw_of(c, P, K + 1);
-  return SCALED ? zw1 : zw1 * zp_of(c, P, K);
-}
-
 // ------------------------------------------------------- reductions ------
-// Every kernel that reduces has blocks of 32 x BY threads, a warp being 32
-// consecutive columns i of one row j.  Each warp writes one partial sum at
-// its canonical index (row j, 32-column chunk), and the last block to finish
-// (atomic ticket) adds the partials in index order with a fixed 64-thread
-// pattern, so the totals do not depend on the block shape of the variant that
-// ran.  Returns true in thread 0 of the last block, which then holds the
-// totals in v.
+// Partial sums of one tile: the block's threads are added in a fixed order.
+constexpr int kThreads = 256, kWarps = kThreads / 32;
+
 template <int NV>
-__device__ bool grid_sum(double (&v)[NV], SolverState* S) {
-  __shared__ double sh[NV * 2];
-  __shared__ bool last;
-  const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
-  const unsigned nchunk = gridDim.x;
-  const unsigned nrow = (unsigned)S->rows;  // JE - 2 rows of unknowns
-  const unsigned row = blockIdx.y * blockDim.y + threadIdx.y;
+__device__ __forceinline__ void tile_partial(const double (&v)[NV], SolverState* S, int tile) {
+  __shared__ double sh[NV][kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
     double x = v[q];
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0 && row < nrow) S->partials[(size_t)q * S->max_blocks + row * nchunk + blockIdx.x] = x;
-  }
-  __threadfence();
-  __syncthreads();
-  const unsigned nb = gridDim.x * gridDim.y;
-  if (tid == 0) {
-    const unsigned t = atomicAdd(&S->ticket, 1u);
-    last = (t == nb - 1);
+    if (lane == 0) sh[q][warp] = x;
   }
   __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  const unsigned n = nrow * nchunk;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
+  if (threadIdx.x < NV) {
     double x = 0.0;
-    if (tid < 64)
-      for (unsigned b = tid; b < n; b += 64)
-        x += ((volatile double*)S->partials)[(size_t)q * S->max_blocks + b];
-    if (tid < 64) {
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) sh[q * 2 + (tid >> 5)] = x;
-    }
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) x += sh[threadIdx.x][w];
+    S->partials[(size_t)threadIdx.x * S->max_blocks + tile] = x;
   }
   __syncthreads();
-  if (tid == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = sh[q * 2] + sh[q * 2 + 1];
-    S->ticket = 0;
-  }
-  return tid == 0;
 }
 
-// The same reduction for blocks whose warps are identified by (row, chunk)
-// directly (blocks wider than 32 columns, or with a warp that owns no
-// columns: writes = false).  The partial index and the summation order are
-// those of grid_sum, so every form's totals agree bit for bit.
+// After a block's last tile: true in thread 0 of the last block to get here,
+// which then holds the totals over all tiles in v.
 template <int NV>
-__device__ bool grid_sum_rows(double (&v)[NV], SolverState* S, unsigned row, unsigned chunk,
-                              unsigned nchunk, bool writes) {
-  __shared__ double sh[NV * 2];
+__device__ bool grid_total(double (&v)[NV], SolverState* S, int ntiles) {
+  __shared__ double sh[NV][kWarps];
   __shared__ bool last;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y, lane = tid & 31;
-  const unsigned nrow = (unsigned)S->rows;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double x = v[q];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (writes && lane == 0 && row < nrow && chunk < nchunk)
-      S->partials[(size_t)q * S->max_blocks + row * nchunk + chunk] = x;
-  }
-  __threadfence();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < NV) __threadfence();
   __syncthreads();
-  const unsigned nb = gridDim.x * gridDim.y;
-  if (tid == 0) {
-    const unsigned t = atomicAdd(&S->ticket, 1u);
-    last = (t == nb - 1);
-  }
+  if (tid == 0) last = atomicAdd(&S->ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  const unsigned n = nrow * nchunk;
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
+    const double* part = S->partials + (size_t)q * S->max_blocks;
     double x = 0.0;
-    if (tid < 64)
-      for (unsigned b = tid; b < n; b += 64)
-        x += ((volatile double*)S->partials)[(size_t)q * S->max_blocks + b];
-    if (tid < 64) {
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) sh[q * 2 + (tid >> 5)] = x;
-    }
+#pragma unroll 8
+    for (int b = tid; b < ntiles; b += kThreads) x += __ldcg(part + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) sh[q][warp] = x;
   }
   __syncthreads();
   if (tid == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = sh[q * 2] + sh[q * 2 + 1];
+    for (int q = 0; q < NV; ++q) {
+      double x = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) x += sh[q][w];
+      v[q] = x;
+    }
     S->ticket = 0;
   }
   return tid == 0;
 }
 
 // ------------------------------------------------------- set-up ---------
+__device__ __forceinline__ int red_i(int m, int j) { return 2 * m + (j & 1); }
+__device__ __forceinline__ int black_i(int m, int j) { return 2 * m + 1 - (j & 1); }
+
 // Pivots of the column tridiagonal of B (constant): dinv(K) = 1/d'(K) with
-// d'(1) = d(1), d'(K) = d(K) - a(K) c(K-1) / d'(K-1).
-__global__ void k_factor(Geo G, PoissonGeo P, double* __restrict__ dinv64,
-                         float* __restrict__ dinv32) {
+// d'(1) = d(1), d'(K) = d(K) - a(K) c(K-1) / d'(K-1), per colour in the
+// compact layout: the red ones in FP64 and FP32 (the elimination is exact to
+// the solve's precision), the black ones, a fixed preconditioner, in FP32 for
+// both forms; and the 2D data of the columns.  Columns that are no unknowns
+// keep kk = 0 (no wet level).
+__global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, double* __restrict__ dr64,
+                           float* __restrict__ dr32, float* __restrict__ db32) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   const int KE = G.L.ke;
   if (i > G.L.ie - 1 || j > G.L.je - 1) return;
   const ColC c = load_col(G, P, i, j);
+  const bool black = (i + j) & 1;
+  const RbColour& q = R.col[black];
+  const int s = (i >> 1) + R.P2 * j;
+  q.kk[s] = (unsigned long long)c.kb | (unsigned long long)c.kbw << 10 |
+            (unsigned long long)c.kbe << 20 | (unsigned long long)c.kbn << 30 |
+            (unsigned long long)c.kbs << 40;
+  q.we[s] = make_double2(c.cw, c.ce);
+  q.ns[s] = make_double2(c.cn, c.cs);
+  q.zw[s] = make_double2(c.zwa, c.zwb);
+  q.iz[s] = make_double2(c.iza, c.izb);
   double dprev = 1.0, cprev = 0.0;
-  for (int K = 1; K <= KE; ++K) {
+  for (int K = 1; K <= c.kb; ++K) {
     const Coef r = row<true>(c, P, K, KE);
     const double d = K == 1 ? r.dc : r.dc - (r.u * dprev) * cprev;
     const double di = 1.0 / d;
-    AT(dinv64, i, j, K) = di;
-    AT(dinv32, i, j, K) = (float)di;
+    const int o = s + R.plane2 * (K - 1);
+    if (black) {
+      db32[o] = (float)di;
+    } else {
+      dr64[o] = di;
+      dr32[o] = (float)di;
+    }
     dprev = di;
     cprev = r.d;
   }
 }
 
 // ------------------------------------------------------- PCG kernels -----
+// Where a thread stands: G lanes per column, LC levels per lane.
+template <typename T, int G, int LC>
+struct Lane {
+  static constexpr int CW = 32 / G;          // columns per warp
+  static constexpr int CT = kWarps * CW;     // columns per tile
+  static constexpr int TAB = G * (LC + 1) + 1;
+  int m, g, K0, tab;                         // column, lane in it, first level - 1, its table entry
+  __device__ __forceinline__ Lane() {
+    const int lane = threadIdx.x & 31;
+    g = lane / CW;
+    m = (threadIdx.x >> 5) * CW + lane % CW;
+    K0 = g * LC;
+    tab = g * (LC + 1);
+  }
+};
 
-// Column kernel: residual update, z = M^-1 r (exact column tridiagonal of B),
-// dots r.z and r.r.
-//   MODE 1 (init, x = 0):   r = b / ZP   (the right-hand side of B x = b / ZP)
-//   MODE 2 (iteration):     x += alpha p ; r -= alpha q
-// The column tridiagonal is symmetric (a(K+1) = c(K) = ZW(K+1)), so
-// M = L D L^T with y = L^-1 r from the forward sweep and r.z = sum dinv y^2:
-// the dot needs no second pass over r.  With SM the forward values y are
-// kept in shared memory ([level][thread], blockDim.x * blockDim.y * KE
-// elements) for the backward sweep; otherwise they go through z.
-template <typename T, int MODE, bool SM, int U>
-__global__ void __launch_bounds__(128) k_pcg_col(Geo G, PoissonGeo P, SolverState* S,
-                                                 const T* __restrict__ b, T* __restrict__ x,
-                                                 T* __restrict__ r, const T* __restrict__ p,
-                                                 const T* __restrict__ q, T* __restrict__ z) {
-  extern __shared__ __align__(16) unsigned char col_smem[];
-  T* ys = reinterpret_cast<T*>(col_smem);
-  __shared__ T szw[kMaxKe + 1];
-  if (S->converged) return;
-  const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y, nt = blockDim.x * blockDim.y;
-  for (int e = tid; e <= KE; e += nt) szw[e] = (T)P.zwn[e];
+// ZW(K) at szw[e + e / LC], e = K - 1 = 0..KE, and 1/ZP(K) alike: the lanes
+// of a column read LC + 1 entries apart (no bank conflicts).
+template <typename T, int G, int LC>
+__device__ __forceinline__ void load_tables(const RbGeo& R, T* szw, T* siz) {
+  for (int e = threadIdx.x; e <= G * LC; e += kThreads) {
+    szw[e + e / LC] = e <= R.ke ? (T)R.zwn[e] : T(0);
+    if (siz) siz[e + e / LC] = e < R.ke ? (T)R.izn[e] : T(0);
+  }
   __syncthreads();
-  // arithmetic in T: the FP32 inner solve computes in FP32 (dots summed in T
-  // over U levels, then in FP64)
-  const T alpha = MODE == 2 ? (T)S->alpha : T(0);
-  // pivots rounded to FP32 in both precisions: a fixed preconditioner that
-  // moves half the bytes (the operator apply and the vectors keep precision T)
-  const float* __restrict__ dinv = P.dinv32;
-  double rz = 0.0, rr = 0.0, bb = 0.0;
-  if (i <= IE - 1 && j <= JE - 1) {
-    const ColC c = load_col(G, P, i, j);
-    const T zwa = (T)c.zwa;
-    const int kb = c.kb;
-    T yprev = 0, dprev = 0;
-    const unsigned base = (unsigned)G.L.at(i, j, 0), plane = (unsigned)G.L.plane;
-    // U: levels whose loads are issued together.  Levels below the bottom
-    // (K > kb) are land rows: decoupled, right-hand side 0, so every vector
-    // holds exact zeros there (k_resid clears x) and their dot terms are +0;
-    // they are neither loaded nor stored, while the lanes of a warp still
-    // march the levels together (their loads stay coalesced).
-    for (int K0 = 1; K0 <= KE; K0 += U) {
-      T lb[U], lr[U], lp[U], lq[U], lx[U], ld[U];
+}
+
+// Couplings a(K) between levels K - 1 and K of the lane's levels and of the one
+// below its last: ZW(K) inside the column (its own value at the bottom),
+// 0 at the surface and below the bottom.
+template <typename T, int G, int LC>
+__device__ __forceinline__ void couplings(const Lane<T, G, LC>& t, const T* szw, int kb, T zwa,
+                                          T (&a)[LC + 1]) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int K = K0 + u;
-        lb[u] = lr[u] = lp[u] = lq[u] = lx[u] = ld[u] = T(0);
-        if (K <= kb) {
-          const unsigned o = base + plane * (unsigned)(K - 1);
-          if (MODE == 1) {
-            lb[u] = b[o];
-          } else {
-            lr[u] = r[o];
-            lp[u] = p[o];
-            lq[u] = q[o];
-            lx[u] = x[o];
-          }
-          ld[u] = (T)dinv[o];
-        }
-      }
-      // partial dots are flushed to FP64 at every fourth level (K = 4, 8, ...)
-      // and at the end, whatever U is
-      T rzt = 0, rrt = 0, bbt = 0;
+  for (int u = 0; u <= LC; ++u) {
+    const int K = t.K0 + 1 + u;
+    const T zw = szw[t.tab + u + (u == LC)];
+    a[u] = (K == 1 || K > kb) ? T(0) : (K == kb ? zwa : zw);
+  }
+}
+
+// v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d and
+// couplings a; returns v.M^-1 v = sum y^2 / d of this lane's levels.
+template <typename T, int G, int LC>
+__device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, T (&v)[LC], const T (&d)[LC],
+                                          const T (&a)[LC + 1]) {
+  constexpr int CW = 32 / G;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the lane's levels as one affine
+  // map y_out = A y_in + B, scanned over the lanes above
+  const T dm = __shfl_up_sync(kAll, d[LC - 1], CW);
+  T A = T(1), B = T(0);
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int K = K0 + u;
-        if (K > KE) break;
-        if (u == 4) {
-          rz += (double)rzt;
-          rr += (double)rrt;
-          bb += (double)bbt;
-          rzt = rrt = bbt = 0;
-        }
-        const unsigned o = base + plane * (unsigned)(K - 1);
-        T rk;
-        const bool wetk = K <= kb;
-        if (MODE == 1) {
-          rk = (T)((double)lb[u] * izp_of(c, P, K));
-          bbt = fma(rk, rk, bbt);
-        } else {
-          if (wetk) x[o] = fma(alpha, lp[u], lx[u]);
-          rk = fma(-alpha, lq[u], lr[u]);
-        }
-        if (wetk) r[o] = rk;
-        rrt = fma(rk, rk, rrt);
-        // a(K) of B: ZW(K) above a wet level below the surface
-        const T up = (K == 1 || K > kb) ? T(0) : (K == kb ? zwa : szw[K - 1]);
-        const T yt = fma(-(up * dprev), yprev, rk);
-        if (SM) ys[(K - 1) * nt + tid] = yt;
-        else if (wetk) z[o] = yt;  // y kept in z until the backward sweep
-        yprev = yt;
-        dprev = ld[u];
-        rzt = fma(yt * yt, dprev, rzt);
-      }
-      rz += (double)rzt;
-      rr += (double)rrt;
-      bb += (double)bbt;
-    }
-    T znext = 0;
-    for (int K1 = KE; K1 >= 1; K1 -= U) {
-      T ly[U], ld[U];
+  for (int u = 0; u < LC; ++u) {
+    const T l = -(a[u] * (u ? d[u - 1] : dm));
+    B = fma(l, B, v[u]);
+    A = l * A;
+  }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int K = K1 - u;
-        ly[u] = ld[u] = T(0);
-        if (K >= 1 && K <= kb) {
-          const unsigned o = base + plane * (unsigned)(K - 1);
-          ly[u] = SM ? ys[(K - 1) * nt + tid] : z[o];
-          ld[u] = (T)dinv[o];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int K = K1 - u;
-        if (K < 1) break;
-        // c(K) of B: ZW(K+1) when level K+1 is wet
-        const T dn = (K >= kb || K == KE) ? T(0) : (K + 1 == kb ? zwa : szw[K]);
-        const T zt = fma(-dn, znext, ly[u]) * ld[u];
-        if (K <= kb) z[base + plane * (unsigned)(K - 1)] = zt;
-        znext = zt;
-      }
+  for (int o = CW; o < 32; o <<= 1) {
+    const T Ap = __shfl_up_sync(kAll, A, o), Bp = __shfl_up_sync(kAll, B, o);
+    if (lane >= o) {
+      B = fma(A, Bp, B);
+      A *= Ap;
     }
   }
-  double v[3] = {rz, rr, bb};
-  // warp (row, 32-column chunk) of this thread, for blocks of any width
-  const unsigned row = blockIdx.y * blockDim.y + threadIdx.y;
-  const unsigned chunk = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-  if (grid_sum_rows<3>(v, S, row, chunk, (unsigned)((IE - 2 + 31) / 32), true)) {
-    if (MODE == 2) {
-      S->beta = v[0] / S->rho;
+  T y = __shfl_up_sync(kAll, B, CW);
+  if (t.g == 0) y = T(0);
+  T rz = T(0);
+#pragma unroll
+  for (int u = 0; u < LC; ++u) {
+    y = fma(-(a[u] * (u ? d[u - 1] : dm)), y, v[u]);
+    v[u] = y * d[u];
+    rz = fma(y, v[u], rz);
+  }
+  // backward: z(K) = y(K) d(K) - a(K+1) d(K) z(K+1)
+  A = T(1);
+  B = T(0);
+#pragma unroll
+  for (int u = LC - 1; u >= 0; --u) {
+    const T l = -(a[u + 1] * d[u]);
+    B = fma(l, B, v[u]);
+    A = l * A;
+  }
+#pragma unroll
+  for (int o = CW; o < 32; o <<= 1) {
+    const T Ap = __shfl_down_sync(kAll, A, o), Bp = __shfl_down_sync(kAll, B, o);
+    if (lane + o < 32) {
+      B = fma(A, Bp, B);
+      A *= Ap;
+    }
+  }
+  T z = __shfl_down_sync(kAll, B, CW);
+  if (t.g == G - 1) z = T(0);
+#pragma unroll
+  for (int u = LC - 1; u >= 0; --u) {
+    z = fma(-(a[u + 1] * d[u]), z, v[u]);
+    v[u] = z;
+  }
+  return rz;
+}
+
+__device__ __forceinline__ int wet_levels(unsigned long long kk, int nb) {
+  return (int)((kk >> (10 * nb)) & 1023u);
+}
+
+// Red columns.
+//   kIter    u = D^-1 C v + beta u          (v = z; u is not read while beta = 0)
+//   kBefore  u = D^-1 (b / ZP)              (b: full layout, scaled); sum of (b / ZP)^2
+//   kAfter   x += scale (u - D^-1 C v)      (v = the black correction; x: full layout)
+enum { kIter = 0, kBefore = 1, kAfter = 2 };
+
+template <typename T, int G, int LC, int MODE>
+__global__ void __launch_bounds__(kThreads) k_rb_red(RbGeo R, SolverState* S,
+                                                     const T* __restrict__ v, T* __restrict__ u,
+                                                     const T* __restrict__ dinv,
+                                                     const double* __restrict__ b,
+                                                     double* __restrict__ x, int ntiles, int nmc) {
+  using Ln = Lane<T, G, LC>;
+  __shared__ T szw[Ln::TAB], siz[Ln::TAB];
+  if (MODE == kIter && S->converged) return;
+  const T beta = MODE == kIter ? (T)S->beta : T(0);
+  double scale = 1.0;
+  if (MODE != kIter && sizeof(T) == 4) {
+    scale = sqrt(S->res_rr);
+    if (MODE == kBefore) scale = scale > 0.0 ? 1.0 / scale : 0.0;
+  }
+  load_tables<T, G, LC>(R, szw, siz);
+  const Ln t;
+  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
+    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
+    unsigned long long kk = 0;
+    if (m < R.M) kk = R.col[0].kk[s2];
+    const int kb = wet_levels(kk, 0);
+    T cw = 0, ce = 0, cn = 0, cs = 0, zwa = 0;
+    double iza = 0, izb = 0;
+    if (kb) {
+      const double2 we = R.col[0].we[s2], ns = R.col[0].ns[s2], iz = R.col[0].iz[s2];
+      cw = (T)we.x; ce = (T)we.y; cn = (T)ns.x; cs = (T)ns.y;
+      zwa = (T)R.col[0].zw[s2].x;
+      iza = iz.x; izb = iz.y;
+    }
+    const unsigned o0 = s2 + plane * (unsigned)t.K0;
+    const unsigned ow = o0 - 1u + (unsigned)(j & 1);
+    T g[LC], d[LC], a[LC + 1];
+    couplings<T, G, LC>(t, szw, kb, zwa, a);
+    double bb = 0.0;
+#pragma unroll
+    for (int q = 0; q < LC; ++q) {
+      const int K = t.K0 + 1 + q;
+      const unsigned l = plane * (unsigned)q;
+      g[q] = d[q] = T(0);
+      if (K <= kb) {
+        d[q] = dinv[o0 + l];
+        if (MODE == kBefore) {
+          const double hs = K == kb ? izb : (K == kb - 1 ? iza : R.izn[K - 1]);
+          const unsigned f = (unsigned)red_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
+          g[q] = (T)((b[f] * scale) * hs);
+          bb = fma((double)g[q], (double)g[q], bb);
+        } else {
+          // values of land cells and outside the unknowns are exact zeros
+          const T hs = K == kb ? (T)izb : (K == kb - 1 ? (T)iza : siz[t.tab + q]);
+          T h = cw * v[ow + l];
+          h = fma(ce, v[ow + l + 1u], h);
+          h = fma(cn, v[o0 + l - P2], h);
+          h = fma(cs, v[o0 + l + P2], h);
+          g[q] = hs * h;
+        }
+      }
+    }
+    column_solve<T, G, LC>(t, g, d, a);
+#pragma unroll
+    for (int q = 0; q < LC; ++q) {
+      const int K = t.K0 + 1 + q;
+      const unsigned o = o0 + plane * (unsigned)q;
+      if (K <= kb) {
+        if (MODE == kIter) {
+          u[o] = beta == T(0) ? g[q] : fma(beta, u[o], g[q]);
+        } else if (MODE == kBefore) {
+          u[o] = g[q];
+        } else {
+          const unsigned f = (unsigned)red_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
+          x[f] = x[f] + scale * (double)(u[o] - g[q]);
+        }
+      }
+    }
+    if (MODE == kBefore) {
+      const double w[1] = {bb};
+      tile_partial<1>(w, S, tile);
+    }
+  }
+  if (MODE == kBefore) {
+    double w[1];
+    if (grid_total<1>(w, S, ntiles)) S->bb = w[0];
+  }
+}
+
+// Black columns: x += alpha p (the previous step's), p = z + beta p,
+// q = D p - C u, and alpha = rho / p.q.  The first iteration (iter = 0) reads
+// neither p nor x.
+template <typename T, int G, int LC>
+__global__ void __launch_bounds__(kThreads) k_rb_black(RbGeo R, SolverState* S,
+                                                       const T* __restrict__ z,
+                                                       const T* __restrict__ u, T* __restrict__ p,
+                                                       T* __restrict__ x, T* __restrict__ q,
+                                                       int ntiles, int nmc) {
+  using Ln = Lane<T, G, LC>;
+  __shared__ T szw[Ln::TAB], siz[Ln::TAB];
+  if (S->converged) return;
+  const T beta = (T)S->beta, alpha = (T)S->alpha_prev;
+  const bool first = S->iter == 0;
+  load_tables<T, G, LC>(R, szw, siz);
+  const Ln t;
+  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
+    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
+    unsigned long long kk = 0;
+    if (m < R.M) kk = R.col[1].kk[s2];
+    const int kb = wet_levels(kk, 0);
+    const int kbw = wet_levels(kk, 1), kbe = wet_levels(kk, 2);
+    const int kbn = wet_levels(kk, 3), kbs = wet_levels(kk, 4);
+    T cw = 0, ce = 0, cn = 0, cs = 0, zwa = 0, zwb = 0, iza = 0, izb = 0;
+    if (kb) {
+      const double2 we = R.col[1].we[s2], ns = R.col[1].ns[s2], iz = R.col[1].iz[s2],
+                    zw = R.col[1].zw[s2];
+      cw = (T)we.x; ce = (T)we.y; cn = (T)ns.x; cs = (T)ns.y;
+      zwa = (T)zw.x; zwb = (T)zw.y;
+      iza = (T)iz.x; izb = (T)iz.y;
+    }
+    const unsigned o0 = s2 + plane * (unsigned)t.K0;
+    const unsigned ow = o0 - (unsigned)(j & 1);
+    T pl[LC];
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const unsigned o = o0 + plane * (unsigned)e;
+      pl[e] = T(0);
+      if (t.K0 + 1 + e <= kb) {
+        T pn = z[o];
+        if (first) {
+          x[o] = T(0);
+        } else {
+          const T po = p[o];
+          x[o] = fma(alpha, po, x[o]);
+          pn = fma(beta, po, pn);
+        }
+        p[o] = pn;
+        pl[e] = pn;
+      }
+    }
+    T pu = __shfl_up_sync(0xffffffffu, pl[LC - 1], Ln::CW);
+    T pb = __shfl_down_sync(0xffffffffu, pl[0], Ln::CW);
+    if (t.g == 0) pu = T(0);
+    if (t.g == G - 1) pb = T(0);
+    T pq = T(0);
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const int K = t.K0 + 1 + e;
+      if (K <= kb) {
+        const unsigned o = o0 + plane * (unsigned)e, w = ow + plane * (unsigned)e;
+        const T p0 = pl[e], pd = e + 1 < LC ? pl[e + 1] : pb;
+        T dh = K <= kbw ? cw : T(0);
+        if (K <= kbe) dh += ce;
+        if (K <= kbn) dh += cn;
+        if (K <= kbs) dh += cs;
+        T h = cw * u[w];
+        h = fma(ce, u[w + 1u], h);
+        h = fma(cn, u[o - P2], h);
+        h = fma(cs, u[o + P2], h);
+        h = fma(dh, p0, h);
+        const T hs = K == kb ? izb : (K == kb - 1 ? iza : siz[t.tab + e]);
+        const T zw0 = K == kb ? zwa : szw[t.tab + e];
+        const T zw1 = K + 1 == kb ? zwa : szw[t.tab + e + 1 + (e + 1 == LC)];
+        T s = zw0 * (pu - p0);
+        if (K < kb) s = fma(zw1, pd - p0, s);
+        else if (K == 1) s = fma(-zwb, p0, s);  // Z_C of the surface row keeps ZW(2)
+        s = fma(-hs, h, s);
+        q[o] = s;
+        pq = fma(p0, s, pq);
+      }
+      pu = pl[e];
+    }
+    const double w[1] = {(double)pq};
+    tile_partial<1>(w, S, tile);
+  }
+  double w[1];
+  if (grid_total<1>(w, S, ntiles)) {
+    S->pq = w[0];
+    S->alpha = S->rho / w[0];
+    if (!(w[0] > 0.0) && !(w[0] < 0.0)) S->converged = 3;  // breakdown
+  }
+}
+
+// Black columns: residual, z = D_b^-1 r with the FP32 pivots, r.z and r.r.
+//   INIT   r = b / ZP - C u     (u = D_r^-1 (b / ZP) of the red columns)
+//   else   r -= alpha q
+template <typename T, int G, int LC, bool INIT>
+__global__ void __launch_bounds__(kThreads) k_rb_col(RbGeo R, SolverState* S, T* __restrict__ r,
+                                                     const T* __restrict__ q, T* __restrict__ z,
+                                                     const float* __restrict__ dinv,
+                                                     const double* __restrict__ b,
+                                                     const T* __restrict__ ub, int ntiles,
+                                                     int nmc) {
+  using Ln = Lane<T, G, LC>;
+  __shared__ T szw[Ln::TAB];
+  if (!INIT && S->converged) return;
+  const T alpha = INIT ? T(0) : (T)S->alpha;
+  double scale = 1.0;
+  if (INIT && sizeof(T) == 4) scale = S->res_rr > 0.0 ? 1.0 / sqrt(S->res_rr) : 0.0;
+  load_tables<T, G, LC>(R, szw, nullptr);
+  const Ln t;
+  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
+    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
+    unsigned long long kk = 0;
+    if (m < R.M) kk = R.col[1].kk[s2];
+    const int kb = wet_levels(kk, 0);
+    const T zwa = kb ? (T)R.col[1].zw[s2].x : T(0);
+    const unsigned o0 = s2 + plane * (unsigned)t.K0;
+    T g[LC], d[LC], a[LC + 1], rr = T(0);
+    double bb = 0.0;
+    couplings<T, G, LC>(t, szw, kb, zwa, a);
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const int K = t.K0 + 1 + e;
+      const unsigned o = o0 + plane * (unsigned)e;
+      g[e] = d[e] = T(0);
+      if (K <= kb) {
+        d[e] = (T)dinv[o];
+        if (INIT) {
+          const double2 we = R.col[1].we[s2], ns = R.col[1].ns[s2], iz = R.col[1].iz[s2];
+          const double hs = K == kb ? iz.y : (K == kb - 1 ? iz.x : R.izn[K - 1]);
+          const unsigned f = (unsigned)black_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
+          const unsigned w = o - (unsigned)(j & 1);
+          const T bs = (T)((b[f] * scale) * hs);
+          T h = (T)we.x * ub[w];
+          h = fma((T)we.y, ub[w + 1u], h);
+          h = fma((T)ns.x, ub[o - P2], h);
+          h = fma((T)ns.y, ub[o + P2], h);
+          bb = fma((double)bs, (double)bs, bb);
+          g[e] = fma(-(T)hs, h, bs);
+        } else {
+          g[e] = fma(-alpha, q[o], r[o]);
+        }
+        r[o] = g[e];
+        rr = fma(g[e], g[e], rr);
+      }
+    }
+    const T rz = column_solve<T, G, LC>(t, g, d, a);
+#pragma unroll
+    for (int e = 0; e < LC; ++e)
+      if (t.K0 + 1 + e <= kb) z[o0 + plane * (unsigned)e] = g[e];
+    if (INIT) {
+      const double w[3] = {(double)rz, (double)rr, bb};
+      tile_partial<3>(w, S, tile);
     } else {
-      S->bb = v[2];
+      const double w[2] = {(double)rz, (double)rr};
+      tile_partial<2>(w, S, tile);
+    }
+  }
+  double v[INIT ? 3 : 2];
+  if (grid_total<INIT ? 3 : 2>(v, S, ntiles)) {
+    if (INIT) {
+      S->bb += v[2];  // the red columns' part is there already
       S->beta = 0.0;
+      S->alpha_prev = 0.0;
+    } else {
+      S->beta = v[0] / S->rho;
+      S->alpha_prev = S->alpha;
+      S->iter += 1;
     }
     S->rho = v[0];
     S->rr = v[1];
-    S->iter += (MODE == 2);
     if (sqrt(v[1]) <= S->tol * sqrt(S->bb) || S->bb == 0.0) S->converged = 1;
     if (!(v[0] == v[0]) || !(v[1] == v[1])) S->converged = 2;  // NaN: stop
   }
 }
 
-// Stencil kernel: p = z + beta p_old (first iteration: p = z), q = B p, and
-// the dot p.q; alpha = rho / (p.q).  A block of 32 x kTy columns marches down
-// the levels; p of its 34 x (kTy+2) halo tile is formed once per level into a
-// three-level shared-memory ring, and the 7-point product reads the ring.
-// Arithmetic is in the storage type T (the FP32 inner solve computes in
-// FP32; the dot is accumulated per thread in T over 8 levels, then in FP64).
-// Offsets are 32-bit: a padded field has fewer than 2^31 elements
-// (checked when the handle is created).
-constexpr int kTx = 32;
-
-template <typename T, int kTy>
-__global__ void __launch_bounds__(kTx * kTy) k_pcg_spmv(Geo G, PoissonGeo P, SolverState* S,
-                                                       const T* __restrict__ z,
-                                                       const T* __restrict__ pold,
-                                                       T* __restrict__ pnew, T* __restrict__ q,
-                                                       int first) {
-  constexpr int kHx = kTx + 2, kHy = kTy + 2;
-  constexpr int kH = kHx * kHy, kNt = kTx * kTy, kF = (kH + kNt - 1) / kNt;
-  __shared__ T ring[3][kH];
-  __shared__ T szw[kMaxKe + 1], siz[kMaxKe];
-  if (S->converged) return;
-  const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const unsigned plane = (unsigned)G.L.plane;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + kTx * ty;
-  for (int e = tid; e <= KE; e += kNt) {
-    szw[e] = (T)P.zwn[e];
-    if (e < KE) siz[e] = (T)P.izn[e];
-  }
-  const int i0 = blockIdx.x * kTx + 2, j0 = blockIdx.y * kTy + 2;
-  const int i = i0 + tx, j = j0 + ty;
-  const bool act = i <= IE - 1 && j <= JE - 1;
-  const T beta = first ? T(0) : (T)S->beta;
-  // the deepest wet level of the block's columns: below it every cell of the
-  // block is a land row, whose p and q are exact zeros already in memory and
-  // whose dot terms are +0, so the march stops there (loads go one level
-  // further, for the level below the deepest wet row)
-  __shared__ int skmax;
-  if (tid == 0) skmax = 0;
-  __syncthreads();
-  if (act) atomicMax(&skmax, (int)G.gp.kb[G.L.at2(i, j)]);
-  __syncthreads();
-  const int kmax = skmax, klim = min(KE, kmax + 1);
-  // halo-tile entries this thread fills: offsets at level 1, validity, and
-  // the entry's wet levels (below them the values are exact zeros)
-  unsigned fo[kF];
-  int fs[kF], fk[kF];
-  bool fv[kF];
-#pragma unroll
-  for (int f = 0; f < kF; ++f) {
-    const int e = tid + f * kNt;
-    const int hy = e / kHx, hx = e - hy * kHx;
-    const int ii = i0 - 1 + hx, jj = j0 - 1 + hy;
-    fs[f] = e < kH ? e : -1;
-    fv[f] = e < kH && ii >= 2 && ii <= IE - 1 && jj >= 2 && jj <= JE - 1;
-    fo[f] = fv[f] ? (unsigned)G.L.at(ii, jj, 0) : 0u;
-    fk[f] = fv[f] ? (int)G.gp.kb[G.L.at2(ii, jj)] : 0;
-  }
-  // the halo values of two levels ahead are held in registers, so the loads of
-  // level K+3 are in flight while level K is computed
-  T qz[2][kF], qp[2][kF];
-  auto load = [&](int slot, int K) {
-#pragma unroll
-    for (int f = 0; f < kF; ++f) {
-      qz[slot][f] = T(0);
-      qp[slot][f] = T(0);
-      if (fv[f] && K <= klim && K <= fk[f]) {
-        const unsigned o = fo[f] + plane * (unsigned)(K - 1);
-        qz[slot][f] = z[o];
-        if (!first) qp[slot][f] = pold[o];
-      }
-    }
-  };
-  auto store = [&](T* dst, int slot) {
-#pragma unroll
-    for (int f = 0; f < kF; ++f)
-      if (fs[f] >= 0) dst[fs[f]] = first ? qz[slot][f] : fma(beta, qp[slot][f], qz[slot][f]);
-  };
-  ColC c;
-  T cw = 0, ce = 0, cn = 0, cs = 0, xyc = 0;
-  int kreg = 0;
-  if (act) {
-    c = load_col(G, P, i, j);
-    cw = c.iw ? (T)c.cw : T(0);
-    ce = c.ie ? (T)c.ce : T(0);
-    cn = c.in ? (T)c.cn : T(0);
-    cs = c.is ? (T)c.cs : T(0);
-    xyc = (T)(c.xcf + c.ycf);
-    kreg = c.kreg;
-  }
-  const unsigned own = act ? (unsigned)G.L.at(i, j, 0) : 0u;
-  const int kown = act ? (int)c.kb : 0;
-  const int me = (ty + 1) * kHx + (tx + 1);
-  T* prv = ring[0];
-  T* cur = ring[1];
-  T* nxt = ring[2];
-  for (int e = tid; e < kH; e += kNt) prv[e] = T(0);
-  load(0, 1);
-  store(cur, 0);
-  load(0, 2);
-  load(1, 3);
-  double pq = 0.0;
-  T pqt = T(0);
-  // one level; SA (the register slot holding level K+1) is a literal at every
-  // call so the register queue is never indexed dynamically
-  auto level = [&](int K, auto sa_c) {
-    constexpr int SA = decltype(sa_c)::value;
-    __syncthreads();  // the slot of level K-2 is free; level K is complete
-    store(nxt, SA);
-    load(SA, K + 3);
-    __syncthreads();
-    // land rows of this column (K > kown): p = 0, q = 0 stays in memory and
-    // the dot term is +0, so nothing is formed there
-    if (act && K <= kown) {
-      const T p0 = cur[me];
-      const T pu = prv[me], pn = cur[me - kHx], pw = cur[me - 1], pe = cur[me + 1];
-      const T ps = cur[me + kHx], pd = nxt[me];
-      T s;
-      if (K >= 2 && K <= kreg) {
-        // regular row: all six neighbours wet, vertical factors from the tables;
-        // B p = hs (cw pw + ce pe + cn pn + cs ps - (xcf+ycf) p0)
-        //       + zw0 (pu - p0) + zw1 (pd - p0)
-        const T zw0 = szw[K - 1], zw1 = szw[K], hs = siz[K - 1];
-        T h = cw * pw;
-        h = fma(ce, pe, h);
-        h = fma(cn, pn, h);
-        h = fma(cs, ps, h);
-        h = fma(-xyc, p0, h);
-        s = zw0 * (pu - p0);
-        s = fma(zw1, pd - p0, s);
-        s = fma(hs, h, s);
-      } else {
-        // entries that are not inserted are exactly 0 and their neighbours finite
-        const Coef rw = row<true>(c, P, K, KE);
-        s = (T)rw.dc * p0;
-        s = fma((T)rw.u, pu, s);
-        s = fma((T)rw.n, pn, s);
-        s = fma((T)rw.w, pw, s);
-        s = fma((T)rw.e, pe, s);
-        s = fma((T)rw.s, ps, s);
-        s = fma((T)rw.d, pd, s);
-      }
-      const unsigned o = own + plane * (unsigned)(K - 1);
-      pnew[o] = p0;
-      q[o] = s;
-      pqt = fma(p0, s, pqt);
-      if ((K & 7) == 0) {
-        pq += (double)pqt;
-        pqt = T(0);
-      }
-    }
-    T* t = prv;
-    prv = cur;
-    cur = nxt;
-    nxt = t;
-  };
-  for (int K = 1; K <= kmax; K += 2) {
-    level(K, std::integral_constant<int, 0>{});
-    if (K + 1 <= kmax) level(K + 1, std::integral_constant<int, 1>{});
-  }
-  pq += (double)pqt;
-  double v[1] = {pq};
-  if (grid_sum<1>(v, S)) {
-    S->pq = v[0];
-    S->alpha = S->rho / v[0];
-    if (!(v[0] > 0.0) && !(v[0] < 0.0)) S->converged = 3;  // breakdown
-  }
-}
-
-// The same product without shared memory or barriers: every thread forms p
-// of its own column and of its four horizontal neighbours from z and p_old
-// (the neighbours' lines are shared by the warps of a block through L1), and
-// keeps its own p of levels K-1, K, K+1 in registers.  Neighbours outside the
-// unknowns hold zeros (the solver vectors are zeroed at allocation and only
-// unknowns are written) and meet zero coefficients.
-template <typename T, int BY>
-__global__ void __launch_bounds__(32 * BY) k_pcg_spmv_l1(Geo G, PoissonGeo P, SolverState* S,
-                                                        const T* __restrict__ z,
-                                                        const T* __restrict__ pold,
-                                                        T* __restrict__ pnew, T* __restrict__ q,
-                                                        int first) {
-  __shared__ T szw[kMaxKe + 1], siz[kMaxKe];
-  if (S->converged) return;
-  const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const unsigned plane = (unsigned)G.L.plane, pitch = (unsigned)G.L.P;
-  const int tid = threadIdx.x + 32 * threadIdx.y;
-  for (int e = tid; e <= KE; e += 32 * BY) {
-    szw[e] = (T)P.zwn[e];
-    if (e < KE) siz[e] = (T)P.izn[e];
-  }
-  __syncthreads();
-  const int i = blockIdx.x * 32 + threadIdx.x + 2, j = blockIdx.y * BY + threadIdx.y + 2;
-  const bool act = i <= IE - 1 && j <= JE - 1;
-  const T beta = first ? T(0) : (T)S->beta;
-  double pq = 0.0;
-  if (act) {
-    const ColC c = load_col(G, P, i, j);
-    const T cw = c.iw ? (T)c.cw : T(0), ce = c.ie ? (T)c.ce : T(0);
-    const T cn = c.in ? (T)c.cn : T(0), cs = c.is ? (T)c.cs : T(0);
-    const T xyc = (T)(c.xcf + c.ycf);
-    const int kreg = c.kreg;
-    const unsigned o0 = (unsigned)G.L.at(i, j, 0);
-    auto pv = [&](unsigned o) -> T { return first ? z[o] : fma(beta, pold[o], z[o]); };
-    T pu = T(0), p0 = pv(o0);
-    T pqt = T(0);
-    for (int K = 1; K <= KE; ++K) {
-      const unsigned o = o0 + plane * (unsigned)(K - 1);
-      const T pd = K < KE ? pv(o + plane) : T(0);
-      const T pw = pv(o - 1), pe = pv(o + 1), pn = pv(o - pitch), ps = pv(o + pitch);
-      T s;
-      if (K >= 2 && K <= kreg) {
-        const T zw0 = szw[K - 1], zw1 = szw[K], hs = siz[K - 1];
-        T h = cw * pw;
-        h = fma(ce, pe, h);
-        h = fma(cn, pn, h);
-        h = fma(cs, ps, h);
-        h = fma(-xyc, p0, h);
-        s = zw0 * (pu - p0);
-        s = fma(zw1, pd - p0, s);
-        s = fma(hs, h, s);
-      } else {
-        const Coef rw = row<true>(c, P, K, KE);
-        s = (T)rw.dc * p0;
-        s = fma((T)rw.u, pu, s);
-        s = fma((T)rw.n, pn, s);
-        s = fma((T)rw.w, pw, s);
-        s = fma((T)rw.e, pe, s);
-        s = fma((T)rw.s, ps, s);
-        s = fma((T)rw.d, pd, s);
-      }
-      pnew[o] = p0;
-      q[o] = s;
-      pqt = fma(p0, s, pqt);
-      if ((K & 7) == 0) {
-        pq += (double)pqt;
-        pqt = T(0);
-      }
-      pu = p0;
-      p0 = pd;
-    }
-    pq += (double)pqt;
-  }
-  double v[1] = {pq};
-  if (grid_sum<1>(v, S)) {
-    S->pq = v[0];
-    S->alpha = S->rho / v[0];
-    if (!(v[0] > 0.0) && !(v[0] < 0.0)) S->converged = 3;  // breakdown
-  }
-}
-
-// Warp-row form: a warp holds 32 consecutive columns of one row j and keeps
-// its own p of levels K-1, K, K+1 in registers; the west and east neighbours
-// come from the adjacent lanes by shuffle (the two edge lanes load theirs),
-// the north and south neighbours are formed from z and p_old of rows j-1 and
-// j+1 (shared with the neighbouring warps through L1).  No shared-memory tile
-// and no barrier in the level loop.  The arithmetic is that of the other
-// forms, so the results are the same bit for bit.
-template <typename T, int BY>
-__global__ void __launch_bounds__(32 * BY) k_pcg_spmv_wr(Geo G, PoissonGeo P, SolverState* S,
-                                                        const T* __restrict__ z,
-                                                        const T* __restrict__ pold,
-                                                        T* __restrict__ pnew, T* __restrict__ q,
-                                                        int first) {
-  __shared__ T szw[kMaxKe + 1], siz[kMaxKe];
-  if (S->converged) return;
-  const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const unsigned plane = (unsigned)G.L.plane, pitch = (unsigned)G.L.P;
-  const int lane = threadIdx.x, tid = threadIdx.x + 32 * threadIdx.y;
-  for (int e = tid; e <= KE; e += 32 * BY) {
-    szw[e] = (T)P.zwn[e];
-    if (e < KE) siz[e] = (T)P.izn[e];
-  }
-  __syncthreads();
-  const int i = blockIdx.x * 32 + lane + 2, j = blockIdx.y * BY + threadIdx.y + 2;
-  const bool row_ok = j <= JE - 1;           // the same for the whole warp
-  const bool in_arr = row_ok && i <= IE;     // column i = IE holds zeros (not an unknown)
-  const bool act = row_ok && i <= IE - 1;
-  const T beta = first ? T(0) : (T)S->beta;
-  double pq = 0.0;
-  if (row_ok) {
-    ColC c;
-    T cw = 0, ce = 0, cn = 0, cs = 0, xyc = 0;
-    int kreg = 0;
-    if (act) {
-      c = load_col(G, P, i, j);
-      cw = c.iw ? (T)c.cw : T(0);
-      ce = c.ie ? (T)c.ce : T(0);
-      cn = c.in ? (T)c.cn : T(0);
-      cs = c.is ? (T)c.cs : T(0);
-      xyc = (T)(c.xcf + c.ycf);
-      kreg = c.kreg;
-    }
-    const unsigned o0 = in_arr ? (unsigned)G.L.at(i, j, 0) : 0u;
-    auto pv = [&](unsigned o) -> T { return first ? z[o] : fma(beta, pold[o], z[o]); };
-    T pu = T(0), p0 = in_arr ? pv(o0) : T(0);
-    T pqt = T(0);
-    for (int K = 1; K <= KE; ++K) {
-      const unsigned o = o0 + plane * (unsigned)(K - 1);
-      const T pd = (in_arr && K < KE) ? pv(o + plane) : T(0);
-      T pn = T(0), ps = T(0);
-      if (act) {
-        pn = pv(o - pitch);
-        ps = pv(o + pitch);
-      }
-      T pw = __shfl_up_sync(0xffffffffu, p0, 1);
-      T pe = __shfl_down_sync(0xffffffffu, p0, 1);
-      if (act && lane == 0) pw = pv(o - 1);
-      if (act && lane == 31) pe = pv(o + 1);
-      if (act) {
-        T s;
-        if (K >= 2 && K <= kreg) {
-          const T zw0 = szw[K - 1], zw1 = szw[K], hs = siz[K - 1];
-          T h = cw * pw;
-          h = fma(ce, pe, h);
-          h = fma(cn, pn, h);
-          h = fma(cs, ps, h);
-          h = fma(-xyc, p0, h);
-          s = zw0 * (pu - p0);
-          s = fma(zw1, pd - p0, s);
-          s = fma(hs, h, s);
-        } else {
-          const Coef rw = row<true>(c, P, K, KE);
-          s = (T)rw.dc * p0;
-          s = fma((T)rw.u, pu, s);
-          s = fma((T)rw.n, pn, s);
-          s = fma((T)rw.w, pw, s);
-          s = fma((T)rw.e, pe, s);
-          s = fma((T)rw.s, ps, s);
-          s = fma((T)rw.d, pd, s);
-        }
-        pnew[o] = p0;
-        q[o] = s;
-        pqt = fma(p0, s, pqt);
-        if ((K & 7) == 0) {
-          pq += (double)pqt;
-          pqt = T(0);
-        }
-      }
-      pu = p0;
-      p0 = pd;
-    }
-    pq += (double)pqt;
-  }
-  double v[1] = {pq};
-  if (grid_sum<1>(v, S)) {
-    S->pq = v[0];
-    S->alpha = S->rho / v[0];
-    if (!(v[0] > 0.0) && !(v[0] < 0.0)) S->converged = 3;  // breakdown
-  }
-}
-
-// TMA-staged form.  A block of TX x TY consumer threads (one column each)
-// and one producer warp marches down the levels.  The producer's first lane
-// issues, for every level, tiled bulk-tensor loads of the (TX+4) x (TY+2)
-// halo tiles of z and p_old into an NS-stage shared-memory ring (the tile
-// starts two columns west of the block so that its first element is 16-byte
-// aligned); a stage is refilled once every consumer warp has released it, so
-// up to NS-2 levels are in flight ahead of the two the consumers read.
-// Consumers form p = z + beta p_old for their column and its four horizontal
-// neighbours from the tile, keep p of the level above in a register and read
-// the level below from the next stage.  No block-wide barrier in the level
-// loop; waits on the stage barriers are bounded (a timeout stops the solve
-// with converged = 4).  Positions outside the unknowns hold zeros (the solver
-// vectors are zeroed at allocation and only unknowns are written; loads past
-// the field's extent are zero-filled) and meet zero coefficients, and the
-// arithmetic and dot order equal the other forms', so the results are the
-// same bit for bit.
-template <typename T, int TX, int TY, int NS>
-struct SpmvTma {
-  static constexpr int HX = TX + 4, HY = TY + 2;
-  static constexpr int kArrBytes = HX * HY * (int)sizeof(T);
-  static constexpr int kArrPitch = (kArrBytes + 127) / 128 * 128;
-  static constexpr int kStage = 2 * kArrPitch;
-  static constexpr int kSmem = NS * kStage + 128;  // + alignment slack
-  static constexpr int kConsumers = TX * TY;
-  static constexpr int kThreads = kConsumers + 32;
-  static_assert(TX % 32 == 0, "a warp covers 32 columns of one row");
-  static_assert((HX * sizeof(T)) % 16 == 0, "TMA box rows are whole 16-byte units");
-  static_assert(NS >= 3, "two stages are read while at least one loads");
-};
-
-// Partial of one warp row (row j, 32-column chunk) at its canonical index,
-// summed with the shuffle pattern of grid_sum (a warp's lanes are 32
-// consecutive columns).
-__device__ __forceinline__ void warp_partial(double x, SolverState* S, unsigned row,
-                                             unsigned chunk, unsigned nchunk, int lane) {
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-  if (lane == 0 && row < (unsigned)S->rows && chunk < nchunk)
-    S->partials[row * nchunk + chunk] = x;
-}
-
-// Totals over all partials by the last block to finish (grid_sum's second
-// half): the same index order and 64-thread pattern.
-__device__ bool grid_total1(double& v, SolverState* S) {
-  __shared__ double sh[2];
-  __shared__ bool last;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y, lane = tid & 31;
-  __threadfence();
-  __syncthreads();
-  const unsigned nb = gridDim.x * gridDim.y;
-  if (tid == 0) last = (atomicAdd(&S->ticket, 1u) == nb - 1);
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  const unsigned n = (unsigned)S->rows * (unsigned)((S->max_blocks) / S->rows);
-  double x = 0.0;
-  if (tid < 64)
-    for (unsigned b = tid; b < n; b += 64) x += ((volatile double*)S->partials)[b];
-  if (tid < 64) {
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[tid >> 5] = x;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    v = sh[0] + sh[1];
-    S->ticket = 0;
-  }
-  return tid == 0;
-}
-
-// The block walks tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (one
-// tile per block when the grid has a block per tile; a persistent grid of a
-// block or two per SM otherwise, so that the producer streams the next
-// tile's first levels while the consumers finish the current one and the
-// block's set-up is paid once).
-template <typename T, int TX, int TY, int NS>
-__global__ void __launch_bounds__(TX * TY + 32, 1)
-    k_pcg_spmv_tma(Geo G, PoissonGeo P, SolverState* S, const __grid_constant__ CUtensorMap mz,
-                   const __grid_constant__ CUtensorMap mpo, T* __restrict__ pnew,
-                   T* __restrict__ q, int first) {
-  using C = SpmvTma<T, TX, TY, NS>;
-  extern __shared__ unsigned char spmv_dsm[];
-  __shared__ __align__(8) uint64_t full[NS], empty[NS];
-  __shared__ T szw[kMaxKe + 1], siz[kMaxKe];
-  if (S->converged) return;
-  const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const unsigned plane = (unsigned)G.L.plane;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int ntx = (IE - 2 + TX - 1) / TX, nty = (JE - 2 + TY - 1) / TY, ntiles = ntx * nty;
-  const unsigned nchunk = (unsigned)((IE - 2 + 31) / 32);
-  unsigned char* ring = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(spmv_dsm) + 127) & ~uintptr_t(127));
-  auto zt = [&](int s) { return reinterpret_cast<T*>(ring + s * C::kStage); };
-  auto pt = [&](int s) { return reinterpret_cast<T*>(ring + s * C::kStage + C::kArrPitch); };
-  for (int e = tid; e <= KE; e += C::kThreads) {
-    szw[e] = (T)P.zwn[e];
-    if (e < KE) siz[e] = (T)P.izn[e];
-  }
-  if (tid == 0) {
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], C::kConsumers / 32);
-    }
-    mbar_init_fence();
-  }
-  __syncthreads();
-  bool ok = true;
-  if (warp == C::kConsumers / 32) {
-    // ---- producer: the whole warp walks the (tile, level) steps so that it
-    // reaches the block's later barriers together; its first lane issues
-    const uint32_t bytes = (first ? 1u : 2u) * (uint32_t)C::kArrBytes;
-    if (lane == 0) {
-      tma_prefetch_desc(&mz);
-      if (!first) tma_prefetch_desc(&mpo);
-    }
-    long long g = 0;  // steps issued
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      const int i0 = (t % ntx) * TX + 2, j0 = (t / ntx) * TY + 2;
-      for (int K = 1; K <= KE; ++K, ++g) {
-        const int s = (int)(g % NS);
-        const long long n = g / NS;
-        if (n > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[s], (unsigned)((n - 1) & 1)))) {
-          ok = false;
-          break;
-        }
-        if (lane == 0) {
-          mbar_arrive_expect_tx(&full[s], bytes);
-          tma_load_3d(zt(s), &mz, i0 - 2, j0 - 1, K - 1, &full[s]);
-          if (!first) tma_load_3d(pt(s), &mpo, i0 - 2, j0 - 1, K - 1, &full[s]);
-        }
-        __syncwarp();
-      }
-    }
-    // the block does not exit with copies in flight into its shared memory
-    for (long long h = g - NS > 0 ? g - NS : 0; h < g; ++h)
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[h % NS], (unsigned)((h / NS) & 1))) && ok;
-  } else {
-    // ---- consumers
-    const int tx = tid % TX, ty = tid / TX;
-    const T beta = first ? T(0) : (T)S->beta;
-    const int me = (ty + 1) * C::HX + (tx + 2);
-    auto pv = [&](int s, int e) -> T {
-      return first ? zt(s)[e] : fma(beta, pt(s)[e], zt(s)[e]);
-    };
-    long long g = 0;  // steps consumed
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      const int i0 = (t % ntx) * TX + 2, j0 = (t / ntx) * TY + 2;
-      const int i = i0 + tx, j = j0 + ty;
-      const bool act = i <= IE - 1 && j <= JE - 1;
-      ColC c;
-      T cw = 0, ce = 0, cn = 0, cs = 0, xyc = 0;
-      int kreg = 0;
-      if (act) {
-        c = load_col(G, P, i, j);
-        cw = c.iw ? (T)c.cw : T(0);
-        ce = c.ie ? (T)c.ce : T(0);
-        cn = c.in ? (T)c.cn : T(0);
-        cs = c.is ? (T)c.cs : T(0);
-        xyc = (T)(c.xcf + c.ycf);
-        kreg = c.kreg;
-      }
-      const unsigned own = act ? (unsigned)G.L.at(i, j, 0) : 0u;
-      double pq = 0.0;
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[g % NS], (unsigned)((g / NS) & 1)));
-      T pu = T(0), p0 = ok ? pv((int)(g % NS), me) : T(0);
-      T pqt = T(0);
-      for (int K = 1; K <= KE && ok; ++K, ++g) {
-        const int s = (int)(g % NS);
-        T pd = T(0);
-        if (K < KE) {
-          const int s1 = (int)((g + 1) % NS);
-          if (!__all_sync(0xffffffffu, mbar_wait(&full[s1], (unsigned)(((g + 1) / NS) & 1)))) {
-            ok = false;
-            break;
-          }
-          pd = pv(s1, me);
-        }
-        if (act) {
-          const T pw = pv(s, me - 1), pe = pv(s, me + 1);
-          const T pn = pv(s, me - C::HX), ps = pv(s, me + C::HX);
-          T sv;
-          if (K >= 2 && K <= kreg) {
-            const T zw0 = szw[K - 1], zw1 = szw[K], hs = siz[K - 1];
-            T h = cw * pw;
-            h = fma(ce, pe, h);
-            h = fma(cn, pn, h);
-            h = fma(cs, ps, h);
-            h = fma(-xyc, p0, h);
-            sv = zw0 * (pu - p0);
-            sv = fma(zw1, pd - p0, sv);
-            sv = fma(hs, h, sv);
-          } else {
-            const Coef rw = row<true>(c, P, K, KE);
-            sv = (T)rw.dc * p0;
-            sv = fma((T)rw.u, pu, sv);
-            sv = fma((T)rw.n, pn, sv);
-            sv = fma((T)rw.w, pw, sv);
-            sv = fma((T)rw.e, pe, sv);
-            sv = fma((T)rw.s, ps, sv);
-            sv = fma((T)rw.d, pd, sv);
-          }
-          const unsigned o = own + plane * (unsigned)(K - 1);
-          pnew[o] = p0;
-          q[o] = sv;
-          pqt = fma(p0, sv, pqt);
-          if ((K & 7) == 0) {
-            pq += (double)pqt;
-            pqt = T(0);
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[s]);
-        pu = p0;
-        p0 = pd;
-      }
-      pq += (double)pqt;
-      // this tile's warp-row partial (a warp is 32 columns of one row)
-      warp_partial(pq, S, (unsigned)(j0 - 2 + ty), (unsigned)((i0 - 2 + tx) / 32), nchunk, lane);
-    }
-  }
-  if (!ok) atomicExch(&S->converged, 4);  // a stage wait timed out: stop the solve
-  double v = 0.0;
-  if (grid_total1(v, S)) {
-    S->pq = v;
-    S->alpha = S->rho / v;
-    if (S->converged == 0 && !(v > 0.0) && !(v < 0.0)) S->converged = 3;  // breakdown
-  }
+// The black correction: the x update that the last iteration left open (none
+// before the first), and its addition to the solution (full layout).
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_rb_after(RbGeo R, SolverState* S,
+                                                       const T* __restrict__ p, T* __restrict__ d,
+                                                       double* __restrict__ x) {
+  const int m = blockIdx.x * 32 + (threadIdx.x & 31), K = blockIdx.z * kWarps + (threadIdx.x >> 5) + 1;
+  const int j = blockIdx.y + 2;
+  if (m >= R.M) return;
+  const int s2 = m + R.P2 * j;
+  if (K > wet_levels(R.col[1].kk[s2], 0)) return;
+  const int o = s2 + R.plane2 * (K - 1);
+  T v = T(0);
+  if (S->iter > 0) v = fma((T)S->alpha_prev, p[o], d[o]);
+  d[o] = v;
+  const double scale = sizeof(T) == 4 ? sqrt(S->res_rr) : 1.0;
+  const int f = black_i(m, j) + 2 * (R.P2 * j + R.plane2 * (K - 1));
+  x[f] = x[f] + scale * (double)v;
 }
 
 // r = b - A x with the exact FP64 entries of compute_matrix, accumulated in
@@ -1026,24 +699,35 @@ __device__ __forceinline__ void dd_sub_prod(DD& s, double c, double x) {
   s.hi = hi;
 }
 
-__global__ void __launch_bounds__(128) k_resid(Geo G, PoissonGeo P, SolverState* S,
-                                               const double* __restrict__ b,
-                                               double* __restrict__ x,
-                                               double* __restrict__ r) {
+// LR levels per thread: the levels of a column are independent here, so the
+// blocks split them (a thread that marches down a whole column waits for its
+// loads level by level: 1.4 ms a launch on 1024 x 1024 x 80).
+constexpr int kResidLevels = 8;
+
+__global__ void __launch_bounds__(kThreads) k_resid(Geo G, PoissonGeo P, SolverState* S,
+                                                    const double* __restrict__ b,
+                                                    double* __restrict__ x,
+                                                    double* __restrict__ r, int nbx, int nby,
+                                                    int ntiles) {
   const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
+  const int tile = blockIdx.x, bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
+  const int i = bx * 32 + (threadIdx.x & 31) + 2, j = by * kWarps + (threadIdx.x >> 5) + 2;
+  const int K0 = bz * kResidLevels + 1, K1 = min(KE, K0 + kResidLevels - 1);
   double rr = 0.0, bb = 0.0;
   if (i <= IE - 1 && j <= JE - 1) {
     const ColC c = load_col(G, P, i, j);
     // land rows (K > kb): diagonal only with a zero right-hand side, so the
-    // solution there is 0; x is set to it and r (0) is not stored, which
-    // keeps every solver vector exactly 0 on land for the PCG kernels
-    for (int K = c.kb + 1; K <= KE; ++K)
+    // solution there is 0 and x is set to it; r is neither stored nor read there
+    for (int K = max(c.kb + 1, K0); K <= K1; ++K)
       if (AT(x, i, j, K) != 0.0) AT(x, i, j, K) = 0.0;
-    double xm = 0.0, x0 = AT(x, i, j, 1), xp = 0.0;
-    for (int K = 1; K <= c.kb; ++K) {
-      xp = K < KE ? AT(x, i, j, K + 1) : 0.0;
+    double xm = 0.0, x0 = 0.0, xp = 0.0;
+    if (K0 <= c.kb) {
+      if (K0 > 1) xm = AT(x, i, j, K0 - 1);
+      x0 = AT(x, i, j, K0);
+    }
+    const int Ke = min(K1, c.kb);
+    for (int K = K0; K <= Ke; ++K) {
+      xp = K < c.kb ? AT(x, i, j, K + 1) : 0.0;
       const Coef rw = row<false>(c, P, K, KE);
       const double bk = AT(b, i, j, K);
       DD s{bk, 0.0};
@@ -1055,47 +739,20 @@ __global__ void __launch_bounds__(128) k_resid(Geo G, PoissonGeo P, SolverState*
       if (rw.s != 0.0) dd_sub_prod(s, rw.s, AT(x, i, j + 1, K));
       if (rw.d != 0.0) dd_sub_prod(s, rw.d, xp);
       const double rk = s.hi + s.lo;
-      if (r) AT(r, i, j, K) = rk;
+      AT(r, i, j, K) = rk;
       rr += rk * rk;
       bb += bk * bk;
       xm = x0;
       x0 = xp;
     }
   }
-  double v[2] = {rr, bb};
-  if (grid_sum<2>(v, S)) {
+  const double w[2] = {rr, bb};
+  tile_partial<2>(w, S, tile);
+  double v[2];
+  if (grid_total<2>(v, S, ntiles)) {
     S->res_rr = v[0];
     S->res_bb = v[1];
   }
-}
-
-// refinement helpers
-__global__ void k_scale_to_f32(Geo G, const double* __restrict__ r, const SolverState* S,
-                               float* __restrict__ r32) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int K = blockIdx.z + 1;
-  if (i > G.L.ie - 1 || j > G.L.je - 1) return;
-  const double s = S->res_rr > 0.0 ? 1.0 / sqrt(S->res_rr) : 0.0;
-  AT(r32, i, j, K) = (float)(AT(r, i, j, K) * s);
-}
-
-__global__ void k_axpy_f32(Geo G, const float* __restrict__ d, const SolverState* S,
-                           double* __restrict__ x) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int K = blockIdx.z + 1;
-  if (i > G.L.ie - 1 || j > G.L.je - 1) return;
-  const double s = sqrt(S->res_rr);
-  AT(x, i, j, K) = AT(x, i, j, K) + s * (double)AT(d, i, j, K);
-}
-
-__global__ void k_axpy_f64(Geo G, const double* __restrict__ d, double* __restrict__ x) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int K = blockIdx.z + 1;
-  if (i > G.L.ie - 1 || j > G.L.je - 1) return;
-  AT(x, i, j, K) = AT(x, i, j, K) + AT(d, i, j, K);
 }
 
 __global__ void k_set_limit(SolverState* S, int limit) { S->limit = limit; }
@@ -1105,290 +762,168 @@ __global__ void k_pcg_continue(cudaGraphConditionalHandle hc, const SolverState*
   cudaGraphSetConditional(hc, (S->converged == 0 && S->iter + chunk <= S->limit) ? 1u : 0u);
 }
 
-__global__ void k_reset(SolverState* S, double tol, int keep_bb) {
+__global__ void k_reset(SolverState* S, double tol) {
   S->converged = 0;
   S->iter = 0;
   S->ticket = 0;
   S->tol = tol;
   S->beta = 0.0;
-  if (!keep_bb) S->bb = 0.0;
+  S->alpha_prev = 0.0;
+  S->bb = 0.0;
 }
 
-const dim3 kColBlock(32, 4);
+// Launch shapes: at most this many blocks per SM (a block then walks several
+// tiles), 0 for a block per tile.
+constexpr int kShapes = 9;
+const int kBlocksPerSm[kShapes] = {0, 2, 3, 4, 6, 8, 1, 5, 12};
 
-}  // namespace
-
-void launch_factor(const Geo& G, const PoissonGeo& P, double* dinv64, float* dinv32,
-                   cudaStream_t st) {
-  k_factor<<<grid2(G.L.ie - 2, G.L.je - 2, kColBlock), kColBlock, 0, st>>>(G, P, dinv64, dinv32);
-  count_launch();
-}
-
-// ---------------------------------------------------------- tensor maps
-namespace {
-
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// cuTensorMapEncodeTiled from the driver, looked up once through the runtime
-// (the library does not link libcuda)
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      return nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-
-constexpr int kTmaTx = 64, kTmaTy = 8, kTmaNs = 6;      // variant 6
-constexpr int kTmaTx2 = 32, kTmaTy2 = 8, kTmaNs2 = 8;   // variant 7
-
-template <typename T, int TX, int TY, int NS>
-cudaError_t tma_optin() {
-  return cudaFuncSetAttribute(k_pcg_spmv_tma<T, TX, TY, NS>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              SpmvTma<T, TX, TY, NS>::kSmem);
-}
-
-// persistent: a grid of one block per SM (the kernels fit one block per SM),
-// otherwise a block per tile
-template <typename T, int TX, int TY, int NS>
-int tma_launch(const Geo& G, const PoissonGeo& P, SolverState* S, const T* z, const T* pold,
-               T* pnew, T* q, int first, bool persistent, cudaStream_t st) {
-  using C = SpmvTma<T, TX, TY, NS>;
-  CUtensorMap mz, mp;
-  const int e1 = encode_field_map(&mz, z, (int)sizeof(T), G.L.P, G.L.JN, G.L.ke, C::HX, C::HY);
-  const int e2 = encode_field_map(&mp, first ? z : pold, (int)sizeof(T), G.L.P, G.L.JN, G.L.ke,
-                                  C::HX, C::HY);
-  if (e1 || e2) return e1 ? e1 : e2;
-  const int ntiles = ((G.L.ie - 2 + TX - 1) / TX) * ((G.L.je - 2 + TY - 1) / TY);
-  int nblk = ntiles;
-  if (persistent) {
-    static int nsm = 0;
-    if (!nsm) {
-      int dev = 0;
-      if (cudaGetDevice(&dev) != cudaSuccess ||
-          cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        nsm = 148;
-    }
-    nblk = ntiles < nsm ? ntiles : nsm;
-  }
-  k_pcg_spmv_tma<T, TX, TY, NS><<<nblk, C::kThreads, C::kSmem, st>>>(G, P, S, mz, mp, pnew, q,
-                                                                      first);
-  return 0;
-}
-
-}  // namespace
-
-int encode_field_map(CUtensorMap* map, const void* base, int elem_bytes, int P, int JN, int nlev,
-                     int bx, int by) {
-  EncodeTiledFn fn = encode_tiled();
-  if (!fn) return (int)CUDA_ERROR_NOT_FOUND;
-  const cuuint64_t dims[3] = {(cuuint64_t)P, (cuuint64_t)JN, (cuuint64_t)nlev};
-  const cuuint64_t strides[2] = {(cuuint64_t)P * elem_bytes, (cuuint64_t)P * JN * elem_bytes};
-  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  return (int)fn(map, elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-}
-
-namespace {
-
-// Variants of the column kernel (chosen per handle by the autotuner):
-// forward values through the output vector or in shared memory, the number
-// of levels whose loads are issued together, and blocks of 32 x 4 columns or
-// of 128 consecutive columns of one row (each warp's segment then adjoins its
-// neighbours', the same DRAM pages).
-struct ColVariant {
-  bool sm;
-  int u;
-  dim3 blk;
+struct Shape {
+  int ntiles, nmc, grid;
 };
-constexpr int kNumColVariants = 6;
-const ColVariant kColVariants[kNumColVariants] = {
-    {false, 4, dim3(32, 4)}, {false, 8, dim3(32, 4)}, {true, 4, dim3(32, 2)}, {true, 8, dim3(32, 2)},
-    {false, 4, dim3(128, 1)}, {false, 8, dim3(128, 1)}};
-// a shared-memory variant is usable while its block's forward values fit here
-constexpr size_t kColSmemMax = 96 * 1024;
 
-template <typename T, int MODE, bool SM, int U>
-void col_launch(dim3 blk, size_t smem, const Geo& G, const PoissonGeo& P, SolverState* S,
-                const T* b, T* x, T* r, const T* p, const T* q, T* z, cudaStream_t st) {
-  k_pcg_col<T, MODE, SM, U><<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, smem, st>>>(G, P, S, b, x,
-                                                                                  r, p, q, z);
+Shape shape_of(const RbGeo& R, int columns_per_tile, int variant) {
+  Shape s;
+  s.nmc = (R.M + columns_per_tile - 1) / columns_per_tile;
+  s.ntiles = s.nmc * (R.je - 2);
+  s.grid = s.ntiles;
+  const int per = kBlocksPerSm[variant >= 0 && variant < kShapes ? variant : 0];
+  if (per) s.grid = std::min(s.ntiles, per * R.sms);
+  return s;
 }
 
-template <typename T, int MODE, int U>
-cudaError_t col_optin() {
-  return cudaFuncSetAttribute(k_pcg_col<T, MODE, true, U>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kColSmemMax);
-}
+// Calls f<T, G, LC> with the split for KE levels: four columns of doubles or
+// eight of floats per warp (32-byte segments) while the lane's share fits
+// registers (up to 13 doubles or 26 floats), 16 lanes per column above.
+template <int N>
+using Int = std::integral_constant<int, N>;
 
-template <typename T, int SM, int U>
-void col_mode(int mode, dim3 blk, size_t smem, const Geo& G, const PoissonGeo& P, SolverState* S,
-              const T* b, T* x, T* r, const T* p, const T* q, T* z, cudaStream_t st) {
-  if (mode == 1)
-    col_launch<T, 1, SM, U>(blk, smem, G, P, S, b, x, r, p, q, z, st);
-  else
-    col_launch<T, 2, SM, U>(blk, smem, G, P, S, b, x, r, p, q, z, st);
+template <typename T, typename F>
+void with_split(int ke, F&& f) {
+  if (ke > 104) {
+    if (ke <= 128) f(Int<16>{}, Int<8>{});
+    else if (ke <= 208) f(Int<16>{}, Int<13>{});
+    else f(Int<16>{}, Int<20>{});
+  } else if constexpr (sizeof(T) == 8) {
+    if (ke <= 40) f(Int<8>{}, Int<5>{});
+    else if (ke <= 48) f(Int<8>{}, Int<6>{});
+    else if (ke <= 64) f(Int<8>{}, Int<8>{});
+    else if (ke <= 80) f(Int<8>{}, Int<10>{});
+    else if (ke <= 88) f(Int<8>{}, Int<11>{});
+    else f(Int<8>{}, Int<13>{});
+  } else {
+    if (ke <= 40) f(Int<4>{}, Int<10>{});
+    else if (ke <= 48) f(Int<4>{}, Int<12>{});
+    else if (ke <= 64) f(Int<4>{}, Int<16>{});
+    else if (ke <= 80) f(Int<4>{}, Int<20>{});
+    else if (ke <= 88) f(Int<4>{}, Int<22>{});
+    else f(Int<4>{}, Int<26>{});
+  }
 }
+static_assert(16 * 20 >= kMaxKe, "the longest column has a split");
+
+template <typename T>
+const T* red_pivots(const RbGeo& R);
+template <>
+const double* red_pivots<double>(const RbGeo& R) { return R.dr64; }
+template <>
+const float* red_pivots<float>(const RbGeo& R) { return R.dr32; }
 
 }  // namespace
 
-template <typename T>
-bool pcg_col_variant_ok(const Geo& G, int variant) {
-  if (variant < 0 || variant >= kNumColVariants) return false;
-  const ColVariant& v = kColVariants[variant];
-  return !v.sm || (size_t)v.blk.x * v.blk.y * G.L.ke * sizeof(T) <= kColSmemMax;
-}
-template bool pcg_col_variant_ok<double>(const Geo&, int);
-template bool pcg_col_variant_ok<float>(const Geo&, int);
-int pcg_col_variants() { return kNumColVariants; }
-
-// The shared-memory variants' dynamic shared memory (plus about 2.6 KB of
-// static) may exceed the 48 KB default, so their opt-in is raised to the
-// variants' fixed maximum on the current device.  Every caller sets the same
-// value (the attribute is process-wide per kernel), so handles created on
-// several threads never lower it under one another's launches.
-cudaError_t pcg_prepare_device() {
-  const cudaError_t e[] = {col_optin<double, 1, 4>(), col_optin<double, 2, 4>(),
-                           col_optin<double, 1, 8>(), col_optin<double, 2, 8>(),
-                           col_optin<float, 1, 4>(),  col_optin<float, 2, 4>(),
-                           col_optin<float, 1, 8>(),  col_optin<float, 2, 8>(),
-                           tma_optin<double, kTmaTx, kTmaTy, kTmaNs>(),
-                           tma_optin<float, kTmaTx, kTmaTy, kTmaNs>(),
-                           tma_optin<double, kTmaTx2, kTmaTy2, kTmaNs2>(),
-                           tma_optin<float, kTmaTx2, kTmaTy2, kTmaNs2>()};
-  for (cudaError_t x : e)
-    if (x != cudaSuccess) return x;
-  return cudaSuccess;
-}
-
-template <typename T, typename TX>
-void launch_pcg_col(const Geo& G, const PoissonGeo& P, SolverState* S, int mode, const T* b, TX* x,
-                    T* r, const T* p, const T* q, T* z, int variant, cudaStream_t st) {
-  if (!pcg_col_variant_ok<T>(G, variant)) variant = 0;
-  const ColVariant& v = kColVariants[variant];
-  const size_t smem = v.sm ? (size_t)v.blk.x * v.blk.y * G.L.ke * sizeof(T) : 0;
-  switch (variant) {
-    case 0: case 4: col_mode<T, false, 4>(mode, v.blk, smem, G, P, S, b, x, r, p, q, z, st); break;
-    case 1: case 5: col_mode<T, false, 8>(mode, v.blk, smem, G, P, S, b, x, r, p, q, z, st); break;
-    case 2: col_mode<T, true, 4>(mode, v.blk, smem, G, P, S, b, x, r, p, q, z, st); break;
-    default: col_mode<T, true, 8>(mode, v.blk, smem, G, P, S, b, x, r, p, q, z, st); break;
-  }
+void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, double* dr64, float* dr32,
+                     float* db32, cudaStream_t st) {
+  const dim3 blk(32, 4);
+  k_rb_setup<<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, 0, st>>>(G, P, R, dr64, dr32, db32);
   count_launch();
 }
-template void launch_pcg_col<double, double>(const Geo&, const PoissonGeo&, SolverState*, int,
-                                             const double*, double*, double*, const double*,
-                                             const double*, double*, int, cudaStream_t);
-template void launch_pcg_col<float, float>(const Geo&, const PoissonGeo&, SolverState*, int,
-                                           const float*, float*, float*, const float*,
-                                           const float*, float*, int, cudaStream_t);
 
-// Variants of the stencil kernel: shared-memory ring with 32 x 8 or 32 x 4
-// tiles, the barrier-free L1 form, or the warp-row form, each with 32 x 8 or
-// 32 x 4 blocks; and the TMA-staged form with 64 x 8 (6 stages) or 32 x 8
-// (8 stages) columns per block, a block per tile, and the 64 x 8 form with a
-// persistent grid of one block per SM.
-int pcg_spmv_variants() { return 9; }
+int pcg_col_variants() { return 6; }
+int pcg_spmv_variants() { return kShapes; }
 
-bool pcg_spmv_variant_ok(int variant) {
-  if (variant < 0 || variant >= pcg_spmv_variants()) return false;
-  return variant < 6 || encode_tiled() != nullptr;
-}
-
-// Returns cudaErrorInvalidValue (nothing launched) when a TMA variant's
-// tensor maps cannot be encoded.
 template <typename T>
-cudaError_t launch_pcg_spmv(const Geo& G, const PoissonGeo& P, SolverState* S, const T* z,
-                            const T* pold, T* pnew, T* q, int first, int variant,
-                            cudaStream_t st) {
-  const int nx = G.L.ie - 2, ny = G.L.je - 2;
-  switch (variant) {
-    case 6:
-      if (tma_launch<T, kTmaTx, kTmaTy, kTmaNs>(G, P, S, z, pold, pnew, q, first, false, st))
-        return cudaErrorInvalidValue;
-      break;
-    case 7:
-      if (tma_launch<T, kTmaTx2, kTmaTy2, kTmaNs2>(G, P, S, z, pold, pnew, q, first, false, st))
-        return cudaErrorInvalidValue;
-      break;
-    case 8:
-      if (tma_launch<T, kTmaTx, kTmaTy, kTmaNs>(G, P, S, z, pold, pnew, q, first, true, st))
-        return cudaErrorInvalidValue;
-      break;
-    case 1:
-      k_pcg_spmv<T, 4><<<grid2(nx, ny, dim3(kTx, 4)), dim3(kTx, 4), 0, st>>>(G, P, S, z, pold,
-                                                                              pnew, q, first);
-      break;
-    case 2:
-      k_pcg_spmv_l1<T, 8><<<grid2(nx, ny, dim3(32, 8)), dim3(32, 8), 0, st>>>(G, P, S, z, pold,
-                                                                               pnew, q, first);
-      break;
-    case 3:
-      k_pcg_spmv_l1<T, 4><<<grid2(nx, ny, dim3(32, 4)), dim3(32, 4), 0, st>>>(G, P, S, z, pold,
-                                                                               pnew, q, first);
-      break;
-    case 4:
-      k_pcg_spmv_wr<T, 8><<<grid2(nx, ny, dim3(32, 8)), dim3(32, 8), 0, st>>>(G, P, S, z, pold,
-                                                                               pnew, q, first);
-      break;
-    case 5:
-      k_pcg_spmv_wr<T, 4><<<grid2(nx, ny, dim3(32, 4)), dim3(32, 4), 0, st>>>(G, P, S, z, pold,
-                                                                               pnew, q, first);
-      break;
-    default:
-      k_pcg_spmv<T, 8><<<grid2(nx, ny, dim3(kTx, 8)), dim3(kTx, 8), 0, st>>>(G, P, S, z, pold,
-                                                                              pnew, q, first);
-      break;
-  }
-  count_launch();
-  return cudaSuccess;
+void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbVectors<T>& v,
+                      cudaStream_t st) {
+  with_split<T>(R.ke, [&](auto gc, auto lc) {
+    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
+    const Shape s = shape_of(R, Lane<T, G, LC>::CT, 0);
+    k_rb_red<T, G, LC, kBefore><<<s.grid, kThreads, 0, st>>>(R, S, nullptr, v.ub, red_pivots<T>(R),
+                                                             b, nullptr, s.ntiles, s.nmc);
+    k_rb_col<T, G, LC, true><<<s.grid, kThreads, 0, st>>>(R, S, v.r, nullptr, v.z, R.db32, b, v.ub,
+                                                          s.ntiles, s.nmc);
+  });
+  add_launches(2);
 }
-template cudaError_t launch_pcg_spmv<double>(const Geo&, const PoissonGeo&, SolverState*,
-                                             const double*, const double*, double*, double*, int,
-                                             int, cudaStream_t);
-template cudaError_t launch_pcg_spmv<float>(const Geo&, const PoissonGeo&, SolverState*,
-                                            const float*, const float*, float*, float*, int, int,
-                                            cudaStream_t);
+
+template <typename T>
+void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
+                   cudaStream_t st) {
+  with_split<T>(R.ke, [&](auto gc, auto lc) {
+    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
+    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
+    k_rb_red<T, G, LC, kIter><<<s.grid, kThreads, 0, st>>>(R, S, v.z, v.u, red_pivots<T>(R), nullptr,
+                                                           nullptr, s.ntiles, s.nmc);
+  });
+  count_launch();
+}
+
+template <typename T>
+void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
+                     cudaStream_t st) {
+  with_split<T>(R.ke, [&](auto gc, auto lc) {
+    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
+    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
+    k_rb_black<T, G, LC><<<s.grid, kThreads, 0, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, s.ntiles, s.nmc);
+  });
+  count_launch();
+}
+
+template <typename T>
+void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
+                   cudaStream_t st) {
+  with_split<T>(R.ke, [&](auto gc, auto lc) {
+    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
+    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
+    k_rb_col<T, G, LC, false><<<s.grid, kThreads, 0, st>>>(R, S, v.r, v.q, v.z, R.db32, nullptr,
+                                                           nullptr, s.ntiles, s.nmc);
+  });
+  count_launch();
+}
+
+template <typename T>
+void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x,
+                     cudaStream_t st) {
+  const dim3 grid((R.M + 31) / 32, R.je - 2, (R.ke + kWarps - 1) / kWarps);
+  k_rb_after<T><<<grid, kThreads, 0, st>>>(R, S, v.p, v.x, x);
+  with_split<T>(R.ke, [&](auto gc, auto lc) {
+    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
+    const Shape s = shape_of(R, Lane<T, G, LC>::CT, 0);
+    k_rb_red<T, G, LC, kAfter><<<s.grid, kThreads, 0, st>>>(R, S, v.x, v.ub, red_pivots<T>(R),
+                                                            nullptr, x, s.ntiles, s.nmc);
+  });
+  add_launches(2);
+}
+
+#define ORCTM_RB(T)                                                                              \
+  template void launch_rb_before<T>(const RbGeo&, SolverState*, const double*, const RbVectors<T>&, \
+                                    cudaStream_t);                                               \
+  template void launch_rb_red<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
+  template void launch_rb_black<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
+  template void launch_rb_col<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
+  template void launch_rb_after<T>(const RbGeo&, SolverState*, const RbVectors<T>&, double*, cudaStream_t);
+ORCTM_RB(double)
+ORCTM_RB(float)
+#undef ORCTM_RB
 
 void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const double* b, double* x,
                   double* r, cudaStream_t st) {
-  k_resid<<<grid2(G.L.ie - 2, G.L.je - 2, kColBlock), kColBlock, 0, st>>>(G, P, S, b, x, r);
+  const int nbx = (G.L.ie - 2 + 31) / 32, nby = (G.L.je - 2 + kWarps - 1) / kWarps;
+  const int nt = nbx * nby * ((G.L.ke + kResidLevels - 1) / kResidLevels);
+  k_resid<<<nt, kThreads, 0, st>>>(G, P, S, b, x, r, nbx, nby, nt);
   count_launch();
 }
 
-void launch_scale_to_f32(const Geo& G, const double* r, const SolverState* S, float* r32,
-                         cudaStream_t st) {
-  const dim3 blk(32, 4);
-  k_scale_to_f32<<<grid3(G.L.ie - 2, G.L.je - 2, G.L.ke, blk), blk, 0, st>>>(G, r, S, r32);
-  count_launch();
-}
-
-void launch_axpy_f32(const Geo& G, const float* d, const SolverState* S, double* x,
-                     cudaStream_t st) {
-  const dim3 blk(32, 4);
-  k_axpy_f32<<<grid3(G.L.ie - 2, G.L.je - 2, G.L.ke, blk), blk, 0, st>>>(G, d, S, x);
-  count_launch();
-}
-
-void launch_axpy_f64(const Geo& G, const double* d, double* x, cudaStream_t st) {
-  const dim3 blk(32, 4);
-  k_axpy_f64<<<grid3(G.L.ie - 2, G.L.je - 2, G.L.ke, blk), blk, 0, st>>>(G, d, x);
-  count_launch();
-}
-
-void launch_solver_reset(SolverState* S, double tol, int keep_bb, cudaStream_t st) {
-  k_reset<<<1, 1, 0, st>>>(S, tol, keep_bb);
+void launch_solver_reset(SolverState* S, double tol, cudaStream_t st) {
+  k_reset<<<1, 1, 0, st>>>(S, tol);
   count_launch();
 }
 
@@ -1404,8 +939,11 @@ void launch_pcg_continue(cudaGraphConditionalHandle hc, const SolverState* S, in
 }
 
 size_t solver_max_blocks(const Geo& G) {
-  // one partial per warp row: 32-column chunks x rows of unknowns
-  return (size_t)((G.L.ie - 2 + 31) / 32) * (size_t)(G.L.je - 2);
+  // tiles of k_resid, and of the PCG kernels at their narrowest (16 columns)
+  const size_t resid = (size_t)((G.L.ie - 2 + 31) / 32) * ((G.L.je - 2 + kWarps - 1) / kWarps) *
+                       ((G.L.ke + kResidLevels - 1) / kResidLevels);
+  const size_t pcg = (size_t)((G.L.ie / 2 + 1 + 15) / 16) * (G.L.je - 2);
+  return std::max(resid, pcg);
 }
 
 }  // namespace orctm
