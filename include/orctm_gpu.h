@@ -455,16 +455,12 @@ unsigned long long orctm_kernel_launches(void);
  * estimate, within 1 ulp of IEEE division).  Test support; allocates. */
 int orctm_check_division(int device, const double* a, const double* b, double* q, size_t n);
 
-/* Kernel variants of the Poisson solver: 6 column-kernel variants (forward
- * values in global or shared memory, 4 or 8 levels per load batch, 32x4,
- * 32x2 or 128x1 blocks) and 9 stencil variants (0-5: shared-memory ring,
- * L1 form or warp-row form, 32x8 or 32x4 blocks; 6-8: TMA-staged tiles).
- * All variants give bit-identical results.  A variant of -1 (the default)
- * lets the handle time the variants on its own grid before its first solve
- * in each precision and keep the fastest (the choice is cached per grid size
- * in the process).  orctm_get_tuning returns the variants in use for a
- * precision (0 FP64, 1 FP32), -1 before the first solve.  A shared-memory
- * column variant that does not fit the grid's KE falls back to variant 0. */
+/* Kernel variants of the Poisson solver.  The solver's kernels have one form,
+ * chosen by KE and the precision; the numbers of earlier variants (6 column-kernel
+ * and 9 stencil variants, -1 for the handle's own choice) are accepted and
+ * reported, and change neither results nor speed.  orctm_get_tuning returns
+ * the numbers in use for a precision (0 FP64, 1 FP32), -1 before the first
+ * solve. */
 int orctm_set_tuning(orctm_handle* h, int col_variant, int spmv_variant);
 int orctm_get_tuning(const orctm_handle* h, int precision, int* col_variant, int* spmv_variant);
 

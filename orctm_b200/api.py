@@ -597,7 +597,7 @@ class Instance:
         _lib.check(self.lib.orctm_synchronize(self.h), self.h)
 
     def set_tuning(self, col: int = -1, spmv: int = -1):
-        """Forces the Poisson kernel variants (-1: autotune on the first solve)."""
+        """Kernel variant numbers (accepted and reported; one form runs)."""
         _lib.check(self.lib.orctm_set_tuning(self.h, col, spmv), self.h)
 
     def tuning(self, precision: str = "fp64") -> tuple:

@@ -160,10 +160,8 @@ struct orctm_handle {
   RbVectors<double> v64{};             // vectors of the reduced system, per precision
   RbVectors<float> v32{};
   SolverState* S = nullptr;
-  SolverState* S_tune = nullptr;  // scratch scalars for the autotuner
-  SolverState* S_tune0 = nullptr; // their initial value
   double* partials = nullptr;
-  // kernel variants per precision (0 FP64, 1 FP32); -1 = not chosen yet
+  // variant numbers reported per precision (0 FP64, 1 FP32); -1 = no solve yet
   int col_var[2] = {-1, -1}, spmv_var[2] = {-1, -1};
   int force_col = -1, force_spmv = -1;  // orctm_set_tuning
   // asynchronous copies (orctm_upload_async / orctm_download_async): a copy
@@ -212,9 +210,8 @@ struct orctm_handle {
   double* occ_contra = nullptr;  // device scalar
   double* h_contra = nullptr;    // its page-locked mirror
   double* trotest_buf = nullptr;  // orctm_trotest's scratch, allocated on first use
-  // replayed chunk of PCG iterations per precision and the variants it holds
+  // replayed chunk of PCG iterations per precision
   cudaGraphExec_t pcg_graph[2] = {nullptr, nullptr};
-  int pcg_graph_key[2][2] = {{-1, -1}, {-1, -1}};
   SolverState* hS = nullptr;  // pinned mirror
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t tm0 = nullptr, tm1 = nullptr;  // orctm_timer_start / _stop
@@ -696,7 +693,8 @@ int setup(orctm_handle* h, const orctm_desc* d) {
   }
   if ((st = h->dev_alloc(&h->zo, n2))) return st;
 
-  // red-black tables and pivots (the operator is constant: factorise once)
+  // red-black view of the operator; its tables and pivots (constant) are formed
+  // with a solver mode's vectors, before its first solve
   {
     RbGeo& R = h->R;
     R.ie = IE; R.je = JE; R.ke = KE;
@@ -706,25 +704,15 @@ int setup(orctm_handle* h, const orctm_desc* d) {
     R.zwn = P.zwn;
     R.izn = P.izn;
     ORCTM_CUDA_OK(cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, h->device));
-    const size_t n2h = (size_t)R.plane2, n3h = (size_t)L.n3() / 2;
+    const size_t n2h = (size_t)R.plane2;
     for (RbColour& c : R.col)
       if ((st = h->dev_alloc(&c.kk, n2h)) || (st = h->dev_alloc(&c.we, n2h)) ||
           (st = h->dev_alloc(&c.ns, n2h)) || (st = h->dev_alloc(&c.zw, n2h)) ||
           (st = h->dev_alloc(&c.iz, n2h)))
         return st;
-    double* r64;
-    float *r32, *b32;
-    if ((st = h->dev_alloc(&r64, n3h)) || (st = h->dev_alloc(&r32, n3h)) ||
-        (st = h->dev_alloc(&b32, n3h)))
-      return st;
-    R.dr64 = r64;
-    R.dr32 = r32;
-    R.db32 = b32;
-    launch_rb_setup(G, P, R, r64, r32, b32, h->stream);
-    ORCTM_CUDA_OK(cudaGetLastError());
   }
   // solver scalars
-  const int maxb = (int)solver_max_blocks(G);
+  const int maxb = solver_max_blocks();
   if ((st = h->dev_alloc(&h->S, 1))) return st;
   if ((st = h->dev_alloc(&h->partials, (size_t)4 * maxb))) return st;
   if (!(h->hS = pinned_state_get())) return h->fail(ORCTM_E_NOMEM, "pinned host memory exhausted");
@@ -742,10 +730,14 @@ int setup(orctm_handle* h, const orctm_desc* d) {
 
 template <typename T>
 int alloc_rb(orctm_handle* h, RbVectors<T>& v) {
-  const size_t n = (size_t)h->L.n3() / 2;  // zero-filled: values outside the unknowns stay 0
+  if (v.db) return ORCTM_OK;
+  const size_t n = rb_elements(h->R, sizeof(T));  // zero-filled: values outside the unknowns stay 0
   int st;
-  for (T** p : {&v.x, &v.r, &v.z, &v.p, &v.q, &v.u, &v.ub})
+  for (T** p : {&v.x, &v.r, &v.z, &v.p, &v.q, &v.u, &v.ub, &v.dr})
     if (!*p && (st = h->dev_alloc(p, n))) return st;
+  if ((st = h->dev_alloc(&v.db, n))) return st;
+  launch_rb_setup<T>(h->G, h->P, h->R, v, h->stream);
+  ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
 }
 
@@ -765,9 +757,8 @@ int read_state(orctm_handle* h) {
 
 // A chunk of PCG iterations (three kernels each) is captured once per
 // precision into the body of a graph's conditional while node: the vectors,
-// the solver scalars and the launch shapes of a handle are fixed.  The graph
-// is rebuilt when the shapes change; with profiling on, the launches go one
-// by one (they are bracketed by events).
+// the solver scalars and the launch shapes of a handle are fixed.  With
+// profiling on, the launches go one by one (they are bracketed by events).
 constexpr int kPcgChunk = 4;
 
 template <typename T>
@@ -778,24 +769,19 @@ template <>
 RbVectors<float>& rb_vectors<float>(orctm_handle* h) { return h->v32; }
 
 template <typename T>
-void pcg_iteration(orctm_handle* h, int cv, int sv) {
+void pcg_iteration(orctm_handle* h) {
   const RbVectors<T>& v = rb_vectors<T>(h);
-  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, cv, h->stream));
-  PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, sv, h->stream));
-  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, cv, h->stream));
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, h->stream));
+  PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, h->stream));
+  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, h->stream));
 }
 
 template <typename T>
 int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
   const int pr = sizeof(T) == 4;
-  const int cv = h->col_var[pr], sv = h->spmv_var[pr];
-  if (h->pcg_graph[pr] && h->pcg_graph_key[pr][0] == cv && h->pcg_graph_key[pr][1] == sv) {
+  if (h->pcg_graph[pr]) {
     *out = h->pcg_graph[pr];
     return ORCTM_OK;
-  }
-  if (h->pcg_graph[pr]) {
-    cudaGraphExecDestroy(h->pcg_graph[pr]);
-    h->pcg_graph[pr] = nullptr;
   }
   // a graph holding one conditional while node; its body is a chunk of
   // kPcgChunk iterations ended by the kernel that sets the loop condition
@@ -822,7 +808,7 @@ int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
     cudaGraphDestroy(g);
     return cuda_status(e);
   }
-  for (int k = 0; k < kPcgChunk; ++k) pcg_iteration<T>(h, cv, sv);
+  for (int k = 0; k < kPcgChunk; ++k) pcg_iteration<T>(h);
   launch_pcg_continue(hc, h->S, kPcgChunk, h->stream);
   const cudaError_t e1 = cudaStreamEndCapture(h->stream, &body);
   // launches are counted from the iterations the solve reports, not here
@@ -836,8 +822,6 @@ int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
   cudaGraphDestroy(g);
   ORCTM_CUDA_OK(e2);
   h->pcg_graph[pr] = ex;
-  h->pcg_graph_key[pr][0] = cv;
-  h->pcg_graph_key[pr][1] = sv;
   *out = ex;
   return ORCTM_OK;
 }
@@ -845,8 +829,6 @@ int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
 // One correction: A d = r (h->r) to the relative residual S->tol, added to h->xs.
 template <typename T>
 int pcg_loop(orctm_handle* h, int maxit, int* iters) {
-  const int pr = sizeof(T) == 4;
-  const int cv = h->col_var[pr], sv = h->spmv_var[pr];
   const RbVectors<T>& v = rb_vectors<T>(h);
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_before<T>(h->R, h->S, h->r, v, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
@@ -869,7 +851,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * (3 * kPcgChunk + 1));
   }
   while (!conv && it < maxit) {
-    pcg_iteration<T>(h, cv, sv);
+    pcg_iteration<T>(h);
     ORCTM_CUDA_OK(cudaGetLastError());  // a rejected launch is reported at once
     if (++it % kPcgChunk == 0 || it == maxit) {
       if ((st = read_state(h))) return st;
@@ -882,99 +864,6 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   return ORCTM_OK;
 }
 
-// Autotuner.  Times every launch shape of the column kernel and of the stencil
-// kernel on this handle's grid in precision T and keeps the fastest
-// (one untimed launch, then two timed with CUDA events).  It runs before
-// the first solve of the precision, on solver vectors that the solve writes
-// before it reads them, with scratch solver scalars.  The shapes compute
-// bit-identical results (the dot products are summed tile by tile in a fixed
-// order), so the choice changes only speed.
-// Choices are cached per grid size and precision for later handles.
-std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune_cache;
-
-template <typename T>
-int autotune(orctm_handle* h) {
-  const Geo& G = h->G;
-  const RbVectors<T>& v = rb_vectors<T>(h);
-  const int pr = sizeof(T) == 4;
-  const auto key = std::make_tuple(G.L.ie, G.L.je, G.L.ke, pr);
-  {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune_cache.find(key);
-    if (it != g_tune_cache.end()) {
-      h->col_var[pr] = h->force_col >= 0 ? h->force_col : it->second.first;
-      h->spmv_var[pr] = h->force_spmv >= 0 ? h->force_spmv : it->second.second;
-      return ORCTM_OK;
-    }
-  }
-  if (!h->S_tune) {
-    int st;
-    if ((st = h->dev_alloc(&h->S_tune, 1)) || (st = h->dev_alloc(&h->S_tune0, 1))) return st;
-    SolverState s0 = *h->hS;
-    s0.converged = 0;
-    s0.alpha = 0.0;
-    s0.alpha_prev = 0.0;
-    s0.beta = 0.0;
-    s0.iter = 1;
-    s0.rho = 1.0;
-    s0.bb = 1.0;
-    s0.tol = 0.0;
-    s0.ticket = 0;
-    ORCTM_CUDA_OK(cudaMemcpyAsync(h->S_tune0, &s0, sizeof(SolverState), cudaMemcpyHostToDevice,
-                                  h->stream));
-  }
-  auto timed = [&](auto launch, float* best_ms) -> int {
-    float tot = 0.f;
-    for (int rep = 0; rep < 3; ++rep) {
-      ORCTM_CUDA_OK(cudaMemcpyAsync(h->S_tune, h->S_tune0, sizeof(SolverState),
-                                    cudaMemcpyDeviceToDevice, h->stream));
-      if (rep >= 1) ORCTM_CUDA_OK(cudaEventRecord(h->ev0, h->stream));
-      launch();
-      ORCTM_CUDA_OK(cudaGetLastError());
-      if (rep >= 1) {
-        ORCTM_CUDA_OK(cudaEventRecord(h->ev1, h->stream));
-        ORCTM_CUDA_OK(cudaEventSynchronize(h->ev1));
-        float ms = 0.f;
-        ORCTM_CUDA_OK(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
-        tot += ms;
-      }
-    }
-    *best_ms = tot;
-    return ORCTM_OK;
-  };
-  int st, best_c = 0, best_s = 0;
-  float bc = 1e30f, bs = 1e30f;
-  for (int c = 0; c < pcg_col_variants(); ++c) {
-    float ms;
-    if ((st = timed([&] { launch_rb_col<T>(h->R, h->S_tune, v, c, h->stream); }, &ms))) return st;
-    if (ms < bc) { bc = ms; best_c = c; }
-  }
-  for (int c = 0; c < pcg_spmv_variants(); ++c) {
-    float ms;
-    if ((st = timed([&] { launch_rb_black<T>(h->R, h->S_tune, v, c, h->stream); }, &ms))) return st;
-    if (ms < bs) { bs = ms; best_s = c; }
-  }
-  {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key] = {best_c, best_s};
-  }
-  h->col_var[pr] = h->force_col >= 0 ? h->force_col : best_c;
-  h->spmv_var[pr] = h->force_spmv >= 0 ? h->force_spmv : best_s;
-  return ORCTM_OK;
-}
-
-int ensure_tuned(orctm_handle* h, bool f32) {
-  const int pr = f32 ? 1 : 0;
-  if (h->col_var[pr] >= 0 && h->spmv_var[pr] >= 0) return ORCTM_OK;
-  if (h->force_col >= 0 && h->force_spmv >= 0) {
-    h->col_var[pr] = h->force_col;
-    h->spmv_var[pr] = h->force_spmv;
-    return ORCTM_OK;
-  }
-  return f32 ? autotune<float>(h) : autotune<double>(h);
-}
-
 // Solves A x = b (b in h->b, x in h->xs holding the warm start) by iterative
 // refinement: r = b - A x in double-double against the exact operator, then
 // a PCG correction on the row-scaled operator (FP64, or FP32 for the refined
@@ -985,7 +874,8 @@ int poisson_solve(orctm_handle* h, orctm_solve_stats* stats) {
   orctm_solve_stats s{};
   const bool f32 = h->solver_mode == ORCTM_SOLVER_FP32_REFINED;
   const size_t n3 = (size_t)h->L.n3();
-  if ((st = ensure_tuned(h, f32))) return st;
+  h->col_var[f32] = std::max(h->force_col, 0);  // reported by orctm_get_tuning
+  h->spmv_var[f32] = std::max(h->force_spmv, 0);
   ORCTM_CUDA_OK(cudaEventRecord(h->ev0, h->stream));
   int total = 0, outer = 0;
   double prev = 1e300, rel = 0.0;
@@ -2637,8 +2527,7 @@ int orctm_profile_get(orctm_handle* h, int kind, long long* launches, double* to
 unsigned long long orctm_kernel_launches(void) { return launch_count(); }
 
 int orctm_set_tuning(orctm_handle* h, int col_variant, int spmv_variant) {
-  if (!h || col_variant < -1 || col_variant >= pcg_col_variants() || spmv_variant < -1 ||
-      spmv_variant >= pcg_spmv_variants())
+  if (!h || col_variant < -1 || col_variant >= 6 || spmv_variant < -1 || spmv_variant >= 9)
     return ORCTM_E_ARG;
   h->force_col = col_variant;
   h->force_spmv = spmv_variant;
@@ -2666,12 +2555,13 @@ int orctm_estimate_device_bytes(const orctm_desc* d, int solver, unsigned long l
   // 3D buffers: 12 state fields and the tracers, the routine temporaries of
   // the field pool (at most max(8, 2 ntracers + 2), the advection of all
   // tracers at once, plus the step's initial transports held for it), 3
-  // FP64 solver vectors, the pivots, and 7 half-length vectors of the
-  // reduced system (in FP64, and for the refined solver in FP32 too: a handle
+  // FP64 solver vectors, and the 7 half-length vectors of the reduced system
+  // and its pivots (in FP64, and for the refined solver in FP32 too: a handle
   // that has solved in both forms holds both)
   const double tmp = std::max(8.0, 2.0 * d->ntracers + 2.0) + 3.0;  // + the held transports
-  const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 1.0 +
-                    (solver == ORCTM_SOLVER_FP32_REFINED ? 5.25 : 3.5);
+  const double m32 = ((d->ie - 1) / 2 + 1 + 31) / 32 * 32;  // FP32 tiles hold 32 columns
+  const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 4.25 +
+                    (solver == ORCTM_SOLVER_FP32_REFINED ? 2.25 * std::max(1.0, 2.0 * m32 / P) : 0.0);
   // 2D tables (compressed columns, metrics, biharmonic and Poisson factors)
   const double f2 = 102.0;
   // every array carries two guard zones of about one plane

@@ -17,8 +17,8 @@ struct PoissonGeo {
 };
 
 // Red-black view of the Poisson columns (poisson.cu): column (i, j) is red when
-// i + j is even; column m = i / 2 of row j in a compact layout of pitch P/2.
-// 2D data of one colour's columns:
+// i + j is even, and is column m = i / 2 of row j.  2D data of one colour's
+// columns, at m + P/2 j:
 struct RbColour {
   unsigned long long* kk;     // wet levels: own, west, east, north, south, 10 bits each
   double2 *we, *ns;           // XU(I-1) XP, XU(I) XP ; YV(J-1) YP, YV(J) YP
@@ -31,14 +31,16 @@ struct RbGeo {
   int sms;                    // multiprocessors of the device
   RbColour col[2];            // red, black
   const double *zwn, *izn;
-  const double* dr64;         // red pivots 1/d'(K) of the column tridiagonal of B
-  const float *dr32, *db32;   // the same rounded to FP32; the black pivots
+  __host__ __device__ int nt(int W) const { return (M + W - 1) / W; }  // tiles per row
 };
-// Vectors of the reduced system (compact layout)
+// Vectors of the reduced system (tiled layout, zero outside the unknowns) and
+// the pivots 1/d'(K) of the column tridiagonal of B
 template <typename T>
 struct RbVectors {
   T *x, *r, *z, *p, *q;       // black
   T *u, *ub;                  // red: D_r^-1 C p ; D_r^-1 b
+  T* dr;                      // red pivots
+  float* db;                  // black pivots
 };
 
 // Device-resident scalars of one Krylov solve.
@@ -192,10 +194,13 @@ void launch_nh_rhs(const Geo& G, const double* uoo, const double* uoo1, const do
                    const double* voe1, const double* wno, const double* wno1, const double* zo,
                    double* b, cudaStream_t st);
 // poisson.cu
-// fills the red-black tables and pivots (once per handle)
-void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, double* dr64, float* dr32,
-                     float* db32, cudaStream_t st);
-size_t solver_max_blocks(const Geo& G);
+// elements of a vector of the reduced system, and the red-black tables and
+// pivots of a precision (once per handle and precision)
+size_t rb_elements(const RbGeo& R, int elem_bytes);
+template <typename T>
+void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, const RbVectors<T>& v,
+                     cudaStream_t st);
+int solver_max_blocks();
 // the reduced system's set-up (r, z and the scalars from b, the full-layout
 // right-hand side), the three kernels of an iteration, and the correction's
 // addition to x (full layout).  The FP32 form scales b by 1/||b||_2.
@@ -203,16 +208,13 @@ template <typename T>
 void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbVectors<T>& v,
                       cudaStream_t st);
 template <typename T>
-void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 template <typename T>
-void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 template <typename T>
-void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant, cudaStream_t st);
+void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x, cudaStream_t st);
-// launch shapes the autotuner chooses between (column kernels, stencil kernel)
-int pcg_col_variants();
-int pcg_spmv_variants();
 // r = b - A x in double-double, and x := 0 on land rows (their solution)
 void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const double* b, double* x,
                   double* r, cudaStream_t st);

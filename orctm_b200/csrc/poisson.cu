@@ -30,25 +30,29 @@
 // twice as many iterations).  Red unknowns are formed from the black ones
 // before and after the iterations.
 //
-// Vectors are stored compactly per colour: column (i, j) at m = i / 2, so both
-// colours use offset m + P/2 (j + JN l).  The in-row neighbours of column
-// (m, j) are (m - 1 + s, j) and (m + s, j) of the other colour, s = 0 or 1 by
-// the parity of the row; north and south are (m, j -+ 1).
+// Vectors are stored per colour, column (i, j) at m = i / 2 of row j, in tiles
+// of W columns (128 bytes of a level) that hold all their levels one after
+// the other: offset ((j NT + m / W) KE + l) W + m mod W.  A tile is some 10 KB
+// of consecutive memory; in the padded layout of the model's fields its levels lie
+// megabytes apart on 1024 x 1024 x 80, where every block then touched some 80
+// pages per vector (stencil kernel 1.65 ms a launch; see below).  The in-row
+// neighbours of column (m, j) are (m - 1 + s, j) and (m + s, j) of the other
+// colour, s = 0 or 1 by the parity of the row; north and south are (m, j -+ 1).
 //
-// A column is shared by G lanes of a warp, each with LC consecutive levels in
-// registers (a warp holds 32/G columns: 32-byte segments of a level's row).
-// The tridiagonal recurrences run level by level inside a lane and as a scan
-// of affine maps across the column's lanes, so the whole column is loaded at
-// once and nothing is spilled.  A thread that marches down a column alone
-// waits a memory latency every few levels: 27 us against 5 per launch on the
-// 512 x 1 x 60 slice, and 0.62 of the copy bandwidth on 1024 x 1024 x 80.
+// A block takes a tile at a time.  A column is shared by G threads, each with LC
+// consecutive levels in registers; consecutive threads hold consecutive
+// columns, so every load is a full 128-byte line and a thread's loads are
+// issued together.  The tridiagonal recurrences run level by level inside a
+// thread and as a scan of affine maps over the column's threads through
+// shared memory, so nothing is spilled or read twice.  A thread that marches
+// down a column alone waits a memory latency every few levels (27 us a launch on
+// the 512 x 1 x 60 slice).
 //
-// Dot products are reduced deterministically: every tile writes a partial sum
-// and the last block to finish (atomic ticket) adds the partials in tile
+// Dot products are reduced deterministically: every block writes a partial sum
+// and the last one to finish (atomic ticket) adds the partials in block
 // order and updates the solver scalars on the device, so an iteration
-// needs no host round trip, and totals do not depend on the launch shape.  A
-// device flag marks convergence; kernels of an already converged solve return
-// at once.
+// needs no host round trip.  A device flag marks convergence; kernels of an
+// already converged solve return at once.
 #include <algorithm>
 #include <type_traits>
 
@@ -172,40 +176,44 @@ __device__ __forceinline__ Coef row(const ColC& c, const PoissonGeo& P, int K, i
 }
 
 // ------------------------------------------------------- reductions ------
-// Partial sums of one tile: the block's threads are added in a fixed order.
-constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr int kMaxBlocks = 4096;  // the largest grid that leaves partial sums
 
-template <int NV>
-__device__ __forceinline__ void tile_partial(const double (&v)[NV], SolverState* S, int tile) {
-  __shared__ double sh[NV][kWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double x = v[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[q][warp] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < NV) {
-    double x = 0.0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) x += sh[threadIdx.x][w];
-    S->partials[(size_t)threadIdx.x * S->max_blocks + tile] = x;
-  }
-  __syncthreads();
-}
-
-// After a block's last tile: true in thread 0 of the last block to get here,
-// which then holds the totals over all tiles in v.
-template <int NV>
-__device__ bool grid_total(double (&v)[NV], SolverState* S, int ntiles) {
+// A block adds its threads' values in a fixed order and writes one partial;
+// true in thread 0 of the last block of the grid to get here, which then holds
+// the totals in v (partials added in block order).  Grids are a function of
+// the sizes and the device alone, so totals are reproducible.
+template <int NV, int kThreads>
+__device__ bool grid_sum(double (&v)[NV], SolverState* S) {
+  constexpr int kWarps = kThreads / 32;
   __shared__ double sh[NV][kWarps];
   __shared__ bool last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < NV) __threadfence();
-  __syncthreads();
-  if (tid == 0) last = atomicAdd(&S->ticket, 1u) == gridDim.x - 1;
+  auto block_sum = [&]() {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double x = v[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) sh[q][warp] = x;
+    }
+    __syncthreads();
+    if (tid == 0) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) x += sh[q][w];
+        v[q] = x;
+      }
+    }
+  };
+  block_sum();
+  if (tid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) S->partials[(size_t)q * S->max_blocks + blockIdx.x] = v[q];
+    __threadfence();
+    last = atomicAdd(&S->ticket, 1u) == gridDim.x - 1;
+  }
   __syncthreads();
   if (!last) return false;
   __threadfence();
@@ -214,22 +222,11 @@ __device__ bool grid_total(double (&v)[NV], SolverState* S, int ntiles) {
     const double* part = S->partials + (size_t)q * S->max_blocks;
     double x = 0.0;
 #pragma unroll 8
-    for (int b = tid; b < ntiles; b += kThreads) x += __ldcg(part + b);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[q][warp] = x;
+    for (int b = tid; b < (int)gridDim.x; b += kThreads) x += __ldcg(part + b);
+    v[q] = x;
   }
-  __syncthreads();
-  if (tid == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double x = 0.0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) x += sh[q][w];
-      v[q] = x;
-    }
-    S->ticket = 0;
-  }
+  block_sum();
+  if (tid == 0) S->ticket = 0;
   return tid == 0;
 }
 
@@ -237,14 +234,22 @@ __device__ bool grid_total(double (&v)[NV], SolverState* S, int ntiles) {
 __device__ __forceinline__ int red_i(int m, int j) { return 2 * m + (j & 1); }
 __device__ __forceinline__ int black_i(int m, int j) { return 2 * m + 1 - (j & 1); }
 
+// Columns per tile: 128 bytes of a level
+template <typename T>
+struct Width {
+  static constexpr int W = 128 / (int)sizeof(T);
+};
+
 // Pivots of the column tridiagonal of B (constant): dinv(K) = 1/d'(K) with
-// d'(1) = d(1), d'(K) = d(K) - a(K) c(K-1) / d'(K-1), per colour in the
-// compact layout: the red ones in FP64 and FP32 (the elimination is exact to
+// d'(1) = d(1), d'(K) = d(K) - a(K) c(K-1) / d'(K-1), in the layout of
+// precision T: the red ones in T (the elimination is exact to
 // the solve's precision), the black ones, a fixed preconditioner, in FP32 for
 // both forms; and the 2D data of the columns.  Columns that are no unknowns
 // keep kk = 0 (no wet level).
-__global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, double* __restrict__ dr64,
-                           float* __restrict__ dr32, float* __restrict__ db32) {
+template <typename T>
+__global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, T* __restrict__ dr,
+                           float* __restrict__ db) {
+  constexpr int W = Width<T>::W;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   const int KE = G.L.ke;
@@ -265,48 +270,35 @@ __global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, double* __restrict__ dr
     const Coef r = row<true>(c, P, K, KE);
     const double d = K == 1 ? r.dc : r.dc - (r.u * dprev) * cprev;
     const double di = 1.0 / d;
-    const int o = s + R.plane2 * (K - 1);
-    if (black) {
-      db32[o] = (float)di;
-    } else {
-      dr64[o] = di;
-      dr32[o] = (float)di;
-    }
+    const int m = i >> 1, o = ((j * R.nt(W) + m / W) * KE + K - 1) * W + m % W;
+    if (black) db[o] = (float)di;
+    else dr[o] = (T)di;
     dprev = di;
     cprev = r.d;
   }
 }
 
 // ------------------------------------------------------- PCG kernels -----
-// Where a thread stands: G lanes per column, LC levels per lane.
+// Where a thread stands: column c of the tile, levels K0 + 1 .. K0 + LC.
 template <typename T, int G, int LC>
 struct Lane {
-  static constexpr int CW = 32 / G;          // columns per warp
-  static constexpr int CT = kWarps * CW;     // columns per tile
-  static constexpr int TAB = G * (LC + 1) + 1;
-  int m, g, K0, tab;                         // column, lane in it, first level - 1, its table entry
-  __device__ __forceinline__ Lane() {
-    const int lane = threadIdx.x & 31;
-    g = lane / CW;
-    m = (threadIdx.x >> 5) * CW + lane % CW;
-    K0 = g * LC;
-    tab = g * (LC + 1);
-  }
+  static constexpr int W = Width<T>::W, NT = W * G;  // columns per tile, threads per block
+  int c, g, K0;
+  __device__ __forceinline__ Lane() : c(threadIdx.x % W), g(threadIdx.x / W), K0(g * LC) {}
 };
 
-// ZW(K) at szw[e + e / LC], e = K - 1 = 0..KE, and 1/ZP(K) alike: the lanes
-// of a column read LC + 1 entries apart (no bank conflicts).
+// ZW(K) at szw[K - 1], K = 1..KE+1, and 1/ZP(K) at siz[K - 1]
 template <typename T, int G, int LC>
 __device__ __forceinline__ void load_tables(const RbGeo& R, T* szw, T* siz) {
-  for (int e = threadIdx.x; e <= G * LC; e += kThreads) {
-    szw[e + e / LC] = e <= R.ke ? (T)R.zwn[e] : T(0);
-    if (siz) siz[e + e / LC] = e < R.ke ? (T)R.izn[e] : T(0);
+  for (int e = threadIdx.x; e <= G * LC; e += Lane<T, G, LC>::NT) {
+    szw[e] = e <= R.ke ? (T)R.zwn[e] : T(0);
+    if (siz) siz[e] = e < R.ke ? (T)R.izn[e] : T(0);
   }
   __syncthreads();
 }
 
-// Couplings a(K) between levels K - 1 and K of the lane's levels and of the one
-// below its last: ZW(K) inside the column (its own value at the bottom),
+// Couplings a(K) between levels K - 1 and K of the thread's levels and of the
+// one below its last: ZW(K) inside the column (its own value at the bottom),
 // 0 at the surface and below the bottom.
 template <typename T, int G, int LC>
 __device__ __forceinline__ void couplings(const Lane<T, G, LC>& t, const T* szw, int kb, T zwa,
@@ -314,22 +306,25 @@ __device__ __forceinline__ void couplings(const Lane<T, G, LC>& t, const T* szw,
 #pragma unroll
   for (int u = 0; u <= LC; ++u) {
     const int K = t.K0 + 1 + u;
-    const T zw = szw[t.tab + u + (u == LC)];
+    const T zw = szw[t.K0 + u];
     a[u] = (K == 1 || K > kb) ? T(0) : (K == kb ? zwa : zw);
   }
 }
 
-// v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d and
-// couplings a; returns v.M^-1 v = sum y^2 / d of this lane's levels.
+// Affine maps of the threads of a column, down and up
+template <typename T, int G, int W>
+struct Scan {
+  T fa[G][W], fb[G][W], ba[G][W], bb[G][W];
+};
+
+// v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d (dm: the
+// pivot above the thread's first level) and couplings a; returns v.M^-1 v =
+// sum y^2 / d of this thread's levels.  Two block barriers.
 template <typename T, int G, int LC>
-__device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, T (&v)[LC], const T (&d)[LC],
-                                          const T (&a)[LC + 1]) {
-  constexpr int CW = 32 / G;
-  constexpr unsigned kAll = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the lane's levels as one affine
-  // map y_out = A y_in + B, scanned over the lanes above
-  const T dm = __shfl_up_sync(kAll, d[LC - 1], CW);
+__device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, Scan<T, G, Lane<T, G, LC>::W>& sc,
+                                          T (&v)[LC], const T (&d)[LC], T dm, const T (&a)[LC + 1]) {
+  // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the thread's levels as one affine
+  // map y_out = A y_in + B, applied in turn to what comes from above
   T A = T(1), B = T(0);
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
@@ -337,16 +332,13 @@ __device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, T (&v)[LC], c
     B = fma(l, B, v[u]);
     A = l * A;
   }
+  sc.fa[t.g][t.c] = A;
+  sc.fb[t.g][t.c] = B;
+  __syncthreads();
+  T y = T(0);
 #pragma unroll
-  for (int o = CW; o < 32; o <<= 1) {
-    const T Ap = __shfl_up_sync(kAll, A, o), Bp = __shfl_up_sync(kAll, B, o);
-    if (lane >= o) {
-      B = fma(A, Bp, B);
-      A *= Ap;
-    }
-  }
-  T y = __shfl_up_sync(kAll, B, CW);
-  if (t.g == 0) y = T(0);
+  for (int k = 0; k < G - 1; ++k)
+    if (k < t.g) y = fma(sc.fa[k][t.c], y, sc.fb[k][t.c]);
   T rz = T(0);
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
@@ -363,16 +355,13 @@ __device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, T (&v)[LC], c
     B = fma(l, B, v[u]);
     A = l * A;
   }
+  sc.ba[t.g][t.c] = A;
+  sc.bb[t.g][t.c] = B;
+  __syncthreads();
+  T z = T(0);
 #pragma unroll
-  for (int o = CW; o < 32; o <<= 1) {
-    const T Ap = __shfl_down_sync(kAll, A, o), Bp = __shfl_down_sync(kAll, B, o);
-    if (lane + o < 32) {
-      B = fma(A, Bp, B);
-      A *= Ap;
-    }
-  }
-  T z = __shfl_down_sync(kAll, B, CW);
-  if (t.g == G - 1) z = T(0);
+  for (int k = G - 1; k > 0; --k)
+    if (k > t.g) z = fma(sc.ba[k][t.c], z, sc.bb[k][t.c]);
 #pragma unroll
   for (int u = LC - 1; u >= 0; --u) {
     z = fma(-(a[u + 1] * d[u]), z, v[u]);
@@ -385,6 +374,64 @@ __device__ __forceinline__ int wet_levels(unsigned long long kk, int nb) {
   return (int)((kk >> (10 * nb)) & 1023u);
 }
 
+// One tile: row j, columns m, the offset o0 of the thread's first level in the
+// tiled layout, and its in-row neighbours of the other colour relative to it.
+// kk of the block's next tile is loaded while this one is computed.
+template <typename T, int G, int LC>
+struct Tiles {
+  static constexpr int W = Width<T>::W;
+  int tile, next_tile;
+  int j, m, s2, o0, west, east;
+  unsigned long long kk, kn;
+  __device__ __forceinline__ Tiles(const RbGeo& R, const RbColour& q, const Lane<T, G, LC>& t,
+                                   int ntiles, int nt)
+      : next_tile(blockIdx.x) {
+    kn = fetch(R, q, t, ntiles, nt);
+  }
+  __device__ __forceinline__ unsigned long long fetch(const RbGeo& R, const RbColour& q,
+                                                      const Lane<T, G, LC>& t, int ntiles, int nt) {
+    const int jn = 2 + next_tile / nt, mn = (next_tile % nt) * W + t.c;
+    return next_tile < ntiles && mn < R.M ? __ldg(q.kk + mn + R.P2 * jn) : 0ull;
+  }
+  // sh: 0 when the west neighbour is column m - 1, 1 when it is column m
+  __device__ __forceinline__ bool next(const RbGeo& R, const RbColour& q, const Lane<T, G, LC>& t,
+                                       int ntiles, int nt, bool red) {
+    tile = next_tile;
+    if (tile >= ntiles) return false;
+    kk = kn;
+    j = 2 + tile / nt;
+    const int b = tile % nt;
+    m = b * W + t.c;
+    s2 = kk ? m + R.P2 * j : 0;
+    o0 = ((j * nt + b) * R.ke + t.K0) * W + t.c;
+    const int sh = red ? (j & 1) : 1 - (j & 1);
+    const int back = t.c == 0 ? (W - 1) - R.ke * W : -1;      // column m - 1
+    const int ahead = t.c == W - 1 ? R.ke * W - (W - 1) : 1;  // column m + 1
+    west = sh ? 0 : back;
+    east = sh ? ahead : 0;
+    next_tile += gridDim.x;
+    kn = fetch(R, q, t, ntiles, nt);
+    return true;
+  }
+};
+
+// Asks for a tile of a vector (tiled layout: consecutive memory) in L2 while the
+// block works on the one before it.
+template <typename T>
+__device__ __forceinline__ void prefetch_tile(const T* a, int tile, int nt, int ke) {
+  const T* p = a + (size_t)(tile + 2 * nt) * ke * Width<T>::W;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(ke * 128) : "memory");
+}
+
+// Offset of level q of the thread, or, for a level that is not wet, of an
+// element whose value and neighbours are 0 in every vector (row 1 holds no unknown and
+// column 0 of row 2 neither): the loads of a thread's levels carry no branch
+// and are issued together.
+template <int W>
+__device__ __forceinline__ int at_level(int o0, int q, bool wet, int zero) {
+  return wet ? o0 + W * q : zero;
+}
+
 // Red columns.
 //   kIter    u = D^-1 C v + beta u          (v = z; u is not read while beta = 0)
 //   kBefore  u = D^-1 (b / ZP)              (b: full layout, scaled); sum of (b / ZP)^2
@@ -392,13 +439,14 @@ __device__ __forceinline__ int wet_levels(unsigned long long kk, int nb) {
 enum { kIter = 0, kBefore = 1, kAfter = 2 };
 
 template <typename T, int G, int LC, int MODE>
-__global__ void __launch_bounds__(kThreads) k_rb_red(RbGeo R, SolverState* S,
+__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_red(RbGeo R, SolverState* S,
                                                      const T* __restrict__ v, T* __restrict__ u,
                                                      const T* __restrict__ dinv,
                                                      const double* __restrict__ b,
-                                                     double* __restrict__ x, int ntiles, int nmc) {
+                                                     double* __restrict__ x, int ntiles, int nt) {
   using Ln = Lane<T, G, LC>;
-  __shared__ T szw[Ln::TAB], siz[Ln::TAB];
+  constexpr int W = Ln::W;
+  __shared__ T szw[G * LC + 1], siz[G * LC + 1];
   if (MODE == kIter && S->converged) return;
   const T beta = MODE == kIter ? (T)S->beta : T(0);
   double scale = 1.0;
@@ -407,74 +455,75 @@ __global__ void __launch_bounds__(kThreads) k_rb_red(RbGeo R, SolverState* S,
     if (MODE == kBefore) scale = scale > 0.0 ? 1.0 / scale : 0.0;
   }
   load_tables<T, G, LC>(R, szw, siz);
+  __shared__ Scan<T, G, W> scan;
   const Ln t;
-  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
-    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
-    unsigned long long kk = 0;
-    if (m < R.M) kk = R.col[0].kk[s2];
-    const int kb = wet_levels(kk, 0);
-    T cw = 0, ce = 0, cn = 0, cs = 0, zwa = 0;
-    double iza = 0, izb = 0;
-    if (kb) {
-      const double2 we = R.col[0].we[s2], ns = R.col[0].ns[s2], iz = R.col[0].iz[s2];
-      cw = (T)we.x; ce = (T)we.y; cn = (T)ns.x; cs = (T)ns.y;
-      zwa = (T)R.col[0].zw[s2].x;
-      iza = iz.x; izb = iz.y;
+  const int row = nt * R.ke * W, zero = row;
+  const int P = 2 * R.P2, plane = 2 * R.plane2;  // full layout
+  double bb = 0.0;
+  Tiles<T, G, LC> it(R, R.col[0], t, ntiles, nt);
+  while (it.next(R, R.col[0], t, ntiles, nt, true)) {
+    if (MODE == kIter && threadIdx.x == 0 && it.next_tile < ntiles) {
+      prefetch_tile(dinv, it.next_tile, nt, R.ke);
+      prefetch_tile(v, it.next_tile, nt, R.ke);
+      prefetch_tile(u, it.next_tile, nt, R.ke);
     }
-    const unsigned o0 = s2 + plane * (unsigned)t.K0;
-    const unsigned ow = o0 - 1u + (unsigned)(j & 1);
+    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
     T g[LC], d[LC], a[LC + 1];
-    couplings<T, G, LC>(t, szw, kb, zwa, a);
-    double bb = 0.0;
 #pragma unroll
-    for (int q = 0; q < LC; ++q) {
-      const int K = t.K0 + 1 + q;
-      const unsigned l = plane * (unsigned)q;
-      g[q] = d[q] = T(0);
-      if (K <= kb) {
-        d[q] = dinv[o0 + l];
-        if (MODE == kBefore) {
-          const double hs = K == kb ? izb : (K == kb - 1 ? iza : R.izn[K - 1]);
-          const unsigned f = (unsigned)red_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
-          g[q] = (T)((b[f] * scale) * hs);
-          bb = fma((double)g[q], (double)g[q], bb);
-        } else {
-          // values of land cells and outside the unknowns are exact zeros
-          const T hs = K == kb ? (T)izb : (K == kb - 1 ? (T)iza : siz[t.tab + q]);
-          T h = cw * v[ow + l];
-          h = fma(ce, v[ow + l + 1u], h);
-          h = fma(cn, v[o0 + l - P2], h);
-          h = fma(cs, v[o0 + l + P2], h);
-          g[q] = hs * h;
-        }
-      }
-    }
-    column_solve<T, G, LC>(t, g, d, a);
-#pragma unroll
-    for (int q = 0; q < LC; ++q) {
-      const int K = t.K0 + 1 + q;
-      const unsigned o = o0 + plane * (unsigned)q;
-      if (K <= kb) {
-        if (MODE == kIter) {
-          u[o] = beta == T(0) ? g[q] : fma(beta, u[o], g[q]);
-        } else if (MODE == kBefore) {
-          u[o] = g[q];
-        } else {
-          const unsigned f = (unsigned)red_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
-          x[f] = x[f] + scale * (double)(u[o] - g[q]);
-        }
-      }
-    }
+    for (int q = 0; q < LC; ++q) d[q] = dinv[at_level<W>(o0, q, t.K0 + 1 + q <= kb, zero)];
+    const T dm = dinv[at_level<W>(o0, -1, t.K0 > 0 && t.K0 <= kb, zero)];
+    const T zwa = (T)R.col[0].zw[it.s2].x;
+    const double2 iz = R.col[0].iz[it.s2];
+    const int f0 = red_i(it.m, it.j) + P * it.j + plane * t.K0;
     if (MODE == kBefore) {
-      const double w[1] = {bb};
-      tile_partial<1>(w, S, tile);
+#pragma unroll
+      for (int q = 0; q < LC; ++q) {
+        const int K = t.K0 + 1 + q;
+        const double hs = K == kb ? iz.y : (K == kb - 1 ? iz.x : (double)R.izn[K <= kb ? K - 1 : 0]);
+        const double bv = b[K <= kb ? f0 + plane * q : 0];
+        g[q] = K <= kb ? (T)((bv * scale) * hs) : T(0);
+        bb = fma((double)g[q], (double)g[q], bb);
+      }
+    } else {
+      const double2 we = R.col[0].we[it.s2], ns = R.col[0].ns[it.s2];
+      const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+#pragma unroll
+      for (int q = 0; q < LC; ++q) {
+        // values of land cells and outside the unknowns are exact zeros
+        const int K = t.K0 + 1 + q, o = at_level<W>(o0, q, K <= kb, zero);
+        const T hs = K == kb ? (T)iz.y : (K == kb - 1 ? (T)iz.x : siz[t.K0 + q]);
+        T h = cw * v[o + it.west];
+        h = fma(ce, v[o + it.east], h);
+        h = fma(cn, v[o - row], h);
+        h = fma(cs, v[o + row], h);
+        g[q] = hs * h;
+      }
+    }
+    couplings<T, G, LC>(t, szw, kb, zwa, a);
+    column_solve<T, G, LC>(t, scan, g, d, dm, a);
+    if (MODE == kIter && beta != T(0)) {
+      T uo[LC];
+#pragma unroll
+      for (int q = 0; q < LC; ++q) uo[q] = u[at_level<W>(o0, q, t.K0 + 1 + q <= kb, zero)];
+#pragma unroll
+      for (int q = 0; q < LC; ++q) g[q] = fma(beta, uo[q], g[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < LC; ++q) {
+      const int o = o0 + W * q;
+      if (t.K0 + 1 + q <= kb) {
+        if (MODE == kAfter) {
+          const int f = f0 + plane * q;
+          x[f] = x[f] + scale * (double)(u[o] - g[q]);
+        } else {
+          u[o] = g[q];
+        }
+      }
     }
   }
   if (MODE == kBefore) {
-    double w[1];
-    if (grid_total<1>(w, S, ntiles)) S->bb = w[0];
+    double w[1] = {bb};
+    if (grid_sum<1, Ln::NT>(w, S)) S->bb = w[0];
   }
 }
 
@@ -482,92 +531,101 @@ __global__ void __launch_bounds__(kThreads) k_rb_red(RbGeo R, SolverState* S,
 // q = D p - C u, and alpha = rho / p.q.  The first iteration (iter = 0) reads
 // neither p nor x.
 template <typename T, int G, int LC>
-__global__ void __launch_bounds__(kThreads) k_rb_black(RbGeo R, SolverState* S,
+__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_black(RbGeo R, SolverState* S,
                                                        const T* __restrict__ z,
                                                        const T* __restrict__ u, T* __restrict__ p,
                                                        T* __restrict__ x, T* __restrict__ q,
-                                                       int ntiles, int nmc) {
+                                                       int ntiles, int nt) {
   using Ln = Lane<T, G, LC>;
-  __shared__ T szw[Ln::TAB], siz[Ln::TAB];
+  constexpr int W = Ln::W;
+  __shared__ T szw[G * LC + 1], siz[G * LC + 1];
   if (S->converged) return;
   const T beta = (T)S->beta, alpha = (T)S->alpha_prev;
   const bool first = S->iter == 0;
   load_tables<T, G, LC>(R, szw, siz);
+  __shared__ T top[2][G][W], bottom[2][G][W];  // p of the threads' first and last levels
   const Ln t;
-  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
-    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
-    unsigned long long kk = 0;
-    if (m < R.M) kk = R.col[1].kk[s2];
-    const int kb = wet_levels(kk, 0);
-    const int kbw = wet_levels(kk, 1), kbe = wet_levels(kk, 2);
-    const int kbn = wet_levels(kk, 3), kbs = wet_levels(kk, 4);
-    T cw = 0, ce = 0, cn = 0, cs = 0, zwa = 0, zwb = 0, iza = 0, izb = 0;
-    if (kb) {
-      const double2 we = R.col[1].we[s2], ns = R.col[1].ns[s2], iz = R.col[1].iz[s2],
-                    zw = R.col[1].zw[s2];
-      cw = (T)we.x; ce = (T)we.y; cn = (T)ns.x; cs = (T)ns.y;
-      zwa = (T)zw.x; zwb = (T)zw.y;
-      iza = (T)iz.x; izb = (T)iz.y;
+  const int row = nt * R.ke * W, zero = row;
+  double pq = 0.0;
+  int buf = 0;
+  Tiles<T, G, LC> it(R, R.col[1], t, ntiles, nt);
+  while (it.next(R, R.col[1], t, ntiles, nt, false)) {
+    if (threadIdx.x == 0 && it.next_tile < ntiles) {
+      prefetch_tile(z, it.next_tile, nt, R.ke);
+      prefetch_tile(p, it.next_tile, nt, R.ke);
+      prefetch_tile(x, it.next_tile, nt, R.ke);
+      prefetch_tile(u, it.next_tile, nt, R.ke);
     }
-    const unsigned o0 = s2 + plane * (unsigned)t.K0;
-    const unsigned ow = o0 - (unsigned)(j & 1);
+    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
+    const int kbw = wet_levels(it.kk, 1), kbe = wet_levels(it.kk, 2);
+    const int kbn = wet_levels(it.kk, 3), kbs = wet_levels(it.kk, 4);
     T pl[LC];
+    {
+      T po[LC], xo[LC];
 #pragma unroll
-    for (int e = 0; e < LC; ++e) {
-      const unsigned o = o0 + plane * (unsigned)e;
-      pl[e] = T(0);
-      if (t.K0 + 1 + e <= kb) {
-        T pn = z[o];
-        if (first) {
-          x[o] = T(0);
-        } else {
-          const T po = p[o];
-          x[o] = fma(alpha, po, x[o]);
-          pn = fma(beta, po, pn);
+      for (int e = 0; e < LC; ++e) pl[e] = z[at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero)];
+#pragma unroll
+      for (int e = 0; e < LC; ++e) {
+        const int o = at_level<W>(o0, e, t.K0 + 1 + e <= kb && !first, zero);
+        po[e] = p[o];
+        xo[e] = x[o];
+      }
+#pragma unroll
+      for (int e = 0; e < LC; ++e) {
+        xo[e] = fma(alpha, po[e], xo[e]);
+        pl[e] = fma(beta, po[e], pl[e]);
+        if (t.K0 + 1 + e <= kb) {
+          x[o0 + W * e] = xo[e];
+          p[o0 + W * e] = pl[e];
         }
-        p[o] = pn;
-        pl[e] = pn;
       }
     }
-    T pu = __shfl_up_sync(0xffffffffu, pl[LC - 1], Ln::CW);
-    T pb = __shfl_down_sync(0xffffffffu, pl[0], Ln::CW);
-    if (t.g == 0) pu = T(0);
-    if (t.g == G - 1) pb = T(0);
-    T pq = T(0);
+    top[buf][t.g][t.c] = pl[0];
+    bottom[buf][t.g][t.c] = pl[LC - 1];
+    const double2 we = R.col[1].we[it.s2], ns = R.col[1].ns[it.s2], iz = R.col[1].iz[it.s2],
+                  zw = R.col[1].zw[it.s2];
+    const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+    const T zwa = (T)zw.x;
+    __syncthreads();
+    T pu = t.g == 0 ? T(0) : bottom[buf][t.g - 1][t.c];
+    const T pb = t.g == G - 1 ? T(0) : top[buf][t.g + 1][t.c];
+    buf ^= 1;
+    T pqt = T(0), v[LC];
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const int K = t.K0 + 1 + e, o = at_level<W>(o0, e, K <= kb, zero);
+      T h = cw * u[o + it.west];
+      h = fma(ce, u[o + it.east], h);
+      h = fma(cn, u[o - row], h);
+      v[e] = fma(cs, u[o + row], h);
+    }
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
       const int K = t.K0 + 1 + e;
-      if (K <= kb) {
-        const unsigned o = o0 + plane * (unsigned)e, w = ow + plane * (unsigned)e;
-        const T p0 = pl[e], pd = e + 1 < LC ? pl[e + 1] : pb;
-        T dh = K <= kbw ? cw : T(0);
-        if (K <= kbe) dh += ce;
-        if (K <= kbn) dh += cn;
-        if (K <= kbs) dh += cs;
-        T h = cw * u[w];
-        h = fma(ce, u[w + 1u], h);
-        h = fma(cn, u[o - P2], h);
-        h = fma(cs, u[o + P2], h);
-        h = fma(dh, p0, h);
-        const T hs = K == kb ? izb : (K == kb - 1 ? iza : siz[t.tab + e]);
-        const T zw0 = K == kb ? zwa : szw[t.tab + e];
-        const T zw1 = K + 1 == kb ? zwa : szw[t.tab + e + 1 + (e + 1 == LC)];
-        T s = zw0 * (pu - p0);
-        if (K < kb) s = fma(zw1, pd - p0, s);
-        else if (K == 1) s = fma(-zwb, p0, s);  // Z_C of the surface row keeps ZW(2)
-        s = fma(-hs, h, s);
-        q[o] = s;
-        pq = fma(p0, s, pq);
-      }
-      pu = pl[e];
+      const T p0 = pl[e], pd = e + 1 < LC ? pl[e + 1] : pb;
+      T dh = K <= kbw ? cw : T(0);
+      dh += K <= kbe ? ce : T(0);
+      dh += K <= kbn ? cn : T(0);
+      dh += K <= kbs ? cs : T(0);
+      const T h = fma(dh, p0, v[e]);
+      const T hs = K == kb ? (T)iz.y : (K == kb - 1 ? (T)iz.x : siz[t.K0 + e]);
+      const T zw0 = K == kb ? zwa : szw[t.K0 + e];
+      // below the bottom nothing couples, but Z_C of the surface row keeps ZW(2)
+      T zw1 = K + 1 == kb ? zwa : szw[t.K0 + e + 1];
+      if (K == kb) zw1 = K == 1 ? (T)zw.y : T(0);
+      v[e] = zw0 * (pu - p0);
+      v[e] = fma(zw1, pd - p0, v[e]);
+      v[e] = fma(-hs, h, v[e]);
+      pqt = fma(p0, v[e], pqt);  // p0 = 0 below the bottom
+      pu = p0;
     }
-    const double w[1] = {(double)pq};
-    tile_partial<1>(w, S, tile);
+#pragma unroll
+    for (int e = 0; e < LC; ++e)
+      if (t.K0 + 1 + e <= kb) q[o0 + W * e] = v[e];
+    pq += (double)pqt;
   }
-  double w[1];
-  if (grid_total<1>(w, S, ntiles)) {
+  double w[1] = {pq};
+  if (grid_sum<1, Ln::NT>(w, S)) {
     S->pq = w[0];
     S->alpha = S->rho / w[0];
     if (!(w[0] > 0.0) && !(w[0] < 0.0)) S->converged = 3;  // breakdown
@@ -578,72 +636,81 @@ __global__ void __launch_bounds__(kThreads) k_rb_black(RbGeo R, SolverState* S,
 //   INIT   r = b / ZP - C u     (u = D_r^-1 (b / ZP) of the red columns)
 //   else   r -= alpha q
 template <typename T, int G, int LC, bool INIT>
-__global__ void __launch_bounds__(kThreads) k_rb_col(RbGeo R, SolverState* S, T* __restrict__ r,
+__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_col(RbGeo R, SolverState* S, T* __restrict__ r,
                                                      const T* __restrict__ q, T* __restrict__ z,
                                                      const float* __restrict__ dinv,
                                                      const double* __restrict__ b,
                                                      const T* __restrict__ ub, int ntiles,
-                                                     int nmc) {
+                                                     int nt) {
   using Ln = Lane<T, G, LC>;
-  __shared__ T szw[Ln::TAB];
+  constexpr int W = Ln::W;
+  __shared__ T szw[G * LC + 1];
   if (!INIT && S->converged) return;
   const T alpha = INIT ? T(0) : (T)S->alpha;
   double scale = 1.0;
   if (INIT && sizeof(T) == 4) scale = S->res_rr > 0.0 ? 1.0 / sqrt(S->res_rr) : 0.0;
   load_tables<T, G, LC>(R, szw, nullptr);
+  __shared__ Scan<T, G, W> scan;
   const Ln t;
-  const unsigned P2 = (unsigned)R.P2, plane = (unsigned)R.plane2;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int j = 2 + tile / nmc, m = (tile % nmc) * Ln::CT + t.m;
-    const unsigned s2 = (unsigned)m + P2 * (unsigned)j;
-    unsigned long long kk = 0;
-    if (m < R.M) kk = R.col[1].kk[s2];
-    const int kb = wet_levels(kk, 0);
-    const T zwa = kb ? (T)R.col[1].zw[s2].x : T(0);
-    const unsigned o0 = s2 + plane * (unsigned)t.K0;
-    T g[LC], d[LC], a[LC + 1], rr = T(0);
-    double bb = 0.0;
-    couplings<T, G, LC>(t, szw, kb, zwa, a);
+  const int row = nt * R.ke * W, zero = row;
+  double rz = 0.0, rr = 0.0, bb = 0.0;
+  Tiles<T, G, LC> it(R, R.col[1], t, ntiles, nt);
+  while (it.next(R, R.col[1], t, ntiles, nt, false)) {
+    if (!INIT && threadIdx.x == 0 && it.next_tile < ntiles) {
+      prefetch_tile(q, it.next_tile, nt, R.ke);
+      prefetch_tile(r, it.next_tile, nt, R.ke);
+    }
+    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
+    T g[LC], d[LC], a[LC + 1], rrt = T(0);
+#pragma unroll
+    for (int e = 0; e < LC; ++e) d[e] = (T)dinv[at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero)];
+    const T dm = (T)dinv[at_level<W>(o0, -1, t.K0 > 0 && t.K0 <= kb, zero)];
+    const T zwa = (T)R.col[1].zw[it.s2].x;
+    if (INIT) {
+      const double2 we = R.col[1].we[it.s2], ns = R.col[1].ns[it.s2], iz = R.col[1].iz[it.s2];
+      const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+      const int plane = 2 * R.plane2;
+      const int f0 = black_i(it.m, it.j) + 2 * R.P2 * it.j + plane * t.K0;
+#pragma unroll
+      for (int e = 0; e < LC; ++e) {
+        const int K = t.K0 + 1 + e, o = at_level<W>(o0, e, K <= kb, zero);
+        const double hs = K == kb ? iz.y : (K == kb - 1 ? iz.x : (double)R.izn[K <= kb ? K - 1 : 0]);
+        const T bs = K <= kb ? (T)((b[f0 + plane * e] * scale) * hs) : T(0);
+        T h = cw * ub[o + it.west];
+        h = fma(ce, ub[o + it.east], h);
+        h = fma(cn, ub[o - row], h);
+        h = fma(cs, ub[o + row], h);
+        g[e] = fma(-(T)hs, h, bs);
+        bb = fma((double)bs, (double)bs, bb);
+      }
+    } else {
+      T ql[LC];
+#pragma unroll
+      for (int e = 0; e < LC; ++e) {
+        const int o = at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero);
+        ql[e] = q[o];
+        g[e] = r[o];
+      }
+#pragma unroll
+      for (int e = 0; e < LC; ++e) g[e] = fma(-alpha, ql[e], g[e]);
+    }
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
-      const int K = t.K0 + 1 + e;
-      const unsigned o = o0 + plane * (unsigned)e;
-      g[e] = d[e] = T(0);
-      if (K <= kb) {
-        d[e] = (T)dinv[o];
-        if (INIT) {
-          const double2 we = R.col[1].we[s2], ns = R.col[1].ns[s2], iz = R.col[1].iz[s2];
-          const double hs = K == kb ? iz.y : (K == kb - 1 ? iz.x : R.izn[K - 1]);
-          const unsigned f = (unsigned)black_i(m, j) + 2u * P2 * (unsigned)j + 2u * plane * (unsigned)(K - 1);
-          const unsigned w = o - (unsigned)(j & 1);
-          const T bs = (T)((b[f] * scale) * hs);
-          T h = (T)we.x * ub[w];
-          h = fma((T)we.y, ub[w + 1u], h);
-          h = fma((T)ns.x, ub[o - P2], h);
-          h = fma((T)ns.y, ub[o + P2], h);
-          bb = fma((double)bs, (double)bs, bb);
-          g[e] = fma(-(T)hs, h, bs);
-        } else {
-          g[e] = fma(-alpha, q[o], r[o]);
-        }
-        r[o] = g[e];
-        rr = fma(g[e], g[e], rr);
-      }
+      if (t.K0 + 1 + e <= kb) r[o0 + W * e] = g[e];
+      rrt = fma(g[e], g[e], rrt);
     }
-    const T rz = column_solve<T, G, LC>(t, g, d, a);
+    couplings<T, G, LC>(t, szw, kb, zwa, a);
+    rz += (double)column_solve<T, G, LC>(t, scan, g, d, dm, a);
+    rr += (double)rrt;
 #pragma unroll
     for (int e = 0; e < LC; ++e)
-      if (t.K0 + 1 + e <= kb) z[o0 + plane * (unsigned)e] = g[e];
-    if (INIT) {
-      const double w[3] = {(double)rz, (double)rr, bb};
-      tile_partial<3>(w, S, tile);
-    } else {
-      const double w[2] = {(double)rz, (double)rr};
-      tile_partial<2>(w, S, tile);
-    }
+      if (t.K0 + 1 + e <= kb) z[o0 + W * e] = g[e];
   }
   double v[INIT ? 3 : 2];
-  if (grid_total<INIT ? 3 : 2>(v, S, ntiles)) {
+  v[0] = rz;
+  v[1] = rr;
+  if (INIT) v[2] = bb;
+  if (grid_sum<INIT ? 3 : 2, Ln::NT>(v, S)) {
     if (INIT) {
       S->bb += v[2];  // the red columns' part is there already
       S->beta = 0.0;
@@ -663,15 +730,13 @@ __global__ void __launch_bounds__(kThreads) k_rb_col(RbGeo R, SolverState* S, T*
 // The black correction: the x update that the last iteration left open (none
 // before the first), and its addition to the solution (full layout).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_rb_after(RbGeo R, SolverState* S,
-                                                       const T* __restrict__ p, T* __restrict__ d,
-                                                       double* __restrict__ x) {
-  const int m = blockIdx.x * 32 + (threadIdx.x & 31), K = blockIdx.z * kWarps + (threadIdx.x >> 5) + 1;
+__global__ void __launch_bounds__(128) k_rb_after(RbGeo R, SolverState* S, const T* __restrict__ p,
+                                                  T* __restrict__ d, double* __restrict__ x) {
+  constexpr int W = Width<T>::W;
+  const int m = blockIdx.x * W + threadIdx.x % W, K = blockIdx.z * (128 / W) + threadIdx.x / W + 1;
   const int j = blockIdx.y + 2;
-  if (m >= R.M) return;
-  const int s2 = m + R.P2 * j;
-  if (K > wet_levels(R.col[1].kk[s2], 0)) return;
-  const int o = s2 + R.plane2 * (K - 1);
+  if (m >= R.M || K > wet_levels(R.col[1].kk[m + R.P2 * j], 0)) return;
+  const int o = ((j * R.nt(W) + (int)blockIdx.x) * R.ke + K - 1) * W + threadIdx.x % W;
   T v = T(0);
   if (S->iter > 0) v = fma((T)S->alpha_prev, p[o], d[o]);
   d[o] = v;
@@ -699,57 +764,72 @@ __device__ __forceinline__ void dd_sub_prod(DD& s, double c, double x) {
   s.hi = hi;
 }
 
-// LR levels per thread: the levels of a column are independent here, so the
+// kResidLevels levels per thread: the levels of a column are independent here, so the
 // blocks split them (a thread that marches down a whole column waits for its
 // loads level by level: 1.4 ms a launch on 1024 x 1024 x 80).
-constexpr int kResidLevels = 8;
+constexpr int kResidLevels = 8, kResidThreads = 128;
 
-__global__ void __launch_bounds__(kThreads) k_resid(Geo G, PoissonGeo P, SolverState* S,
+__global__ void __launch_bounds__(kResidThreads) k_resid(Geo G, PoissonGeo P, SolverState* S,
                                                     const double* __restrict__ b,
                                                     double* __restrict__ x,
                                                     double* __restrict__ r, int nbx, int nby,
                                                     int ntiles) {
   const int KE = G.L.ke, IE = G.L.ie, JE = G.L.je;
-  const int tile = blockIdx.x, bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
-  const int i = bx * 32 + (threadIdx.x & 31) + 2, j = by * kWarps + (threadIdx.x >> 5) + 2;
-  const int K0 = bz * kResidLevels + 1, K1 = min(KE, K0 + kResidLevels - 1);
   double rr = 0.0, bb = 0.0;
-  if (i <= IE - 1 && j <= JE - 1) {
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int bx = tile % nbx, by = (tile / nbx) % nby, bz = tile / (nbx * nby);
+    const int i = bx * 32 + (threadIdx.x & 31) + 2, j = by * (kResidThreads / 32) + (threadIdx.x >> 5) + 2;
+    const int K0 = bz * kResidLevels + 1, K1 = min(KE, K0 + kResidLevels - 1);
+    if (i > IE - 1 || j > JE - 1) continue;
     const ColC c = load_col(G, P, i, j);
     // land rows (K > kb): diagonal only with a zero right-hand side, so the
     // solution there is 0 and x is set to it; r is neither stored nor read there
     for (int K = max(c.kb + 1, K0); K <= K1; ++K)
       if (AT(x, i, j, K) != 0.0) AT(x, i, j, K) = 0.0;
-    double xm = 0.0, x0 = 0.0, xp = 0.0;
+    double xm = 0.0, x0 = 0.0;
     if (K0 <= c.kb) {
       if (K0 > 1) xm = AT(x, i, j, K0 - 1);
       x0 = AT(x, i, j, K0);
     }
-    const int Ke = min(K1, c.kb);
-    for (int K = K0; K <= Ke; ++K) {
-      xp = K < c.kb ? AT(x, i, j, K + 1) : 0.0;
-      const Coef rw = row<false>(c, P, K, KE);
-      const double bk = AT(b, i, j, K);
-      DD s{bk, 0.0};
-      if (rw.u != 0.0) dd_sub_prod(s, rw.u, xm);
-      if (rw.n != 0.0) dd_sub_prod(s, rw.n, AT(x, i, j - 1, K));
-      if (rw.w != 0.0) dd_sub_prod(s, rw.w, AT(x, i - 1, j, K));
-      dd_sub_prod(s, rw.dc, x0);
-      if (rw.e != 0.0) dd_sub_prod(s, rw.e, AT(x, i + 1, j, K));
-      if (rw.s != 0.0) dd_sub_prod(s, rw.s, AT(x, i, j + 1, K));
-      if (rw.d != 0.0) dd_sub_prod(s, rw.d, xp);
-      const double rk = s.hi + s.lo;
-      AT(r, i, j, K) = rk;
-      rr += rk * rk;
-      bb += bk * bk;
-      xm = x0;
-      x0 = xp;
+    // the loads of four levels are issued together; an entry that the reference
+    // does not insert is 0 and its neighbour's value is not used
+#pragma unroll 1
+    for (int Kb = K0; Kb <= min(K1, c.kb); Kb += 4) {
+      double vb[4], vw[4], ve[4], vn[4], vs[4], vd[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int K = min(Kb + e, c.kb);
+        vb[e] = AT(b, i, j, K);
+        vw[e] = AT(x, i - 1, j, K);
+        ve[e] = AT(x, i + 1, j, K);
+        vn[e] = AT(x, i, j - 1, K);
+        vs[e] = AT(x, i, j + 1, K);
+        vd[e] = AT(x, i, j, min(K + 1, c.kb));
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int K = Kb + e;
+        if (K > min(K1, c.kb)) break;
+        const Coef rw = row<false>(c, P, K, KE);
+        DD s{vb[e], 0.0};
+        if (rw.u != 0.0) dd_sub_prod(s, rw.u, xm);
+        if (rw.n != 0.0) dd_sub_prod(s, rw.n, vn[e]);
+        if (rw.w != 0.0) dd_sub_prod(s, rw.w, vw[e]);
+        dd_sub_prod(s, rw.dc, x0);
+        if (rw.e != 0.0) dd_sub_prod(s, rw.e, ve[e]);
+        if (rw.s != 0.0) dd_sub_prod(s, rw.s, vs[e]);
+        if (rw.d != 0.0) dd_sub_prod(s, rw.d, vd[e]);
+        const double rk = s.hi + s.lo;
+        AT(r, i, j, K) = rk;
+        rr += rk * rk;
+        bb += vb[e] * vb[e];
+        xm = x0;
+        x0 = vd[e];
+      }
     }
   }
-  const double w[2] = {rr, bb};
-  tile_partial<2>(w, S, tile);
-  double v[2];
-  if (grid_total<2>(v, S, ntiles)) {
+  double v[2] = {rr, bb};
+  if (grid_sum<2, kResidThreads>(v, S)) {
     S->res_rr = v[0];
     S->res_bb = v[1];
   }
@@ -772,119 +852,107 @@ __global__ void k_reset(SolverState* S, double tol) {
   S->bb = 0.0;
 }
 
-// Launch shapes: at most this many blocks per SM (a block then walks several
-// tiles), 0 for a block per tile.
-constexpr int kShapes = 9;
-const int kBlocksPerSm[kShapes] = {0, 2, 3, 4, 6, 8, 1, 5, 12};
-
 struct Shape {
-  int ntiles, nmc, grid;
+  int ntiles, nt, grid;
 };
 
-Shape shape_of(const RbGeo& R, int columns_per_tile, int variant) {
+// A persistent grid: as many blocks as run at once, each walking tiles.
+template <auto Kernel, typename L>
+Shape shape_of(const RbGeo& R) {
+  static const int per_sm = [] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, L::NT, 0) != cudaSuccess) n = 1;
+    return std::max(n, 1);
+  }();
   Shape s;
-  s.nmc = (R.M + columns_per_tile - 1) / columns_per_tile;
-  s.ntiles = s.nmc * (R.je - 2);
-  s.grid = s.ntiles;
-  const int per = kBlocksPerSm[variant >= 0 && variant < kShapes ? variant : 0];
-  if (per) s.grid = std::min(s.ntiles, per * R.sms);
+  s.nt = R.nt(L::W);
+  s.ntiles = s.nt * (R.je - 2);
+  s.grid = std::min({s.ntiles, per_sm * R.sms, kMaxBlocks});
   return s;
 }
 
-// Calls f<T, G, LC> with the split for KE levels: four columns of doubles or
-// eight of floats per warp (32-byte segments) while the lane's share fits
-// registers (up to 13 doubles or 26 floats), 16 lanes per column above.
 template <int N>
 using Int = std::integral_constant<int, N>;
 
-template <typename T, typename F>
+// Calls f with the split of a column of KE levels: 8 threads of up to 13
+// levels, 16 of up to 20 above.  More levels per thread take more than the 255
+// registers; fewer, the shared work of a thread (its column's 2D data, the
+// scan) outweighs its levels.
+template <typename F>
 void with_split(int ke, F&& f) {
-  if (ke > 104) {
-    if (ke <= 128) f(Int<16>{}, Int<8>{});
-    else if (ke <= 208) f(Int<16>{}, Int<13>{});
-    else f(Int<16>{}, Int<20>{});
-  } else if constexpr (sizeof(T) == 8) {
-    if (ke <= 40) f(Int<8>{}, Int<5>{});
-    else if (ke <= 48) f(Int<8>{}, Int<6>{});
-    else if (ke <= 64) f(Int<8>{}, Int<8>{});
-    else if (ke <= 80) f(Int<8>{}, Int<10>{});
-    else if (ke <= 88) f(Int<8>{}, Int<11>{});
-    else f(Int<8>{}, Int<13>{});
-  } else {
-    if (ke <= 40) f(Int<4>{}, Int<10>{});
-    else if (ke <= 48) f(Int<4>{}, Int<12>{});
-    else if (ke <= 64) f(Int<4>{}, Int<16>{});
-    else if (ke <= 80) f(Int<4>{}, Int<20>{});
-    else if (ke <= 88) f(Int<4>{}, Int<22>{});
-    else f(Int<4>{}, Int<26>{});
-  }
+  if (ke <= 40) f(Int<8>{}, Int<5>{});
+  else if (ke <= 48) f(Int<8>{}, Int<6>{});
+  else if (ke <= 64) f(Int<8>{}, Int<8>{});
+  else if (ke <= 80) f(Int<8>{}, Int<10>{});
+  else if (ke <= 88) f(Int<8>{}, Int<11>{});
+  else if (ke <= 104) f(Int<8>{}, Int<13>{});
+  else if (ke <= 160) f(Int<16>{}, Int<10>{});
+  else f(Int<16>{}, Int<20>{});
 }
 static_assert(16 * 20 >= kMaxKe, "the longest column has a split");
 
-template <typename T>
-const T* red_pivots(const RbGeo& R);
-template <>
-const double* red_pivots<double>(const RbGeo& R) { return R.dr64; }
-template <>
-const float* red_pivots<float>(const RbGeo& R) { return R.dr32; }
-
 }  // namespace
 
-void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, double* dr64, float* dr32,
-                     float* db32, cudaStream_t st) {
-  const dim3 blk(32, 4);
-  k_rb_setup<<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, 0, st>>>(G, P, R, dr64, dr32, db32);
-  count_launch();
+size_t rb_elements(const RbGeo& R, int elem_bytes) {
+  const int W = 128 / elem_bytes;
+  return (size_t)R.nt(W) * W * R.ke * (R.je + 1);
 }
 
-int pcg_col_variants() { return 6; }
-int pcg_spmv_variants() { return kShapes; }
+template <typename T>
+void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, const RbVectors<T>& v,
+                     cudaStream_t st) {
+  const dim3 blk(32, 4);
+  k_rb_setup<T><<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, 0, st>>>(G, P, R, v.dr, v.db);
+  count_launch();
+}
 
 template <typename T>
 void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbVectors<T>& v,
                       cudaStream_t st) {
-  with_split<T>(R.ke, [&](auto gc, auto lc) {
+  with_split(R.ke, [&](auto gc, auto lc) {
     constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    const Shape s = shape_of(R, Lane<T, G, LC>::CT, 0);
-    k_rb_red<T, G, LC, kBefore><<<s.grid, kThreads, 0, st>>>(R, S, nullptr, v.ub, red_pivots<T>(R),
-                                                             b, nullptr, s.ntiles, s.nmc);
-    k_rb_col<T, G, LC, true><<<s.grid, kThreads, 0, st>>>(R, S, v.r, nullptr, v.z, R.db32, b, v.ub,
-                                                          s.ntiles, s.nmc);
+    using L = Lane<T, G, LC>;
+    const Shape s = shape_of<k_rb_red<T, G, LC, kBefore>, L>(R);
+    k_rb_red<T, G, LC, kBefore><<<s.grid, L::NT, 0, st>>>(R, S, nullptr, v.ub, v.dr, b, nullptr,
+                                                          s.ntiles, s.nt);
+    const Shape c = shape_of<k_rb_col<T, G, LC, true>, L>(R);
+    k_rb_col<T, G, LC, true><<<c.grid, L::NT, 0, st>>>(R, S, v.r, nullptr, v.z, v.db, b, v.ub,
+                                                       c.ntiles, c.nt);
   });
   add_launches(2);
 }
 
 template <typename T>
-void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
-                   cudaStream_t st) {
-  with_split<T>(R.ke, [&](auto gc, auto lc) {
+void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
+  with_split(R.ke, [&](auto gc, auto lc) {
     constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
-    k_rb_red<T, G, LC, kIter><<<s.grid, kThreads, 0, st>>>(R, S, v.z, v.u, red_pivots<T>(R), nullptr,
-                                                           nullptr, s.ntiles, s.nmc);
+    using L = Lane<T, G, LC>;
+    const Shape s = shape_of<k_rb_red<T, G, LC, kIter>, L>(R);
+    k_rb_red<T, G, LC, kIter><<<s.grid, L::NT, 0, st>>>(R, S, v.z, v.u, v.dr, nullptr, nullptr,
+                                                        s.ntiles, s.nt);
   });
   count_launch();
 }
 
 template <typename T>
-void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
-                     cudaStream_t st) {
-  with_split<T>(R.ke, [&](auto gc, auto lc) {
+void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
+  with_split(R.ke, [&](auto gc, auto lc) {
     constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
-    k_rb_black<T, G, LC><<<s.grid, kThreads, 0, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, s.ntiles, s.nmc);
+    using L = Lane<T, G, LC>;
+    const Shape s = shape_of<k_rb_black<T, G, LC>, L>(R);
+    k_rb_black<T, G, LC><<<s.grid, L::NT, 0, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, s.ntiles, s.nt);
   });
   count_launch();
 }
 
 template <typename T>
-void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int variant,
-                   cudaStream_t st) {
-  with_split<T>(R.ke, [&](auto gc, auto lc) {
+void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
+  with_split(R.ke, [&](auto gc, auto lc) {
     constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    const Shape s = shape_of(R, Lane<T, G, LC>::CT, variant);
-    k_rb_col<T, G, LC, false><<<s.grid, kThreads, 0, st>>>(R, S, v.r, v.q, v.z, R.db32, nullptr,
-                                                           nullptr, s.ntiles, s.nmc);
+    using L = Lane<T, G, LC>;
+    const Shape s = shape_of<k_rb_col<T, G, LC, false>, L>(R);
+    k_rb_col<T, G, LC, false><<<s.grid, L::NT, 0, st>>>(R, S, v.r, v.q, v.z, v.db, nullptr, nullptr,
+                                                        s.ntiles, s.nt);
   });
   count_launch();
 }
@@ -892,23 +960,27 @@ void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int va
 template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x,
                      cudaStream_t st) {
-  const dim3 grid((R.M + 31) / 32, R.je - 2, (R.ke + kWarps - 1) / kWarps);
-  k_rb_after<T><<<grid, kThreads, 0, st>>>(R, S, v.p, v.x, x);
-  with_split<T>(R.ke, [&](auto gc, auto lc) {
+  constexpr int W = Width<T>::W;
+  const dim3 grid(R.nt(W), R.je - 2, (R.ke + 128 / W - 1) / (128 / W));
+  k_rb_after<T><<<grid, 128, 0, st>>>(R, S, v.p, v.x, x);
+  with_split(R.ke, [&](auto gc, auto lc) {
     constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    const Shape s = shape_of(R, Lane<T, G, LC>::CT, 0);
-    k_rb_red<T, G, LC, kAfter><<<s.grid, kThreads, 0, st>>>(R, S, v.x, v.ub, red_pivots<T>(R),
-                                                            nullptr, x, s.ntiles, s.nmc);
+    using L = Lane<T, G, LC>;
+    const Shape s = shape_of<k_rb_red<T, G, LC, kAfter>, L>(R);
+    k_rb_red<T, G, LC, kAfter><<<s.grid, L::NT, 0, st>>>(R, S, v.x, v.ub, v.dr, nullptr, x, s.ntiles,
+                                                         s.nt);
   });
   add_launches(2);
 }
 
 #define ORCTM_RB(T)                                                                              \
+  template void launch_rb_setup<T>(const Geo&, const PoissonGeo&, const RbGeo&, const RbVectors<T>&, \
+                                   cudaStream_t);                                                \
   template void launch_rb_before<T>(const RbGeo&, SolverState*, const double*, const RbVectors<T>&, \
                                     cudaStream_t);                                               \
-  template void launch_rb_red<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
-  template void launch_rb_black<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
-  template void launch_rb_col<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
+  template void launch_rb_red<T>(const RbGeo&, SolverState*, const RbVectors<T>&, cudaStream_t); \
+  template void launch_rb_black<T>(const RbGeo&, SolverState*, const RbVectors<T>&, cudaStream_t); \
+  template void launch_rb_col<T>(const RbGeo&, SolverState*, const RbVectors<T>&, cudaStream_t); \
   template void launch_rb_after<T>(const RbGeo&, SolverState*, const RbVectors<T>&, double*, cudaStream_t);
 ORCTM_RB(double)
 ORCTM_RB(float)
@@ -916,9 +988,10 @@ ORCTM_RB(float)
 
 void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const double* b, double* x,
                   double* r, cudaStream_t st) {
-  const int nbx = (G.L.ie - 2 + 31) / 32, nby = (G.L.je - 2 + kWarps - 1) / kWarps;
+  const int nbx = (G.L.ie - 2 + 31) / 32, nby = (G.L.je - 2 + kResidThreads / 32 - 1) / (kResidThreads / 32);
   const int nt = nbx * nby * ((G.L.ke + kResidLevels - 1) / kResidLevels);
-  k_resid<<<nt, kThreads, 0, st>>>(G, P, S, b, x, r, nbx, nby, nt);
+  const int grid = std::min(nt, kMaxBlocks);
+  k_resid<<<grid, kResidThreads, 0, st>>>(G, P, S, b, x, r, nbx, nby, nt);
   count_launch();
 }
 
@@ -938,12 +1011,6 @@ void launch_pcg_continue(cudaGraphConditionalHandle hc, const SolverState* S, in
   count_launch();
 }
 
-size_t solver_max_blocks(const Geo& G) {
-  // tiles of k_resid, and of the PCG kernels at their narrowest (16 columns)
-  const size_t resid = (size_t)((G.L.ie - 2 + 31) / 32) * ((G.L.je - 2 + kWarps - 1) / kWarps) *
-                       ((G.L.ke + kResidLevels - 1) / kResidLevels);
-  const size_t pcg = (size_t)((G.L.ie / 2 + 1 + 15) / 16) * (G.L.je - 2);
-  return std::max(resid, pcg);
-}
+int solver_max_blocks() { return kMaxBlocks; }
 
 }  // namespace orctm
