@@ -700,7 +700,8 @@ int setup(orctm_handle* h, const orctm_desc* d) {
     R.ie = IE; R.je = JE; R.ke = KE;
     R.P2 = L.P / 2;
     R.plane2 = L.plane / 2;
-    R.M = (IE - 1) / 2 + 1;
+    R.M = (IE - 1) / 2;
+    R.device = h->device;
     R.zwn = P.zwn;
     R.izn = P.izn;
     ORCTM_CUDA_OK(cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -735,7 +736,7 @@ int alloc_rb(orctm_handle* h, RbVectors<T>& v) {
   int st;
   for (T** p : {&v.x, &v.r, &v.z, &v.p, &v.q, &v.u, &v.ub, &v.dr})
     if (!*p && (st = h->dev_alloc(p, n))) return st;
-  if ((st = h->dev_alloc(&v.db, n))) return st;
+  if ((st = h->dev_alloc(&v.km, rb_tiles(h->R, sizeof(T)))) || (st = h->dev_alloc(&v.db, n))) return st;
   launch_rb_setup<T>(h->G, h->P, h->R, v, h->stream);
   ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
@@ -859,6 +860,10 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     }
   }
   *iters = h->hS->iter;
+  if (conv == 4) {  // a bounded wait inside a kernel gave up
+    h->err = "a device-side wait for a staged copy timed out in the Poisson solver";
+    return ORCTM_E_CUDA;
+  }
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_after<T>(h->R, h->S, v, h->xs, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
@@ -2559,7 +2564,7 @@ int orctm_estimate_device_bytes(const orctm_desc* d, int solver, unsigned long l
   // and its pivots (in FP64, and for the refined solver in FP32 too: a handle
   // that has solved in both forms holds both)
   const double tmp = std::max(8.0, 2.0 * d->ntracers + 2.0) + 3.0;  // + the held transports
-  const double m32 = ((d->ie - 1) / 2 + 1 + 31) / 32 * 32;  // FP32 tiles hold 32 columns
+  const double m32 = ((d->ie - 1) / 2 + 31) / 32 * 32;  // FP32 tiles hold 32 columns
   const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 4.25 +
                     (solver == ORCTM_SOLVER_FP32_REFINED ? 2.25 * std::max(1.0, 2.0 * m32 / P) : 0.0);
   // 2D tables (compressed columns, metrics, biharmonic and Poisson factors)

@@ -27,10 +27,13 @@ struct RbColour {
 struct RbGeo {
   int ie, je, ke;
   int P2, plane2;             // P / 2, P / 2 * JN
-  int M;                      // columns m = 0..M-1 hold every unknown of a row
-  int sms;                    // multiprocessors of the device
+  int M;                      // columns m = 1..M hold every unknown of a row
+  int device, sms;            // the device and its multiprocessors
   RbColour col[2];            // red, black
   const double *zwn, *izn;
+  // columns per tile: 128 bytes of a level, half of it in long columns
+  static constexpr int kWide = 160;
+  __host__ __device__ int width(int elem_bytes) const { return (ke <= kWide ? 128 : 64) / elem_bytes; }
   __host__ __device__ int nt(int W) const { return (M + W - 1) / W; }  // tiles per row
 };
 // Vectors of the reduced system (tiled layout, zero outside the unknowns) and
@@ -41,12 +44,13 @@ struct RbVectors {
   T *u, *ub;                  // red: D_r^-1 C p ; D_r^-1 b
   T* dr;                      // red pivots
   float* db;                  // black pivots
+  int* km;                    // deepest wet level of each tile, red then black
 };
 
 // Device-resident scalars of one Krylov solve.
 struct SolverState {
   double rho, beta, alpha, alpha_prev, pq, rr, bb, tol, res_rr, res_bb;
-  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown
+  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown, 4 a staged copy timed out
   int iter;
   int limit;      // iteration limit of the device-side loop (orctm handle's maxit)
   unsigned ticket;
@@ -197,6 +201,7 @@ void launch_nh_rhs(const Geo& G, const double* uoo, const double* uoo1, const do
 // elements of a vector of the reduced system, and the red-black tables and
 // pivots of a precision (once per handle and precision)
 size_t rb_elements(const RbGeo& R, int elem_bytes);
+size_t rb_tiles(const RbGeo& R, int elem_bytes);
 template <typename T>
 void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, const RbVectors<T>& v,
                      cudaStream_t st);

@@ -32,7 +32,7 @@
 //
 // Vectors are stored per colour, column (i, j) at m = i / 2 of row j, in tiles
 // of W columns (128 bytes of a level) that hold all their levels one after
-// the other: offset ((j NT + m / W) KE + l) W + m mod W.  A tile is some 10 KB
+// the other: offset ((j NT + b) KE + l) W + c, b W + c = m - 1.  A tile is some 10 KB
 // of consecutive memory; in the padded layout of the model's fields its levels lie
 // megabytes apart on 1024 x 1024 x 80, where every block then touched some 80
 // pages per vector (stencil kernel 1.65 ms a launch; see below).  The in-row
@@ -54,10 +54,12 @@
 // needs no host round trip.  A device flag marks convergence; kernels of an
 // already converged solve return at once.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
 #include "ops.h"
+#include "tma.cuh"
 
 namespace orctm {
 
@@ -234,22 +236,18 @@ __device__ bool grid_sum(double (&v)[NV], SolverState* S) {
 __device__ __forceinline__ int red_i(int m, int j) { return 2 * m + (j & 1); }
 __device__ __forceinline__ int black_i(int m, int j) { return 2 * m + 1 - (j & 1); }
 
-// Columns per tile: 128 bytes of a level
-template <typename T>
-struct Width {
-  static constexpr int W = 128 / (int)sizeof(T);
-};
 
 // Pivots of the column tridiagonal of B (constant): dinv(K) = 1/d'(K) with
 // d'(1) = d(1), d'(K) = d(K) - a(K) c(K-1) / d'(K-1), in the layout of
 // precision T: the red ones in T (the elimination is exact to
 // the solve's precision), the black ones, a fixed preconditioner, in FP32 for
-// both forms; and the 2D data of the columns.  Columns that are no unknowns
-// keep kk = 0 (no wet level).
+// both forms; the 2D data of the columns, kk with the wet levels of the column
+// and of its neighbours; and the deepest wet level km of each tile.  Columns that
+// are no unknowns keep kk = 0 (no wet level).
 template <typename T>
 __global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, T* __restrict__ dr,
-                           float* __restrict__ db) {
-  constexpr int W = Width<T>::W;
+                           float* __restrict__ db, int* __restrict__ km) {
+  const int W = R.width((int)sizeof(T));
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   const int KE = G.L.ke;
@@ -265,12 +263,14 @@ __global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, T* __restrict__ dr,
   q.ns[s] = make_double2(c.cn, c.cs);
   q.zw[s] = make_double2(c.zwa, c.zwb);
   q.iz[s] = make_double2(c.iza, c.izb);
+  const int m = (i >> 1) - 1, nt = R.nt(W);
+  atomicMax(km + (black ? nt * (G.L.je + 1) : 0) + j * nt + m / W, c.kb);
   double dprev = 1.0, cprev = 0.0;
   for (int K = 1; K <= c.kb; ++K) {
     const Coef r = row<true>(c, P, K, KE);
     const double d = K == 1 ? r.dc : r.dc - (r.u * dprev) * cprev;
     const double di = 1.0 / d;
-    const int m = i >> 1, o = ((j * R.nt(W) + m / W) * KE + K - 1) * W + m % W;
+    const int o = ((j * nt + m / W) * KE + K - 1) * W + m % W;
     if (black) db[o] = (float)di;
     else dr[o] = (T)di;
     dprev = di;
@@ -280,31 +280,31 @@ __global__ void k_rb_setup(Geo G, PoissonGeo P, RbGeo R, T* __restrict__ dr,
 
 // ------------------------------------------------------- PCG kernels -----
 // Where a thread stands: column c of the tile, levels K0 + 1 .. K0 + LC.
-template <typename T, int G, int LC>
+template <typename T, int G, int LC, int H>
 struct Lane {
-  static constexpr int W = Width<T>::W, NT = W * G;  // columns per tile, threads per block
+  using V = T;
+  static constexpr int W = (128 >> H) / (int)sizeof(T);  // columns per tile
+  static constexpr int NT = W * G, ROWS = G * LC, L = LC, GROUPS = G;
   int c, g, K0;
   __device__ __forceinline__ Lane() : c(threadIdx.x % W), g(threadIdx.x / W), K0(g * LC) {}
 };
 
 // ZW(K) at szw[K - 1], K = 1..KE+1, and 1/ZP(K) at siz[K - 1]
-template <typename T, int G, int LC>
+template <typename Ln, typename T>
 __device__ __forceinline__ void load_tables(const RbGeo& R, T* szw, T* siz) {
-  for (int e = threadIdx.x; e <= G * LC; e += Lane<T, G, LC>::NT) {
+  for (int e = threadIdx.x; e <= Ln::ROWS; e += Ln::NT) {
     szw[e] = e <= R.ke ? (T)R.zwn[e] : T(0);
     if (siz) siz[e] = e < R.ke ? (T)R.izn[e] : T(0);
   }
-  __syncthreads();
 }
 
 // Couplings a(K) between levels K - 1 and K of the thread's levels and of the
 // one below its last: ZW(K) inside the column (its own value at the bottom),
 // 0 at the surface and below the bottom.
-template <typename T, int G, int LC>
-__device__ __forceinline__ void couplings(const Lane<T, G, LC>& t, const T* szw, int kb, T zwa,
-                                          T (&a)[LC + 1]) {
+template <typename Ln, typename T, int LC>
+__device__ __forceinline__ void couplings(const Ln& t, const T* szw, int kb, T zwa, T (&a)[LC]) {
 #pragma unroll
-  for (int u = 0; u <= LC; ++u) {
+  for (int u = 0; u < LC; ++u) {
     const int K = t.K0 + 1 + u;
     const T zw = szw[t.K0 + u];
     a[u] = (K == 1 || K > kb) ? T(0) : (K == kb ? zwa : zw);
@@ -312,17 +312,20 @@ __device__ __forceinline__ void couplings(const Lane<T, G, LC>& t, const T* szw,
 }
 
 // Affine maps of the threads of a column, down and up
-template <typename T, int G, int W>
+template <typename Ln>
 struct Scan {
-  T fa[G][W], fb[G][W], ba[G][W], bb[G][W];
+  typename Ln::V fa[Ln::GROUPS][Ln::W], fb[Ln::GROUPS][Ln::W], ba[Ln::GROUPS][Ln::W],
+      bb[Ln::GROUPS][Ln::W];
 };
 
 // v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d (dm: the
 // pivot above the thread's first level) and couplings a; returns v.M^-1 v =
-// sum y^2 / d of this thread's levels.  Two block barriers.
-template <typename T, int G, int LC>
-__device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, Scan<T, G, Lane<T, G, LC>::W>& sc,
-                                          T (&v)[LC], const T (&d)[LC], T dm, const T (&a)[LC + 1]) {
+// sum y^2 / d of this thread's levels.  Two block barriers; between() runs
+// after the first, when every thread has its inputs in registers.
+template <typename Ln, typename T, int LC, typename F>
+__device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC], const T (&d)[LC],
+                                          T dm, const T (&a)[LC + 1], F&& between) {
+  constexpr int G = Ln::GROUPS;
   // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the thread's levels as one affine
   // map y_out = A y_in + B, applied in turn to what comes from above
   T A = T(1), B = T(0);
@@ -335,6 +338,7 @@ __device__ __forceinline__ T column_solve(const Lane<T, G, LC>& t, Scan<T, G, La
   sc.fa[t.g][t.c] = A;
   sc.fb[t.g][t.c] = B;
   __syncthreads();
+  between();
   T y = T(0);
 #pragma unroll
   for (int k = 0; k < G - 1; ++k)
@@ -374,79 +378,169 @@ __device__ __forceinline__ int wet_levels(unsigned long long kk, int nb) {
   return (int)((kk >> (10 * nb)) & 1023u);
 }
 
-// One tile: row j, columns m, the offset o0 of the thread's first level in the
-// tiled layout, and its in-row neighbours of the other colour relative to it.
-// kk of the block's next tile is loaded while this one is computed.
-template <typename T, int G, int LC>
+// The tiles of one colour and what a thread sees of one: row j, the column
+// m = i / 2, the offset o0 of its first level in the tiled layout, and whether
+// its west neighbour of the other colour is column m (sh) or m - 1.
+struct Tile {
+  int j, b, m, o0;
+  bool sh;
+  unsigned long long kk;
+};
+template <typename Ln>
 struct Tiles {
-  static constexpr int W = Width<T>::W;
-  int tile, next_tile;
-  int j, m, s2, o0, west, east;
-  unsigned long long kk, kn;
-  __device__ __forceinline__ Tiles(const RbGeo& R, const RbColour& q, const Lane<T, G, LC>& t,
-                                   int ntiles, int nt)
-      : next_tile(blockIdx.x) {
-    kn = fetch(R, q, t, ntiles, nt);
+  const RbGeo& R;
+  const RbColour& q;
+  const Ln& t;
+  int ntiles, nt;
+  bool red;
+  __device__ __forceinline__ unsigned long long kk(int tile) const {
+    const int m = 1 + (tile % nt) * Ln::W + t.c;
+    return tile < ntiles && m <= R.M ? __ldg(q.kk + m + R.P2 * (2 + tile / nt)) : 0ull;
   }
-  __device__ __forceinline__ unsigned long long fetch(const RbGeo& R, const RbColour& q,
-                                                      const Lane<T, G, LC>& t, int ntiles, int nt) {
-    const int jn = 2 + next_tile / nt, mn = (next_tile % nt) * W + t.c;
-    return next_tile < ntiles && mn < R.M ? __ldg(q.kk + mn + R.P2 * jn) : 0ull;
-  }
-  // sh: 0 when the west neighbour is column m - 1, 1 when it is column m
-  __device__ __forceinline__ bool next(const RbGeo& R, const RbColour& q, const Lane<T, G, LC>& t,
-                                       int ntiles, int nt, bool red) {
-    tile = next_tile;
-    if (tile >= ntiles) return false;
-    kk = kn;
-    j = 2 + tile / nt;
-    const int b = tile % nt;
-    m = b * W + t.c;
-    s2 = kk ? m + R.P2 * j : 0;
-    o0 = ((j * nt + b) * R.ke + t.K0) * W + t.c;
-    const int sh = red ? (j & 1) : 1 - (j & 1);
-    const int back = t.c == 0 ? (W - 1) - R.ke * W : -1;      // column m - 1
-    const int ahead = t.c == W - 1 ? R.ke * W - (W - 1) : 1;  // column m + 1
-    west = sh ? 0 : back;
-    east = sh ? ahead : 0;
-    next_tile += gridDim.x;
-    kn = fetch(R, q, t, ntiles, nt);
-    return true;
+  __device__ __forceinline__ Tile at(int tile, unsigned long long kk) const {
+    Tile a;
+    a.j = 2 + tile / nt;
+    a.b = tile % nt;
+    a.m = 1 + a.b * Ln::W + t.c;
+    a.o0 = ((a.j * nt + a.b) * R.ke + t.K0) * Ln::W + t.c;
+    a.sh = (a.j & 1) == (red ? 1 : 0);
+    a.kk = kk;
+    return a;
   }
 };
 
-// Asks for a tile of a vector (tiled layout: consecutive memory) in L2 while the
-// block works on the one before it.
-template <typename T>
-__device__ __forceinline__ void prefetch_tile(const T* a, int tile, int nt, int ke) {
-  const T* p = a + (size_t)(tile + 2 * nt) * ke * Width<T>::W;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(ke * 128) : "memory");
-}
-
-// Offset of level q of the thread, or, for a level that is not wet, of an
-// element whose value and neighbours are 0 in every vector (row 1 holds no unknown and
-// column 0 of row 2 neither): the loads of a thread's levels carry no branch
-// and are issued together.
-template <int W>
-__device__ __forceinline__ int at_level(int o0, int q, bool wet, int zero) {
-  return wet ? o0 + W * q : zero;
-}
+// Staging.  A block's next tile is copied to shared memory while it computes
+// this one: one thread issues a bulk copy per array (a tile is consecutive
+// memory; down to the tile's deepest wet level), all wait on an mbarrier.  NA
+// arrays of T, the pivots (D, ND = 1 or 0) and the four pairs of 2D data; the
+// in-row neighbours across the tile's edge come by a copy per level.
+// Loads straight to registers left the kernels waiting for most of the time
+// (black kernel 106 us at 448 x 448 x 80, 10 of 14 cycles of a warp in
+// long-scoreboard stalls), copies by every thread cost as many instructions as the
+// computation (red kernel 67 -> 80 us).
+template <typename Ln, typename D, int NA, int ND>
+struct Stage {
+  using T = typename Ln::V;
+  static constexpr int ROWS = Ln::ROWS, W = Ln::W, N = ROWS * W;
+  static constexpr size_t smem =
+      16 * 4 * W + sizeof(T) * N * NA + sizeof(D) * N * ND + sizeof(T) * ROWS;
+  double2* pairs;
+  T *data, *edge;
+  D* piv;
+  uint64_t* bar;
+  uint32_t phase;
+  bool ok;
+  __device__ __forceinline__ Stage(unsigned char* dsm, uint64_t* b) : bar(b), phase(0), ok(true) {
+    pairs = reinterpret_cast<double2*>(dsm);
+    data = reinterpret_cast<T*>(dsm + 16 * 4 * W);
+    piv = reinterpret_cast<D*>(dsm + 16 * 4 * W + sizeof(T) * N * NA);
+    edge = reinterpret_cast<T*>(dsm + 16 * 4 * W + sizeof(T) * N * NA + sizeof(D) * N * ND);
+    if (threadIdx.x == 0) {
+      mbar_init(bar, 1);
+      mbar_init_fence();
+    }
+  }
+  // Issues the copies of tile a (the block has read the slots' last contents):
+  // arrays n = 0..NA-1 from v[n] at the tile's own place plus rows[n] rows.
+  template <int NV>
+  __device__ __forceinline__ void issue(const Tiles<Ln>& s, const Tile& a, const int* __restrict__ km,
+                                        const T* const (&v)[NV], const int (&rows)[NV],
+                                        const D* dinv, const T* edge_of) {
+    static_assert(NV == NA || NA == 0, "");
+    const int ke = s.R.ke;
+    if (threadIdx.x == 0) {
+      const uint32_t n = (uint32_t)__ldg(km + (s.red ? 0 : s.nt * (s.R.je + 1)) + a.j * s.nt + a.b);
+      mbar_arrive_expect_tx(bar, 16 * 4 * W + n * W * (uint32_t)(sizeof(T) * NA + sizeof(D) * ND));
+      const int s2 = 1 + a.b * W + s.R.P2 * a.j;
+      bulk_load(pairs, s.q.zw + s2, 16 * W, bar);
+      bulk_load(pairs + W, s.q.iz + s2, 16 * W, bar);
+      bulk_load(pairs + 2 * W, s.q.we + s2, 16 * W, bar);
+      bulk_load(pairs + 3 * W, s.q.ns + s2, 16 * W, bar);
+      if (n) {
+#pragma unroll
+        for (int e = 0; e < NA; ++e)
+          bulk_load(data + e * N, v[e] + (size_t)((a.j + rows[e]) * s.nt + a.b) * ke * W,
+                    n * W * (uint32_t)sizeof(T), bar);
+        if (ND)
+          bulk_load(piv, dinv + (size_t)(a.j * s.nt + a.b) * ke * W, n * W * (uint32_t)sizeof(D), bar);
+      }
+    }
+    if (NA > 0 && edge_of && s.t.c == (a.sh ? W - 1 : 0)) {
+      // this column's neighbour is in the tile to the west (c = 0) or east
+      const bool there = a.sh ? a.b + 1 < s.nt : a.b > 0;
+      const int o = a.o0 + (a.sh ? ke * W - (W - 1) : (W - 1) - ke * W);
+      const int kb = wet_levels(a.kk, 0);
+#pragma unroll
+      for (int q = 0; q < Ln::L; ++q) {
+        const bool get = there && s.t.K0 + 1 + q <= kb;
+        copy_async(edge + s.t.K0 + q, edge_of + (get ? o + W * q : 0), get);
+      }
+    }
+  }
+  __device__ __forceinline__ void wait() {
+    copies_wait();
+    if (ok) ok = mbar_wait(bar, phase);
+    phase ^= 1;
+  }
+  __device__ __forceinline__ T get(const Ln& t, int n, int q) const {
+    return data[n * N + (t.K0 + q) * W + t.c];
+  }
+  // C v of the thread's levels without the factor 1/ZP, 0 below the bottom
+  // (values of land cells and outside the unknowns are exact zeros); arrays
+  // n, n+1, n+2: the tile itself and the ones north and south of it
+  __device__ __forceinline__ void neighbour_sum(const Ln& t, const Tile& a, int n, double2 we,
+                                                double2 ns, T (&h)[Ln::L]) const {
+    const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+    const T co = a.sh ? cw : ce, cx = a.sh ? ce : cw;  // column m, and the other one
+    const int cc = a.sh ? min(t.c + 1, W - 1) : max(t.c - 1, 0);
+    const bool across = t.c == (a.sh ? W - 1 : 0);
+    const int kb = wet_levels(a.kk, 0);
+    const T* d = data + n * N + t.K0 * W;
+#pragma unroll
+    for (int q = 0; q < Ln::L; ++q) {
+      h[q] = co * d[q * W + t.c];
+      T x = d[q * W + cc];
+      if (across) x = edge[t.K0 + q];
+      h[q] = fma(cx, x, h[q]);
+      h[q] = fma(cn, d[N + q * W + t.c], h[q]);
+      h[q] = fma(cs, d[2 * N + q * W + t.c], h[q]);
+      if (t.K0 + 1 + q > kb) h[q] = T(0);
+    }
+  }
+  // pivots of the thread's levels and the one above the first
+  __device__ __forceinline__ void pivots(const Ln& t, int kb, T& dm, T (&d)[Ln::L]) const {
+    dm = t.K0 > 0 && t.K0 <= kb ? (T)piv[(t.K0 - 1) * W + t.c] : T(0);
+#pragma unroll
+    for (int q = 0; q < Ln::L; ++q)
+      d[q] = t.K0 + 1 + q <= kb ? (T)piv[(t.K0 + q) * W + t.c] : T(0);
+  }
+  // a copy that never landed stops the solve
+  __device__ __forceinline__ void report(SolverState* S) const {
+    if (!ok && threadIdx.x == 0) atomicExch(&S->converged, 4);
+  }
+};
 
 // Red columns.
-//   kIter    u = D^-1 C v + beta u          (v = z; u is not read while beta = 0)
+//   kIter    u = D^-1 C v + beta u          (v = z; u is not used while beta = 0)
 //   kBefore  u = D^-1 (b / ZP)              (b: full layout, scaled); sum of (b / ZP)^2
 //   kAfter   x += scale (u - D^-1 C v)      (v = the black correction; x: full layout)
 enum { kIter = 0, kBefore = 1, kAfter = 2 };
 
-template <typename T, int G, int LC, int MODE>
-__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_red(RbGeo R, SolverState* S,
-                                                     const T* __restrict__ v, T* __restrict__ u,
-                                                     const T* __restrict__ dinv,
-                                                     const double* __restrict__ b,
-                                                     double* __restrict__ x, int ntiles, int nt) {
-  using Ln = Lane<T, G, LC>;
-  constexpr int W = Ln::W;
-  __shared__ T szw[G * LC + 1], siz[G * LC + 1];
+template <typename Ln, int MODE>
+using RedStage = Stage<Ln, typename Ln::V, MODE == kBefore ? 0 : 3, 1>;
+
+template <typename Ln, int MODE, typename T = typename Ln::V>
+__global__ void __launch_bounds__(Ln::NT) k_rb_red(RbGeo R, SolverState* S,
+                                                   const T* __restrict__ v, T* __restrict__ u,
+                                                   const T* __restrict__ dinv,
+                                                   const int* __restrict__ km,
+                                                   const double* __restrict__ b,
+                                                   double* __restrict__ x, int ntiles, int nt) {
+  constexpr int W = Ln::W, LC = Ln::L;
+  extern __shared__ __align__(128) unsigned char dsm[];
+  __shared__ T szw[Ln::ROWS + 1], siz[Ln::ROWS + 1];
+  __shared__ Scan<Ln> scan;
+  __shared__ __align__(8) uint64_t bar;
   if (MODE == kIter && S->converged) return;
   const T beta = MODE == kIter ? (T)S->beta : T(0);
   double scale = 1.0;
@@ -454,27 +548,35 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_red(RbGeo R, SolverSt
     scale = sqrt(S->res_rr);
     if (MODE == kBefore) scale = scale > 0.0 ? 1.0 / scale : 0.0;
   }
-  load_tables<T, G, LC>(R, szw, siz);
-  __shared__ Scan<T, G, W> scan;
   const Ln t;
-  const int row = nt * R.ke * W, zero = row;
-  const int P = 2 * R.P2, plane = 2 * R.plane2;  // full layout
+  const Tiles<Ln> tiles{R, R.col[0], t, ntiles, nt, true};
+  RedStage<Ln, MODE> st(dsm, &bar);
+  load_tables<Ln>(R, szw, siz);
+  __syncthreads();
+  auto issue = [&](const Tile& a) { st.issue(tiles, a, km, {v, v, v}, {0, -1, 1}, dinv, v); };
+  int tile = blockIdx.x;
+  Tile next = tiles.at(tile, tiles.kk(tile));
+  issue(next);
+  unsigned long long kn = tiles.kk(tile + gridDim.x);
+  const int plane = 2 * R.plane2;  // full layout
   double bb = 0.0;
-  Tiles<T, G, LC> it(R, R.col[0], t, ntiles, nt);
-  while (it.next(R, R.col[0], t, ntiles, nt, true)) {
-    if (MODE == kIter && threadIdx.x == 0 && it.next_tile < ntiles) {
-      prefetch_tile(dinv, it.next_tile, nt, R.ke);
-      prefetch_tile(v, it.next_tile, nt, R.ke);
-      prefetch_tile(u, it.next_tile, nt, R.ke);
-    }
-    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
-    T g[LC], d[LC], a[LC + 1];
+  for (; tile < ntiles; tile += gridDim.x) {
+    const Tile a = next;
+    const int kb = wet_levels(a.kk, 0);
+    T g[LC], d[LC], uo[LC], cp[LC + 1], dm;
+    if (MODE != kBefore) {
 #pragma unroll
-    for (int q = 0; q < LC; ++q) d[q] = dinv[at_level<W>(o0, q, t.K0 + 1 + q <= kb, zero)];
-    const T dm = dinv[at_level<W>(o0, -1, t.K0 > 0 && t.K0 <= kb, zero)];
-    const T zwa = (T)R.col[0].zw[it.s2].x;
-    const double2 iz = R.col[0].iz[it.s2];
-    const int f0 = red_i(it.m, it.j) + P * it.j + plane * t.K0;
+      for (int q = 0; q < LC; ++q) uo[q] = t.K0 + 1 + q <= kb ? u[a.o0 + W * q] : T(0);
+    }
+    const int f0 = red_i(a.m, a.j) + 2 * R.P2 * a.j + plane * t.K0;
+    if (MODE == kBefore) {
+#pragma unroll
+      for (int q = 0; q < LC; ++q) g[q] = T(0);
+    }
+    st.wait();
+    const T zwa = (T)st.pairs[t.c].x;
+    const double2 iz = st.pairs[W + t.c];
+    st.pivots(t, kb, dm, d);
     if (MODE == kBefore) {
 #pragma unroll
       for (int q = 0; q < LC; ++q) {
@@ -485,42 +587,34 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_red(RbGeo R, SolverSt
         bb = fma((double)g[q], (double)g[q], bb);
       }
     } else {
-      const double2 we = R.col[0].we[it.s2], ns = R.col[0].ns[it.s2];
-      const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+      st.neighbour_sum(t, a, 0, st.pairs[2 * W + t.c], st.pairs[3 * W + t.c], g);
 #pragma unroll
       for (int q = 0; q < LC; ++q) {
-        // values of land cells and outside the unknowns are exact zeros
-        const int K = t.K0 + 1 + q, o = at_level<W>(o0, q, K <= kb, zero);
-        const T hs = K == kb ? (T)iz.y : (K == kb - 1 ? (T)iz.x : siz[t.K0 + q]);
-        T h = cw * v[o + it.west];
-        h = fma(ce, v[o + it.east], h);
-        h = fma(cn, v[o - row], h);
-        h = fma(cs, v[o + row], h);
-        g[q] = hs * h;
+        const int K = t.K0 + 1 + q;
+        g[q] *= K == kb ? (T)iz.y : (K == kb - 1 ? (T)iz.x : siz[t.K0 + q]);
       }
     }
-    couplings<T, G, LC>(t, szw, kb, zwa, a);
-    column_solve<T, G, LC>(t, scan, g, d, dm, a);
-    if (MODE == kIter && beta != T(0)) {
-      T uo[LC];
-#pragma unroll
-      for (int q = 0; q < LC; ++q) uo[q] = u[at_level<W>(o0, q, t.K0 + 1 + q <= kb, zero)];
-#pragma unroll
-      for (int q = 0; q < LC; ++q) g[q] = fma(beta, uo[q], g[q]);
-    }
+    couplings(t, szw, kb, kb ? zwa : T(0), cp);
+    column_solve(t, scan, g, d, dm, cp, [&] {
+      if (tile + (int)gridDim.x < ntiles) {
+        next = tiles.at(tile + gridDim.x, kn);
+        issue(next);
+        kn = tiles.kk(tile + 2 * gridDim.x);
+      }
+    });
 #pragma unroll
     for (int q = 0; q < LC; ++q) {
-      const int o = o0 + W * q;
       if (t.K0 + 1 + q <= kb) {
         if (MODE == kAfter) {
           const int f = f0 + plane * q;
-          x[f] = x[f] + scale * (double)(u[o] - g[q]);
+          x[f] = x[f] + scale * (double)(uo[q] - g[q]);
         } else {
-          u[o] = g[q];
+          u[a.o0 + W * q] = MODE == kIter && beta != T(0) ? fma(beta, uo[q], g[q]) : g[q];
         }
       }
     }
   }
+  st.report(S);
   if (MODE == kBefore) {
     double w[1] = {bb};
     if (grid_sum<1, Ln::NT>(w, S)) S->bb = w[0];
@@ -528,77 +622,75 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_red(RbGeo R, SolverSt
 }
 
 // Black columns: x += alpha p (the previous step's), p = z + beta p,
-// q = D p - C u, and alpha = rho / p.q.  The first iteration (iter = 0) reads
+// q = D p - C u, and alpha = rho / p.q.  The first iteration (iter = 0) uses
 // neither p nor x.
-template <typename T, int G, int LC>
-__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_black(RbGeo R, SolverState* S,
-                                                       const T* __restrict__ z,
-                                                       const T* __restrict__ u, T* __restrict__ p,
-                                                       T* __restrict__ x, T* __restrict__ q,
-                                                       int ntiles, int nt) {
-  using Ln = Lane<T, G, LC>;
-  constexpr int W = Ln::W;
-  __shared__ T szw[G * LC + 1], siz[G * LC + 1];
+template <typename Ln>
+using BlackStage = Stage<Ln, typename Ln::V, 6, 0>;
+
+template <typename Ln, typename T = typename Ln::V>
+__global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
+                                                     const T* __restrict__ z,
+                                                     const T* __restrict__ u, T* __restrict__ p,
+                                                     T* __restrict__ x, T* __restrict__ q,
+                                                     const int* __restrict__ km, int ntiles, int nt) {
+  constexpr int W = Ln::W, LC = Ln::L, G = Ln::GROUPS;
+  extern __shared__ __align__(128) unsigned char dsm[];
+  __shared__ T szw[Ln::ROWS + 1], siz[Ln::ROWS + 1];
+  __shared__ T top[2][G][W], bottom[2][G][W];  // p of the threads' first and last levels
+  __shared__ __align__(8) uint64_t bar;
   if (S->converged) return;
   const T beta = (T)S->beta, alpha = (T)S->alpha_prev;
   const bool first = S->iter == 0;
-  load_tables<T, G, LC>(R, szw, siz);
-  __shared__ T top[2][G][W], bottom[2][G][W];  // p of the threads' first and last levels
   const Ln t;
-  const int row = nt * R.ke * W, zero = row;
+  const Tiles<Ln> tiles{R, R.col[1], t, ntiles, nt, false};
+  BlackStage<Ln> st(dsm, &bar);
+  load_tables<Ln>(R, szw, siz);
+  __syncthreads();
+  auto issue = [&](const Tile& a) {
+    st.issue(tiles, a, km, {u, u, u, z, p, x}, {0, -1, 1, 0, 0, 0}, u, u);
+  };
+  int tile = blockIdx.x;
+  Tile next = tiles.at(tile, tiles.kk(tile));
+  issue(next);
+  unsigned long long kn = tiles.kk(tile + gridDim.x);
   double pq = 0.0;
   int buf = 0;
-  Tiles<T, G, LC> it(R, R.col[1], t, ntiles, nt);
-  while (it.next(R, R.col[1], t, ntiles, nt, false)) {
-    if (threadIdx.x == 0 && it.next_tile < ntiles) {
-      prefetch_tile(z, it.next_tile, nt, R.ke);
-      prefetch_tile(p, it.next_tile, nt, R.ke);
-      prefetch_tile(x, it.next_tile, nt, R.ke);
-      prefetch_tile(u, it.next_tile, nt, R.ke);
+  for (; tile < ntiles; tile += gridDim.x) {
+    const Tile a = next;
+    const int kb = wet_levels(a.kk, 0);
+    T pl[LC], xo[LC], v[LC];
+    st.wait();
+    const double2 zw = st.pairs[t.c], iz = st.pairs[W + t.c];
+    const double2 we = st.pairs[2 * W + t.c], ns = st.pairs[3 * W + t.c];
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const bool old = !first && t.K0 + 1 + e <= kb;
+      const T po = old ? st.get(t, 4, e) : T(0);
+      xo[e] = fma(alpha, po, old ? st.get(t, 5, e) : T(0));
+      pl[e] = fma(beta, po, t.K0 + 1 + e <= kb ? st.get(t, 3, e) : T(0));
     }
-    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
-    const int kbw = wet_levels(it.kk, 1), kbe = wet_levels(it.kk, 2);
-    const int kbn = wet_levels(it.kk, 3), kbs = wet_levels(it.kk, 4);
-    T pl[LC];
-    {
-      T po[LC], xo[LC];
-#pragma unroll
-      for (int e = 0; e < LC; ++e) pl[e] = z[at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero)];
-#pragma unroll
-      for (int e = 0; e < LC; ++e) {
-        const int o = at_level<W>(o0, e, t.K0 + 1 + e <= kb && !first, zero);
-        po[e] = p[o];
-        xo[e] = x[o];
-      }
-#pragma unroll
-      for (int e = 0; e < LC; ++e) {
-        xo[e] = fma(alpha, po[e], xo[e]);
-        pl[e] = fma(beta, po[e], pl[e]);
-        if (t.K0 + 1 + e <= kb) {
-          x[o0 + W * e] = xo[e];
-          p[o0 + W * e] = pl[e];
-        }
-      }
-    }
+    st.neighbour_sum(t, a, 0, we, ns, v);
     top[buf][t.g][t.c] = pl[0];
     bottom[buf][t.g][t.c] = pl[LC - 1];
-    const double2 we = R.col[1].we[it.s2], ns = R.col[1].ns[it.s2], iz = R.col[1].iz[it.s2],
-                  zw = R.col[1].zw[it.s2];
-    const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
-    const T zwa = (T)zw.x;
     __syncthreads();
+    if (tile + (int)gridDim.x < ntiles) {
+      next = tiles.at(tile + gridDim.x, kn);
+      issue(next);
+      kn = tiles.kk(tile + 2 * gridDim.x);
+    }
+#pragma unroll
+    for (int e = 0; e < LC; ++e)
+      if (t.K0 + 1 + e <= kb) {
+        x[a.o0 + W * e] = xo[e];
+        p[a.o0 + W * e] = pl[e];
+      }
     T pu = t.g == 0 ? T(0) : bottom[buf][t.g - 1][t.c];
     const T pb = t.g == G - 1 ? T(0) : top[buf][t.g + 1][t.c];
     buf ^= 1;
-    T pqt = T(0), v[LC];
-#pragma unroll
-    for (int e = 0; e < LC; ++e) {
-      const int K = t.K0 + 1 + e, o = at_level<W>(o0, e, K <= kb, zero);
-      T h = cw * u[o + it.west];
-      h = fma(ce, u[o + it.east], h);
-      h = fma(cn, u[o - row], h);
-      v[e] = fma(cs, u[o + row], h);
-    }
+    const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y, zwa = (T)zw.x;
+    const int kbw = wet_levels(a.kk, 1), kbe = wet_levels(a.kk, 2);
+    const int kbn = wet_levels(a.kk, 3), kbs = wet_levels(a.kk, 4);
+    T pqt = T(0);
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
       const int K = t.K0 + 1 + e;
@@ -613,99 +705,106 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_black(RbGeo R, Solver
       // below the bottom nothing couples, but Z_C of the surface row keeps ZW(2)
       T zw1 = K + 1 == kb ? zwa : szw[t.K0 + e + 1];
       if (K == kb) zw1 = K == 1 ? (T)zw.y : T(0);
-      v[e] = zw0 * (pu - p0);
-      v[e] = fma(zw1, pd - p0, v[e]);
-      v[e] = fma(-hs, h, v[e]);
-      pqt = fma(p0, v[e], pqt);  // p0 = 0 below the bottom
+      T s = zw0 * (pu - p0);
+      s = fma(zw1, pd - p0, s);
+      s = fma(-hs, h, s);
+      if (K <= kb) {
+        q[a.o0 + W * e] = s;
+        pqt = fma(p0, s, pqt);
+      }
       pu = p0;
     }
-#pragma unroll
-    for (int e = 0; e < LC; ++e)
-      if (t.K0 + 1 + e <= kb) q[o0 + W * e] = v[e];
     pq += (double)pqt;
   }
+  st.report(S);
   double w[1] = {pq};
   if (grid_sum<1, Ln::NT>(w, S)) {
     S->pq = w[0];
     S->alpha = S->rho / w[0];
-    if (!(w[0] > 0.0) && !(w[0] < 0.0)) S->converged = 3;  // breakdown
+    if (S->converged == 0 && !(w[0] > 0.0) && !(w[0] < 0.0)) S->converged = 3;  // breakdown
   }
 }
 
 // Black columns: residual, z = D_b^-1 r with the FP32 pivots, r.z and r.r.
 //   INIT   r = b / ZP - C u     (u = D_r^-1 (b / ZP) of the red columns)
 //   else   r -= alpha q
-template <typename T, int G, int LC, bool INIT>
-__global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_col(RbGeo R, SolverState* S, T* __restrict__ r,
-                                                     const T* __restrict__ q, T* __restrict__ z,
-                                                     const float* __restrict__ dinv,
-                                                     const double* __restrict__ b,
-                                                     const T* __restrict__ ub, int ntiles,
-                                                     int nt) {
-  using Ln = Lane<T, G, LC>;
-  constexpr int W = Ln::W;
-  __shared__ T szw[G * LC + 1];
+template <typename Ln, bool INIT>
+using ColStage = Stage<Ln, float, INIT ? 3 : 2, 1>;
+
+template <typename Ln, bool INIT, typename T = typename Ln::V>
+__global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* __restrict__ r,
+                                                   const T* __restrict__ q, T* __restrict__ z,
+                                                   const float* __restrict__ dinv,
+                                                   const int* __restrict__ km,
+                                                   const double* __restrict__ b,
+                                                   const T* __restrict__ ub, int ntiles, int nt) {
+  constexpr int W = Ln::W, LC = Ln::L;
+  extern __shared__ __align__(128) unsigned char dsm[];
+  __shared__ T szw[Ln::ROWS + 1];
+  __shared__ Scan<Ln> scan;
+  __shared__ __align__(8) uint64_t bar;
   if (!INIT && S->converged) return;
   const T alpha = INIT ? T(0) : (T)S->alpha;
   double scale = 1.0;
   if (INIT && sizeof(T) == 4) scale = S->res_rr > 0.0 ? 1.0 / sqrt(S->res_rr) : 0.0;
-  load_tables<T, G, LC>(R, szw, nullptr);
-  __shared__ Scan<T, G, W> scan;
   const Ln t;
-  const int row = nt * R.ke * W, zero = row;
+  const Tiles<Ln> tiles{R, R.col[1], t, ntiles, nt, false};
+  ColStage<Ln, INIT> st(dsm, &bar);
+  load_tables<Ln, T>(R, szw, nullptr);
+  __syncthreads();
+  auto issue = [&](const Tile& a) {
+    if constexpr (INIT) st.issue(tiles, a, km, {ub, ub, ub}, {0, -1, 1}, dinv, ub);
+    else st.issue(tiles, a, km, {q, (const T*)r}, {0, 0}, dinv, nullptr);
+  };
+  int tile = blockIdx.x;
+  Tile next = tiles.at(tile, tiles.kk(tile));
+  issue(next);
+  unsigned long long kn = tiles.kk(tile + gridDim.x);
   double rz = 0.0, rr = 0.0, bb = 0.0;
-  Tiles<T, G, LC> it(R, R.col[1], t, ntiles, nt);
-  while (it.next(R, R.col[1], t, ntiles, nt, false)) {
-    if (!INIT && threadIdx.x == 0 && it.next_tile < ntiles) {
-      prefetch_tile(q, it.next_tile, nt, R.ke);
-      prefetch_tile(r, it.next_tile, nt, R.ke);
-    }
-    const int kb = wet_levels(it.kk, 0), o0 = it.o0;
-    T g[LC], d[LC], a[LC + 1], rrt = T(0);
-#pragma unroll
-    for (int e = 0; e < LC; ++e) d[e] = (T)dinv[at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero)];
-    const T dm = (T)dinv[at_level<W>(o0, -1, t.K0 > 0 && t.K0 <= kb, zero)];
-    const T zwa = (T)R.col[1].zw[it.s2].x;
-    if (INIT) {
-      const double2 we = R.col[1].we[it.s2], ns = R.col[1].ns[it.s2], iz = R.col[1].iz[it.s2];
-      const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+  for (; tile < ntiles; tile += gridDim.x) {
+    const Tile a = next;
+    const int kb = wet_levels(a.kk, 0);
+    T g[LC], d[LC], cp[LC + 1], dm, rrt = T(0);
+    st.wait();
+    const T zwa = (T)st.pairs[t.c].x;
+    st.pivots(t, kb, dm, d);
+    if constexpr (INIT) {
+      const double2 iz = st.pairs[W + t.c];
       const int plane = 2 * R.plane2;
-      const int f0 = black_i(it.m, it.j) + 2 * R.P2 * it.j + plane * t.K0;
+      const int f0 = black_i(a.m, a.j) + 2 * R.P2 * a.j + plane * t.K0;
+      st.neighbour_sum(t, a, 0, st.pairs[2 * W + t.c], st.pairs[3 * W + t.c], g);
 #pragma unroll
       for (int e = 0; e < LC; ++e) {
-        const int K = t.K0 + 1 + e, o = at_level<W>(o0, e, K <= kb, zero);
+        const int K = t.K0 + 1 + e;
         const double hs = K == kb ? iz.y : (K == kb - 1 ? iz.x : (double)R.izn[K <= kb ? K - 1 : 0]);
-        const T bs = K <= kb ? (T)((b[f0 + plane * e] * scale) * hs) : T(0);
-        T h = cw * ub[o + it.west];
-        h = fma(ce, ub[o + it.east], h);
-        h = fma(cn, ub[o - row], h);
-        h = fma(cs, ub[o + row], h);
-        g[e] = fma(-(T)hs, h, bs);
+        const T bs = K <= kb ? (T)((b[K <= kb ? f0 + plane * e : 0] * scale) * hs) : T(0);
+        g[e] = K <= kb ? fma(-(T)hs, g[e], bs) : T(0);
         bb = fma((double)bs, (double)bs, bb);
       }
     } else {
-      T ql[LC];
 #pragma unroll
-      for (int e = 0; e < LC; ++e) {
-        const int o = at_level<W>(o0, e, t.K0 + 1 + e <= kb, zero);
-        ql[e] = q[o];
-        g[e] = r[o];
-      }
-#pragma unroll
-      for (int e = 0; e < LC; ++e) g[e] = fma(-alpha, ql[e], g[e]);
+      for (int e = 0; e < LC; ++e)
+        g[e] = t.K0 + 1 + e <= kb ? fma(-alpha, st.get(t, 0, e), st.get(t, 1, e)) : T(0);
     }
+    couplings(t, szw, kb, kb ? zwa : T(0), cp);
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
-      if (t.K0 + 1 + e <= kb) r[o0 + W * e] = g[e];
+      if (t.K0 + 1 + e <= kb) r[a.o0 + W * e] = g[e];
       rrt = fma(g[e], g[e], rrt);
     }
-    couplings<T, G, LC>(t, szw, kb, zwa, a);
-    rz += (double)column_solve<T, G, LC>(t, scan, g, d, dm, a);
+    rz += (double)column_solve(t, scan, g, d, dm, cp, [&] {
+      if (tile + (int)gridDim.x < ntiles) {
+        next = tiles.at(tile + gridDim.x, kn);
+        issue(next);
+        kn = tiles.kk(tile + 2 * gridDim.x);
+      }
+    });
     rr += (double)rrt;
 #pragma unroll
     for (int e = 0; e < LC; ++e)
-      if (t.K0 + 1 + e <= kb) z[o0 + W * e] = g[e];
+      if (t.K0 + 1 + e <= kb) z[a.o0 + W * e] = g[e];
   }
+  st.report(S);
   double v[INIT ? 3 : 2];
   v[0] = rz;
   v[1] = rr;
@@ -722,8 +821,10 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_col(RbGeo R, SolverSt
     }
     S->rho = v[0];
     S->rr = v[1];
-    if (sqrt(v[1]) <= S->tol * sqrt(S->bb) || S->bb == 0.0) S->converged = 1;
-    if (!(v[0] == v[0]) || !(v[1] == v[1])) S->converged = 2;  // NaN: stop
+    if (S->converged == 0) {
+      if (sqrt(v[1]) <= S->tol * sqrt(S->bb) || S->bb == 0.0) S->converged = 1;
+      if (!(v[0] == v[0]) || !(v[1] == v[1])) S->converged = 2;  // NaN: stop
+    }
   }
 }
 
@@ -732,10 +833,10 @@ __global__ void __launch_bounds__(Lane<T, G, LC>::NT) k_rb_col(RbGeo R, SolverSt
 template <typename T>
 __global__ void __launch_bounds__(128) k_rb_after(RbGeo R, SolverState* S, const T* __restrict__ p,
                                                   T* __restrict__ d, double* __restrict__ x) {
-  constexpr int W = Width<T>::W;
-  const int m = blockIdx.x * W + threadIdx.x % W, K = blockIdx.z * (128 / W) + threadIdx.x / W + 1;
-  const int j = blockIdx.y + 2;
-  if (m >= R.M || K > wet_levels(R.col[1].kk[m + R.P2 * j], 0)) return;
+  const int W = R.width((int)sizeof(T));
+  const int m = 1 + blockIdx.x * W + threadIdx.x % W;
+  const int K = blockIdx.z * (128 / W) + threadIdx.x / W + 1, j = blockIdx.y + 2;
+  if (m > R.M || K > wet_levels(R.col[1].kk[m + R.P2 * j], 0)) return;
   const int o = ((j * R.nt(W) + (int)blockIdx.x) * R.ke + K - 1) * W + threadIdx.x % W;
   T v = T(0);
   if (S->iter > 0) v = fma((T)S->alpha_prev, p[o], d[o]);
@@ -856,103 +957,114 @@ struct Shape {
   int ntiles, nt, grid;
 };
 
-// A persistent grid: as many blocks as run at once, each walking tiles.
+// A persistent grid: as many blocks as run at once, each walking tiles.  The
+// blocks per SM are asked for once per kernel and device, after the opt-in to
+// the staging's shared memory (a fixed size per kernel).
+constexpr int kMaxDevices = 64;
+
 template <auto Kernel, typename L>
-Shape shape_of(const RbGeo& R) {
-  static const int per_sm = [] {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, L::NT, 0) != cudaSuccess) n = 1;
-    return std::max(n, 1);
-  }();
+Shape shape_of(const RbGeo& R, size_t smem) {
+  static std::atomic<int> per_sm[kMaxDevices];
+  const int dev = R.device & (kMaxDevices - 1);
+  int n = per_sm[dev].load(std::memory_order_acquire);
+  if (!n) {
+    cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, L::NT, smem) != cudaSuccess || n < 1) n = 1;
+    per_sm[dev].store(n, std::memory_order_release);
+  }
   Shape s;
   s.nt = R.nt(L::W);
   s.ntiles = s.nt * (R.je - 2);
-  s.grid = std::min({s.ntiles, per_sm * R.sms, kMaxBlocks});
+  s.grid = std::min({s.ntiles, n * R.sms, kMaxBlocks});
   return s;
 }
 
-template <int N>
-using Int = std::integral_constant<int, N>;
-
-// Calls f with the split of a column of KE levels: 8 threads of up to 13
-// levels, 16 of up to 20 above.  More levels per thread take more than the 255
-// registers; fewer, the shared work of a thread (its column's 2D data, the
+// Calls f with the Lane type for columns of KE levels: 8 threads of 5 to 13
+// levels, in longer columns more threads of 10, beyond 160 levels in tiles of half
+// the width (a tile of six arrays has to fit shared memory).  A thread's
+// registers hold some 4 values per level; with fewer levels per
+// thread the work that a thread does once (its column's 2D data, the
 // scan) outweighs its levels.
-template <typename F>
+template <typename T, typename F>
 void with_split(int ke, F&& f) {
-  if (ke <= 40) f(Int<8>{}, Int<5>{});
-  else if (ke <= 48) f(Int<8>{}, Int<6>{});
-  else if (ke <= 64) f(Int<8>{}, Int<8>{});
-  else if (ke <= 80) f(Int<8>{}, Int<10>{});
-  else if (ke <= 88) f(Int<8>{}, Int<11>{});
-  else if (ke <= 104) f(Int<8>{}, Int<13>{});
-  else if (ke <= 160) f(Int<16>{}, Int<10>{});
-  else f(Int<16>{}, Int<20>{});
+  if (ke <= 40) f((Lane<T, 8, 5, 0>*)nullptr);
+  else if (ke <= 48) f((Lane<T, 8, 6, 0>*)nullptr);
+  else if (ke <= 64) f((Lane<T, 8, 8, 0>*)nullptr);
+  else if (ke <= 80) f((Lane<T, 8, 10, 0>*)nullptr);
+  else if (ke <= 88) f((Lane<T, 8, 11, 0>*)nullptr);
+  else if (ke <= 104) f((Lane<T, 8, 13, 0>*)nullptr);
+  else if (ke <= RbGeo::kWide) f((Lane<T, 16, 10, 0>*)nullptr);
+  else f((Lane<T, 32, 10, 1>*)nullptr);
 }
-static_assert(16 * 20 >= kMaxKe, "the longest column has a split");
+static_assert(32 * 10 >= kMaxKe && 16 * 10 >= RbGeo::kWide, "the longest column has a split");
 
 }  // namespace
 
 size_t rb_elements(const RbGeo& R, int elem_bytes) {
-  const int W = 128 / elem_bytes;
+  const int W = R.width(elem_bytes);
   return (size_t)R.nt(W) * W * R.ke * (R.je + 1);
+}
+size_t rb_tiles(const RbGeo& R, int elem_bytes) {
+  return (size_t)2 * R.nt(R.width(elem_bytes)) * (R.je + 1);
 }
 
 template <typename T>
 void launch_rb_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, const RbVectors<T>& v,
                      cudaStream_t st) {
   const dim3 blk(32, 4);
-  k_rb_setup<T><<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, 0, st>>>(G, P, R, v.dr, v.db);
+  k_rb_setup<T><<<grid2(G.L.ie - 2, G.L.je - 2, blk), blk, 0, st>>>(G, P, R, v.dr, v.db, v.km);
   count_launch();
 }
+
+#define ORCTM_LANE(l) std::remove_pointer_t<decltype(l)>
 
 template <typename T>
 void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbVectors<T>& v,
                       cudaStream_t st) {
-  with_split(R.ke, [&](auto gc, auto lc) {
-    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    using L = Lane<T, G, LC>;
-    const Shape s = shape_of<k_rb_red<T, G, LC, kBefore>, L>(R);
-    k_rb_red<T, G, LC, kBefore><<<s.grid, L::NT, 0, st>>>(R, S, nullptr, v.ub, v.dr, b, nullptr,
-                                                          s.ntiles, s.nt);
-    const Shape c = shape_of<k_rb_col<T, G, LC, true>, L>(R);
-    k_rb_col<T, G, LC, true><<<c.grid, L::NT, 0, st>>>(R, S, v.r, nullptr, v.z, v.db, b, v.ub,
-                                                       c.ntiles, c.nt);
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    constexpr size_t m1 = RedStage<L, kBefore>::smem, m2 = ColStage<L, true>::smem;
+    const Shape s = shape_of<k_rb_red<L, kBefore>, L>(R, m1);
+    k_rb_red<L, kBefore><<<s.grid, L::NT, m1, st>>>(R, S, (const T*)nullptr, v.ub, v.dr, v.km, b, nullptr,
+                                                    s.ntiles, s.nt);
+    const Shape c = shape_of<k_rb_col<L, true>, L>(R, m2);
+    k_rb_col<L, true><<<c.grid, L::NT, m2, st>>>(R, S, v.r, (const T*)nullptr, v.z, v.db, v.km, b, v.ub,
+                                                 c.ntiles, c.nt);
   });
   add_launches(2);
 }
 
 template <typename T>
 void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
-  with_split(R.ke, [&](auto gc, auto lc) {
-    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    using L = Lane<T, G, LC>;
-    const Shape s = shape_of<k_rb_red<T, G, LC, kIter>, L>(R);
-    k_rb_red<T, G, LC, kIter><<<s.grid, L::NT, 0, st>>>(R, S, v.z, v.u, v.dr, nullptr, nullptr,
-                                                        s.ntiles, s.nt);
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    constexpr size_t m = RedStage<L, kIter>::smem;
+    const Shape s = shape_of<k_rb_red<L, kIter>, L>(R, m);
+    k_rb_red<L, kIter><<<s.grid, L::NT, m, st>>>(R, S, v.z, v.u, v.dr, v.km, nullptr, nullptr,
+                                                 s.ntiles, s.nt);
   });
   count_launch();
 }
 
 template <typename T>
 void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
-  with_split(R.ke, [&](auto gc, auto lc) {
-    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    using L = Lane<T, G, LC>;
-    const Shape s = shape_of<k_rb_black<T, G, LC>, L>(R);
-    k_rb_black<T, G, LC><<<s.grid, L::NT, 0, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, s.ntiles, s.nt);
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    constexpr size_t m = BlackStage<L>::smem;
+    const Shape s = shape_of<k_rb_black<L>, L>(R, m);
+    k_rb_black<L><<<s.grid, L::NT, m, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, v.km, s.ntiles, s.nt);
   });
   count_launch();
 }
 
 template <typename T>
 void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
-  with_split(R.ke, [&](auto gc, auto lc) {
-    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    using L = Lane<T, G, LC>;
-    const Shape s = shape_of<k_rb_col<T, G, LC, false>, L>(R);
-    k_rb_col<T, G, LC, false><<<s.grid, L::NT, 0, st>>>(R, S, v.r, v.q, v.z, v.db, nullptr, nullptr,
-                                                        s.ntiles, s.nt);
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    constexpr size_t m = ColStage<L, false>::smem;
+    const Shape s = shape_of<k_rb_col<L, false>, L>(R, m);
+    k_rb_col<L, false><<<s.grid, L::NT, m, st>>>(R, S, v.r, v.q, v.z, v.db, v.km, nullptr, (const T*)nullptr,
+                                                 s.ntiles, s.nt);
   });
   count_launch();
 }
@@ -960,15 +1072,15 @@ void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaSt
 template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x,
                      cudaStream_t st) {
-  constexpr int W = Width<T>::W;
+  const int W = R.width((int)sizeof(T));
   const dim3 grid(R.nt(W), R.je - 2, (R.ke + 128 / W - 1) / (128 / W));
   k_rb_after<T><<<grid, 128, 0, st>>>(R, S, v.p, v.x, x);
-  with_split(R.ke, [&](auto gc, auto lc) {
-    constexpr int G = decltype(gc)::value, LC = decltype(lc)::value;
-    using L = Lane<T, G, LC>;
-    const Shape s = shape_of<k_rb_red<T, G, LC, kAfter>, L>(R);
-    k_rb_red<T, G, LC, kAfter><<<s.grid, L::NT, 0, st>>>(R, S, v.x, v.ub, v.dr, nullptr, x, s.ntiles,
-                                                         s.nt);
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    constexpr size_t m = RedStage<L, kAfter>::smem;
+    const Shape s = shape_of<k_rb_red<L, kAfter>, L>(R, m);
+    k_rb_red<L, kAfter><<<s.grid, L::NT, m, st>>>(R, S, v.x, v.ub, v.dr, v.km, nullptr, x, s.ntiles,
+                                                  s.nt);
   });
   add_launches(2);
 }
