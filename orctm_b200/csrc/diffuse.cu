@@ -2,8 +2,9 @@
 // octdiff_ts.f90:51-59, 294-407) and momentum diffusion with quadratic
 // bottom drag (OCVISC, FREESLIP branch: ocvisc.f90:37-478, 615-688).
 //
-// Implicit vertical diffusion is one Thomas solve per water column, one
-// thread per column.  The tracers' horizontal biharmonic operator is one
+// Implicit vertical diffusion is one tridiagonal solve per water column, by one
+// thread for the tracers and u, v, shared by the threads of a block for w
+// (tridiag.cuh).  The tracers' horizontal biharmonic operator is one
 // fused pass (the first Laplacian formed per level in shared memory, never
 // stored); the momentum one is two passes (a Laplacian into a scratch field,
 // then the flux-form update).  Arithmetic follows the reference's operation order in IEEE binary64,
@@ -11,8 +12,11 @@
 // reciprocal metrics and per-face coefficients computed once at set-up
 // instead of dividing by the metrics, and the remaining divisions (by
 // thicknesses and Thomas pivots) use div_nr (within 1 ulp of IEEE division).
+#include <type_traits>
+
 #include "common.cuh"
 #include "ops.h"
+#include "tridiag.cuh"
 
 namespace orctm {
 
@@ -395,83 +399,13 @@ __global__ void k_visc_speed(Geo G, const double* __restrict__ uoo, const double
 }
 
 // implicit vertical diffusion of u (DIR = 0, ocvisc.f90:168-218) or v
-// (DIR = 1, ocvisc.f90:114-165) with quadratic bottom drag in the last row
-template <int DIR>
-__global__ void __launch_bounds__(kVertBlock) k_visc_uv(Geo G, const double* __restrict__ X,
-                                                        const double* __restrict__ keep,
-                                                        const double* __restrict__ avo,
-                                                        const double* __restrict__ speed,
-                                                        double* __restrict__ O) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
-  if (i > IE || j > JE) return;
-  const bool interior = DIR == 0 ? (i >= 1 && i <= IE - 1 && j >= 2 && j <= JE - 1)
-                                 : (i >= 2 && i <= IE - 1 && j >= 1 && j <= JE - 1);
-  const bool valid = DIR == 0 ? (j >= 1) : (i >= 1);
-  if (!valid) return;
-  if (!interior) {
-    for (int K = 1; K <= KE; ++K) AT(O, i, j, K) = AT(keep, i, j, K);
-    return;
-  }
-  const ColGeo& cg = DIR == 0 ? G.gu : G.gv;
-  const int ij = G.L.at2(i, j);
-  const int ij2 = DIR == 0 ? G.L.at2(i + 1, j) : G.L.at2(i, j + 1);
-  const double BOFRIC = 3.E-3, RAYFRIC = 3.E-3;
-  const double sp = speed[ij];
-  auto avo_at = [&](int q, int K) { return avo[q + G.L.plane * (K - 1)]; };
-  // TRIDSY(K,1) and TRIDSY(K,3) (after the AMS(K+1) factor) of
-  // ocvisc.f90:117-140 / 171-193
-  auto tri = [&](int K, double& t1, double& t3) {
-    const double am = wet(cg, ij, K), dd = thick(cg, G.dzw, ij, K);
-    const double avup = 0.5 * (avo_at(ij, K) + avo_at(ij2, K)) * am;
-    if (K < KE) {
-      const double am1 = wet(cg, ij, K + 1);
-      const double avlo = 0.5 * (avo_at(ij, K + 1) + avo_at(ij2, K + 1)) * am1 +
-                          (BOFRIC + RAYFRIC * dd * sp) * (am - am1);
-      t1 = div_nr(-G.dt * avup * am * G.di[K - 1], G.almzer + dd);
-      t3 = div_nr(-G.dt * avlo * am * G.di[K], G.almzer + dd);
-    } else {
-      const double avlo = (BOFRIC + RAYFRIC * dd * sp) * am;
-      t1 = div_nr(-G.dt * avup * am * G.di[K - 1], G.almzer + dd);
-      t3 = div_nr(-G.dt * avlo * am * G.di[K], G.almzer + dd);
-    }
-  };
-  double t2p[kMaxKe];
-  double t2prev = 1.0, t3prev = 0.0, yprev = 0.0;
-  for (int K = 1; K <= KE; ++K) {
-    double t1, t3;
-    tri(K, t1, t3);
-    double t2 = 1. - t1 - t3;
-    t3 = K < KE ? t3 * wet(cg, ij, K + 1) : 0.;
-    const double xk = AT(X, i, j, K);
-    double y = xk;
-    if (K >= 2) {
-      const double m = div_nr(t1, t2prev);
-      t2 = t2 - div_nr(t3prev * t1, t2prev);
-      y = xk - m * yprev;
-    }
-    t2p[K - 1] = t2;
-    AT(O, i, j, K) = y;
-    yprev = y;
-    t2prev = t2;
-    t3prev = t3;
-  }
-  double nxt = div_nr(wet(cg, ij, KE) * AT(O, i, j, KE), t2p[KE - 1]);
-  AT(O, i, j, KE) = nxt;
-  for (int l = KE - 1; l >= 1; --l) {
-    double t1, t3;
-    tri(l, t1, t3);
-    t3 = t3 * wet(cg, ij, l + 1);
-    nxt = div_nr((AT(O, i, j, l) - t3 * nxt) * wet(cg, ij, l), t2p[l - 1]);
-    AT(O, i, j, l) = nxt;
-  }
-}
-
-// k_visc_uv with the loads of U levels issued together before they are used
-// (X and AVO of both columns in the forward sweep, the forward values and AVO
-// in the backward one); the same expressions in the same order, so the
-// results equal k_visc_uv's bit for bit.
+// (DIR = 1, ocvisc.f90:114-165) with quadratic bottom drag in the last row.
+// The loads of U levels are issued together before they are used (X and AVO of
+// both columns in the forward sweep, the forward values and AVO in the
+// backward one).  The tracers and u, v keep the reference's elimination level
+// by level: the scans of tridiag.cuh differ from it in the last digits, which the
+// convective switches of the whole step amplify (to 4e-8 of u after twenty
+// steps of the laboratory tank, where this form stays bit for bit).
 template <int DIR, int U>
 __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* __restrict__ X,
                                                           const double* __restrict__ keep,
@@ -573,93 +507,73 @@ __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* _
   }
 }
 
-// implicit vertical diffusion of w, levels 2..KE (ocvisc.f90:225-270).  One
-// forward sweep forms each level's coefficients, eliminates (the multiplier
-// TRIDSY(K-1,1)/TRIDSY(K-1,2) and the new diagonal, in the reference's
-// operation order) and substitutes; only the eliminated diagonal is kept per
-// level, and the backward sweep recomputes TRIDSY(K,3) by the same expression.
-// The loads of U levels are issued together (the results do not depend on U).
-template <int U>
-__global__ void __launch_bounds__(kVertBlock) k_visc_w_b(Geo G, const double* __restrict__ W,
-                                                         const double* __restrict__ avo,
-                                                         double* __restrict__ O) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
-  if (i > IE || j > JE) return;
-  const int pl = G.L.plane;
-  const int base = G.L.at(i, j, 0);
-  const bool interior = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1 && KE >= 2;
-  if (!interior) {
-    for (int K = 1; K <= KE + 1; ++K) O[base + (K - 1) * pl] = W[base + (K - 1) * pl];
-    return;
+// implicit vertical diffusion of w, levels 2..KE (ocvisc.f90:225-270); the
+// levels 1 and KEP are carried.  Row K of the solve is level K + 1.
+template <typename Ln>
+__global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restrict__ Wi,
+                                                   const double* __restrict__ avo,
+                                                   double* __restrict__ O) {
+  constexpr int LC = Ln::LC;
+  __shared__ TriScan<Ln, 1> scan;
+  const Ln t;
+  const int i = blockIdx.x * Ln::W + t.c, j = blockIdx.y + 1;
+  const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke, pl = G.L.plane;
+  const bool valid = i >= 1 && i <= IE;
+  const bool interior = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
+  const int base = G.L.at(i, j, t.K0 + 1), ij = G.L.at2(i, j);  // level K0 + 2
+  double x[1][LC], a[LC], b[LC], c[LC], av[LC + 2];
+#pragma unroll
+  for (int u = 0; u < LC + 2; ++u) {  // AVO of levels K0 + 1 ...
+    const int K = t.K0 + 1 + u;
+    av[u] = interior && K <= KE ? avo[base + (u - 1) * pl] : 0.;
   }
-  const int ij = G.L.at2(i, j);
-  auto den = [&](int K) {
-    return 2.0 * G.almzer + thick(G.gp, G.dzw, ij, K - 1) + thick(G.gp, G.dzw, ij, K);
-  };
-  // AVO of levels K-1 (am), K (a0), K+1 (a1)
-  auto tri1 = [&](int K, double dn, double am, double a0) {
-    const double avup = 0.5 * (am + a0) * wet(G.gp, ij, K - 1);
-    return div_nr(-2.0 * G.dt * avup * wet(G.gp, ij, K) * G.di[K - 2], dn);
-  };
-  auto tri3 = [&](int K, double dn, double a0, double a1) {
-    const double avlo = K < KE ? 0.5 * (a1 + a0) * wet(G.gp, ij, K) : 0.0;
-    return div_nr(-2.0 * G.dt * avlo * wet(G.gp, ij, K) * G.di[K - 1], dn);
-  };
-  double t2p[kMaxKe];
-  O[base] = W[base];
-  O[base + KE * pl] = W[base + KE * pl];
-  double prev = 0.0, t2prev = 1.0, t3prev = 0.0;
-  for (int K0 = 2; K0 <= KE; K0 += U) {
-    double la[U + 2], lw[U];
 #pragma unroll
-    for (int u = 0; u < U + 2; ++u) {
-      const int K = K0 - 1 + u;  // K0-1 .. K0+U
-      la[u] = K <= KE ? avo[base + (K - 1) * pl] : 0.0;
-    }
+  for (int u = 0; u < LC; ++u) x[0][u] = valid && t.K0 + 2 + u <= KE ? Wi[base + u * pl] : 0.;
+  if (valid && t.g == 0) {
+    const int top = G.L.at(i, j, 0);
+    O[top] = Wi[top];
+    O[top + KE * pl] = Wi[top + KE * pl];
+  }
+  const int kb = interior ? G.gp.kb[ij] : 0;
+  const double bot = interior ? G.gp.bot[ij] : 0.;
+  auto thickness = [&](int K) { return K < kb ? G.dzw[K - 1] : (K == kb ? bot : 0.0); };
+  auto rden = [&](int K) {
+    return div_nr(1., 2.0 * G.almzer + thickness(K - 1) + thickness(K));
+  };
+  // TRIDSY(K,3) from AVO of levels K and K + 1
+  auto lower = [&](int K, double a0, double a1, double rd) {
+    const double avlo = K < KE && K <= kb ? 0.5 * (a1 + a0) : 0.0;
+    return -2.0 * G.dt * avlo * G.di[K - 1] * rd;
+  };
 #pragma unroll
-    for (int u = 0; u < U; ++u) lw[u] = K0 + u <= KE ? W[base + (K0 + u - 1) * pl] : 0.0;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int K = K0 + u;
-      if (K > KE) break;
-      const double dn = den(K);
-      const double t1 = tri1(K, dn, la[u], la[u + 1]), t3 = tri3(K, dn, la[u + 1], la[u + 2]);
-      double t2 = 1. - t1 - t3;
-      double y = lw[u];
-      if (K >= 3) {
-        const double m = div_nr(t1, t2prev);
-        t2 = t2 - div_nr(t3prev * t1, t2prev);
-        y = y - m * prev;
-      }
-      t2p[K - 1] = t2;
-      O[base + (K - 1) * pl] = y;
-      prev = y;
-      t2prev = t2;
-      t3prev = K < KE ? t3 : 0.;
+  for (int u = 0; u < LC; ++u) {
+    const int K = t.K0 + 2 + u;
+    a[u] = c[u] = 0.;
+    b[u] = 1.;
+    if (K <= KE && K <= kb) {
+      const double rd = rden(K);
+      a[u] = -2.0 * G.dt * (0.5 * (av[u] + av[u + 1])) * G.di[K - 2] * rd;
+      c[u] = lower(K, av[u + 1], av[u + 2], rd);
+      b[u] = 1. - a[u] - c[u];
+      if (K == 2) a[u] = 0.;
     }
   }
-  double nxt = div_nr(wet(G.gp, ij, KE) * prev, t2p[KE - 1]);
-  O[base + (KE - 1) * pl] = nxt;
-  for (int K0 = KE - 1; K0 >= 2; K0 -= U) {
-    double la[U], la1[U], ly[U];
+  const int Kp = t.K0 + 1;  // the level above the thread's first
+  const double cprev = Kp >= 2 && Kp < KE && Kp <= kb ? lower(Kp, av[0], av[1], rden(Kp)) : 0.;
+  if (valid && !interior) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int K = K0 - u;
-      const bool ok = K >= 2;
-      la[u] = ok ? avo[base + (K - 1) * pl] : 0.0;
-      la1[u] = ok ? avo[base + K * pl] : 0.0;
-      ly[u] = ok ? O[base + (K - 1) * pl] : 0.0;
-    }
+    for (int u = 0; u < LC; ++u)
+      if (t.K0 + 2 + u <= KE) O[base + u * pl] = x[0][u];
+  }
+  // levels below the bottom end as 0
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int K = K0 - u;
-      if (K < 2) break;
-      const double t3 = tri3(K, den(K), la[u], la1[u]);
-      nxt = div_nr((ly[u] - t3 * nxt) * wet(G.gp, ij, K), t2p[K - 1]);
-      O[base + (K - 1) * pl] = nxt;
-    }
+  for (int u = 0; u < LC; ++u)
+    if (t.K0 + 2 + u > kb) x[0][u] = 0.;
+  tri_solve<Ln, 1>(t, scan, a, b, c, cprev, x);
+  if (interior) {
+#pragma unroll
+    for (int u = 0; u < LC; ++u)
+      if (t.K0 + 2 + u <= KE) O[base + u * pl] = x[0][u];
   }
 }
 
@@ -902,7 +816,11 @@ void launch_ocvisc(const Geo& G, const double* uoo, const double* voe, const dou
   count_launch();
   k_visc_uv_b<1, 4><<<grid2(IE + 1, JE + 1, bc), bc, 0, st>>>(G, voe, vke, avo, spv, vkv);
   count_launch();
-  k_visc_w_b<4><<<grid2(IE, JE, bc), bc, 0, st>>>(G, wno, avo, wnv);
+  with_tri_split(KE, [&](auto* l) {
+    using Ln = std::remove_pointer_t<decltype(l)>;
+    const int nb = (IE + Ln::W) / Ln::W;
+    k_visc_w<Ln><<<dim3(nb, JE), Ln::NT, 0, st>>>(G, wno, avo, wnv);
+  });
   count_launch();
   dim3 gl = grid2(IE + 1, JE + 1, b3);
   gl.z = KE;

@@ -26,10 +26,12 @@
 // rejected with ORCTM_E_TOO_LARGE before anything is launched.
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "../../include/orctm_gpu.h"
 #include "common.cuh"
 #include "ops.h"
+#include "tridiag.cuh"
 
 namespace orctm {
 
@@ -65,100 +67,142 @@ __device__ __forceinline__ long long v2(const NaArgs& a, int i, int j) {
 
 // implicit vertical diffusion (octdiff_base.f90:182-204, octdiff_ts.f90:294-324);
 // columns outside the interior are copied
-__global__ void k_na_vert(NaArgs a, const double* __restrict__ T, double* __restrict__ O) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int IE = a.IE, JE = a.JE, KE = a.KE;
-  if (i > IE || j > JE) return;
-  if (!(i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1)) {
-    for (int K = 1; K <= KE; ++K) O[p3(a, i, j, K)] = T[p3(a, i, j, K)];
-    return;
+template <typename Ln>
+__global__ void __launch_bounds__(Ln::NT) k_na_vert(NaArgs a, const double* __restrict__ T,
+                                                    double* __restrict__ O) {
+  constexpr int LC = Ln::LC;
+  __shared__ TriScan<Ln, 1> scan;
+  const Ln t;
+  const int i = blockIdx.x * Ln::W + t.c + 1, j = blockIdx.y + 1;
+  const int IE = a.IE, JE = a.JE, KE = a.KE, pl = IE * JE;
+  const bool valid = i <= IE;
+  const bool interior = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
+  const int base = (int)p3(a, i, j, t.K0 + 1);
+  double x[1][LC], ta[LC], tb[LC], tc[LC], d[LC + 1], th[LC], wt[LC];
+#pragma unroll
+  for (int u = 0; u <= LC; ++u)
+    d[u] = interior && t.K0 + 1 + u <= KE + 1 ? a.dvo[base + u * pl] : 0.;
+#pragma unroll
+  for (int u = 0; u < LC; ++u) {
+    const bool ok = t.K0 + 1 + u <= KE;
+    x[0][u] = valid && ok ? T[base + u * pl] : 0.;
+    th[u] = interior && ok ? a.ddpo[base + u * pl] : 0.;
+    wt[u] = interior && ok ? a.weto[base + u * pl] : 0.;
   }
-  double t1[kMaxKe], t2[kMaxKe], t3[kMaxKe];
-  const double zo = a.zo[p2(a, i, j)];
-  for (int K = 1; K <= KE; ++K) {
+  const bool above = interior && t.K0 > 0 && t.K0 < KE;
+  const double thp = above ? a.ddpo[base - pl] : 0.;
+  const double zo = interior ? a.zo[p2(a, i, j)] : 0.;
+  auto rden = [&](int K, double dd) {
     const double zzsurf = K == 1 ? 1. : 0.;
-    const double den = a.ddpo[p3(a, i, j, K)] + zzsurf * (zo) + a.almzer;
-    t1[K - 1] = -a.dt * a.dvo[p3(a, i, j, K)] * a.weto[p3(a, i, j, K)] * a.di[K - 1] / den;
-    t3[K - 1] = -a.dt * a.dvo[p3(a, i, j, K + 1)] * a.di[K] / den;
-    t2[K - 1] = 1. - t1[K - 1] - t3[K - 1];
+    return 1. / (dd + zzsurf * (zo) + a.almzer);
+  };
+#pragma unroll
+  for (int u = 0; u < LC; ++u) {
+    const int K = t.K0 + 1 + u;
+    ta[u] = tc[u] = 0.;
+    tb[u] = 1.;
+    if (interior && K <= KE) {
+      const double rd = rden(K, th[u]);
+      ta[u] = -a.dt * d[u] * wt[u] * a.di[K - 1] * rd;
+      tc[u] = -a.dt * d[u + 1] * a.di[K] * rd;
+      tb[u] = 1. - ta[u] - tc[u];
+      if (K == 1) ta[u] = 0.;
+    }
   }
-  for (int K = 2; K <= KE; ++K) {
-    const double m = t1[K - 1];
-    t1[K - 2] = m / t2[K - 2];
-    t2[K - 1] = t2[K - 1] - t3[K - 2] * m / t2[K - 2];
+  const double cprev = above ? -a.dt * d[0] * a.di[t.K0] * rden(t.K0, thp) : 0.;
+  if (valid && !interior) {
+#pragma unroll
+    for (int u = 0; u < LC; ++u)
+      if (t.K0 + 1 + u <= KE) O[base + u * pl] = x[0][u];
   }
-  double prev = T[p3(a, i, j, 1)];
-  O[p3(a, i, j, 1)] = prev;
-  for (int K = 2; K <= KE; ++K) {
-    prev = T[p3(a, i, j, K)] - t1[K - 2] * prev;
-    O[p3(a, i, j, K)] = prev;
-  }
-  double nxt = O[p3(a, i, j, KE)] / t2[KE - 1];
-  O[p3(a, i, j, KE)] = nxt;
-  for (int l = KE - 1; l >= 1; --l) {
-    nxt = (O[p3(a, i, j, l)] - t3[l - 1] * nxt) / t2[l - 1];
-    O[p3(a, i, j, l)] = nxt;
+  tri_solve<Ln, 1>(t, scan, ta, tb, tc, cprev, x);
+  if (interior) {
+#pragma unroll
+    for (int u = 0; u < LC; ++u)
+      if (t.K0 + 1 + u <= KE) O[base + u * pl] = x[0][u];
   }
 }
 
+// The horizontal passes: a thread takes kNaLevels levels of a column, so that
+// the divisions by the metrics are made once for them.
+constexpr int kNaLevels = 6;
+
 // masked Laplacian (octdiff_ts.f90:346-362); halo cells are written as 0
-__global__ void k_na_lap(NaArgs a, const double* __restrict__ T, double* __restrict__ L1) {
+__global__ void __launch_bounds__(128) k_na_lap(NaArgs a, const double* __restrict__ T,
+                                                double* __restrict__ L1) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int K = blockIdx.z + 1;
-  const int IE = a.IE, JE = a.JE;
+  const int IE = a.IE, JE = a.JE, pl = IE * JE, K0 = blockIdx.z * kNaLevels;
   if (i > IE || j > JE) return;
-  double r = 0.0;
-  if (i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1) {
-    const double c = T[p3(a, i, j, K)];
-    auto w = [&](int ii, int jj) { return a.weto[p3(a, ii, jj, K)]; };
-    r = w(i, j) *
-        ((w(i - 1, j) * (T[p3(a, i - 1, j, K)] - c) / a.dlxu[u2(a, i - 1, j)] +
-          w(i + 1, j) * (T[p3(a, i + 1, j, K)] - c) / a.dlxu[u2(a, i, j)]) /
-             a.dlxp[p2(a, i, j)] +
-         (w(i, j - 1) * (T[p3(a, i, j - 1, K)] - c) / a.dlyv[v2(a, i, j - 1)] +
-          w(i, j + 1) * (T[p3(a, i, j + 1, K)] - c) / a.dlyv[v2(a, i, j)]) /
-             a.dlyp[p2(a, i, j)]);
+  const bool inner = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
+  double rxw = 0., rxe = 0., rxp = 0., ryn = 0., rys = 0., ryp = 0.;
+  if (inner) {
+    rxw = 1. / a.dlxu[u2(a, i - 1, j)];
+    rxe = 1. / a.dlxu[u2(a, i, j)];
+    rxp = 1. / a.dlxp[p2(a, i, j)];
+    ryn = 1. / a.dlyv[v2(a, i, j - 1)];
+    rys = 1. / a.dlyv[v2(a, i, j)];
+    ryp = 1. / a.dlyp[p2(a, i, j)];
   }
-  L1[p3(a, i, j, K)] = r;
+  const int c = (int)p3(a, i, j, K0 + 1);
+#pragma unroll
+  for (int q = 0; q < kNaLevels; ++q) {
+    const int o = c + q * pl;
+    if (K0 + q >= a.KE) break;
+    double r = 0.0;
+    if (inner) {
+      const double t = T[o];
+      r = a.weto[o] * ((a.weto[o - 1] * (T[o - 1] - t) * rxw + a.weto[o + 1] * (T[o + 1] - t) * rxe) * rxp +
+                       (a.weto[o - IE] * (T[o - IE] - t) * ryn + a.weto[o + IE] * (T[o + IE] - t) * rys) * ryp);
+    }
+    L1[o] = r;
+  }
 }
 
 // biharmonic update (octdiff_ts.f90:369-399)
-__global__ void k_na_bih(NaArgs a, const double* __restrict__ T, const double* __restrict__ L1,
-                         double* __restrict__ O) {
+__global__ void __launch_bounds__(128) k_na_bih(NaArgs a, const double* __restrict__ T,
+                                                const double* __restrict__ L1,
+                                                double* __restrict__ O) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const int K = blockIdx.z + 1;
-  const int IE = a.IE, JE = a.JE;
+  const int IE = a.IE, JE = a.JE, pl = IE * JE, K0 = blockIdx.z * kNaLevels;
   if (i > IE || j > JE) return;
-  const double t = T[p3(a, i, j, K)];
-  double r = t;
-  if (i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1) {
-    auto w = [&](int ii, int jj) { return a.weto[p3(a, ii, jj, K)]; };
-    auto aulx = [&](int ii, int jj) {
-      const double x = a.dlxu[u2(a, ii, jj)];
-      return a.aulapts * ((x * x) * (x * x));
+  const bool inner = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
+  double fw = 0., fe = 0., fn = 0., fs = 0., area = 0., z = 0.;
+  if (inner) {
+    // AULX DLYU / DLXU and AULY DLXV / DLYV of the four faces
+    auto fx = [&](int ii) {
+      const double x = a.dlxu[u2(a, ii, j)];
+      return a.aulapts * ((x * x) * (x * x)) * a.dlyu[u2(a, ii, j)] / x;
     };
-    auto auly = [&](int ii, int jj) {
-      const double y = a.dlyv[v2(a, ii, jj)];
-      return a.aulapts * ((y * y) * (y * y));
+    auto fy = [&](int jj) {
+      const double y = a.dlyv[v2(a, i, jj)];
+      return a.aulapts * ((y * y) * (y * y)) * a.dlxv[v2(a, i, jj)] / y;
     };
-    const double zzsurf = K == 1 ? 1. : 0.;
-    const double c = L1[p3(a, i, j, K)];
-    const double den = (a.ddpo[p3(a, i, j, K)] + a.almzer + zzsurf * (a.zo[p2(a, i, j)])) *
-                       a.dlxp[p2(a, i, j)] * a.dlyp[p2(a, i, j)];
-    r = t - (w(i, j) / den) * a.dzw[K - 1] *
-                (w(i - 1, j) * aulx(i - 1, j) * a.dlyu[u2(a, i - 1, j)] *
-                     (L1[p3(a, i - 1, j, K)] - c) / a.dlxu[u2(a, i - 1, j)] +
-                 w(i + 1, j) * aulx(i, j) * a.dlyu[u2(a, i, j)] * (L1[p3(a, i + 1, j, K)] - c) /
-                     a.dlxu[u2(a, i, j)] +
-                 w(i, j - 1) * auly(i, j - 1) * a.dlxv[v2(a, i, j - 1)] *
-                     (L1[p3(a, i, j - 1, K)] - c) / a.dlyv[v2(a, i, j - 1)] +
-                 w(i, j + 1) * auly(i, j) * a.dlxv[v2(a, i, j)] * (L1[p3(a, i, j + 1, K)] - c) /
-                     a.dlyv[v2(a, i, j)]);
+    fw = fx(i - 1);
+    fe = fx(i);
+    fn = fy(j - 1);
+    fs = fy(j);
+    area = a.dlxp[p2(a, i, j)] * a.dlyp[p2(a, i, j)];
+    z = a.zo[p2(a, i, j)];
   }
-  O[p3(a, i, j, K)] = r;
+  const int o0 = (int)p3(a, i, j, K0 + 1);
+#pragma unroll
+  for (int q = 0; q < kNaLevels; ++q) {
+    const int o = o0 + q * pl, K = K0 + q + 1;
+    if (K > a.KE) break;
+    const double t = T[o];
+    double r = t;
+    if (inner) {
+      const double zzsurf = K == 1 ? 1. : 0.;
+      const double c = L1[o];
+      const double den = (a.ddpo[o] + a.almzer + zzsurf * (z)) * area;
+      r = t - (a.weto[o] / den) * a.dzw[K - 1] *
+                  (a.weto[o - 1] * fw * (L1[o - 1] - c) + a.weto[o + 1] * fe * (L1[o + 1] - c) +
+                   a.weto[o - IE] * fn * (L1[o - IE] - c) + a.weto[o + IE] * fs * (L1[o + IE] - c));
+    }
+    O[o] = r;
+  }
 }
 
 // Device address of the scratch array on the current device.  The first call
@@ -243,11 +287,14 @@ extern "C" int orctm_octdiff_noalloc(const orctm_octdiff_noalloc_args* in) {
   double* lap = scratch + kNoAllocMaxCells;    // first Laplacian T1O
   NaArgs a{in->ie, in->je, in->ke, in->dt, in->almzer, in->aulapts, in->dvo, in->ddpo, in->weto,
            in->di, in->dzw, in->dlxp, in->dlyp, in->dlxu, in->dlyu, in->dlxv, in->dlyv, in->zo};
-  const dim3 bc(32, 2), b3(32, 4);
-  const dim3 gc((in->ie + 31) / 32, (in->je + 1) / 2, 1);
-  const dim3 g3((in->ie + 31) / 32, (in->je + 3) / 4, in->ke);
+  const dim3 b3(32, 4);
+  const dim3 g3((in->ie + 31) / 32, (in->je + 3) / 4, (in->ke + kNaLevels - 1) / kNaLevels);
   const bool bih = in->aulapts > in->almzer;
-  k_na_vert<<<gc, bc, 0, s>>>(a, in->tracer_in, bih ? vdiff : in->tracer_out);
+  with_tri_split(in->ke, [&](auto* l) {
+    using Ln = std::remove_pointer_t<decltype(l)>;
+    const dim3 gc((in->ie + Ln::W - 1) / Ln::W, in->je);
+    k_na_vert<Ln><<<gc, Ln::NT, 0, s>>>(a, in->tracer_in, bih ? vdiff : in->tracer_out);
+  });
   count_launch();
   if (bih) {
     k_na_lap<<<g3, b3, 0, s>>>(a, vdiff, lap);
