@@ -154,6 +154,8 @@ struct orctm_handle {
   int solver_mode = ORCTM_SOLVER_FP64;
   double rtol = 1e-10;
   int maxit = 5000;
+  double* stage = nullptr;  // uploads in their host layout (copy_field)
+  size_t stage_n = 0;
   double* b = nullptr;
   double *xs = nullptr, *r = nullptr;  // solution and outer residual
   RbGeo R{};                           // red-black view of the columns
@@ -361,22 +363,44 @@ void extent(const orctm_handle* h, int f, int& i0, int& ni, int& j0, int& nj, in
   }
 }
 
-// One copy between a field's host layout (ni x nj x nk from the first element)
-// and its padded device layout.  (A copy per level, the form before, cost the
-// host some 8 us each: 68 ms a step on 256 x 256 x 60 with every field copied
-// in and seven out, where the copies take 13 ms on the bus.)
-cudaError_t copy_field(const orctm_handle* h, double* host, const double* dev, int i0, int ni,
-                       int j0, int nj, int nk, cudaMemcpyKind kind, cudaStream_t st) {
+// Copies a field between its host layout (ni x nj x nk from the first element)
+// and its padded device layout.  To the host: one strided copy (51 GB/s on
+// 256 x 256 x 60).  To the device a strided copy runs at 17 GB/s there (rows of
+// 2 KB; 39 at 5.6 KB), a plain one at 54, so fields come through a staging buffer
+// of at most kStageBytes, a part at a time, and a kernel spreads the rows.
+constexpr size_t kStageBytes = 64u << 20;
+
+int copy_field(orctm_handle* h, double* host, const double* dev, int i0, int ni, int j0, int nj,
+               int nk, cudaMemcpyKind kind, cudaStream_t st) {
   const Layout& L = h->L;
-  const cudaPitchedPtr hp = make_cudaPitchedPtr(host, sizeof(double) * ni, ni, nj);
-  const cudaPitchedPtr dp = make_cudaPitchedPtr(const_cast<double*>(dev) + L.at(i0, j0, 0),
-                                                sizeof(double) * L.P, ni, L.JN);
-  cudaMemcpy3DParms p{};
-  p.srcPtr = kind == cudaMemcpyHostToDevice ? hp : dp;
-  p.dstPtr = kind == cudaMemcpyHostToDevice ? dp : hp;
-  p.extent = make_cudaExtent(sizeof(double) * ni, nj, nk);
-  p.kind = kind;
-  return cudaMemcpy3DAsync(&p, st);
+  double* first = const_cast<double*>(dev) + L.at(i0, j0, 0);
+  if (kind == cudaMemcpyDeviceToHost) {
+    cudaMemcpy3DParms p{};
+    p.srcPtr = make_cudaPitchedPtr(first, sizeof(double) * L.P, ni, L.JN);
+    p.dstPtr = make_cudaPitchedPtr(host, sizeof(double) * ni, ni, nj);
+    p.extent = make_cudaExtent(sizeof(double) * ni, nj, nk);
+    p.kind = kind;
+    ORCTM_CUDA_OK(cudaMemcpy3DAsync(&p, st));
+    return ORCTM_OK;
+  }
+  const size_t level = (size_t)ni * nj;
+  if (!h->stage) {  // the largest field's host layout, or the limit (one level at least)
+    const size_t all = (size_t)(L.ie + 1) * (L.je + 1) * (L.ke + 1);
+    const size_t one = (size_t)(L.ie + 1) * (L.je + 1);
+    h->stage_n = std::max(one, std::min(all, kStageBytes / sizeof(double)));
+    int s2;
+    if ((s2 = h->dev_alloc(&h->stage, h->stage_n))) return s2;
+    // allocated and cleared on the compute stream; the copies may run on the other
+    ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
+  }
+  const int per = (int)std::min<size_t>(nk, h->stage_n / level);
+  for (int k = 0; k < nk; k += per) {
+    const int n = std::min(per, nk - k), rows = n * nj;
+    ORCTM_CUDA_OK(cudaMemcpyAsync(h->stage, host + level * k, sizeof(double) * level * n, kind, st));
+    launch_unpack(h->stage, first + (size_t)L.plane * k, ni, nj, rows, L.P, L.plane, st);
+    ORCTM_CUDA_OK(cudaGetLastError());
+  }
+  return ORCTM_OK;
 }
 
 // Geometry checks and compression -------------------------------------------
@@ -978,7 +1002,10 @@ int download_async(orctm_handle* h, int f, double* host) {
   extent(h, f, i0, ni, j0, nj, nk);
   double* src = f == ORCTM_F_ZO ? h->zo : h->slot[f];
   if ((st = copy_after_compute(h))) return st;
-  ORCTM_CUDA_OK(copy_field(h, host, src, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->cstream));
+  {
+    const int sc = copy_field(h, host, src, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->cstream);
+    if (sc) return sc;
+  }
   // routines never write a buffer in place, and a referenced buffer is never
   // handed out again: holding a reference keeps the source intact until the
   // copy has ended
@@ -1357,7 +1384,10 @@ int orctm_upload(orctm_handle* h, int f, const double* host, size_t n) {
     }
     dst = h->slot[f];
   }
-  ORCTM_CUDA_OK(copy_field(h, const_cast<double*>(host), dst, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->stream));
+  {
+    const int sc = copy_field(h, const_cast<double*>(host), dst, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->stream);
+    if (sc) return sc;
+  }
   ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
   return ORCTM_OK;
 }
@@ -1373,7 +1403,10 @@ int orctm_download(orctm_handle* h, int f, double* host, size_t n) {
   int i0, ni, j0, nj, nk;
   extent(h, f, i0, ni, j0, nj, nk);
   const double* src = f == ORCTM_F_ZO ? h->zo : h->slot[f];
-  ORCTM_CUDA_OK(copy_field(h, host, src, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->stream));
+  {
+    const int sc = copy_field(h, host, src, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->stream);
+    if (sc) return sc;
+  }
   ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
   return ORCTM_OK;
 }
@@ -1398,7 +1431,10 @@ int orctm_upload_async(orctm_handle* h, int f, const double* host, size_t n) {
   // after the kernels queued so far (which may still read the old contents)
   // and after the allocation above, which is ordered on the compute stream
   if ((st = copy_after_compute(h))) return st;
-  ORCTM_CUDA_OK(copy_field(h, const_cast<double*>(host), dst, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->cstream));
+  {
+    const int sc = copy_field(h, const_cast<double*>(host), dst, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->cstream);
+    if (sc) return sc;
+  }
   if (!h->field_ready[f]) ORCTM_CUDA_OK(cudaEventCreateWithFlags(&h->field_ready[f], cudaEventDisableTiming));
   ORCTM_CUDA_OK(cudaEventRecord(h->field_ready[f], h->cstream));
   h->pending[f] = true;
@@ -2384,7 +2420,10 @@ int orctm_upload_baroclinic(orctm_handle* h, int which, const double* host, size
   if ((st = baroclinic_array(h, which, &p, &i0, &ni, &j0, &nj, &nk))) return st;
   if (!host || n != (size_t)ni * nj * nk) return h->fail(ORCTM_E_ARG, "orctm_upload_baroclinic: size");
   if ((st = compute_after_copies(h))) return st;
-  ORCTM_CUDA_OK(copy_field(h, const_cast<double*>(host), p, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->stream));
+  {
+    const int sc = copy_field(h, const_cast<double*>(host), p, i0, ni, j0, nj, nk, cudaMemcpyHostToDevice, h->stream);
+    if (sc) return sc;
+  }
   ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
   return ORCTM_OK;
 }
@@ -2396,7 +2435,10 @@ int orctm_download_baroclinic(orctm_handle* h, int which, double* host, size_t n
   int i0, ni, j0, nj, nk, st;
   if ((st = baroclinic_array(h, which, &p, &i0, &ni, &j0, &nj, &nk))) return st;
   if (!host || n != (size_t)ni * nj * nk) return h->fail(ORCTM_E_ARG, "orctm_download_baroclinic: size");
-  ORCTM_CUDA_OK(copy_field(h, host, p, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->stream));
+  {
+    const int sc = copy_field(h, host, p, i0, ni, j0, nj, nk, cudaMemcpyDeviceToHost, h->stream);
+    if (sc) return sc;
+  }
   ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
   return ORCTM_OK;
 }
@@ -2563,7 +2605,7 @@ int orctm_estimate_device_bytes(const orctm_desc* d, int solver, unsigned long l
   // FP64 solver vectors, and the 7 half-length vectors of the reduced system
   // and its pivots (in FP64, and for the refined solver in FP32 too: a handle
   // that has solved in both forms holds both)
-  const double tmp = std::max(8.0, 2.0 * d->ntracers + 2.0) + 3.0;  // + the held transports
+  const double tmp = std::max(8.0, 2.0 * d->ntracers + 2.0) + 3.0 + 1.0;  // + the held transports, the staging
   const double m32 = ((d->ie - 1) / 2 + 31) / 32 * 32;  // FP32 tiles hold 32 columns
   const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 4.25 +
                     (solver == ORCTM_SOLVER_FP32_REFINED ? 2.25 * std::max(1.0, 2.0 * m32 / P) : 0.0);

@@ -155,4 +155,29 @@ void launch_nh_post(const Geo& G, const double* x, const double* pold, double* p
   count_launch();
 }
 
+namespace {
+// Rows of a field from consecutive memory to the padded layout; one thread per
+// element of kUnpackRows rows.
+constexpr int kUnpackRows = 8;
+__global__ void __launch_bounds__(128) k_unpack(const double* __restrict__ src,
+                                                double* __restrict__ dst, int ni, int nj, int rows,
+                                                int P, int plane) {
+  const int i = blockIdx.y * 128 + threadIdx.x;
+  if (i >= ni) return;
+#pragma unroll
+  for (int q = 0; q < kUnpackRows; ++q) {
+    const int row = blockIdx.x * kUnpackRows + q;  // of all levels
+    if (row >= rows) return;
+    dst[i + P * (row % nj) + plane * (row / nj)] = src[(size_t)row * ni + i];
+  }
+}
+}  // namespace
+
+void launch_unpack(const double* src, double* dst, int ni, int nj, int rows, int P, int plane,
+                   cudaStream_t st) {
+  const dim3 grid((rows + kUnpackRows - 1) / kUnpackRows, (ni + 127) / 128);
+  k_unpack<<<grid, 128, 0, st>>>(src, dst, ni, nj, rows, P, plane);
+  count_launch();
+}
+
 }  // namespace orctm

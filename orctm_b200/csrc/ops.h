@@ -197,6 +197,9 @@ void launch_obc_ts(const Geo& G, const ObcArgs& a, double* tracer, cudaStream_t 
 void launch_nh_rhs(const Geo& G, const double* uoo, const double* uoo1, const double* voe,
                    const double* voe1, const double* wno, const double* wno1, const double* zo,
                    double* b, cudaStream_t st);
+// rows (of all levels, nj per level) of ni values each to the padded layout
+void launch_unpack(const double* src, double* dst, int ni, int nj, int rows, int P, int plane,
+                   cudaStream_t st);
 // poisson.cu
 // elements of a vector of the reduced system, and the red-black tables and
 // pivots of a precision (once per handle and precision)
