@@ -881,7 +881,11 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   // pass maxit, with no host round trip in between; the iterations left before
   // maxit, and all of them while profiling, one by one
   int it = 0, conv = 0;
-  if (!h->prof && maxit >= kPcgChunk) {
+  if (!h->prof && launch_rb_small<T>(h->R, h->S, v, maxit, h->stream)) {
+    if ((st = read_state(h))) return st;
+    it = h->hS->iter;
+    conv = h->hS->converged;
+  } else if (!h->prof && maxit >= kPcgChunk) {
     cudaGraphExec_t ex;
     if ((st = pcg_loop_graph<T>(h, &ex))) return st;
     launch_set_limit(h->S, maxit, h->stream);

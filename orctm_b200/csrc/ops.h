@@ -54,6 +54,7 @@ struct SolverState {
   int iter;
   int limit;      // iteration limit of the device-side loop (orctm handle's maxit)
   unsigned ticket;
+  unsigned gbar;  // arrivals at the barriers of the one-kernel loop
   int max_blocks;    // partial sums per quantity: the most tiles of a kernel
   double* partials;  // [4 * max_blocks]
 };
@@ -221,6 +222,9 @@ template <typename T>
 void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 template <typename T>
 void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
+// the whole loop in one kernel, on small grids; false: not launched
+template <typename T>
+bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit, cudaStream_t st);
 template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x, cudaStream_t st);
 // r = b - A x in double-double, and x := 0 on land rows (their solution)

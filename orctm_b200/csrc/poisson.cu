@@ -828,6 +828,275 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
   }
 }
 
+// ------------------------------------------------------- small grids -----
+// The whole PCG loop in one cooperative kernel, a block per tile: the block keeps
+// its red and its black tile in shared memory from the first iteration to the
+// last, and only u and z go through L2, to the neighbouring tiles.  The three
+// kernels of an iteration cost some 10 us each on such grids whatever the
+// work (launch, first loads, last block's sum); here a phase ends with a grid-wide barrier that also carries
+// its dot products.  The arithmetic and the order of the sums are those of
+// the three kernels with a block per tile.  Waits are bounded by a clock budget
+// (converged = 4).
+struct GridSync {
+  SolverState* S;
+  unsigned target;
+  bool ok;
+};
+
+// All blocks' values added in block order, the same total for every thread of
+// the grid (NV = 0: the barrier alone).
+template <int NV, int NT>
+__device__ __forceinline__ void grid_all(double (&v)[NV ? NV : 1], GridSync& g, int slot) {
+  constexpr int kWarps = NT / 32;
+  __shared__ double sh[NV ? NV : 1][kWarps];
+  __shared__ bool up;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  SolverState* S = g.S;
+  auto block_sum = [&]() {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double x = v[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) sh[q][warp] = x;
+    }
+    __syncthreads();
+  };
+  block_sum();
+  g.target += gridDim.x;
+  if (tid == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      double x = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) x += sh[q][w];
+      S->partials[(size_t)(slot + q) * S->max_blocks + blockIdx.x] = x;
+    }
+    __threadfence();
+    atomicAdd(&S->gbar, 1u);
+    const long long t0 = clock64();
+    bool there = false;
+    while (!there) {
+      unsigned n;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(n) : "l"(&S->gbar) : "memory");
+      there = (int)(n - g.target) >= 0;
+      if (!there && clock64() - t0 > kWaitCycles) break;
+    }
+    up = there;
+  }
+  __syncthreads();
+  g.ok = up;
+  if constexpr (NV == 0) return;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const double* part = S->partials + (size_t)(slot + q) * S->max_blocks;
+    double x = 0.0;
+#pragma unroll 4
+    for (int b = tid; b < (int)gridDim.x; b += NT) x += __ldcg(part + b);
+    v[q] = x;
+  }
+  block_sum();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    double x = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) x += sh[q][w];
+    v[q] = x;
+  }
+  __syncthreads();
+}
+
+template <typename Ln>
+constexpr size_t small_smem() {
+  return (size_t)Ln::ROWS * Ln::W * (sizeof(typename Ln::V) * 6 + sizeof(float));
+}
+
+template <typename Ln, typename T = typename Ln::V>
+__global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 : 3))
+    k_rb_small(RbGeo R, SolverState* S, RbVectors<T> vec,
+                                                     int ntiles, int nt, int maxit) {
+  constexpr int W = Ln::W, LC = Ln::L, N = Ln::ROWS * W;
+  extern __shared__ __align__(128) unsigned char dsm[];
+  __shared__ T szw[Ln::ROWS + 1], siz[Ln::ROWS + 1];
+  __shared__ Scan<Ln> scan;
+  T* zt = reinterpret_cast<T*>(dsm);  // z, u, p: the tile as its neighbouring threads see it
+  T *ut = zt + N, *ps = ut + N, *xs = ps + N, *rs = xs + N, *ds = rs + N;
+  float* db = reinterpret_cast<float*>(ds + N);
+  if (S->converged) return;
+  const Ln t;
+  const Tiles<Ln> reds{R, R.col[0], t, ntiles, nt, true}, blacks{R, R.col[1], t, ntiles, nt, false};
+  const Tile a = reds.at(blockIdx.x, reds.kk(blockIdx.x));
+  const Tile k = blacks.at(blockIdx.x, blacks.kk(blockIdx.x));
+  load_tables<Ln>(R, szw, siz);
+  const int row = nt * R.ke * W;
+  const int me = t.K0 * W + t.c;
+  const int kba = wet_levels(a.kk, 0), kbk = wet_levels(k.kk, 0);
+  auto s2 = [&](const Tile& q) { return q.kk ? q.m + R.P2 * q.j : 0; };
+  const double2 we0 = R.col[0].we[s2(a)], ns0 = R.col[0].ns[s2(a)], iz0 = R.col[0].iz[s2(a)];
+  const double2 we1 = R.col[1].we[s2(k)], ns1 = R.col[1].ns[s2(k)], iz1 = R.col[1].iz[s2(k)];
+  const T zwa0 = kba ? (T)R.col[0].zw[s2(a)].x : T(0);
+  const double2 zw1 = R.col[1].zw[s2(k)];
+  const T zwa1 = kbk ? (T)zw1.x : T(0);
+#pragma unroll
+  for (int q = 0; q < LC; ++q) {
+    const int K = t.K0 + 1 + q, o = me + W * q;
+    zt[o] = K <= kbk ? vec.z[k.o0 + W * q] : T(0);
+    rs[o] = K <= kbk ? vec.r[k.o0 + W * q] : T(0);
+    db[o] = K <= kbk ? vec.db[k.o0 + W * q] : 0.f;
+    ds[o] = K <= kba ? vec.dr[a.o0 + W * q] : T(0);
+    ut[o] = ps[o] = xs[o] = T(0);
+  }
+  __syncthreads();
+  // C v of the thread's levels without 1/ZP: the tile itself from shared memory,
+  // its neighbours' tiles from L2 (written by other blocks before the last barrier)
+  auto neighbours = [&](const Tile& q, int kb, const T* tile, const T* all, double2 we, double2 ns,
+                        T (&h)[LC]) {
+    const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y;
+    const T co = q.sh ? cw : ce, cx = q.sh ? ce : cw;
+    const bool across = t.c == (q.sh ? W - 1 : 0);
+    const int cc = (q.sh ? min(t.c + 1, W - 1) : max(t.c - 1, 0)) - t.c;
+    const int ko = across && (q.sh ? q.b + 1 < nt : q.b > 0) ? kb : 0;
+    const int oo = q.o0 + (q.sh ? R.ke * W - (W - 1) : (W - 1) - R.ke * W);
+    const int kn = min(kb, wet_levels(q.kk, 3)), ks = min(kb, wet_levels(q.kk, 4));
+    T vn[LC], vs[LC], vo[LC];
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      const int K = t.K0 + 1 + e;
+      vn[e] = K <= kn ? __ldcg(all + q.o0 - row + W * e) : T(0);
+      vs[e] = K <= ks ? __ldcg(all + q.o0 + row + W * e) : T(0);
+      vo[e] = K <= ko ? __ldcg(all + oo + W * e) : T(0);
+    }
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      h[e] = co * tile[me + W * e];
+      const T x = across ? vo[e] : tile[me + W * e + cc];
+      h[e] = fma(cx, x, h[e]);
+      h[e] = fma(cn, vn[e], h[e]);
+      h[e] = fma(cs, vs[e], h[e]);
+      if (t.K0 + 1 + e > kb) h[e] = T(0);
+    }
+  };
+  GridSync g{S, 0u, true};
+  double rho = S->rho, rr = S->rr, alpha = 0.0, beta = 0.0;
+  const double tol = S->tol, bb = S->bb;
+  int iter = 0, conv = 0;
+  while (!conv && iter < maxit) {
+    // ---- red: u = D^-1 C z + beta u
+    T h[LC], d[LC], cp[LC + 1];
+    neighbours(a, kba, zt, vec.z, we0, ns0, h);
+#pragma unroll
+    for (int q = 0; q < LC; ++q) {
+      const int K = t.K0 + 1 + q;
+      h[q] *= K == kba ? (T)iz0.y : (K == kba - 1 ? (T)iz0.x : siz[t.K0 + q]);
+      d[q] = ds[me + W * q];
+    }
+    T dm = t.K0 > 0 ? ds[me - W] : T(0);
+    couplings(t, szw, kba, zwa0, cp);
+    column_solve(t, scan, h, d, dm, cp, [] {});
+#pragma unroll
+    for (int q = 0; q < LC; ++q)
+      if (t.K0 + 1 + q <= kba) {
+        const T u = beta != 0.0 ? fma((T)beta, ut[me + W * q], h[q]) : h[q];
+        ut[me + W * q] = u;
+        vec.u[a.o0 + W * q] = u;
+      }
+    // ---- black: x += alpha p, p = z + beta p (both of this block alone)
+#pragma unroll
+    for (int q = 0; q < LC; ++q) {
+      const int o = me + W * q;
+      const T po = ps[o];
+      xs[o] = fma((T)alpha, po, xs[o]);
+      ps[o] = fma((T)beta, po, zt[o]);
+    }
+    double none[1];
+    grid_all<0, Ln::NT>(none, g, 0);
+    if (!g.ok) break;
+    // q = D p - C u
+    neighbours(k, kbk, ut, vec.u, we1, ns1, h);
+    T qv[LC], pqt = T(0);
+    {
+      const T cw = (T)we1.x, ce = (T)we1.y, cn = (T)ns1.x, cs = (T)ns1.y;
+      const int kbw = wet_levels(k.kk, 1), kbe = wet_levels(k.kk, 2);
+      const int kbn = wet_levels(k.kk, 3), kbs = wet_levels(k.kk, 4);
+      T pu = t.K0 > 0 ? ps[me - W] : T(0);
+      const T pb = t.g < Ln::GROUPS - 1 ? ps[me + W * LC] : T(0);
+#pragma unroll
+      for (int e = 0; e < LC; ++e) {
+        const int K = t.K0 + 1 + e;
+        const T p0 = ps[me + W * e], pd = e + 1 < LC ? ps[me + W * (e + 1)] : pb;
+        T dh = K <= kbw ? cw : T(0);
+        dh += K <= kbe ? ce : T(0);
+        dh += K <= kbn ? cn : T(0);
+        dh += K <= kbs ? cs : T(0);
+        const T hh = fma(dh, p0, h[e]);
+        const T hs = K == kbk ? (T)iz1.y : (K == kbk - 1 ? (T)iz1.x : siz[t.K0 + e]);
+        const T zw0 = K == kbk ? zwa1 : szw[t.K0 + e];
+        T zwn = K + 1 == kbk ? zwa1 : szw[t.K0 + e + 1];
+        if (K == kbk) zwn = K == 1 ? (T)zw1.y : T(0);
+        T s = zw0 * (pu - p0);
+        s = fma(zwn, pd - p0, s);
+        s = fma(-hs, hh, s);
+        qv[e] = K <= kbk ? s : T(0);
+        if (K <= kbk) pqt = fma(p0, s, pqt);
+        pu = p0;
+      }
+    }
+    double w1[1] = {(double)pqt};
+    grid_all<1, Ln::NT>(w1, g, 0);
+    if (!g.ok) break;
+    alpha = rho / w1[0];
+    if (!(w1[0] > 0.0) && !(w1[0] < 0.0)) {
+      conv = 3;
+      alpha = 0.0;  // breakdown: x keeps the last full step
+      break;
+    }
+    // ---- column: r -= alpha q, z = D^-1 r
+    T rrt = T(0);
+#pragma unroll
+    for (int e = 0; e < LC; ++e) {
+      h[e] = fma(-(T)alpha, qv[e], rs[me + W * e]);
+      rs[me + W * e] = h[e];
+      rrt = fma(h[e], h[e], rrt);
+      d[e] = (T)db[me + W * e];
+    }
+    dm = t.K0 > 0 ? (T)db[me - W] : T(0);
+    couplings(t, szw, kbk, zwa1, cp);
+    const T rz = column_solve(t, scan, h, d, dm, cp, [] {});
+#pragma unroll
+    for (int e = 0; e < LC; ++e)
+      if (t.K0 + 1 + e <= kbk) {
+        zt[me + W * e] = h[e];
+        vec.z[k.o0 + W * e] = h[e];
+      }
+    double w2[2] = {(double)rz, (double)rrt};
+    grid_all<2, Ln::NT>(w2, g, 1);
+    if (!g.ok) break;
+    beta = w2[0] / rho;
+    rho = w2[0];
+    rr = w2[1];
+    ++iter;
+    if (sqrt(rr) <= tol * sqrt(bb)) conv = 1;
+    if (!(rho == rho) || !(rr == rr)) conv = 2;  // NaN: stop
+  }
+  if (!g.ok) conv = 4;
+  // x without its last update, which k_rb_after makes with p and alpha_prev
+#pragma unroll
+  for (int q = 0; q < LC; ++q)
+    if (t.K0 + 1 + q <= kbk) {
+      vec.x[k.o0 + W * q] = xs[me + W * q];
+      vec.p[k.o0 + W * q] = ps[me + W * q];
+    }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    S->iter = iter;
+    S->rho = rho;
+    S->rr = rr;
+    S->beta = beta;
+    S->alpha_prev = alpha;
+    if (conv != 4) S->converged = conv;
+  }
+  if (conv == 4 && threadIdx.x == 0) atomicExch(&S->converged, 4);
+}
+
 // The black correction: the x update that the last iteration left open (none
 // before the first), and its addition to the solution (full layout).
 template <typename T>
@@ -947,6 +1216,7 @@ __global__ void k_reset(SolverState* S, double tol) {
   S->converged = 0;
   S->iter = 0;
   S->ticket = 0;
+  S->gbar = 0;
   S->tol = tol;
   S->beta = 0.0;
   S->alpha_prev = 0.0;
@@ -1085,7 +1355,33 @@ void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, doub
   add_launches(2);
 }
 
+// Whether the grid is small enough for k_rb_small (a tile per resident block, and
+// columns of up to 104 levels: one shape of block), which it then launches.
+template <typename T>
+bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit,
+                     cudaStream_t st) {
+  bool done = false;
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    if constexpr (L::GROUPS == 8) {
+      constexpr size_t m = small_smem<L>();
+      const Shape s = shape_of<k_rb_small<L>, L>(R, m);
+      if (s.grid < s.ntiles) return;
+      RbGeo r = R;
+      RbVectors<T> vec = v;
+      int ntiles = s.ntiles, nt = s.nt;
+      void* args[] = {&r, &S, &vec, &ntiles, &nt, &maxit};
+      done = cudaLaunchCooperativeKernel((const void*)&k_rb_small<L>, dim3(s.grid), dim3(L::NT), args,
+                                         m, st) == cudaSuccess;
+      if (done) count_launch();
+      else (void)cudaGetLastError();  // the three kernels take its place
+    }
+  });
+  return done;
+}
+
 #define ORCTM_RB(T)                                                                              \
+  template bool launch_rb_small<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
   template void launch_rb_setup<T>(const Geo&, const PoissonGeo&, const RbGeo&, const RbVectors<T>&, \
                                    cudaStream_t);                                                \
   template void launch_rb_before<T>(const RbGeo&, SolverState*, const double*, const RbVectors<T>&, \
