@@ -1034,16 +1034,15 @@ int r_ocadpo(orctm_handle* h, int n) {
   int st;
   if ((st = wait_uploads(h, {ORCTM_F_THO + n, ORCTM_F_UKO, ORCTM_F_VKE, ORCTM_F_WO, ORCTM_F_ZO})))
     return st;
-  double *out, *tA, *vA, *vB;
-  if ((st = h->alloc(&out)) || (st = h->alloc(&tA)) || (st = h->alloc(&vA)) || (st = h->alloc(&vB)))
-    return st;
+  double *out, *mid, *vol;
+  if ((st = h->alloc(&out)) || (st = h->alloc(&mid)) || (st = h->alloc(&vol))) return st;
   const int f = ORCTM_F_THO + n;
   PROF(h, ORCTM_PROF_OCADPO,
        launch_ocadpo(h->G, h->slot[f], h->slot[ORCTM_F_UKO], h->slot[ORCTM_F_VKE],
-                     h->slot[ORCTM_F_WO], h->zo, out, tA, vA, vB, h->stream));
+                     h->slot[ORCTM_F_WO], h->zo, out, mid, vol, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   h->bind(f, out);
-  h->unref(tA); h->unref(vA); h->unref(vB);
+  h->unref(mid); h->unref(vol);
   return ORCTM_OK;
 }
 
@@ -1063,22 +1062,21 @@ int r_ocadpo_all(orctm_handle* h, const double* uko = nullptr, const double* vke
     vke = h->slot[ORCTM_F_VKE];
     wo = h->slot[ORCTM_F_WO];
   }
-  double *out[kMaxTracers] = {}, *mid[kMaxTracers] = {}, *vA = nullptr, *vB = nullptr;
+  double *out[kMaxTracers] = {}, *mid[kMaxTracers] = {}, *vol = nullptr;
   const double* in[kMaxTracers] = {};
   for (int n = 0; n < ntr; ++n) {
     if ((st = h->alloc(&out[n])) || (st = h->alloc(&mid[n]))) return st;
     in[n] = h->slot[ORCTM_F_THO + n];
   }
-  if ((st = h->alloc(&vA)) || (st = h->alloc(&vB))) return st;
+  if ((st = h->alloc(&vol))) return st;
   PROF(h, ORCTM_PROF_OCADPO,
-       launch_ocadpo_all(h->G, ntr, in, out, mid, uko, vke, wo, h->zo, vA, vB, h->stream));
+       launch_ocadpo_all(h->G, ntr, in, out, mid, uko, vke, wo, h->zo, vol, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   for (int n = 0; n < ntr; ++n) {
     h->bind(ORCTM_F_THO + n, out[n]);
     h->unref(mid[n]);
   }
-  h->unref(vA);
-  h->unref(vB);
+  h->unref(vol);
   return ORCTM_OK;
 }
 
@@ -1090,24 +1088,23 @@ int r_momadv(orctm_handle* h) {
     if (st0) return st0;
   }
   int st;
-  double *out, *tA, *vA, *vB;
-  if ((st = h->alloc(&out)) || (st = h->alloc(&tA)) || (st = h->alloc(&vA)) || (st = h->alloc(&vB)))
-    return st;
+  double *out, *mid, *vol;
+  if ((st = h->alloc(&out)) || (st = h->alloc(&mid)) || (st = h->alloc(&vol))) return st;
   const double *uko = h->slot[ORCTM_F_UKO], *vke = h->slot[ORCTM_F_VKE], *wo = h->slot[ORCTM_F_WO];
   int f;
   if (WHICH == 0) {
     f = ORCTM_F_UOO;
-    PROF(h, ORCTM_PROF_OCUAD, launch_ocuad(h->G, h->slot[f], uko, vke, wo, out, tA, vA, vB, h->stream));
+    PROF(h, ORCTM_PROF_OCUAD, launch_ocuad(h->G, h->slot[f], uko, vke, wo, out, mid, vol, h->stream));
   } else if (WHICH == 1) {
     f = ORCTM_F_VOE;
-    PROF(h, ORCTM_PROF_OCVAD, launch_ocvad(h->G, h->slot[f], uko, vke, wo, out, tA, vA, vB, h->stream));
+    PROF(h, ORCTM_PROF_OCVAD, launch_ocvad(h->G, h->slot[f], uko, vke, wo, out, mid, vol, h->stream));
   } else {
     f = ORCTM_F_WNO;
-    PROF(h, ORCTM_PROF_OCWAD, launch_ocwad(h->G, h->slot[f], uko, vke, wo, h->zo, out, tA, vA, vB, h->stream));
+    PROF(h, ORCTM_PROF_OCWAD, launch_ocwad(h->G, h->slot[f], uko, vke, wo, h->zo, out, mid, vol, h->stream));
   }
   ORCTM_CUDA_OK(cudaGetLastError());
   h->bind(f, out);
-  h->unref(tA); h->unref(vA); h->unref(vB);
+  h->unref(mid); h->unref(vol);
   return ORCTM_OK;
 }
 

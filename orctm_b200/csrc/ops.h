@@ -153,26 +153,22 @@ void launch_occlit(const Geo& G, const BaroArgs& b, const ThermoFields& f, const
                    double* uko, double* vke, double* uk1o, double* vk1e, double* wo, double* wpo,
                    double* t1o, double* bruva, double* contrij, double* contra, cudaStream_t st);
 
-// advect.cu
+// advect.cu: mid and vol are scratch fields
 void launch_ocadpo(const Geo& G, const double* T, const double* uko, const double* vke,
-                   const double* wo, const double* zo, double* out, double* tA, double* vA,
-                   double* vB, cudaStream_t st);
+                   const double* wo, const double* zo, double* out, double* mid, double* vol,
+                   cudaStream_t st);
 // OCADPO for ntr tracers at once (shared transports and volumes); equals
 // ntr launch_ocadpo calls bit for bit
 void launch_ocadpo_all(const Geo& G, int ntr, const double* const* T, double* const* out,
                        double* const* mid, const double* uko, const double* vke,
-                       const double* wo, const double* zo, double* vA, double* vB,
-                       cudaStream_t st);
-int adpo_max_fused();
+                       const double* wo, const double* zo, double* vol, cudaStream_t st);
 void launch_ocuad(const Geo& G, const double* T, const double* uko, const double* vke,
-                  const double* wo, double* out, double* tA, double* vA, double* vB,
-                  cudaStream_t st);
+                  const double* wo, double* out, double* mid, double* vol, cudaStream_t st);
 void launch_ocvad(const Geo& G, const double* T, const double* uko, const double* vke,
-                  const double* wo, double* out, double* tA, double* vA, double* vB,
-                  cudaStream_t st);
+                  const double* wo, double* out, double* mid, double* vol, cudaStream_t st);
 void launch_ocwad(const Geo& G, const double* T, const double* uko, const double* vke,
-                  const double* wo, const double* zo, double* out, double* tA, double* vA,
-                  double* vB, cudaStream_t st);
+                  const double* wo, const double* zo, double* out, double* mid, double* vol,
+                  cudaStream_t st);
 
 // diffuse.cu
 void launch_octdiff_vert(const Geo& G, int ntr, const double* const* in, double* const* out,
