@@ -81,15 +81,25 @@ __device__ __forceinline__ Fl<N> zero_fl() {
 
 // The limited upwind pair: TRP takes the average with ta, TRM with tb; SCHA is
 // multiplied by the masks' product w (0 or 1), SCH capped by cap, and 0 with
-// flat.  (ocadpo.f90:107-125, 203-232; ocuad.f90:41-52 without masks)
+// flat.  (ocadpo.f90:107-125, 203-232; ocuad.f90:41-52 without masks)  Where a
+// factor makes the result 0 (no outflow: land; SCHA = 0: a uniform field, a
+// local extremum) the steps it makes idle are passed by, which a whole warp often can.
 __device__ __forceinline__ void limited(double up, double um, double t, double ta, double tb,
-                                        double vol, double cap, double w, bool flat, double& trp,
+                                        double vol, double cap, bool w, bool flat, double& trp,
                                         double& trm) {
-  const double abl = fabs(ta - tb);
-  const double zwabl = fabs(ta + tb - 2. * t);
-  const double scha = fmx(0., div_nr(abl - zwabl, abl + 1.E-20)) * w;
-  double sch = fmn(cap, div_nr(scha * vol, up + um + 1.E-20));
-  if (flat) sch = 0.;
+  trp = trm = 0.;
+  const double out = up + um;
+  if (out == 0.) return;
+  double sch = 0.;
+  if (w && !flat) {
+    const double abl = fabs(ta - tb);
+    const double zwabl = fabs(ta + tb - 2. * t);
+    const double num = abl - zwabl;
+    if (!(num <= 0.)) {
+      const double scha = fmx(0., div_in_range(num, abl + 1.E-20));
+      sch = fmn(cap, div_in_range(scha * vol, out + 1.E-20));
+    }
+  }
   const double schi = 1. - sch;
   trp = up * (schi * t + sch * 0.5 * (t + ta));
   trm = um * (schi * t + sch * 0.5 * (t + tb));
@@ -132,7 +142,7 @@ __global__ void __launch_bounds__(32 * kZxRows)
   const ColGeo& cg = cell_columns<VAR>(G);
   const int kb = cell ? cg.kb[ij] : 0;
   const double bot = cell ? cg.bot[ij] : 0.;
-  auto thick_c = [&](int K) { return K < kb ? G.dzw[K - 1] : (K == kb ? bot : 0.0); };
+  auto thick_c = [&](int K) { return K < kb ? __ldg(G.dzw + K - 1) : (K == kb ? bot : 0.0); };
 
   // ---- z: metrics, volumes, interface velocity ww(K) between levels K - 1 and K
   const bool zin = cell && i >= R::iL && i <= IE - 1 && j >= R::jL && j <= JE - 1;
@@ -175,10 +185,10 @@ __global__ void __launch_bounds__(32 * kZxRows)
   const bool uin = i >= 0 && i <= IE && xrow;           // u-points that may be read
   const int kbu = uin ? G.gu.kb[ij] : 0;
   const double botu = uin ? G.gu.bot[ij] : 0.;
-  auto thick_u = [&](int K) { return K < kbu ? G.dzw[K - 1] : (K == kbu ? botu : 0.0); };
+  auto thick_u = [&](int K) { return K < kbu ? __ldg(G.dzw + K - 1) : (K == kbu ? botu : 0.0); };
   const int kbu2 = VAR == V_VAD && uin ? G.gu.kb[ij + G.L.P] : 0;
   const double botu2 = VAR == V_VAD && uin ? G.gu.bot[ij + G.L.P] : 0.;
-  auto thick_u2 = [&](int K) { return K < kbu2 ? G.dzw[K - 1] : (K == kbu2 ? botu2 : 0.0); };
+  auto thick_u2 = [&](int K) { return K < kbu2 ? __ldg(G.dzw + K - 1) : (K == kbu2 ? botu2 : 0.0); };
   const double hdt = 0.5 * G.dt;
   double cup = 0., cum = 0.;  // factors of the eastward and the westward transport
   bool flux_here, edge = false;
@@ -231,7 +241,7 @@ __global__ void __launch_bounds__(32 * kZxRows)
     const bool flat = VAR == V_ADPO && (K == 1 || K == KE);
 #pragma unroll
     for (int n = 0; n < N; ++n)
-      limited(f.wtp, f.wtm, c[n], a[n], b[n], vol, cap, 1., flat, f.trp[n], f.trm[n]);
+      limited(f.wtp, f.wtm, c[n], a[n], b[n], vol, cap, true, flat, f.trp[n], f.trm[n]);
     return f;
   };
   // transports of the level above the first and below the last one of WAD
@@ -340,7 +350,7 @@ __global__ void __launch_bounds__(32 * kZxRows)
     const bool live = flux_here && K >= R::kL && K <= KE;
     if (!live) up = um = 0.;
     const double wtp_w = from_west(up), wtm_e = from_east(um);
-    const double w3 = VAR == V_ADPO || VAR == V_WAD ? (K <= kb3 ? 1. : 0.) : 1.;
+    const bool w3 = VAR == V_ADPO || VAR == V_WAD ? K <= kb3 : true;
     const bool upd = xup && K >= R::kL && K <= KE && K <= kb;
     double v2 = v1;
 #pragma unroll
@@ -458,7 +468,7 @@ __global__ void __launch_bounds__(32 * kYLevels)
         f.trp[n] = f.wtp * t[n];
         f.trm[n] = f.wtm * t[n];
       } else {
-        limited(f.wtp, f.wtm, t[n], tb[n], ta[n], vol, 1., masked ? (w3 ? 1. : 0.) : 1., false,
+        limited(f.wtp, f.wtm, t[n], tb[n], ta[n], vol, 1., masked ? w3 : true, false,
                 f.trp[n], f.trm[n]);
       }
     }

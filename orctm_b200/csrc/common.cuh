@@ -88,10 +88,12 @@ __device__ __forceinline__ bool wetb(const ColGeo& c, int ij, int K) { return K 
 // System/6000 processor", IBM J. Res. Develop. 34 (1990) 111-119).  The
 // result is within 1 ulp of the correctly rounded quotient (checked against
 // IEEE division by orctm_check_division).  Denominators that are zero,
-// subnormal, infinite or NaN take the IEEE division.
-__device__ __forceinline__ double div_nr(double a, double b) {
-  const double ab = fabs(b);
-  if (!(ab >= 1e-300 && ab <= 1e300)) return a / b;
+// subnormal, infinite, NaN or near the ends of the range take the IEEE division.
+static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+
+// the refinement alone, for denominators known to be no smaller than 1e-290
+// (up to 1e300; an infinity or NaN gives NaN, as a quotient of infinities does)
+__device__ __forceinline__ double div_in_range(double a, double b) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
   double e = __fma_rn(-b, r, 1.0);
@@ -100,6 +102,14 @@ __device__ __forceinline__ double div_nr(double a, double b) {
   r = __fma_rn(r, e, r);
   const double q = a * r;
   return __fma_rn(r, __fma_rn(-b, q, a), q);
+}
+
+__device__ __forceinline__ double div_nr(double a, double b) {
+  // exponent between -991 and 992, by the integer pipe: the double-precision
+  // comparisons cost as much as the refinement's steps
+  const unsigned e = ((unsigned)__double2hiint(b) & 0x7ff00000u) - (32u << 20);
+  if (e > (1983u << 20)) return div_ieee(a, b);
+  return div_in_range(a, b);
 }
 
 // Fortran MAX/MIN for non-NaN operands, evaluated exactly as the oracle does.
