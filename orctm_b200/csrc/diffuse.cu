@@ -577,197 +577,217 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
   }
 }
 
-__device__ __forceinline__ double rdlypsi(const Geo& G, int i, int j) { return G.rdlypsi[G.L.at2(i, j)]; }
-__device__ __forceinline__ double rdlxpsi(const Geo& G, int i, int j) { return G.rdlxpsi[G.L.at2(i, j)]; }
+// The horizontal passes of OCVISC: a thread takes kViscLevels levels of a point,
+// so the geometry of the point and its four neighbours (some 15 values for each
+// staggering) is loaded once for them; the loads of four levels are issued together.
+// (A thread per point and level reloaded it every level: 5.4 ms for the two
+// passes on 1024 x 1024 x 80.)  Where a neighbour is outside the staggering's range,
+// its term, which the reference omits, is 0.
+constexpr int kViscLevels = 8;
+enum { S_U = 0, S_V = 1, S_W = 2 };
 
-// first Laplacians UK1O (u), VK1E (v), WN1O (w), ocvisc.f90:350-438, 617-669.
-// (Fusing this pass with the next through shared-memory tiles, as the tracer
-// kernel above does, was measured on c3 and not kept: with the geometry of
-// the edge cases reloaded every level the fused form was 5% slower, and one
-// launch per level 1.7x slower, than these two level-parallel passes.)
-__global__ void k_visc_lap(Geo G, const double* __restrict__ uk, const double* __restrict__ vk,
-                           const double* __restrict__ wn, double* __restrict__ u1,
-                           double* __restrict__ v1, double* __restrict__ w1) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int K = blockIdx.z + 1;
-  const int IE = G.L.ie, JE = G.L.je;
-  if (i > IE || j > JE) return;
-  // ---- u-points
-  if (j >= 1) {
-    auto AO = [&](int ii, int jj) { return wet(G.gu, G.L.at2(ii, jj), K); };
-    auto UK = [&](int ii, int jj) { return AT(uk, ii, jj, K); };
-    const bool jin = j >= 2 && j <= JE - 1, iin = i >= 1 && i <= IE - 1;
-    double r = 0.0;
-    auto ypart = [&]() {
-      return (AO(i, j - 1) * (UK(i, j - 1) - UK(i, j)) * rdlypsi(G, i, j - 1) -
-              AO(i, j + 1) * (UK(i, j) - UK(i, j + 1)) * rdlypsi(G, i, j)) *
-             G.rdlyu[G.L.at2(i, j)];
-    };
-    auto xpart = [&]() {
-      return (AO(i + 1, j) * (UK(i + 1, j) - UK(i, j)) * G.rdlxp[G.L.at2(i + 1, j)] -
-              AO(i - 1, j) * (UK(i, j) - UK(i - 1, j)) * G.rdlxp[G.L.at2(i, j)]) *
-             G.rdlxu[G.L.at2(i, j)];
-    };
-    if (jin && iin) {
-      r = AO(i, j) * (xpart() + ypart());
-    } else if (jin && i == 0) {
-      r = AO(i, j) * ((AO(i + 1, j) * (UK(i + 1, j) - UK(i, j)) * G.rdlxp[G.L.at2(i + 1, j)]) *
-                          G.rdlxu[G.L.at2(i, j)] +
-                      ypart());
-    } else if (jin && i == IE) {
-      r = AO(i, j) * ((-AO(i - 1, j) * (UK(i, j) - UK(i - 1, j)) * G.rdlxp[G.L.at2(i, j)]) *
-                          G.rdlxu[G.L.at2(i, j)] +
-                      ypart());
-    } else if (iin && j == 1) {
-      r = AO(i, j) * (xpart() + (-AO(i, j + 1) * (UK(i, j) - UK(i, j + 1)) * rdlypsi(G, i, j)) *
-                                    G.rdlyu[G.L.at2(i, j)]);
-    } else if (iin && j == JE) {
-      r = AO(i, j) * (xpart() + (AO(i, j - 1) * (UK(i, j - 1) - UK(i, j)) * rdlypsi(G, i, j - 1)) *
-                                    G.rdlyu[G.L.at2(i, j)]);
+// wet levels of a point's neighbours (0: no term) and the loads of its stencil
+struct Cross {
+  int c, e, w, n, s;
+};
+template <int ST>
+__device__ __forceinline__ Cross cross_kb(const Geo& G, int i, int j) {
+  const ColGeo& cg = ST == S_U ? G.gu : ST == S_V ? G.gv : G.gp;
+  const int ij = G.L.at2(i, j);
+  constexpr int i0 = ST == S_U ? 0 : 1, j0 = ST == S_V ? 0 : 1;
+  Cross k;
+  k.c = cg.kb[ij];
+  k.e = i < G.L.ie ? cg.kb[ij + 1] : 0;
+  k.w = i > i0 ? cg.kb[ij - 1] : 0;
+  k.n = j > j0 ? cg.kb[ij - G.L.P] : 0;
+  k.s = j < G.L.je ? cg.kb[ij + G.L.P] : 0;
+  return k;
+}
+
+// first Laplacians UK1O (u), VK1E (v), WN1O (w), ocvisc.f90:350-438, 617-669
+template <int ST>
+__device__ __forceinline__ void visc_lap(const Geo& G, const double* __restrict__ f,
+                                         double* __restrict__ out, int i, int j, int K0) {
+  const int IE = G.L.ie, JE = G.L.je, P = G.L.P, pl = G.L.plane;
+  constexpr int i0 = ST == S_U ? 0 : 1, j0 = ST == S_V ? 0 : 1;
+  if (i < i0 || j < j0) return;
+  const bool iin = i > i0 && i < IE, jin = j > j0 && j < JE;
+  const int ij = G.L.at2(i, j);
+  Cross k = cross_kb<ST>(G, i, j);
+  double ce = 0., cw = 0., cn = 0., cs = 0., rx = 0., ry = 0.;
+  if (iin || jin) {
+    if (ST == S_U) {
+      ce = i < IE ? G.rdlxp[ij + 1] : 0.;
+      cw = G.rdlxp[ij];
+      rx = G.rdlxu[ij];
+      cn = G.rdlypsi[ij - P];
+      cs = G.rdlypsi[ij];
+      ry = G.rdlyu[ij];
+    } else if (ST == S_V) {
+      ce = G.rdlxpsi[ij];
+      cw = G.rdlxpsi[ij - 1];
+      rx = G.rdlxv[ij];
+      cn = G.rdlyp[ij];
+      cs = j < JE ? G.rdlyp[ij + P] : 0.;
+      ry = G.rdlyv[ij];
+    } else {
+      ce = G.rdlxu[ij];
+      cw = G.rdlxu[ij - 1];
+      rx = G.rdlxp[ij];
+      cn = G.rdlyv[ij - P];
+      cs = G.rdlyv[ij];
+      ry = G.rdlyp[ij];
     }
-    AT(u1, i, j, K) = r;
+  } else {
+    k.c = 0;  // a corner
   }
-  // ---- v-points
-  if (i >= 1) {
-    auto AE = [&](int ii, int jj) { return wet(G.gv, G.L.at2(ii, jj), K); };
-    auto VK = [&](int ii, int jj) { return AT(vk, ii, jj, K); };
-    const bool jin = j >= 1 && j <= JE - 1, iin = i >= 2 && i <= IE - 1;
-    double r = 0.0;
-    auto xpart = [&]() {
-      return (AE(i + 1, j) * (VK(i + 1, j) - VK(i, j)) * rdlxpsi(G, i, j) -
-              AE(i - 1, j) * (VK(i, j) - VK(i - 1, j)) * rdlxpsi(G, i - 1, j)) *
-             G.rdlxv[G.L.at2(i, j)];
-    };
-    auto ypart = [&]() {
-      return (AE(i, j - 1) * (VK(i, j - 1) - VK(i, j)) * G.rdlyp[G.L.at2(i, j)] -
-              AE(i, j + 1) * (VK(i, j) - VK(i, j + 1)) * G.rdlyp[G.L.at2(i, j + 1)]) *
-             G.rdlyv[G.L.at2(i, j)];
-    };
-    if (jin && iin) {
-      r = AE(i, j) * (xpart() + ypart());
-    } else if (jin && i == 1) {
-      r = AE(i, j) * ((AE(i + 1, j) * (VK(i + 1, j) - VK(i, j)) * rdlxpsi(G, i, j)) *
-                          G.rdlxv[G.L.at2(i, j)] +
-                      ypart());
-    } else if (jin && i == IE) {
-      r = AE(i, j) * ((-AE(i - 1, j) * (VK(i, j) - VK(i - 1, j)) * rdlxpsi(G, i - 1, j)) *
-                          G.rdlxv[G.L.at2(i, j)] +
-                      ypart());
-    } else if (iin && j == 0) {
-      r = AE(i, j) * (xpart() + (-AE(i, j + 1) * (VK(i, j) - VK(i, j + 1)) * G.rdlyp[G.L.at2(i, j + 1)]) *
-                                    G.rdlyv[G.L.at2(i, j)]);
-    } else if (iin && j == JE) {
-      r = AE(i, j) * (xpart() + (AE(i, j - 1) * (VK(i, j - 1) - VK(i, j)) * G.rdlyp[G.L.at2(i, j)]) *
-                                    G.rdlyv[G.L.at2(i, j)]);
+  const int o0 = G.L.at(i, j, K0 - 1), n = min(kViscLevels, G.L.ke + 1 - K0);
+  for (int q0 = 0; q0 < n; q0 += 4) {
+    double c[4], e[4], w[4], no[4], so[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int K = K0 + q0 + q, o = o0 + (q0 + q) * pl;
+      const bool wet = K <= k.c;  // (k.c <= KE)
+      c[q] = wet ? f[o] : 0.;
+      e[q] = wet && K <= k.e ? f[o + 1] : c[q];
+      w[q] = wet && K <= k.w ? f[o - 1] : c[q];
+      no[q] = wet && K <= k.n ? f[o - P] : c[q];
+      so[q] = wet && K <= k.s ? f[o + P] : c[q];
     }
-    AT(v1, i, j, K) = r;
-  }
-  // ---- w-points (levels 1..KE)
-  if (i >= 1 && j >= 1) {
-    auto WE = [&](int ii, int jj) { return wet(G.gp, G.L.at2(ii, jj), K); };
-    auto WN = [&](int ii, int jj) { return AT(wn, ii, jj, K); };
-    const bool jin = j >= 2 && j <= JE - 1, iin = i >= 2 && i <= IE - 1;
-    double r = 0.0;
-    auto xpart = [&]() {
-      return (WE(i + 1, j) * (WN(i + 1, j) - WN(i, j)) * G.rdlxu[G.L.at2(i, j)] -
-              WE(i - 1, j) * (WN(i, j) - WN(i - 1, j)) * G.rdlxu[G.L.at2(i - 1, j)]) *
-             G.rdlxp[G.L.at2(i, j)];
-    };
-    auto ypart = [&]() {
-      return (WE(i, j - 1) * (WN(i, j - 1) - WN(i, j)) * G.rdlyv[G.L.at2(i, j - 1)] -
-              WE(i, j + 1) * (WN(i, j) - WN(i, j + 1)) * G.rdlyv[G.L.at2(i, j)]) *
-             G.rdlyp[G.L.at2(i, j)];
-    };
-    if (jin && iin) {
-      r = WE(i, j) * (xpart() + ypart());
-    } else if (jin && i == 1) {
-      r = WE(i, j) * ((WE(i + 1, j) * (WN(i + 1, j) - WN(i, j)) * G.rdlxu[G.L.at2(i, j)]) *
-                          G.rdlxp[G.L.at2(i, j)] +
-                      ypart());
-    } else if (jin && i == IE) {
-      r = WE(i, j) * ((-WE(i - 1, j) * (WN(i, j) - WN(i - 1, j)) * G.rdlxu[G.L.at2(i - 1, j)]) *
-                          G.rdlxp[G.L.at2(i, j)] +
-                      ypart());
-    } else if (iin && j == 1) {
-      r = WE(i, j) * (xpart() + (-WE(i, j + 1) * (WN(i, j) - WN(i, j + 1)) * G.rdlyv[G.L.at2(i, j)]) *
-                                    G.rdlyp[G.L.at2(i, j)]);
-    } else if (iin && j == JE) {
-      r = WE(i, j) * (xpart() + (WE(i, j - 1) * (WN(i, j - 1) - WN(i, j)) * G.rdlyv[G.L.at2(i, j - 1)]) *
-                                    G.rdlyp[G.L.at2(i, j)]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (q0 + q >= n) break;
+      // a neighbour without water gives c - c = 0, as its mask does
+      const double x = ((e[q] - c[q]) * ce - (c[q] - w[q]) * cw) * rx;
+      const double y = ((no[q] - c[q]) * cn - (c[q] - so[q]) * cs) * ry;
+      out[o0 + (q0 + q) * pl] = K0 + q0 + q <= k.c ? x + y : 0.;
     }
-    AT(w1, i, j, K) = r;
   }
 }
 
-// second passes, ocvisc.f90:445-477 (u, v) and 673-688 (w)
-__global__ void k_visc_bih(Geo G, const double* __restrict__ uoo, const double* __restrict__ voe,
-                           const double* __restrict__ uk, const double* __restrict__ vk,
-                           const double* __restrict__ wn, const double* __restrict__ u1,
-                           const double* __restrict__ v1, const double* __restrict__ w1,
-                           double* __restrict__ uo, double* __restrict__ vo,
-                           double* __restrict__ wo) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int K = blockIdx.z + 1;  // 1..KE+1
-  const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
-  if (i > IE || j > JE) return;
-  const double mv = G.minvalue;
-  // The face terms AUL.. * width / length of ocvisc.f90:445-477, 673-688 are
-  // precomputed per face (G.ugx .. G.wgy) and the cell areas' reciprocals per
-  // cell, so a cell needs no division except by its thickness (w).
-  if (K <= KE) {
-    // ---- u
-    if (j >= 1) {
-      double r = AT(uoo, i, j, K);
-      if (i >= 1 && i <= IE - 1 && j >= 2 && j <= JE - 1) {
-        auto AO = [&](int ii, int jj) { return wet(G.gu, G.L.at2(ii, jj), K); };
-        auto U1 = [&](int ii, int jj) { return AT(u1, ii, jj, K); };
-        const int ij = G.L.at2(i, j);
-        r = (AO(i, j) * G.rareau[ij]) *
-            (G.dlxu[ij] * G.dlyu[ij] * AT(uk, i, j, K) -
-             (G.ugx[G.L.at2(i + 1, j)] * AO(i + 1, j) * (U1(i + 1, j) - U1(i, j)) -
-              G.ugx[ij] * AO(i - 1, j) * (U1(i, j) - U1(i - 1, j)) +
-              G.ugy[G.L.at2(i, j - 1)] * AO(i, j - 1) * (U1(i, j - 1) - U1(i, j)) -
-              G.ugy[ij] * AO(i, j + 1) * (U1(i, j) - U1(i, j + 1))));
-      }
-      AT(uo, i, j, K) = r;
+__global__ void __launch_bounds__(128) k_visc_lap(Geo G, const double* __restrict__ uk,
+                                                  const double* __restrict__ vk,
+                                                  const double* __restrict__ wn,
+                                                  double* __restrict__ u1,
+                                                  double* __restrict__ v1,
+                                                  double* __restrict__ w1, int chunks) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  if (i > G.L.ie || j > G.L.je) return;
+  const int K0 = (blockIdx.z % chunks) * kViscLevels + 1;
+  switch (blockIdx.z / chunks) {
+    case 0: visc_lap<S_U>(G, uk, u1, i, j, K0); break;
+    case 1: visc_lap<S_V>(G, vk, v1, i, j, K0); break;
+    default: visc_lap<S_W>(G, wn, w1, i, j, K0); break;
+  }
+}
+
+// second passes, ocvisc.f90:445-477 (u, v) and 673-688 (w).  The face terms
+// AUL.. * width / length are precomputed per face (G.ugx .. G.wgy) and the cell
+// areas' reciprocals per cell, so a cell needs no division except by its
+// thickness (w).  keep: the values of points outside the update range.
+template <int ST>
+__device__ __forceinline__ void visc_bih(const Geo& G, const double* __restrict__ keep,
+                                         const double* __restrict__ f,
+                                         const double* __restrict__ l, double* __restrict__ out,
+                                         int i, int j, int K0) {
+  const int IE = G.L.ie, JE = G.L.je, P = G.L.P, pl = G.L.plane;
+  constexpr int i0 = ST == S_U ? 0 : 1, j0 = ST == S_V ? 0 : 1;
+  if (i < i0 || j < j0) return;
+  const int kbot = G.L.ke + (ST == S_W);  // KEP of w is carried
+  const int o0 = G.L.at(i, j, K0 - 1), n = min(kViscLevels, kbot + 1 - K0);
+  if (!(i > i0 && i < IE && j > j0 && j < JE)) {
+    for (int q = 0; q < n; ++q) out[o0 + q * pl] = keep[o0 + q * pl];
+    return;
+  }
+  const int ij = G.L.at2(i, j);
+  const Cross k = cross_kb<ST>(G, i, j);
+  double ge, gw, gn, gs, area, rarea;
+  if (ST == S_U) {
+    ge = G.ugx[ij + 1];
+    gw = G.ugx[ij];
+    gn = G.ugy[ij - P];
+    gs = G.ugy[ij];
+    area = G.dlxu[ij] * G.dlyu[ij];
+    rarea = G.rareau[ij];
+  } else if (ST == S_V) {
+    ge = G.vgx[ij];
+    gw = G.vgx[ij - 1];
+    gn = G.vgy[ij];
+    gs = G.vgy[ij + P];
+    area = G.dlxv[ij] * G.dlyv[ij];
+    rarea = G.rareav[ij];
+  } else {
+    ge = G.wgx[ij];
+    gw = G.wgx[ij - 1];
+    gn = G.wgy[ij - P];
+    gs = G.wgy[ij];
+    area = G.dlxp[ij] * G.dlyp[ij];
+    rarea = G.rareap[ij];
+  }
+  // w: thicknesses of the cell and its faces, at least MINVALUE
+  int kue = 0, kuw = 0, kvn = 0, kvs = 0;
+  double bc = 0., bue = 0., buw = 0., bvn = 0., bvs = 0.;
+  if (ST == S_W) {
+    kue = G.gu.kb[ij];
+    kuw = G.gu.kb[ij - 1];
+    kvn = G.gv.kb[ij - P];
+    kvs = G.gv.kb[ij];
+    bc = G.gp.bot[ij];
+    bue = G.gu.bot[ij];
+    buw = G.gu.bot[ij - 1];
+    bvn = G.gv.bot[ij - P];
+    bvs = G.gv.bot[ij];
+  }
+  for (int q0 = 0; q0 < n; q0 += 4) {
+    double v[4], c[4], e[4], w[4], no[4], so[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int K = K0 + q0 + q, o = o0 + (q0 + q) * pl;
+      const bool wet = K <= k.c;
+      v[q] = K <= kbot ? f[o] : 0.;
+      c[q] = wet ? l[o] : 0.;
+      e[q] = wet && K <= k.e ? l[o + 1] : c[q];
+      w[q] = wet && K <= k.w ? l[o - 1] : c[q];
+      no[q] = wet && K <= k.n ? l[o - P] : c[q];
+      so[q] = wet && K <= k.s ? l[o + P] : c[q];
     }
-    // ---- v
-    if (i >= 1) {
-      double r = AT(voe, i, j, K);
-      if (i >= 2 && i <= IE - 1 && j >= 1 && j <= JE - 1) {
-        auto AE = [&](int ii, int jj) { return wet(G.gv, G.L.at2(ii, jj), K); };
-        auto V1 = [&](int ii, int jj) { return AT(v1, ii, jj, K); };
-        const int ij = G.L.at2(i, j);
-        r = (AE(i, j) * G.rareav[ij]) *
-            (G.dlxv[ij] * G.dlyv[ij] * AT(vk, i, j, K) -
-             (G.vgx[ij] * AE(i + 1, j) * (V1(i + 1, j) - V1(i, j)) -
-              G.vgx[G.L.at2(i - 1, j)] * AE(i - 1, j) * (V1(i, j) - V1(i - 1, j)) +
-              G.vgy[ij] * AE(i, j - 1) * (V1(i, j - 1) - V1(i, j)) -
-              G.vgy[G.L.at2(i, j + 1)] * AE(i, j + 1) * (V1(i, j) - V1(i, j + 1))));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int K = K0 + q0 + q;
+      if (q0 + q >= n) break;
+      double r = 0.;
+      if (K <= k.c) {
+        if (ST == S_W) {
+          const double mv = G.minvalue, dz = __ldg(G.dzw + K - 1);
+          auto th = [&](int kb, double bot) { return fmx(K < kb ? dz : (K == kb ? bot : 0.0), mv); };
+          const double dzp = th(k.c, bc);
+          r = div_nr(rarea, dzp) *
+              (area * dzp * v[q] -
+               (ge * th(kue, bue) * (e[q] - c[q]) - gw * th(kuw, buw) * (c[q] - w[q]) +
+                gn * th(kvn, bvn) * (no[q] - c[q]) - gs * th(kvs, bvs) * (c[q] - so[q])));
+        } else {
+          r = rarea * (area * v[q] - (ge * (e[q] - c[q]) - gw * (c[q] - w[q]) +
+                                      gn * (no[q] - c[q]) - gs * (c[q] - so[q])));
+        }
       }
-      AT(vo, i, j, K) = r;
+      if (ST == S_W && K > G.L.ke) r = v[q];
+      out[o0 + (q0 + q) * pl] = r;
     }
   }
-  // ---- w (levels 1..KE updated, KEP carried)
-  if (i >= 1 && j >= 1) {
-    double r = AT(wn, i, j, K);
-    if (K <= KE && i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1) {
-      auto WE = [&](int ii, int jj) { return wet(G.gp, G.L.at2(ii, jj), K); };
-      auto W1 = [&](int ii, int jj) { return AT(w1, ii, jj, K); };
-      auto dzu = [&](int ii, int jj) { return fmx(thick(G.gu, G.dzw, G.L.at2(ii, jj), K), mv); };
-      auto dzv = [&](int ii, int jj) { return fmx(thick(G.gv, G.dzw, G.L.at2(ii, jj), K), mv); };
-      const int ij = G.L.at2(i, j);
-      const double dzp = fmx(thick(G.gp, G.dzw, ij, K), mv);
-      r = div_nr(WE(i, j) * G.rareap[ij], dzp) *
-          (G.dlxp[ij] * G.dlyp[ij] * dzp * AT(wn, i, j, K) -
-           (G.wgx[ij] * dzu(i, j) * WE(i + 1, j) * (W1(i + 1, j) - W1(i, j)) -
-            G.wgx[G.L.at2(i - 1, j)] * dzu(i - 1, j) * WE(i - 1, j) * (W1(i, j) - W1(i - 1, j)) +
-            G.wgy[G.L.at2(i, j - 1)] * dzv(i, j - 1) * WE(i, j - 1) * (W1(i, j - 1) - W1(i, j)) -
-            G.wgy[ij] * dzv(i, j) * WE(i, j + 1) * (W1(i, j) - W1(i, j + 1))));
-    }
-    AT(wo, i, j, K) = r;
+}
+
+__global__ void __launch_bounds__(128) k_visc_bih(
+    Geo G, const double* __restrict__ uoo, const double* __restrict__ voe,
+    const double* __restrict__ uk, const double* __restrict__ vk, const double* __restrict__ wn,
+    const double* __restrict__ u1, const double* __restrict__ v1, const double* __restrict__ w1,
+    double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ wo, int chunks) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  if (i > G.L.ie || j > G.L.je) return;
+  const int K0 = (blockIdx.z % chunks) * kViscLevels + 1;
+  switch (blockIdx.z / chunks) {
+    case 0: visc_bih<S_U>(G, uoo, uk, u1, uo, i, j, K0); break;
+    case 1: visc_bih<S_V>(G, voe, vk, v1, vo, i, j, K0); break;
+    default: visc_bih<S_W>(G, wn, wn, w1, wo, i, j, K0); break;
   }
 }
 
@@ -822,12 +842,12 @@ void launch_ocvisc(const Geo& G, const double* uoo, const double* voe, const dou
     k_visc_w<Ln><<<dim3(nb, JE), Ln::NT, 0, st>>>(G, wno, avo, wnv);
   });
   count_launch();
+  const int chunks = (KE + 1 + kViscLevels - 1) / kViscLevels;
   dim3 gl = grid2(IE + 1, JE + 1, b3);
-  gl.z = KE;
-  k_visc_lap<<<gl, b3, 0, st>>>(G, ukv, vkv, wnv, u1, v1, w1);
+  gl.z = 3 * chunks;
+  k_visc_lap<<<gl, b3, 0, st>>>(G, ukv, vkv, wnv, u1, v1, w1, chunks);
   count_launch();
-  gl.z = KE + 1;
-  k_visc_bih<<<gl, b3, 0, st>>>(G, uoo, voe, ukv, vkv, wnv, u1, v1, w1, uo, vo, wo);
+  k_visc_bih<<<gl, b3, 0, st>>>(G, uoo, voe, ukv, vkv, wnv, u1, v1, w1, uo, vo, wo, chunks);
   count_launch();
 }
 
