@@ -194,11 +194,11 @@ struct orctm_handle {
   size_t obc_exp_cap = 0;
   const double* obc_exp_sao_south = nullptr;
   // barotropic solve (orctm_set_barotropic): its constants, its 2D device
-  // fields and TRONEU's SOR sweeps captured once as a graph
+  // fields
   bool baro_ready = false;
   BaroArgs baro{};
   BaroFields bf{};
-  cudaGraphExec_t sor_graph = nullptr;
+  double* sor_z = nullptr;  // TRONEU's second plane, allocated on first use
   WindFields wind{};  // OCWIND's forcing (orctm_ocwind), allocated on first use
   bool wind_ready = false;
   // OCTHER (orctm_set_thermo), OCMODMOM's Coriolis factors
@@ -1289,7 +1289,6 @@ int orctm_destroy(orctm_handle* h) {
   }
   for (int pr = 0; pr < 2; ++pr)
     if (h->pcg_graph[pr]) cudaGraphExecDestroy(h->pcg_graph[pr]);
-  if (h->sor_graph) cudaGraphExecDestroy(h->sor_graph);
   if (h->hS) pinned_state_put(h->hS);
   if (h->h_contra) cudaFreeHost(h->h_contra);
   for (int k = 0; k < ORCTM_PROF_KINDS; ++k)
@@ -1881,41 +1880,10 @@ int orctm_set_barotropic(orctm_handle* h, const orctm_barotropic* b) {
   BaroArgs a{b->grav, b->stabn, b->conn, b->rlsa1, b->sorpar, b->minvalue, b->niter, b->eta_forc ? 1 : 0};
   launch_itprep(h->G, a, h->bf.u1o, h->bf.v1e, h->bf, h->stream);
   ORCTM_CUDA_OK(cudaGetLastError());
-  // the new constants change the SOR launches: capture them again
-  if (h->sor_graph) {
-    ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
-    cudaGraphExecDestroy(h->sor_graph);
-    h->sor_graph = nullptr;
-  }
   h->baro = a;
   h->baro_ready = true;
   return ORCTM_OK;
 }
-
-namespace {
-int sor_graph(orctm_handle* h, cudaGraphExec_t* out) {
-  if (h->sor_graph) {
-    *out = h->sor_graph;
-    return ORCTM_OK;
-  }
-  const unsigned long long before = launch_count();
-  ORCTM_CUDA_OK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  for (int it = 0; it < h->baro.niter; ++it) {
-    launch_sor(h->G, h->baro, h->bf, 0, h->stream);
-    launch_sor(h->G, h->baro, h->bf, 1, h->stream);
-  }
-  cudaGraph_t g = nullptr;
-  const cudaError_t e1 = cudaStreamEndCapture(h->stream, &g);
-  add_launches(-(long long)(launch_count() - before));  // counted when the graph runs
-  ORCTM_CUDA_OK(e1);
-  cudaGraphExec_t ex = nullptr;
-  const cudaError_t e2 = cudaGraphInstantiate(&ex, g, 0ULL);
-  cudaGraphDestroy(g);
-  ORCTM_CUDA_OK(e2);
-  h->sor_graph = *out = ex;
-  return ORCTM_OK;
-}
-}  // namespace
 
 int orctm_troneu(orctm_handle* h, const double* u1o, const double* v1e, const double* uzo,
                  const double* vze) {
@@ -1935,12 +1903,9 @@ int orctm_troneu(orctm_handle* h, const double* u1o, const double* v1e, const do
   ORCTM_CUDA_OK(cudaMemsetAsync(h->bf.z1o, 0, sizeof(double) * (size_t)h->L.plane, h->stream));
   launch_troneu_rhs(h->G, h->baro, h->bf, h->stream);
   ORCTM_CUDA_OK(cudaGetLastError());
-  if (h->baro.niter > 0) {
-    cudaGraphExec_t ex;
-    if ((st = sor_graph(h, &ex))) return st;
-    ORCTM_CUDA_OK(cudaGraphLaunch(ex, h->stream));
-    add_launches(2LL * h->baro.niter);
-  }
+  if (!h->sor_z && (st = h->dev_alloc(&h->sor_z, (size_t)h->L.plane))) return st;
+  launch_sor(h->G, h->baro, h->bf, h->sor_z, h->baro.niter, h->stream);
+  ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
 }
 
@@ -2034,11 +1999,6 @@ int orctm_trotest(orctm_handle* h, int ntry, int niter, double* sorpar_out) {
   cudaGraphExecDestroy(ex);
   if (rc != ORCTM_OK) return rc;
   *sorpar_out = sorpmin;
-  // TRONEU uses the chosen value from now on
-  if (h->sor_graph) {
-    cudaGraphExecDestroy(h->sor_graph);
-    h->sor_graph = nullptr;
-  }
   h->baro.sorpar = sorpmin;
   return ORCTM_OK;
 }

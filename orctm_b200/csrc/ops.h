@@ -105,7 +105,8 @@ void launch_ocwind(const Geo& G, const WindFields& w, double* uoo, double* voe, 
 void launch_itprep(const Geo& G, const BaroArgs& a, const double* deuto, const double* deute,
                    const BaroFields& f, cudaStream_t st);
 void launch_troneu_rhs(const Geo& G, const BaroArgs& a, const BaroFields& f, cudaStream_t st);
-void launch_sor(const Geo& G, const BaroArgs& a, const BaroFields& f, int parity, cudaStream_t st);
+void launch_sor(const Geo& G, const BaroArgs& a, const BaroFields& f, double* zt, int niter,
+                cudaStream_t st);
 void launch_ocvtro(const Geo& G, const BaroArgs& a, const BaroFields& f, double* zo,
                    cudaStream_t st);
 void launch_ocvtot(const Geo& G, const BaroArgs& a, const double* uso, const double* vse,
