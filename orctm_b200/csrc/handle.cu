@@ -208,7 +208,7 @@ struct orctm_handle {
   ThermoFields tf{};
   CorFields cf{};
   double *uk1o = nullptr, *vk1e = nullptr;
-  double *occ_wpo = nullptr, *occ_t1o = nullptr, *occ_bruva = nullptr, *occ_contrij = nullptr;
+  double *occ_wpo = nullptr, *occ_bruva = nullptr, *occ_contrij = nullptr;
   double* occ_contra = nullptr;  // device scalar
   double* h_contra = nullptr;    // its page-locked mirror
   double* trotest_buf = nullptr;  // orctm_trotest's scratch, allocated on first use
@@ -2305,13 +2305,12 @@ int r_occlit(orctm_handle* h) {
     return st;
   if (!h->occ_wpo) {
     const size_t n3 = (size_t)h->L.n3(), n2 = (size_t)h->L.plane;
-    if ((st = h->dev_alloc(&h->occ_wpo, n3)) || (st = h->dev_alloc(&h->occ_t1o, n3)) ||
-        (st = h->dev_alloc(&h->occ_bruva, n2)) || (st = h->dev_alloc(&h->occ_contrij, n2)) ||
+    if ((st = h->dev_alloc(&h->occ_wpo, n3)) || (st = h->dev_alloc(&h->occ_bruva, n2)) || (st = h->dev_alloc(&h->occ_contrij, n2)) ||
         (st = h->dev_alloc(&h->occ_contra, 1)))
       return st;
   }
   launch_occlit(h->G, h->baro, h->tf, h->bf, h->slot[ORCTM_F_UKO], h->slot[ORCTM_F_VKE], h->uk1o,
-                h->vk1e, h->slot[ORCTM_F_WO], h->occ_wpo, h->occ_t1o, h->occ_bruva,
+                h->vk1e, h->slot[ORCTM_F_WO], h->occ_wpo, h->occ_bruva,
                 h->occ_contrij, h->occ_contra, h->stream);
   ORCTM_CUDA_OK(cudaGetLastError());
   ORCTM_CUDA_OK(cudaMemcpyAsync(h->h_contra, h->occ_contra, sizeof(double), cudaMemcpyDeviceToHost,

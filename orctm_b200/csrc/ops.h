@@ -147,12 +147,13 @@ void launch_stabio_rescale(const Geo& G, const ThermoFields& f, cudaStream_t st)
 void launch_ocmodmom(const Geo& G, const BaroArgs& b, const ThermoFields& f, const CorFields& c,
                      const BaroFields& bf, const double* zo, const double* uoo, const double* voe,
                      double* uko, double* vke, double* uk1o, double* vk1e, double* wno,
-                     double* ub, double* vb, double* wb, double* dw, cudaStream_t st);
-// OCCLIT; scratch: wpo, t1o (3D), bruva, contrij (2D); *contra receives the
+                     double* ub, double* vb, double* wb, double* dw,
+                     cudaStream_t st);
+// OCCLIT; scratch: wpo (3D), bruva, contrij (2D); *contra receives the
 // sum of CONTRIJ (device scalar)
 void launch_occlit(const Geo& G, const BaroArgs& b, const ThermoFields& f, const BaroFields& bf,
                    double* uko, double* vke, double* uk1o, double* vk1e, double* wo, double* wpo,
-                   double* t1o, double* bruva, double* contrij, double* contra, cudaStream_t st);
+                   double* bruva, double* contrij, double* contra, cudaStream_t st);
 
 // advect.cu: mid and vol are scratch fields
 void launch_ocadpo(const Geo& G, const double* T, const double* uko, const double* vke,
