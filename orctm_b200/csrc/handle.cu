@@ -717,8 +717,43 @@ int setup(orctm_handle* h, const orctm_desc* d) {
     dst = p;
     return ORCTM_OK;
   };
+  // The vertical profiles of the coarse space: the lowest two modes of T phi =
+  // lambda W phi on the deepest column, T the vertical part of B (its nominal
+  // ZW), W the weights 1/ZP, by inverse iteration
+  std::vector<double> phi((size_t)RbCoarse::kModes * KE, 0.0);
+  {
+    int n = 0;
+    for (size_t s = 0; s < n2; ++s) n = std::max(n, kbp[s]);
+    std::vector<double> piv(n), y(n);
+    for (int K = 0; K < n; ++K) {
+      const double up = K ? zwn[K] : 0.0;
+      piv[K] = zwn[K] + (K + 1 < n ? zwn[K + 1] : 0.0) - (K ? up * up / piv[K - 1] : 0.0);
+    }
+    for (int q = 0; q < std::min(n, (int)RbCoarse::kModes); ++q) {
+      double* f = phi.data() + (size_t)q * KE;
+      for (int K = 0; K < n; ++K) f[K] = q ? (2 * K < n ? 1.0 : -1.0) : 1.0;
+      for (int it = 0; it < 40; ++it) {
+        for (int p = 0; p < q; ++p) {
+          const double* g = phi.data() + (size_t)p * KE;
+          double fg = 0.0, gg = 0.0;
+          for (int K = 0; K < n; ++K) {
+            fg += izn[K] * f[K] * g[K];
+            gg += izn[K] * g[K] * g[K];
+          }
+          for (int K = 0; K < n; ++K) f[K] -= fg / gg * g[K];
+        }
+        for (int K = 0; K < n; ++K) y[K] = izn[K] * f[K] + (K ? zwn[K] / piv[K - 1] * y[K - 1] : 0.0);
+        double top = 0.0;
+        for (int K = n - 1; K >= 0; --K) {
+          f[K] = (y[K] + (K + 1 < n ? zwn[K + 1] * f[K + 1] : 0.0)) / piv[K];
+          top = std::max(top, std::fabs(f[K]));
+        }
+        for (int K = 0; K < n; ++K) f[K] /= top;
+      }
+    }
+  }
   PoissonGeo& P = h->P;
-  if ((st = upv(P.xu, xu)) || (st = upv(P.xp, xp)) || (st = upv(P.yv, yv)) ||
+  if ((st = upv(h->R.phi, phi)) || (st = upv(P.xu, xu)) || (st = upv(P.xp, xp)) || (st = upv(P.yv, yv)) ||
       (st = upv(P.yp, yp)) || (st = upv(P.zwa, zwa)) || (st = upv(P.zwb, zwb)) ||
       (st = upv(P.zpa, zpa)) || (st = upv(P.zpb, zpb)) || (st = upv(P.zpc, zpc)) ||
       (st = upv(P.zwn, zwn)) || (st = upv(P.zpn, zpn)) || (st = upv(P.iza, iza)) ||
@@ -778,6 +813,20 @@ int alloc_rb(orctm_handle* h, RbVectors<T>& v) {
   int st;
   for (T** p : {&v.x, &v.r, &v.z, &v.p, &v.q, &v.u, &v.ub, &v.dr})
     if (!*p && (st = h->dev_alloc(p, n))) return st;
+  if (!h->R.co.mu) {  // the coarse operator, one for both precisions
+    RbCoarse& co = h->R.co;
+    const size_t n2 = (size_t)RbCoarse::kModes * h->L.plane;
+    if ((st = h->dev_alloc(&co.ce, n2)) || (st = h->dev_alloc(&co.cs, n2)) ||
+        (st = h->dev_alloc(&co.sc, n2)) || (st = h->dev_alloc(&co.mu, RbCoarse::kModes)))
+      return st;
+    launch_coarse_setup(h->G, h->P, h->R, h->stream);
+    float mu[RbCoarse::kModes];
+    ORCTM_CUDA_OK(cudaMemcpyAsync(mu, co.mu, sizeof(mu), cudaMemcpyDeviceToHost, h->stream));
+    ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
+    coarse_plan(co, mu);
+  }
+  const size_t n2 = (size_t)RbCoarse::kModes * h->R.plane2;
+  if ((!v.rho && (st = h->dev_alloc(&v.rho, n2))) || (!v.cc && (st = h->dev_alloc(&v.cc, n2)))) return st;
   if ((st = h->dev_alloc(&v.km, rb_tiles(h->R, sizeof(T)))) || (st = h->dev_alloc(&v.db, n))) return st;
   launch_rb_setup<T>(h->G, h->P, h->R, v, h->stream);
   ORCTM_CUDA_OK(cudaGetLastError());
@@ -798,7 +847,7 @@ int read_state(orctm_handle* h) {
   return ORCTM_OK;
 }
 
-// A chunk of PCG iterations (three kernels each) is captured once per
+// A chunk of PCG iterations (three or four kernels each) is captured once per
 // precision into the body of a graph's conditional while node: the vectors,
 // the solver scalars and the launch shapes of a handle are fixed.  With
 // profiling on, the launches go one by one (they are bracketed by events).
@@ -817,6 +866,7 @@ void pcg_iteration(orctm_handle* h) {
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, h->stream));
+  if (h->R.co.on) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
 }
 
 template <typename T>
@@ -881,11 +931,16 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   // pass maxit, with no host round trip in between; the iterations left before
   // maxit, and all of them while profiling, one by one
   int it = 0, conv = 0;
-  if (!h->prof && launch_rb_small<T>(h->R, h->S, v, maxit, h->stream)) {
+  const bool small = !h->prof && launch_rb_small<T>(h->R, h->S, v, maxit, h->stream);
+  if (small) {
     if ((st = read_state(h))) return st;
     it = h->hS->iter;
     conv = h->hS->converged;
-  } else if (!h->prof && maxit >= kPcgChunk) {
+  } else {
+    if (h->R.co.on) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
+    ORCTM_CUDA_OK(cudaGetLastError());
+  }
+  if (!small && !h->prof && maxit >= kPcgChunk) {
     cudaGraphExec_t ex;
     if ((st = pcg_loop_graph<T>(h, &ex))) return st;
     launch_set_limit(h->S, maxit, h->stream);
@@ -895,7 +950,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     // convergence the chunk's remaining kernels return at once
     it = h->hS->iter;
     conv = h->hS->converged;
-    add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * (3 * kPcgChunk + 1));
+    add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * ((h->R.co.on ? 4 : 3) * kPcgChunk + 1));
   }
   while (!conv && it < maxit) {
     pcg_iteration<T>(h);
@@ -2570,7 +2625,7 @@ int orctm_estimate_device_bytes(const orctm_desc* d, int solver, unsigned long l
   const double f3 = 12.0 + d->ntracers + tmp + 3.0 + 4.25 +
                     (solver == ORCTM_SOLVER_FP32_REFINED ? 2.25 * std::max(1.0, 2.0 * m32 / P) : 0.0);
   // 2D tables (compressed columns, metrics, biharmonic and Poisson factors)
-  const double f2 = 102.0;
+  const double f2 = 108.0;
   // every array carries two guard zones of about one plane
   const double guard = 2.0 * (plane + 2.0 * P + 64.0);
   *bytes = (unsigned long long)((f3 * (n3 + guard) + f2 * (plane + guard) + 16.0 * guard) * 8.0) +

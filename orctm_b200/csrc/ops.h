@@ -24,6 +24,17 @@ struct RbColour {
   double2 *we, *ns;           // XU(I-1) XP, XU(I) XP ; YV(J-1) YP, YV(J) YP
   double2 *zw, *iz;           // ZW at levels kb, kb+1 ; 1/ZP at levels kb-1, kb
 };
+// The coarse operator of the reduced system (poisson.cu): per vertical profile
+// the 2D Galerkin operator, scaled to a unit diagonal, at the model's 2D layout.
+struct RbCoarse {
+  static constexpr int kModes = 2;
+  float *ce, *cs;             // couplings to (i + 1, j) and (i, j + 1)
+  float* sc;                  // diagonal^(-1/2), 0 on land
+  float* mu;                  // largest sum of a column's couplings over its diagonal
+  bool on;                    // whether the iterations use it
+  int steps[kModes];          // Chebyshev steps, for eigenvalues from lmin to 1
+  float lmin[kModes], gain[kModes];
+};
 struct RbGeo {
   int ie, je, ke;
   int P2, plane2;             // P / 2, P / 2 * JN
@@ -31,6 +42,8 @@ struct RbGeo {
   int device, sms;            // the device and its multiprocessors
   RbColour col[2];            // red, black
   const double *zwn, *izn;
+  const double* phi;          // vertical profiles [kModes][ke]
+  RbCoarse co;
   // columns per tile: 128 bytes of a level, half of it in long columns
   static constexpr int kWide = 160;
   __host__ __device__ int width(int elem_bytes) const { return (ke <= kWide ? 128 : 64) / elem_bytes; }
@@ -45,11 +58,13 @@ struct RbVectors {
   T* dr;                      // red pivots
   float* db;                  // black pivots
   int* km;                    // deepest wet level of each tile, red then black
+  T* rho;                     // the residual's products with the profiles (2D, per profile)
+  float* cc;                  // the coarse correction z + sum phi cc
 };
 
 // Device-resident scalars of one Krylov solve.
 struct SolverState {
-  double rho, beta, alpha, alpha_prev, pq, rr, bb, tol, res_rr, res_bb;
+  double rho, beta, alpha, alpha_prev, pq, rz, rr, bb, tol, res_rr, res_bb;
   int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown, 4 a staged copy timed out
   int iter;
   int limit;      // iteration limit of the device-side loop (orctm handle's maxit)
@@ -220,6 +235,10 @@ template <typename T>
 void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 template <typename T>
 void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
+template <typename T>
+void launch_rb_coarse(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
+void launch_coarse_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, cudaStream_t st);
+void coarse_plan(RbCoarse& co, const float* mu);
 // the whole loop in one kernel, on small grids; false: not launched
 template <typename T>
 bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit, cudaStream_t st);
