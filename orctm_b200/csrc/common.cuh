@@ -112,6 +112,22 @@ __device__ __forceinline__ double div_nr(double a, double b) {
   return div_in_range(a, b);
 }
 
+// 1 / b for div_by, NaN outside the range where its steps are exact enough
+__device__ __forceinline__ double rcp_for(double b) {
+  const double m = fabs(b);
+  return m >= 1e-100 && m <= 1e100 ? 1. / b : __longlong_as_double(0x7ff8000000000000LL);
+}
+// a / b with r = rcp_for(b), for several a and one b: a r with one residual
+// correction (Markstein, IBM J. Res. Develop. 34 (1990) 111-119), the quotient rounded to
+// nearest.  Quotients near the ends of the range, infinities and NaN take the division.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q0 = a * r, q = __fma_rn(__fma_rn(-b, q0, a), r, q0);
+  // exponent between -500 and 500
+  const unsigned e = ((unsigned)__double2hiint(q) & 0x7ff00000u) - (523u << 20);
+  if (e > (1000u << 20) && a != 0.) return div_ieee(a, b);
+  return q;
+}
+
 // Fortran MAX/MIN for non-NaN operands, evaluated exactly as the oracle does.
 __device__ __forceinline__ double fmx(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double fmn(double a, double b) { return b < a ? b : a; }
