@@ -582,18 +582,19 @@ __global__ void k_occlit_prep(Geo G, ThermoFields f, double* __restrict__ uko,
 // and its part that is added to the level below on loaded velocities: ua =
 // UKO(I-1), ub = UKO(I), va = VKE(J), vb = VKE(J-1)
 struct DivMetrics {
-  double dti, dtdxpo, dlyuw, dlyue, dlyp, dtdyo, dlxvs, dlxvn, dlxp;
+  double dti, dtdxpo, dlyuw, dlyue, dlyp, dtdyo, dlxvs, dlxvn, dlxp, rlyp, rlxp;
 };
 __device__ __forceinline__ DivMetrics div_metrics(const Geo& G, int ij) {
   const int P = G.L.P;
   return DivMetrics{G.dti, G.dtdxpo[ij], G.dlyu[ij - 1], G.dlyu[ij], G.dlyp[ij],
-                    G.dtdyo[ij], G.dlxv[ij], G.dlxv[ij - P], G.dlxp[ij]};
+                    G.dtdyo[ij], G.dlxv[ij], G.dlxv[ij - P], G.dlxp[ij],
+                    rcp_for(G.dlyp[ij]), rcp_for(G.dlxp[ij])};
 }
 __device__ __forceinline__ double div_part(const DivMetrics& m, double w, double ua, double ub,
                                            double va, double vb) {
   return m.dti * w *
-         (m.dtdxpo * (ua * m.dlyuw - ub * m.dlyue) / m.dlyp +
-          m.dtdyo * (va * m.dlxvs - vb * m.dlxvn) / m.dlxp);
+         (div_by(m.dtdxpo * (ua * m.dlyuw - ub * m.dlyue), m.dlyp, m.rlyp) +
+          div_by(m.dtdyo * (va * m.dlxvs - vb * m.dlxvn), m.dlxp, m.rlxp));
 }
 
 // The column passes of OCCLIT.  A block holds 32 neighbouring columns of one
