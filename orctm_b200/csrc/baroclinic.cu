@@ -875,7 +875,7 @@ void launch_occlit(const Geo& G, const BaroArgs& b, const ThermoFields& f, const
   const dim3 ob(32, kOcG);
   const int nb = (G.L.ie + 32) / 32;
   const size_t sm1 = sizeof(double) * 32 * G.L.ke;
-  if (2 * sm1 > 48 * 1024) {  // columns above 96 levels: the opt-in, one value for every caller
+  if (2 * sm1 + 1024 > 48 * 1024) {  // with the static part: the opt-in, one value for every caller
     const int most = (int)(sizeof(double) * 32 * kMaxKe);
     cudaFuncSetAttribute(k_occlit_wo, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_occlit_wpo, cudaFuncAttributeMaxDynamicSharedMemorySize, most);

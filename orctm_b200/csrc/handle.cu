@@ -825,6 +825,7 @@ int alloc_rb(orctm_handle* h, RbVectors<T>& v) {
     ORCTM_CUDA_OK(cudaStreamSynchronize(h->stream));
     coarse_plan(co, mu);
   }
+  v.coarse = h->R.co.on && !rb_small<T>(h->R);
   const size_t n2 = (size_t)RbCoarse::kModes * h->R.plane2;
   if ((!v.rho && (st = h->dev_alloc(&v.rho, n2))) || (!v.cc && (st = h->dev_alloc(&v.cc, n2)))) return st;
   if ((st = h->dev_alloc(&v.km, rb_tiles(h->R, sizeof(T)))) || (st = h->dev_alloc(&v.db, n))) return st;
@@ -866,7 +867,7 @@ void pcg_iteration(orctm_handle* h) {
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, h->stream));
-  if (h->R.co.on) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
+  if (v.coarse) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
 }
 
 template <typename T>
@@ -937,7 +938,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     it = h->hS->iter;
     conv = h->hS->converged;
   } else {
-    if (h->R.co.on) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
+    if (v.coarse) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
     ORCTM_CUDA_OK(cudaGetLastError());
   }
   if (!small && !h->prof && maxit >= kPcgChunk) {
@@ -950,7 +951,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     // convergence the chunk's remaining kernels return at once
     it = h->hS->iter;
     conv = h->hS->converged;
-    add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * ((h->R.co.on ? 4 : 3) * kPcgChunk + 1));
+    add_launches((long long)((it + kPcgChunk - 1) / kPcgChunk) * ((v.coarse ? 4 : 3) * kPcgChunk + 1));
   }
   while (!conv && it < maxit) {
     pcg_iteration<T>(h);

@@ -31,7 +31,7 @@ struct RbCoarse {
   float *ce, *cs;             // couplings to (i + 1, j) and (i, j + 1)
   float* sc;                  // diagonal^(-1/2), 0 on land
   float* mu;                  // largest sum of a column's couplings over its diagonal
-  bool on;                    // whether the iterations use it
+  bool on;                    // whether it saves iterations
   int steps[kModes];          // Chebyshev steps, for eigenvalues from lmin to 1
   float lmin[kModes], gain[kModes];
 };
@@ -60,6 +60,7 @@ struct RbVectors {
   int* km;                    // deepest wet level of each tile, red then black
   T* rho;                     // the residual's products with the profiles (2D, per profile)
   float* cc;                  // the coarse correction z + sum phi cc
+  bool coarse;                // whether the iterations make it
 };
 
 // Device-resident scalars of one Krylov solve.
@@ -239,7 +240,9 @@ template <typename T>
 void launch_rb_coarse(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st);
 void launch_coarse_setup(const Geo& G, const PoissonGeo& P, const RbGeo& R, cudaStream_t st);
 void coarse_plan(RbCoarse& co, const float* mu);
-// the whole loop in one kernel, on small grids; false: not launched
+// the whole loop in one kernel, on small grids (rb_small); false: not launched
+template <typename T>
+bool rb_small(const RbGeo& R);
 template <typename T>
 bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit, cudaStream_t st);
 template <typename T>

@@ -1554,7 +1554,7 @@ void launch_rb_before(const RbGeo& R, SolverState* S, const double* b, const RbV
                                                     (const float*)nullptr, s.ntiles, s.nt);
     const Shape c = shape_of<k_rb_col<L, true>, L>(R, m2);
     k_rb_col<L, true><<<c.grid, L::NT, m2, st>>>(R, S, v.r, (const T*)nullptr, v.z, v.db, v.km, b, v.ub,
-                                                 R.co.on ? v.rho : (T*)nullptr, c.ntiles, c.nt);
+                                                 v.coarse ? v.rho : (T*)nullptr, c.ntiles, c.nt);
   });
   add_launches(2);
 }
@@ -1566,7 +1566,7 @@ void launch_rb_red(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaSt
     constexpr size_t m = RedStage<L, kIter>::smem;
     const Shape s = shape_of<k_rb_red<L, kIter>, L>(R, m);
     k_rb_red<L, kIter><<<s.grid, L::NT, m, st>>>(R, S, v.z, v.u, v.dr, v.km, nullptr, nullptr,
-                                                 R.co.on ? v.cc : (const float*)nullptr, s.ntiles, s.nt);
+                                                 v.coarse ? v.cc : (const float*)nullptr, s.ntiles, s.nt);
   });
   count_launch();
 }
@@ -1578,7 +1578,7 @@ void launch_rb_black(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cuda
     constexpr size_t m = BlackStage<L>::smem;
     const Shape s = shape_of<k_rb_black<L>, L>(R, m);
     k_rb_black<L><<<s.grid, L::NT, m, st>>>(R, S, v.z, v.u, v.p, v.x, v.q, v.km,
-                                           R.co.on ? v.cc : (const float*)nullptr, s.ntiles, s.nt);
+                                           v.coarse ? v.cc : (const float*)nullptr, s.ntiles, s.nt);
   });
   count_launch();
 }
@@ -1590,7 +1590,7 @@ void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaSt
     constexpr size_t m = ColStage<L, false>::smem;
     const Shape s = shape_of<k_rb_col<L, false>, L>(R, m);
     k_rb_col<L, false><<<s.grid, L::NT, m, st>>>(R, S, v.r, v.q, v.z, v.db, v.km, nullptr, (const T*)nullptr,
-                                                 R.co.on ? v.rho : (T*)nullptr, s.ntiles, s.nt);
+                                                 v.coarse ? v.rho : (T*)nullptr, s.ntiles, s.nt);
   });
   count_launch();
 }
@@ -1598,7 +1598,7 @@ void launch_rb_col(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaSt
 // The coarse correction of z; follows every k_rb_col of the iterations, and the first
 template <typename T>
 void launch_rb_coarse(const RbGeo& R, SolverState* S, const RbVectors<T>& v, cudaStream_t st) {
-  if (!R.co.on) return;
+  if (!v.coarse) return;
   const int inner = kCoEdge - 4 * (std::max(R.co.steps[0], R.co.steps[1]) - 1);
   const int ntx = (R.ie - 2 + inner - 1) / inner, nty = (R.je - 2 + inner - 1) / inner;
   const long long n = (long long)ntx * nty * RbCoarse::kModes;
@@ -1649,8 +1649,23 @@ void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, doub
   add_launches(2);
 }
 
-// Whether the grid is small enough for k_rb_small (a tile per resident block, and
-// columns of up to 104 levels: one shape of block), which it then launches.
+// Whether the grid is small enough for k_rb_small: a tile per resident block, and
+// columns of up to 104 levels (one shape of block).  It does without the coarse
+// space: with it the separate kernels take as long at the largest such grids (97 x 131
+// x 41: 1.9 ms a step both ways) and longer on a slice (640 x 1 x 50: 9.4 ms against 4.9).
+template <typename T>
+bool rb_small(const RbGeo& R) {
+  bool fits = false;
+  with_split<T>(R.ke, [&](auto* l) {
+    using L = ORCTM_LANE(l);
+    if constexpr (L::GROUPS == 8) {
+      const Shape s = shape_of<k_rb_small<L>, L>(R, small_smem<L>());
+      fits = s.grid >= s.ntiles;
+    }
+  });
+  return fits;
+}
+
 template <typename T>
 bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit,
                      cudaStream_t st) {
@@ -1675,6 +1690,7 @@ bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int 
 }
 
 #define ORCTM_RB(T)                                                                              \
+  template bool rb_small<T>(const RbGeo&);                                                      \
   template bool launch_rb_small<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
   template void launch_rb_setup<T>(const Geo&, const PoissonGeo&, const RbGeo&, const RbVectors<T>&, \
                                    cudaStream_t);                                                \
