@@ -406,12 +406,13 @@ __global__ void k_visc_speed(Geo G, const double* __restrict__ uoo, const double
 // by level: the scans of tridiag.cuh differ from it in the last digits, which the
 // convective switches of the whole step amplify (to 4e-8 of u after twenty
 // steps of the laboratory tank, where this form stays bit for bit).
+// Both directions are one launch, the grid's z index: 256 x 256 columns fill a fifth
+// of the chip's warps.
 template <int DIR, int U>
-__global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* __restrict__ X,
-                                                          const double* __restrict__ keep,
-                                                          const double* __restrict__ avo,
-                                                          const double* __restrict__ speed,
-                                                          double* __restrict__ O) {
+__device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__ X,
+                                        const double* __restrict__ keep,
+                                        const double* __restrict__ avo,
+                                        const double* __restrict__ speed, double* __restrict__ O) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
@@ -505,6 +506,19 @@ __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* _
       O[base + (l - 1) * pl] = nxt;
     }
   }
+}
+template <int U>
+__global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* __restrict__ xu,
+                                                          const double* __restrict__ xv,
+                                                          const double* __restrict__ keepu,
+                                                          const double* __restrict__ keepv,
+                                                          const double* __restrict__ avo,
+                                                          const double* __restrict__ spu,
+                                                          const double* __restrict__ spv,
+                                                          double* __restrict__ ou,
+                                                          double* __restrict__ ov) {
+  if (blockIdx.z == 0) visc_uv<0, U>(G, xu, keepu, avo, spu, ou);
+  else visc_uv<1, U>(G, xv, keepv, avo, spv, ov);
 }
 
 // implicit vertical diffusion of w, levels 2..KE (ocvisc.f90:225-270); the
@@ -832,9 +846,9 @@ void launch_ocvisc(const Geo& G, const double* uoo, const double* voe, const dou
   const dim3 b2(32, 4), bc(32, kVertBlock / 32), b3(32, 4);
   k_visc_speed<<<grid2(IE + 1, JE + 1, b2), b2, 0, st>>>(G, uoo, voe, spu, spv);
   count_launch();
-  k_visc_uv_b<0, 4><<<grid2(IE + 1, JE + 1, bc), bc, 0, st>>>(G, uoo, uko, avo, spu, ukv);
-  count_launch();
-  k_visc_uv_b<1, 4><<<grid2(IE + 1, JE + 1, bc), bc, 0, st>>>(G, voe, vke, avo, spv, vkv);
+  dim3 gv = grid2(IE + 1, JE + 1, bc);
+  gv.z = 2;
+  k_visc_uv_b<4><<<gv, bc, 0, st>>>(G, uoo, voe, uko, vke, avo, spu, spv, ukv, vkv);
   count_launch();
   with_tri_split(KE, [&](auto* l) {
     using Ln = std::remove_pointer_t<decltype(l)>;
