@@ -14,6 +14,8 @@
 // thicknesses and Thomas pivots) use div_nr (within 1 ulp of IEEE division).
 #include <type_traits>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "ops.h"
 #include "tridiag.cuh"
@@ -234,7 +236,8 @@ constexpr int kHbLx = kHbX + 2, kHbLy = kHbY + 2;   // Laplacian tile
 constexpr int kHbT = kHbTx * kHbTy, kHbL = kHbLx * kHbLy, kHbN = kHbX * kHbY;
 constexpr int kHbTf = (kHbT + kHbN - 1) / kHbN, kHbLf = (kHbL + kHbN - 1) / kHbN;
 
-__global__ void __launch_bounds__(kHbN) k_tdiff_hbih(Geo G, TrPtrs tp, int ntr,
+template <bool SPLIT>
+__global__ void __launch_bounds__(kHbN) k_tdiff_hbih(Geo G, TrPtrs tp, int ntr, int levels,
                                                      const double* __restrict__ zo) {
   __shared__ double ts[kHbT];
   __shared__ double ls[kHbL];
@@ -310,24 +313,28 @@ __global__ void __launch_bounds__(kHbN) k_tdiff_hbih(Geo G, TrPtrs tp, int ntr,
   const int me_t = (ty + 2) * kHbTx + (tx + 2), me_l = (ty + 1) * kHbLx + (tx + 1);
   const int own = cell ? G.L.at(i, j, 0) : 0;
   auto wet_at = [](int kb, int K) { return K <= kb ? 1.0 : 0.0; };
-  for (int n = 0; n < ntr; ++n) {
+  // all tracers and levels, or (SPLIT) a tracer and a part of the levels
+  const int n0 = SPLIT ? blockIdx.z % ntr : 0, n1 = SPLIT ? n0 + 1 : ntr;
+  const int K0 = SPLIT ? 1 + (blockIdx.z / ntr) * levels : 1;
+  const int K1 = SPLIT ? min(KE, K0 + levels - 1) : KE;
+  for (int n = n0; n < n1; ++n) {
     const double* __restrict__ T = tp.in[n];
     double* __restrict__ O = tp.out[n];
     double nx[kHbTf];
-#pragma unroll
-    for (int f = 0; f < kHbTf; ++f) nx[f] = tin[f] ? T[toff[f]] : 0.0;
-    for (int K = 1; K <= KE; ++K) {
+  #pragma unroll
+    for (int f = 0; f < kHbTf; ++f) nx[f] = tin[f] ? T[toff[f] + plane * (K0 - 1)] : 0.0;
+    for (int K = K0; K <= K1; ++K) {
       __syncthreads();  // the previous level's tiles are no longer read
-#pragma unroll
+  #pragma unroll
       for (int f = 0; f < kHbTf; ++f)
         if (tval[f]) ts[tid + f * kHbN] = nx[f];
-      if (K < KE) {
-#pragma unroll
+      if (K < K1) {
+  #pragma unroll
         for (int f = 0; f < kHbTf; ++f)
           if (tin[f]) nx[f] = T[toff[f] + plane * K];
       }
       __syncthreads();
-#pragma unroll
+  #pragma unroll
       for (int f = 0; f < kHbLf; ++f) {
         const LapPos& L = lp[f];
         if (L.e >= kHbL) continue;
@@ -834,7 +841,21 @@ void launch_octdiff_hbih(const Geo& G, int ntr, const double* const* in, double*
     tp.out[n] = out[n];
   }
   const dim3 b(kHbX, kHbY);
-  k_tdiff_hbih<<<grid2(G.L.ie, G.L.je, b), b, 0, st>>>(G, tp, ntr, zo);
+  dim3 gr = grid2(G.L.ie, G.L.je, b);
+  // On planes of less than three blocks per SM a block takes one tracer and a part of
+  // the levels, at least eight: four rounds of blocks, where one block for all left
+  // the chip waiting (OCTDIFF of 512 x 1 x 60 0.131 ms, now 0.071, 97 x 131 x 41 0.150 and
+  // 0.100, 256 x 256 x 60 0.38 and 0.33); on larger ones it marches through all, its
+  // geometry loaded once (413 x 311 x 83 0.79 ms against 0.81 in parts).
+  const int blocks = gr.x * gr.y;
+  if (blocks < 3 * 148) {
+    const int parts = std::min((4 * 2 * 148 + blocks * ntr - 1) / (blocks * ntr), (G.L.ke + 7) / 8);
+    const int levels = (G.L.ke + parts - 1) / parts;
+    gr.z = ntr * ((G.L.ke + levels - 1) / levels);
+    k_tdiff_hbih<true><<<gr, b, 0, st>>>(G, tp, ntr, levels, zo);
+  } else {
+    k_tdiff_hbih<false><<<gr, b, 0, st>>>(G, tp, ntr, G.L.ke, zo);
+  }
   count_launch();
 }
 
