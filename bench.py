@@ -34,11 +34,15 @@ FALLBACK_HBM_GBS = 6650.0
 
 # Algorithmic bytes per interior cell per launch of each launcher group
 # (each distinct array the math needs read once, each output written once;
-# thickness/mask geometry is compressed to 2D and counts 0 B).
+# thickness/mask geometry is compressed to 2D and counts 0 B).  The Poisson
+# iteration works on the black columns' vectors (half of the cells): "pcg_spmv" is
+# the black kernel (x, p, z, u in; x, p, q out), "pcg_col" the average over the red
+# kernel (z, u in; u out; pivots in doubles), the column kernel (r, q in; r, z out; pivots
+# in floats) and the coarse correction, which moves planes only.
 BYTES_PER_CELL_F64 = {
     "ocuad": 40, "ocvad": 40, "ocwad": 40, "ocadpo": 40,
     "ocvisc": 56, "nh_rhs": 56, "nh_post": 56,
-    "pcg_spmv": 32, "pcg_col": 56, "resid": 24,
+    "pcg_spmv": 28, "pcg_col": (16 + 18 + 0) / 3, "resid": 24,
 }
 
 
@@ -388,8 +392,8 @@ def main():
     ap.add_argument("--no-whole-step", action="store_true",
                     help="skip the whole-step (orctm_step_full) measurement")
     ap.add_argument("--tuning", type=lambda s: tuple(int(v) for v in s.split(",")), default=None,
-                    help="COL,SPMV: pin the FP64 Poisson kernel variants instead of autotuning "
-                         "(profiling a given variant)")
+                    help="COL,SPMV: variant numbers passed to orctm_set_tuning (accepted; "
+                         "the Poisson kernels have one form)")
     ap.add_argument("--nvtx", action="store_true",
                     help="wrap the event-timed FP64 steps (every solver iteration launched "
                          "on its own) in the NVTX range fp64_steps, for an ncu launch list "
@@ -467,7 +471,7 @@ def main():
     mixed["solver_speedup_vs_fp64"] = poisson_ms / mixed["poisson_ms"]
     mixed["vs_fp64"] = compare_forms(inst, gpu, gpu2, nsteps)
     tuning = {"fp64": list(gpu.tuning("fp64")), "fp32_refined": list(gpu2.tuning("fp32_refined")),
-              "meaning": "(column-kernel variant, stencil-kernel variant) picked by the autotuner"}
+              "meaning": "variant numbers as reported by orctm_get_tuning; the kernels have one form"}
     gpu2.close()
 
     # ---- roofline of the dominant kernel --------------------------------
@@ -483,13 +487,8 @@ def main():
     traffic = None
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
-            tj = json.load(f)
-        if top in tj:
-            # measured per variant (DRAM bytes per cell of the whole grid):
-            # reported only for the variant the tuner picked
-            var = str(tuning["fp64"][0] if top == "pcg_col" else tuning["fp64"][1])
-            per = tj[top].get("by_variant", {}).get(var)
-            traffic = per * cells if per is not None else None
+            per = json.load(f).get(top, {}).get("bytes_per_cell")
+        traffic = per * cells if per is not None else None
     except Exception:
         pass
     roofline = {"bound": "hbm", "kernel": top, "achieved": round(achieved, 1), "peak": hbm,

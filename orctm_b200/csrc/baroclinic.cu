@@ -22,10 +22,10 @@
 //
 // Work per launch: OCTHER is one thread per water column (the level loops
 // carry running values: PO, the wind-mixing decay); OCMODMOM is one launch
-// per Coriolis iteration over all points, ping-ponging UK1O / VK1E / W
+// per three Coriolis iterations over all points, ping-ponging UK1O / VK1E / W
 // between two buffers, plus a column pass for the vertical sums; OCCLIT is a
 // column pass per iteration for the velocities (their vertical sums) and one
-// for WPO (its running sums in both directions).
+// for WPO (its running sums in both directions), eight threads to a column.
 #include "common.cuh"
 #include "ops.h"
 
