@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(32 * kOcG) k_occlit_wo(Geo G, ThermoFields f,
   extern __shared__ double oc_sm[];
   double (*s)[32] = reinterpret_cast<double (*)[32]>(oc_sm);
   const int c = threadIdx.x, g = threadIdx.y;
-  const int i = blockIdx.x * 32 + c, j = blockIdx.y + 1;
+  const int nb = (G.L.ie + 32) / 32;
+  const int i = blockIdx.x % nb * 32 + c, j = blockIdx.x / nb + 1;
   const int IE = G.L.ie, KE = G.L.ke;
   const bool in = i >= 1 && i <= IE;
   const int ij = G.L.at2(in ? i : 1, j), pl = G.L.plane, P = G.L.P;
@@ -671,7 +672,8 @@ __global__ void __launch_bounds__(32 * kOcG) k_occlit_uv(Geo G, BaroArgs b, Baro
   double (*dw)[32] = s + G.L.ke;  // metric * WPO difference
   __shared__ double tot[32];
   const int c = threadIdx.x, g = threadIdx.y;
-  const int i = blockIdx.x * 32 + c, j = blockIdx.y + 1;
+  const int nb = (G.L.ie + 32) / 32;
+  const int i = blockIdx.x % nb * 32 + c, j = blockIdx.x / nb + 1;
   const int IE = G.L.ie, KE = G.L.ke;
   const bool u = blockIdx.z == 0;
   if (u && j < 2) return;  // j <= JE - 1 by the grid
@@ -724,7 +726,8 @@ __global__ void __launch_bounds__(32 * kOcG) k_occlit_wpo(
   extern __shared__ double oc_sm[];
   double (*s)[32] = reinterpret_cast<double (*)[32]>(oc_sm);
   const int c = threadIdx.x, g = threadIdx.y;
-  const int i = blockIdx.x * 32 + c, j = blockIdx.y + 1;
+  const int nb = (G.L.ie + 32) / 32;
+  const int i = blockIdx.x % nb * 32 + c, j = blockIdx.x / nb + 1;
   const int IE = G.L.ie, KE = G.L.ke;
   const bool in = i >= 1 && i <= IE;
   const int ij = G.L.at2(in ? i : 1, j), pl = G.L.plane, P = G.L.P;
@@ -873,7 +876,7 @@ void launch_occlit(const Geo& G, const BaroArgs& b, const ThermoFields& f, const
   const dim3 cb(32, 4);
   k_occlit_prep<<<grid3(G.L.ie + 1, G.L.je + 1, G.L.ke, cb), cb, 0, st>>>(G, f, uko, vke, uk1o, vk1e, bruva);
   const dim3 ob(32, kOcG);
-  const int nb = (G.L.ie + 32) / 32;
+  const int nb = (G.L.ie + 32) / 32;  // rows in x: y ends at 65535
   const size_t sm1 = sizeof(double) * 32 * G.L.ke;
   if (2 * sm1 + 1024 > 48 * 1024) {  // with the static part: the opt-in, one value for every caller
     const int most = (int)(sizeof(double) * 32 * kMaxKe);
@@ -881,15 +884,15 @@ void launch_occlit(const Geo& G, const BaroArgs& b, const ThermoFields& f, const
     cudaFuncSetAttribute(k_occlit_wpo, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(k_occlit_uv, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * most);
   }
-  k_occlit_wo<<<dim3(nb, G.L.je), ob, sm1, st>>>(G, f, uko, vke, wo, wpo);
+  k_occlit_wo<<<nb * G.L.je, ob, sm1, st>>>(G, f, uko, vke, wo, wpo);
   count_launch();
   count_launch();
   const int itermax = 8;
   for (int iter = 1; iter <= itermax; ++iter) {
-    k_occlit_uv<<<dim3(nb, G.L.je - 1, 2), ob, 2 * sm1, st>>>(G, b, bf, uko, vke, uk1o, vk1e, wpo);
+    k_occlit_uv<<<dim3(nb * (G.L.je - 1), 1, 2), ob, 2 * sm1, st>>>(G, b, bf, uko, vke, uk1o, vk1e, wpo);
     count_launch();
     if (iter == itermax) break;
-    k_occlit_wpo<<<dim3(nb, G.L.je), ob, sm1, st>>>(G, b, f, uko, vke, wo, bruva, wpo, contrij,
+    k_occlit_wpo<<<nb * G.L.je, ob, sm1, st>>>(G, b, f, uko, vke, wo, bruva, wpo, contrij,
                                                     iter == 1 ? 0. : 1.);
     count_launch();
   }

@@ -537,8 +537,9 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
   constexpr int LC = Ln::LC;
   __shared__ TriScan<Ln, 1> scan;
   const Ln t;
-  const int i = blockIdx.x * Ln::W + t.c, j = blockIdx.y + 1;
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke, pl = G.L.plane;
+  const int nb = (IE + Ln::W) / Ln::W;
+  const int i = blockIdx.x % nb * Ln::W + t.c, j = blockIdx.x / nb + 1;
   const bool valid = i >= 1 && i <= IE;
   const bool interior = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
   const int base = G.L.at(i, j, t.K0 + 1), ij = G.L.at2(i, j);  // level K0 + 2
@@ -873,8 +874,8 @@ void launch_ocvisc(const Geo& G, const double* uoo, const double* voe, const dou
   count_launch();
   with_tri_split(KE, [&](auto* l) {
     using Ln = std::remove_pointer_t<decltype(l)>;
-    const int nb = (IE + Ln::W) / Ln::W;
-    k_visc_w<Ln><<<dim3(nb, JE), Ln::NT, 0, st>>>(G, wno, avo, wnv);
+    const int nb = (IE + Ln::W) / Ln::W;  // rows in x: y ends at 65535
+    k_visc_w<Ln><<<nb * JE, Ln::NT, 0, st>>>(G, wno, avo, wnv);
   });
   count_launch();
   const int chunks = (KE + 1 + kViscLevels - 1) / kViscLevels;

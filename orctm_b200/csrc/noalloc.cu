@@ -73,8 +73,9 @@ __global__ void __launch_bounds__(Ln::NT) k_na_vert(NaArgs a, const double* __re
   constexpr int LC = Ln::LC;
   __shared__ TriScan<Ln, 1> scan;
   const Ln t;
-  const int i = blockIdx.x * Ln::W + t.c + 1, j = blockIdx.y + 1;
   const int IE = a.IE, JE = a.JE, KE = a.KE, pl = IE * JE;
+  const int nb = (IE + Ln::W - 1) / Ln::W;
+  const int i = blockIdx.x % nb * Ln::W + t.c + 1, j = blockIdx.x / nb + 1;
   const bool valid = i <= IE;
   const bool interior = i >= 2 && i <= IE - 1 && j >= 2 && j <= JE - 1;
   const int base = (int)p3(a, i, j, t.K0 + 1);
@@ -292,7 +293,7 @@ extern "C" int orctm_octdiff_noalloc(const orctm_octdiff_noalloc_args* in) {
   const bool bih = in->aulapts > in->almzer;
   with_tri_split(in->ke, [&](auto* l) {
     using Ln = std::remove_pointer_t<decltype(l)>;
-    const dim3 gc((in->ie + Ln::W - 1) / Ln::W, in->je);
+    const int gc = (in->ie + Ln::W - 1) / Ln::W * in->je;  // rows in x: y ends at 65535
     k_na_vert<Ln><<<gc, Ln::NT, 0, s>>>(a, in->tracer_in, bih ? vdiff : in->tracer_out);
   });
   count_launch();

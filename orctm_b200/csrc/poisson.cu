@@ -1356,10 +1356,11 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_rb_after(RbGeo R, SolverState* S, const T* __restrict__ p,
                                                   T* __restrict__ d, double* __restrict__ x) {
   const int W = R.width((int)sizeof(T));
-  const int m = 1 + blockIdx.x * W + threadIdx.x % W;
-  const int K = blockIdx.z * (128 / W) + threadIdx.x / W + 1, j = blockIdx.y + 2;
+  const int nb = R.nt(W), b = blockIdx.x % nb;
+  const int m = 1 + b * W + threadIdx.x % W;
+  const int K = blockIdx.z * (128 / W) + threadIdx.x / W + 1, j = blockIdx.x / nb + 2;
   if (m > R.M || K > wet_levels(R.col[1].kk[m + R.P2 * j], 0)) return;
-  const int o = ((j * R.nt(W) + (int)blockIdx.x) * R.ke + K - 1) * W + threadIdx.x % W;
+  const int o = ((j * nb + b) * R.ke + K - 1) * W + threadIdx.x % W;
   T v = T(0);
   if (S->iter > 0) v = fma((T)S->alpha_prev, p[o], d[o]);
   d[o] = v;
@@ -1637,7 +1638,7 @@ template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x,
                      cudaStream_t st) {
   const int W = R.width((int)sizeof(T));
-  const dim3 grid(R.nt(W), R.je - 2, (R.ke + 128 / W - 1) / (128 / W));
+  const dim3 grid(R.nt(W) * (R.je - 2), 1, (R.ke + 128 / W - 1) / (128 / W));
   k_rb_after<T><<<grid, 128, 0, st>>>(R, S, v.p, v.x, x);
   with_split<T>(R.ke, [&](auto* l) {
     using L = ORCTM_LANE(l);

@@ -124,6 +124,16 @@ def test_troneu_bit_identical_at_tile_edges(nx, ny, niter):
     gpu.close()
 
 
+def test_planes_of_more_rows_than_a_grid_has_in_y(monkeypatch):
+    """66 000 rows: launches that take rows one by one count them in x."""
+    tall = _make("c2", 2, 66000, 7, dx=2e4)  # within the scratch-free entry's cells
+    monkeypatch.setattr(test_zz_no_alloc, "instance", lambda case: tall)
+    test_zz_no_alloc.test_octdiff_noalloc_matches_handle_path_and_oracle("edge", False)
+    test_gpu_parity.test_momentum_diffusion(("edge", tall))
+    test_gpu_baroclinic.test_octher_ocmodmom_occlit_bit_identical("c2", dict(nx=2, ny=66000, nz=7, dx=2e4), 0, False)
+    test_poisson_residual_by_the_oracles_matrix(("c2", 2, 66000, 7, 2e4), "fp64")
+
+
 def test_copies_of_fields_larger_than_the_staging_buffer():
     """A field of 80 MB in several stagings, at every staggering, there and back."""
     inst = _make("c2", 401, 307, 80)
