@@ -778,7 +778,10 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
   if (grid_sum<1, Ln::NT>(w, S)) {
     S->pq = w[0];
     S->alpha = S->rho / w[0];
-    if (S->converged == 0 && !(w[0] > 0.0) && !(w[0] < 0.0)) S->converged = 3;  // breakdown
+    if (S->converged == 0 && !(w[0] > 0.0) && !(w[0] < 0.0)) {
+      S->converged = 3;  // breakdown: x has the last full step, and p is no direction to follow
+      S->alpha_prev = 0.0;
+    }
   }
 }
 
@@ -1351,7 +1354,8 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
 }
 
 // The black correction: the x update that the last iteration left open (none
-// before the first), and its addition to the solution (full layout).
+// before the first, nor with alpha_prev = 0 after a breakdown, where p need not be
+// finite), and its addition to the solution (full layout).
 template <typename T>
 __global__ void __launch_bounds__(128) k_rb_after(RbGeo R, SolverState* S, const T* __restrict__ p,
                                                   T* __restrict__ d, double* __restrict__ x) {
@@ -1361,8 +1365,9 @@ __global__ void __launch_bounds__(128) k_rb_after(RbGeo R, SolverState* S, const
   const int K = blockIdx.z * (128 / W) + threadIdx.x / W + 1, j = blockIdx.x / nb + 2;
   if (m > R.M || K > wet_levels(R.col[1].kk[m + R.P2 * j], 0)) return;
   const int o = ((j * nb + b) * R.ke + K - 1) * W + threadIdx.x % W;
-  T v = T(0);
-  if (S->iter > 0) v = fma((T)S->alpha_prev, p[o], d[o]);
+  const T alpha = (T)S->alpha_prev;
+  T v = S->iter > 0 ? d[o] : T(0);
+  if (S->iter > 0 && alpha != T(0)) v = fma(alpha, p[o], v);
   d[o] = v;
   const double scale = sizeof(T) == 4 ? sqrt(S->res_rr) : 1.0;
   const int f = black_i(m, j) + 2 * (R.P2 * j + R.plane2 * (K - 1));
