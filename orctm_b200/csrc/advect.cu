@@ -79,25 +79,47 @@ __device__ __forceinline__ Fl<N> zero_fl() {
   return f;
 }
 
+// Infinities and NaN.  In the reference's expressions a transport without outflow is
+// 0 times an average, which is NaN if that is not finite, and MIN(cap, NaN) is cap.
+// The short cuts of `limited` do not show that, so a march notes whether one of its
+// values was not finite (Seen), and is then done again in full, without short cuts.
+// The values are noted where they are used: noted at its load, a value in flight is
+// waited for.  OCUAD + OCVAD + OCWAD + OCADPO of three tracers on 301 x 403 x 67: 1.86 ms,
+// as without the note; 2.27 with short cuts that are safe one by one.
+struct Seen {
+  unsigned top = 0;  // the largest high word without its sign
+  __device__ __forceinline__ double operator()(double x) {
+    top = max(top, (unsigned)__double2hiint(x) & 0x7fffffffu);
+    return x;
+  }
+  // a value that is 0 or above, or NaN
+  __device__ __forceinline__ void nonneg(double x) { top = max(top, (unsigned)__double2hiint(x)); }
+  __device__ __forceinline__ bool nonfinite() const { return top >= 0x7ff00000u; }
+};
+
 // The limited upwind pair: TRP takes the average with ta, TRM with tb; SCHA is
 // multiplied by the masks' product w (0 or 1), SCH capped by cap, and 0 with
 // flat.  (ocadpo.f90:107-125, 203-232; ocuad.f90:41-52 without masks)  Where a
 // factor makes the result 0 (no outflow: land; SCHA = 0: a uniform field, a
-// local extremum) the steps it makes idle are passed by, which a whole warp often can.
-__device__ __forceinline__ void limited(double up, double um, double t, double ta, double tb,
-                                        double vol, double cap, bool w, bool flat, double& trp,
-                                        double& trm) {
+// local extremum) the steps it makes idle are passed by, which a whole warp often
+// can; in full they are not (an outflow of infinity divides to 0 there, NaN stays).
+__device__ __forceinline__ void limited(bool full, double up, double um, double t, double ta,
+                                        double tb, double vol, double cap, bool w, bool flat,
+                                        double& trp, double& trm) {
   trp = trm = 0.;
   const double out = up + um;
-  if (out == 0.) return;
+  if (out == 0. && !full) return;
   double sch = 0.;
-  if (w && !flat) {
+  if ((w || full) && !flat) {
     const double abl = fabs(ta - tb);
     const double zwabl = fabs(ta + tb - 2. * t);
     const double num = abl - zwabl;
-    if (!(num <= 0.)) {
-      const double scha = fmx(0., div_in_range(num, abl + 1.E-20));
-      sch = fmn(cap, div_in_range(scha * vol, out + 1.E-20));
+    if (!(num <= 0.) || full) {
+      double scha = fmx(0., div_in_range(num, abl + 1.E-20));
+      if (!w) scha = 0. * scha;
+      const double x = scha * vol;
+      sch = fmn(cap, div_in_range(x, out + 1.E-20));
+      if (full && out > 1e300) sch = fmn(cap, 0. * x);
     }
   }
   const double schi = 1. - sch;
@@ -122,20 +144,23 @@ __device__ __forceinline__ double from_east(double x) { return __shfl_down_sync(
 constexpr int kZxCells = 28, kZxRows = 4;
 
 // ocadpo.f90:94-232, ocuad.f90:20-148, ocvad.f90:20-148, ocwad.f90:14-...;
-// the block's levels are klen from 1 + klen blockIdx.z
+// the block's levels are klen from 1 + klen blockIdx.z (full: without short cuts).
+// Returns whether a value of the march was not finite, for the whole warp
 template <int VAR, int N>
-__global__ void __launch_bounds__(32 * kZxRows)
-    k_adv_zx(Geo G, TrIO io, const double* __restrict__ wo, const double* __restrict__ zo,
-             const double* __restrict__ uko, double* __restrict__ Vo, int klen) {
+__device__ __forceinline__ bool march_zx(const Geo& G, const TrIO& io, const double* __restrict__ wo,
+                                         const double* __restrict__ zo,
+                                         const double* __restrict__ uko, double* __restrict__ Vo,
+                                         int klen, bool full) {
   using R = Rng<VAR>;
+  Seen seen;
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke, pl = G.L.plane;
   const int lane = threadIdx.x;
   const int i = R::i0 + blockIdx.x * kZxCells + lane - 2;
   const int j = R::j0 + blockIdx.y * kZxRows + threadIdx.y;
-  if (j > JE) return;  // the whole warp
+  if (j > JE) return false;  // the whole warp
   const int kbot = VAR == V_WAD ? KE + 1 : KE;  // levels of the field
   const int Ka = 1 + blockIdx.z * klen, Kb = min(kbot, Ka + klen - 1);
-  if (Ka > kbot) return;
+  if (Ka > kbot) return false;
   const bool cell = i >= R::i0 && i <= IE;             // a point of the field
   const bool own = cell && lane >= 2 && lane < 2 + kZxCells;
   const int ij = G.L.at2(i, j), b0 = G.L.at(i, j, 0);
@@ -150,8 +175,8 @@ __global__ void __launch_bounds__(32 * kZxRows)
   const double dlyc = !cell ? 0. : VAR == V_UAD ? G.dlyu[ij] : VAR == V_VAD ? G.dlyv[ij] : G.dlyp[ij];
   const double area = dlxc * dlyc;
   const double cdt = zin ? 0.5 * G.dt * G.dlyp[ij] * G.dlxp[ij] : 0.;
-  const double zij = cell && (VAR == V_ADPO || VAR == V_WAD) ? zo[ij] : 0.;
-  const double wsurf = VAR == V_ADPO && cell ? wo[b0] : 0.;
+  const double zij = cell && (VAR == V_ADPO || VAR == V_WAD) ? seen(zo[ij]) : 0.;
+  const double wsurf = VAR == V_ADPO && cell ? seen(wo[b0]) : 0.;
   auto v0 = [&](int K) {
     if (K > kb) return 0.;
     if (VAR == V_WAD) {
@@ -235,13 +260,14 @@ __global__ void __launch_bounds__(32 * kZxRows)
     Fl<N> f;
     f.wtp = cdt * (w0 + fabs(w0));
     f.wtm = cdt * (fabs(w1) - w1);
+    seen.nonneg(f.wtp + f.wtm);
     const int klo = K + 1 < KE ? K + 1 : KE;
     const double cap = VAR == V_ADPO ? (klo <= kb ? 1. : 0.)
                        : VAR == V_WAD ? (K + 1 <= KE && K + 1 <= kb ? 1. : 0.) : 1.;
     const bool flat = VAR == V_ADPO && (K == 1 || K == KE);
 #pragma unroll
     for (int n = 0; n < N; ++n)
-      limited(f.wtp, f.wtm, c[n], a[n], b[n], vol, cap, true, flat, f.trp[n], f.trm[n]);
+      limited(full, f.wtp, f.wtm, c[n], a[n], b[n], vol, cap, true, flat, f.trp[n], f.trm[n]);
     return f;
   };
   // transports of the level above the first and below the last one of WAD
@@ -271,12 +297,15 @@ __global__ void __launch_bounds__(32 * kZxRows)
       t0[n] = load_t(n, Ka);
       tu[n] = !kLast && Ka == 1 ? t0[n] : load_t(n, Ka - 1);
       tl[n] = !kLast && Ka == KE ? t0[n] : load_t(n, Ka + 1);
+      seen(tu[n]);
+      seen(t0[n]);
+      seen(tl[n]);
     }
     if (Ka > Kz) {
       const int Km = Ka - 1;
       double tuu[N];
 #pragma unroll
-      for (int n = 0; n < N; ++n) tuu[n] = !kLast && Km == 1 ? tu[n] : load_t(n, Km - 1);
+      for (int n = 0; n < N; ++n) tuu[n] = seen(!kLast && Km == 1 ? tu[n] : load_t(n, Km - 1));
       const double wu = VAR == V_WAD ? raw_w(Km - 1) : 0.;
       fm = zflux(Km, face_w(Km, wu), w0, tuu, tu, t0, v0(Km));
     } else if (VAR == V_WAD && Ka == 1) {
@@ -301,7 +330,7 @@ __global__ void __launch_bounds__(32 * kZxRows)
     double vn = 0., ww2 = 0., tll[N];
 #pragma unroll
     for (int n = 0; n < N; ++n) {
-      tll[n] = !kLast && K + 1 >= KE ? tl[n] : tn2[n];
+      tll[n] = seen(!kLast && K + 1 >= KE ? tl[n] : tn2[n]);
       tn2[n] = load_t(n, K + 3);
     }
     if (K < KE) {
@@ -349,12 +378,14 @@ __global__ void __launch_bounds__(32 * kZxRows)
     }
     const bool live = flux_here && K >= R::kL && K <= KE;
     if (!live) up = um = 0.;
+    seen.nonneg(up + um);
     const double wtp_w = from_west(up), wtm_e = from_east(um);
     const bool w3 = VAR == V_ADPO || VAR == V_WAD ? K <= kb3 : true;
     const bool upd = xup && K >= R::kL && K <= KE && K <= kb;
     double v2 = v1;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
+      seen(t1[n]);
       const double te = from_east(t1[n]), tw = from_west(t1[n]);
       double trp = 0., trm = 0.;
       if (live) {
@@ -362,7 +393,7 @@ __global__ void __launch_bounds__(32 * kZxRows)
           trp = up * t1[n];
           trm = um * t1[n];
         } else {
-          limited(up, um, t1[n], te, tw, v1, 1., w3, false, trp, trm);
+          limited(full, up, um, t1[n], te, tw, v1, 1., w3, false, trp, trm);
         }
       }
       // RN = V + WTP(I-1) - WTP(I) - WTM(I) + WTM(I+1)
@@ -383,6 +414,18 @@ __global__ void __launch_bounds__(32 * kZxRows)
       tl[n] = tll[n];
     }
   }
+  return __any_sync(kAll, seen.nonfinite());
+}
+
+// Blocks per SM: one momentum field fits 80 registers a thread, which hides more
+// latency than 96 (OCVAD's 250 us on 301 x 403 x 67 are 230 so)
+template <int VAR, int N>
+__global__ void __launch_bounds__(32 * kZxRows, N == 1 ? (VAR == V_ADPO ? 5 : 6) : 7 - N)
+    k_adv_zx(Geo G, TrIO io, const double* __restrict__ wo, const double* __restrict__ zo,
+             const double* __restrict__ uko, double* __restrict__ Vo, int klen) {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass)
+    if (!march_zx<VAR, N>(G, io, wo, zo, uko, Vo, klen, pass)) return;
 }
 
 // ---------------------------------------------------------------- y sweep ---
@@ -391,17 +434,19 @@ constexpr int kYLevels = 8;
 // ocadpo.f90:264-348, ocuad.f90:184-271, ocvad.f90:184-271, ocwad.f90:160-238;
 // jlen rows per block.  The J = 0 edge of OCVAD reads DLXU(I,0) in the
 // reference, outside DLXU's bounds; DLXV(I,0) is used.
+// Returns as march_zx, for the thread's own column.
 template <int VAR, int N>
-__global__ void __launch_bounds__(32 * kYLevels)
-    k_adv_y(Geo G, TrIO io, const double* __restrict__ V, const double* __restrict__ vke, int jlen) {
+__device__ __forceinline__ bool march_y(const Geo& G, const TrIO& io, const double* __restrict__ V,
+                                        const double* __restrict__ vke, int jlen, bool full) {
   using R = Rng<VAR>;
+  Seen seen;
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke, P = G.L.P;
   const int i = blockIdx.x * 32 + threadIdx.x;
   const int K = blockIdx.z * kYLevels + threadIdx.y + 1;
   const int kbot = VAR == V_WAD ? KE + 1 : KE;
-  if (K > kbot || i < R::i0 || i > IE) return;
+  if (K > kbot || i < R::i0 || i > IE) return false;
   const int ja = R::j0 + blockIdx.y * jlen, jb = min(JE, ja + jlen - 1);
-  if (ja > JE) return;
+  if (ja > JE) return false;
   const int lev = (K - 1) * G.L.plane + i;  // offset of row 0
   const bool klev = K >= R::kL && K <= KE;
   const bool col = klev && i >= R::iL && i <= IE - 1;  // columns that the sweep updates
@@ -409,7 +454,7 @@ __global__ void __launch_bounds__(32 * kYLevels)
     for (int j = ja; j <= jb; ++j)
 #pragma unroll
       for (int n = 0; n < N; ++n) io.out[n][lev + P * j] = io.in[n][lev + P * j];
-    return;
+    return false;
   }
   const double hdt = 0.5 * G.dt;
   const double dz = G.dzw[K - 1], dzu = VAR == V_WAD ? G.dzw[K - 2] : 0.;
@@ -461,6 +506,7 @@ __global__ void __launch_bounds__(32 * kYLevels)
     }
     f.wtp = cu * (vno + fabs(vno));
     f.wtm = cd * (fabs(fa.v) - fa.v);
+    seen.nonneg(f.wtp + f.wtm);
     const bool edge = VAR == V_UAD ? (q == 1 || q == JE) : VAR == V_VAD ? (q == 0 || q == JE) : false;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
@@ -468,7 +514,7 @@ __global__ void __launch_bounds__(32 * kYLevels)
         f.trp[n] = f.wtp * t[n];
         f.trm[n] = f.wtm * t[n];
       } else {
-        limited(f.wtp, f.wtm, t[n], tb[n], ta[n], vol, 1., masked ? w3 : true, false,
+        limited(full, f.wtp, f.wtm, t[n], tb[n], ta[n], vol, 1., masked ? w3 : true, false,
                 f.trp[n], f.trm[n]);
       }
     }
@@ -488,15 +534,19 @@ __global__ void __launch_bounds__(32 * kYLevels)
       tp[n] = t_at(n, ja - 1);
       t0[n] = t_at(n, ja);
       tn[n] = t_at(n, ja + 1);
+      seen(tpp[n]);
+      seen(tp[n]);
+      seen(t0[n]);
+      seen(tn[n]);
     }
     const int kpp = kb_at(ja - 2);
     kp = kb_at(ja - 1);
     k0 = kb_at(ja);
     kn = kb_at(ja + 1);
-    v0 = v_at(ja);
+    v0 = seen(v_at(ja));
     const Face f2 = face(ja - 2), f1 = face(ja - 1);
     fa = face(ja);
-    fp = flux(ja - 1, f2, f1, tpp, tp, t0, v_at(ja - 1), K <= min(kpp, min(kp, k0)));
+    fp = flux(ja - 1, f2, f1, tpp, tp, t0, seen(v_at(ja - 1)), K <= min(kpp, min(kp, k0)));
     fc = flux(ja, f1, fa, tp, t0, tn, v0, K <= min(kp, min(k0, kn)));
   }
   // values of the row after next, one step ahead
@@ -513,6 +563,9 @@ __global__ void __launch_bounds__(32 * kYLevels)
     for (int n = 0; n < N; ++n) t3[n] = t_at(n, j + 3);
     const Face fb = fa;
     fa = face(j + 1);
+    seen(v1);
+#pragma unroll
+    for (int n = 0; n < N; ++n) seen(tnn[n]);
     const Fl<N> fn = flux(j + 1, fb, fa, t0, tn, tnn, v1, K <= min(k0, min(kn, knn)));
     // RN = V + WTP(J+1) - WTP(J) - WTM(J) + WTM(J-1)
     const bool upd = j >= R::jL && j <= JE - 1 && K <= k0;
@@ -533,6 +586,15 @@ __global__ void __launch_bounds__(32 * kYLevels)
     kn = knn;
     knn = k3;
   }
+  return seen.nonfinite();
+}
+
+template <int VAR, int N>
+__global__ void __launch_bounds__(32 * kYLevels, N == 1 ? 4 : 2)
+    k_adv_y(Geo G, TrIO io, const double* __restrict__ V, const double* __restrict__ vke, int jlen) {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass)
+    if (!march_y<VAR, N>(G, io, V, vke, jlen, pass)) return;
 }
 
 // Levels per block of k_adv_zx and rows per block of k_adv_y: a march
