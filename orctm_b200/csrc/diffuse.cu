@@ -373,6 +373,15 @@ __global__ void __launch_bounds__(kHbN) k_tdiff_hbih(Geo G, TrPtrs tp, int ntr, 
 }
 
 // -------------------------------------------------------------- OCVISC ----
+// Infinities and NaN on land.  A mask is a factor 0 in the reference's expressions, and
+// 0 times such a value is NaN, in its own cell and in its neighbours.  The horizontal
+// passes do not load land cells unless the vertical solves, which write every level,
+// have met a value that is not finite: they note it at `bad` (element (0, 0) of SPEEDU,
+// no u-point, which k_visc_speed clears).
+__device__ __forceinline__ bool finite(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+
 // bottom speeds SPEEDU/SPEEDV (ocvisc.f90:53-104): evaluated at the single
 // level where the mask drops from 1 to 0 (or at KE when the column is full)
 __global__ void k_visc_speed(Geo G, const double* __restrict__ uoo, const double* __restrict__ voe,
@@ -419,11 +428,13 @@ template <int DIR, int U>
 __device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__ X,
                                         const double* __restrict__ keep,
                                         const double* __restrict__ avo,
-                                        const double* __restrict__ speed, double* __restrict__ O) {
+                                        const double* __restrict__ speed, double* __restrict__ O,
+                                        double* bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
   if (i > IE || j > JE) return;
+  bool ok = true;
   const bool interior = DIR == 0 ? (i >= 1 && i <= IE - 1 && j >= 2 && j <= JE - 1)
                                  : (i >= 2 && i <= IE - 1 && j >= 1 && j <= JE - 1);
   const bool valid = DIR == 0 ? (j >= 1) : (i >= 1);
@@ -431,7 +442,12 @@ __device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__
   const int pl = G.L.plane;
   const int base = G.L.at(i, j, 0);
   if (!interior) {
-    for (int K = 1; K <= KE; ++K) O[base + (K - 1) * pl] = keep[base + (K - 1) * pl];
+    for (int K = 1; K <= KE; ++K) {
+      const double v = keep[base + (K - 1) * pl];
+      ok &= finite(v);
+      O[base + (K - 1) * pl] = v;
+    }
+    if (!ok) *bad = 1.;
     return;
   }
   const ColGeo& cg = DIR == 0 ? G.gu : G.gv;
@@ -489,6 +505,7 @@ __device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__
     }
   }
   double nxt = div_nr(wet(cg, ij, KE) * yprev, t2p[KE - 1]);
+  ok &= finite(nxt);
   O[base + (KE - 1) * pl] = nxt;
   for (int l0 = KE - 1; l0 >= 1; l0 -= U) {
     double la[U], lb[U], la1[U], lb1[U], ly[U];
@@ -510,9 +527,11 @@ __device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__
       tri(l, la[u], lb[u], la1[u], lb1[u], t1, t3);
       t3 = t3 * wet(cg, ij, l + 1);
       nxt = div_nr((ly[u] - t3 * nxt) * wet(cg, ij, l), t2p[l - 1]);
+      ok &= finite(nxt);
       O[base + (l - 1) * pl] = nxt;
     }
   }
+  if (!ok) *bad = 1.;
 }
 template <int U>
 __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* __restrict__ xu,
@@ -523,9 +542,9 @@ __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* _
                                                           const double* __restrict__ spu,
                                                           const double* __restrict__ spv,
                                                           double* __restrict__ ou,
-                                                          double* __restrict__ ov) {
-  if (blockIdx.z == 0) visc_uv<0, U>(G, xu, keepu, avo, spu, ou);
-  else visc_uv<1, U>(G, xv, keepv, avo, spv, ov);
+                                                          double* __restrict__ ov, double* bad) {
+  if (blockIdx.z == 0) visc_uv<0, U>(G, xu, keepu, avo, spu, ou, bad);
+  else visc_uv<1, U>(G, xv, keepv, avo, spv, ov, bad);
 }
 
 // implicit vertical diffusion of w, levels 2..KE (ocvisc.f90:225-270); the
@@ -533,7 +552,7 @@ __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* _
 template <typename Ln>
 __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restrict__ Wi,
                                                    const double* __restrict__ avo,
-                                                   double* __restrict__ O) {
+                                                   double* __restrict__ O, double* bad) {
   constexpr int LC = Ln::LC;
   __shared__ TriScan<Ln, 1> scan;
   const Ln t;
@@ -570,8 +589,10 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
     const int K = t.K0 + 2 + u;
-    a[u] = c[u] = 0.;
-    b[u] = 1.;
+    // land: the masks' factor 0 of the coefficients
+    a[u] = 0. * (av[u] + av[u + 1]);
+    c[u] = 0. * (av[u + 1] + av[u + 2]);
+    b[u] = 1. - a[u] - c[u];
     if (K <= KE && K <= kb) {
       const double rd = rden(K);
       a[u] = -2.0 * G.dt * (0.5 * (av[u] + av[u + 1])) * G.di[K - 2] * rd;
@@ -582,21 +603,30 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
   }
   const int Kp = t.K0 + 1;  // the level above the thread's first
   const double cprev = Kp >= 2 && Kp < KE && Kp <= kb ? lower(Kp, av[0], av[1], rden(Kp)) : 0.;
+  bool ok = true;
+  if (valid && t.g == 0) ok = finite(Wi[G.L.at(i, j, 0)]);
   if (valid && !interior) {
 #pragma unroll
     for (int u = 0; u < LC; ++u)
-      if (t.K0 + 2 + u <= KE) O[base + u * pl] = x[0][u];
+      if (t.K0 + 2 + u <= KE) {
+        ok &= finite(x[0][u]);
+        O[base + u * pl] = x[0][u];
+      }
   }
-  // levels below the bottom end as 0
+  // levels below the bottom end as 0 (NaN where the mask's factor 0 gives it)
 #pragma unroll
   for (int u = 0; u < LC; ++u)
-    if (t.K0 + 2 + u > kb) x[0][u] = 0.;
+    if (t.K0 + 2 + u > kb) x[0][u] = 0. * x[0][u];
   tri_solve<Ln, 1>(t, scan, a, b, c, cprev, x);
   if (interior) {
 #pragma unroll
     for (int u = 0; u < LC; ++u)
-      if (t.K0 + 2 + u <= KE) O[base + u * pl] = x[0][u];
+      if (t.K0 + 2 + u <= KE) {
+        ok &= finite(x[0][u]);
+        O[base + u * pl] = x[0][u];
+      }
   }
+  if (!ok) *bad = 1.;
 }
 
 // The horizontal passes of OCVISC: a thread takes kViscLevels levels of a point,
@@ -627,7 +657,7 @@ __device__ __forceinline__ Cross cross_kb(const Geo& G, int i, int j) {
 }
 
 // first Laplacians UK1O (u), VK1E (v), WN1O (w), ocvisc.f90:350-438, 617-669
-template <int ST>
+template <int ST, bool ALL>
 __device__ __forceinline__ void visc_lap(const Geo& G, const double* __restrict__ f,
                                          double* __restrict__ out, int i, int j, int K0) {
   const int IE = G.L.ie, JE = G.L.je, P = G.L.P, pl = G.L.plane;
@@ -663,51 +693,66 @@ __device__ __forceinline__ void visc_lap(const Geo& G, const double* __restrict_
   } else {
     k.c = 0;  // a corner
   }
+  const bool all = ALL && (iin || jin);
   const int o0 = G.L.at(i, j, K0 - 1), n = min(kViscLevels, G.L.ke + 1 - K0);
   for (int q0 = 0; q0 < n; q0 += 4) {
     double c[4], e[4], w[4], no[4], so[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int K = K0 + q0 + q, o = o0 + (q0 + q) * pl;
-      const bool wet = K <= k.c;  // (k.c <= KE)
-      c[q] = wet ? f[o] : 0.;
-      e[q] = wet && K <= k.e ? f[o + 1] : c[q];
-      w[q] = wet && K <= k.w ? f[o - 1] : c[q];
-      no[q] = wet && K <= k.n ? f[o - P] : c[q];
-      so[q] = wet && K <= k.s ? f[o + P] : c[q];
+      const bool land = all && q0 + q < n, wet = K <= k.c;  // (k.c <= KE)
+      c[q] = wet || land ? f[o] : 0.;
+      e[q] = (wet && K <= k.e) || (land && i < IE) ? f[o + 1] : c[q];
+      w[q] = (wet && K <= k.w) || (land && i > i0) ? f[o - 1] : c[q];
+      no[q] = (wet && K <= k.n) || (land && j > j0) ? f[o - P] : c[q];
+      so[q] = (wet && K <= k.s) || (land && j < JE) ? f[o + P] : c[q];
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (q0 + q >= n) break;
-      // a neighbour without water gives c - c = 0, as its mask does
-      const double x = ((e[q] - c[q]) * ce - (c[q] - w[q]) * cw) * rx;
-      const double y = ((no[q] - c[q]) * cn - (c[q] - so[q]) * cs) * ry;
-      out[o0 + (q0 + q) * pl] = K0 + q0 + q <= k.c ? x + y : 0.;
+      const int K = K0 + q0 + q;
+      double r;
+      if (!all) {  // a neighbour without water gives c - c = 0, as its mask does
+        const double x = ((e[q] - c[q]) * ce - (c[q] - w[q]) * cw) * rx;
+        const double y = ((no[q] - c[q]) * cn - (c[q] - so[q]) * cs) * ry;
+        r = K <= k.c ? x + y : 0.;
+      } else {
+        const double x = ((K <= k.e ? ce : 0.) * (e[q] - c[q]) - (K <= k.w ? cw : 0.) * (c[q] - w[q])) * rx;
+        const double y = ((K <= k.n ? cn : 0.) * (no[q] - c[q]) - (K <= k.s ? cs : 0.) * (c[q] - so[q])) * ry;
+        r = (K <= k.c ? 1. : 0.) * (x + y);
+      }
+      out[o0 + (q0 + q) * pl] = r;
     }
   }
 }
 
-__global__ void __launch_bounds__(128) k_visc_lap(Geo G, const double* __restrict__ uk,
+__global__ void __launch_bounds__(128, 7) k_visc_lap(Geo G, const double* __restrict__ uk,
                                                   const double* __restrict__ vk,
                                                   const double* __restrict__ wn,
                                                   double* __restrict__ u1,
                                                   double* __restrict__ v1,
-                                                  double* __restrict__ w1, int chunks) {
+                                                  double* __restrict__ w1, const double* bad,
+                                                  int chunks) {
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
   if (i > G.L.ie || j > G.L.je) return;
   const int K0 = (blockIdx.z % chunks) * kViscLevels + 1;
-  switch (blockIdx.z / chunks) {
-    case 0: visc_lap<S_U>(G, uk, u1, i, j, K0); break;
-    case 1: visc_lap<S_V>(G, vk, v1, i, j, K0); break;
-    default: visc_lap<S_W>(G, wn, w1, i, j, K0); break;
-  }
+  auto run = [&](auto all) {
+    constexpr bool A = decltype(all)::value;
+    switch (blockIdx.z / chunks) {
+      case 0: visc_lap<S_U, A>(G, uk, u1, i, j, K0); break;
+      case 1: visc_lap<S_V, A>(G, vk, v1, i, j, K0); break;
+      default: visc_lap<S_W, A>(G, wn, w1, i, j, K0); break;
+    }
+  };
+  if (*bad == 0.) run(std::false_type{});
+  else run(std::true_type{});
 }
 
 // second passes, ocvisc.f90:445-477 (u, v) and 673-688 (w).  The face terms
 // AUL.. * width / length are precomputed per face (G.ugx .. G.wgy) and the cell
 // areas' reciprocals per cell, so a cell needs no division except by its
 // thickness (w).  keep: the values of points outside the update range.
-template <int ST>
+template <int ST, bool ALL>
 __device__ __forceinline__ void visc_bih(const Geo& G, const double* __restrict__ keep,
                                          const double* __restrict__ f,
                                          const double* __restrict__ l, double* __restrict__ out,
@@ -765,31 +810,39 @@ __device__ __forceinline__ void visc_bih(const Geo& G, const double* __restrict_
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int K = K0 + q0 + q, o = o0 + (q0 + q) * pl;
-      const bool wet = K <= k.c;
+      const bool land = ALL && K <= G.L.ke, wet = K <= k.c;
       v[q] = K <= kbot ? f[o] : 0.;
-      c[q] = wet ? l[o] : 0.;
-      e[q] = wet && K <= k.e ? l[o + 1] : c[q];
-      w[q] = wet && K <= k.w ? l[o - 1] : c[q];
-      no[q] = wet && K <= k.n ? l[o - P] : c[q];
-      so[q] = wet && K <= k.s ? l[o + P] : c[q];
+      c[q] = wet || land ? l[o] : 0.;
+      e[q] = (wet && K <= k.e) || land ? l[o + 1] : c[q];
+      w[q] = (wet && K <= k.w) || land ? l[o - 1] : c[q];
+      no[q] = (wet && K <= k.n) || land ? l[o - P] : c[q];
+      so[q] = (wet && K <= k.s) || land ? l[o + P] : c[q];
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int K = K0 + q0 + q;
       if (q0 + q >= n) break;
       double r = 0.;
-      if (K <= k.c) {
+      if (K <= k.c || (ALL && K <= G.L.ke)) {
+        const double wet = K <= k.c ? 1. : 0.;
+        double fe = ge, fw = gw, fn = gn, fs = gs;
+        if (ALL) {
+          fe = K <= k.e ? fe : 0.;
+          fw = K <= k.w ? fw : 0.;
+          fn = K <= k.n ? fn : 0.;
+          fs = K <= k.s ? fs : 0.;
+        }
         if (ST == S_W) {
           const double mv = G.minvalue, dz = __ldg(G.dzw + K - 1);
           auto th = [&](int kb, double bot) { return fmx(K < kb ? dz : (K == kb ? bot : 0.0), mv); };
           const double dzp = th(k.c, bc);
-          r = div_nr(rarea, dzp) *
+          r = div_nr(wet * rarea, dzp) *
               (area * dzp * v[q] -
-               (ge * th(kue, bue) * (e[q] - c[q]) - gw * th(kuw, buw) * (c[q] - w[q]) +
-                gn * th(kvn, bvn) * (no[q] - c[q]) - gs * th(kvs, bvs) * (c[q] - so[q])));
+               (fe * th(kue, bue) * (e[q] - c[q]) - fw * th(kuw, buw) * (c[q] - w[q]) +
+                fn * th(kvn, bvn) * (no[q] - c[q]) - fs * th(kvs, bvs) * (c[q] - so[q])));
         } else {
-          r = rarea * (area * v[q] - (ge * (e[q] - c[q]) - gw * (c[q] - w[q]) +
-                                      gn * (no[q] - c[q]) - gs * (c[q] - so[q])));
+          r = wet * rarea * (area * v[q] - (fe * (e[q] - c[q]) - fw * (c[q] - w[q]) +
+                                            fn * (no[q] - c[q]) - fs * (c[q] - so[q])));
         }
       }
       if (ST == S_W && K > G.L.ke) r = v[q];
@@ -802,15 +855,21 @@ __global__ void __launch_bounds__(128) k_visc_bih(
     Geo G, const double* __restrict__ uoo, const double* __restrict__ voe,
     const double* __restrict__ uk, const double* __restrict__ vk, const double* __restrict__ wn,
     const double* __restrict__ u1, const double* __restrict__ v1, const double* __restrict__ w1,
-    double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ wo, int chunks) {
+    double* __restrict__ uo, double* __restrict__ vo, double* __restrict__ wo, const double* bad,
+    int chunks) {
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
   if (i > G.L.ie || j > G.L.je) return;
   const int K0 = (blockIdx.z % chunks) * kViscLevels + 1;
-  switch (blockIdx.z / chunks) {
-    case 0: visc_bih<S_U>(G, uoo, uk, u1, uo, i, j, K0); break;
-    case 1: visc_bih<S_V>(G, voe, vk, v1, vo, i, j, K0); break;
-    default: visc_bih<S_W>(G, wn, wn, w1, wo, i, j, K0); break;
-  }
+  auto run = [&](auto all) {
+    constexpr bool A = decltype(all)::value;
+    switch (blockIdx.z / chunks) {
+      case 0: visc_bih<S_U, A>(G, uoo, uk, u1, uo, i, j, K0); break;
+      case 1: visc_bih<S_V, A>(G, voe, vk, v1, vo, i, j, K0); break;
+      default: visc_bih<S_W, A>(G, wn, wn, w1, wo, i, j, K0); break;
+    }
+  };
+  if (*bad == 0.) run(std::false_type{});
+  else run(std::true_type{});
 }
 
 }  // namespace
@@ -866,24 +925,25 @@ void launch_ocvisc(const Geo& G, const double* uoo, const double* voe, const dou
                    double* w1, double* uo, double* vo, double* wo, cudaStream_t st) {
   const int IE = G.L.ie, JE = G.L.je, KE = G.L.ke;
   const dim3 b2(32, 4), bc(32, kVertBlock / 32), b3(32, 4);
+  double* bad = spu + G.L.at2(0, 0);  // cleared by k_visc_speed
   k_visc_speed<<<grid2(IE + 1, JE + 1, b2), b2, 0, st>>>(G, uoo, voe, spu, spv);
   count_launch();
   dim3 gv = grid2(IE + 1, JE + 1, bc);
   gv.z = 2;
-  k_visc_uv_b<4><<<gv, bc, 0, st>>>(G, uoo, voe, uko, vke, avo, spu, spv, ukv, vkv);
+  k_visc_uv_b<4><<<gv, bc, 0, st>>>(G, uoo, voe, uko, vke, avo, spu, spv, ukv, vkv, bad);
   count_launch();
   with_tri_split(KE, [&](auto* l) {
     using Ln = std::remove_pointer_t<decltype(l)>;
     const int nb = (IE + Ln::W) / Ln::W;  // rows in x: y ends at 65535
-    k_visc_w<Ln><<<nb * JE, Ln::NT, 0, st>>>(G, wno, avo, wnv);
+    k_visc_w<Ln><<<nb * JE, Ln::NT, 0, st>>>(G, wno, avo, wnv, bad);
   });
   count_launch();
   const int chunks = (KE + 1 + kViscLevels - 1) / kViscLevels;
   dim3 gl = grid2(IE + 1, JE + 1, b3);
   gl.z = 3 * chunks;
-  k_visc_lap<<<gl, b3, 0, st>>>(G, ukv, vkv, wnv, u1, v1, w1, chunks);
+  k_visc_lap<<<gl, b3, 0, st>>>(G, ukv, vkv, wnv, u1, v1, w1, bad, chunks);
   count_launch();
-  k_visc_bih<<<gl, b3, 0, st>>>(G, uoo, voe, ukv, vkv, wnv, u1, v1, w1, uo, vo, wo, chunks);
+  k_visc_bih<<<gl, b3, 0, st>>>(G, uoo, voe, ukv, vkv, wnv, u1, v1, w1, uo, vo, wo, bad, chunks);
   count_launch();
 }
 

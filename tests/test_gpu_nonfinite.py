@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 ROUTINES = {"ocuad": ("uoo", "uko", "vke", "wo"), "ocvad": ("voe", "uko", "vke", "wo"),
             "ocwad": ("wno", "uko", "vke", "wo", "zo"), "ocadpo": ("tracer0", "uko", "vke", "wo", "zo"),
-            "octdiff": ("tracer0", "dvo", "zo")}
+            "octdiff": ("tracer0", "dvo", "zo"), "ocvisc": ("uoo", "voe", "wno", "avo")}
 
 
 @pytest.fixture(scope="module")
@@ -55,14 +55,17 @@ def _oracle(orc, routine, st):
     if routine == "ocadpo":
         orc.ocadpo(st["tracers"][0], *a, st["zo"])
         return {"tracer0": st["tracers"][0]}
-    orc.octdiff(st["tracers"], st["dvo"], st["zo"])
-    return {"tracer0": st["tracers"][0]}
+    if routine == "octdiff":
+        orc.octdiff(st["tracers"], st["dvo"], st["zo"])
+        return {"tracer0": st["tracers"][0]}
+    orc.ocvisc(*(st[k] for k in ("uoo", "voe", "wno", "uko", "vke", "avo")))
+    return {k: st[k] for k in ("uoo", "voe", "wno")}
 
 
 # (an infinity in a column solve is no case: the kernels' quotient by refinement gives
 # NaN where IEEE division gives an infinity, and the two part ways from there)
 @pytest.mark.parametrize("routine,value", [(r, v) for r in sorted(ROUTINES) for v in (np.nan, np.inf)
-                                           if np.isnan(v) or r != "octdiff"])
+                                           if np.isnan(v) or r not in ("octdiff", "ocvisc")])
 def test_nonfinite_values_spread_as_in_the_oracle(inst, routine, value):
     orc = O.Oracle(inst)
     gpu = Instance(inst)
