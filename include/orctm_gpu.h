@@ -455,6 +455,12 @@ unsigned long long orctm_kernel_launches(void);
  * estimate, within 1 ulp of IEEE division).  Test support; allocates. */
 int orctm_check_division(int device, const double* a, const double* b, double* q, size_t n);
 
+/* Test support: the clock cycles, at most the two billion (about one second) a
+ * handle is created with, after which a wait inside a solver kernel gives up (0:
+ * at once).  The solve then returns ORCTM_E_CUDA without changing the fields, and
+ * the handle stays usable. */
+int orctm_set_wait_cycles(orctm_handle* h, long long cycles);
+
 /* Kernel variants of the Poisson solver.  The solver's kernels have one form,
  * chosen by KE and the precision; the numbers of earlier variants (6 column-kernel
  * and 9 stencil variants, -1 for the handle's own choice) are accepted and

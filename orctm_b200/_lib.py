@@ -122,6 +122,7 @@ EXPORTS = (
     "orctm_synchronize", "orctm_build_grid", "orctm_timer_start", "orctm_timer_stop",
     "orctm_set_profiling", "orctm_profile_get", "orctm_kernel_launches", "orctm_device_bytes",
     "orctm_trim_device_memory", "orctm_set_tuning", "orctm_get_tuning",
+    "orctm_set_wait_cycles",
     "orctm_serve_create", "orctm_serve_submit", "orctm_serve_wait", "orctm_serve_poll",
     "orctm_serve_drain", "orctm_serve_get_stats", "orctm_serve_destroy", "orctm_batch_run",
     "orctm_estimate_device_bytes", "orctm_check_division", "orctm_ocadpo_all",
@@ -157,6 +158,7 @@ def load(build_if_missing: bool = True):
     lib.orctm_last_error.restype = C.c_char_p
     lib.orctm_last_error.argtypes = [C.c_void_p]
     lib.orctm_create.argtypes = [C.POINTER(Desc), C.POINTER(C.c_void_p)]
+    lib.orctm_set_wait_cycles.argtypes = [C.c_void_p, C.c_longlong]
     for name in ("orctm_destroy", "orctm_ocuad", "orctm_ocvad", "orctm_ocwad", "orctm_octdiff",
                  "orctm_octimf", "orctm_ocvisc", "orctm_synchronize", "orctm_ocadpo_all"):
         getattr(lib, name).argtypes = [C.c_void_p]

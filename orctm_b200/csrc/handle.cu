@@ -797,6 +797,7 @@ int setup(orctm_handle* h, const orctm_desc* d) {
   std::memset(h->hS, 0, sizeof(SolverState));
   h->hS->max_blocks = maxb;
   h->hS->partials = h->partials;
+  h->hS->wait = solver_wait_cycles();
   ORCTM_CUDA_OK(cudaMemcpyAsync(h->S, h->hS, sizeof(SolverState), cudaMemcpyHostToDevice, h->stream));
   ORCTM_CUDA_OK(cudaEventCreate(&h->ev0));
   ORCTM_CUDA_OK(cudaEventCreate(&h->ev1));
@@ -920,6 +921,11 @@ int pcg_loop_graph(orctm_handle* h, cudaGraphExec_t* out) {
   return ORCTM_OK;
 }
 
+// whether a bounded wait inside a kernel gave up, as of the last read_state
+int check_waits(orctm_handle* h) {
+  return h->hS->gave_up ? h->fail(ORCTM_E_CUDA, "a device-side wait timed out in the Poisson solver") : ORCTM_OK;
+}
+
 // One correction: A d = r (h->r) to the relative residual S->tol, added to h->xs.
 template <typename T>
 int pcg_loop(orctm_handle* h, int maxit, int* iters) {
@@ -962,10 +968,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     }
   }
   *iters = h->hS->iter;
-  if (conv == 4) {  // a bounded wait inside a kernel gave up
-    h->err = "a device-side wait for a staged copy timed out in the Poisson solver";
-    return ORCTM_E_CUDA;
-  }
+  if ((st = check_waits(h))) return st;
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_after<T>(h->R, h->S, v, h->xs, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
@@ -987,10 +990,10 @@ int poisson_solve(orctm_handle* h, orctm_solve_stats* stats) {
   int total = 0, outer = 0;
   double prev = 1e300, rel = 0.0;
   for (;; ++outer) {
-    launch_solver_reset(h->S, h->rtol, h->stream);
+    launch_solver_reset(h->S, h->rtol, outer == 0, h->stream);
     PROF(h, ORCTM_PROF_RESID, launch_resid(G, h->P, h->S, h->b, h->xs, h->r, h->stream));
     ORCTM_CUDA_OK(cudaGetLastError());
-    if ((st = read_state(h))) return st;
+    if ((st = read_state(h)) || (st = check_waits(h))) return st;
     const double bnorm = std::sqrt(h->hS->res_bb);
     if (bnorm == 0.0) {  // zero right-hand side: the solution is zero
       ORCTM_CUDA_OK(cudaMemsetAsync(h->xs, 0, sizeof(double) * n3, h->stream));
@@ -1005,7 +1008,7 @@ int poisson_solve(orctm_handle* h, orctm_solve_stats* stats) {
     double inner = 0.3 * h->rtol / rel;
     inner = std::min(0.5, std::max(inner, f32 ? 2e-5 : 1e-13));
     int its = 0;
-    launch_solver_reset(h->S, inner, h->stream);
+    launch_solver_reset(h->S, inner, false, h->stream);
     if ((st = f32 ? pcg_loop<float>(h, h->maxit - total, &its)
                   : pcg_loop<double>(h, h->maxit - total, &its)))
       return st;
@@ -2588,6 +2591,15 @@ int orctm_profile_get(orctm_handle* h, int kind, long long* launches, double* to
 }
 
 unsigned long long orctm_kernel_launches(void) { return launch_count(); }
+
+int orctm_set_wait_cycles(orctm_handle* h, long long cycles) {
+  ORCTM_ENTER(h);
+  if (cycles < 0 || cycles > solver_wait_cycles())
+    return h->fail(ORCTM_E_ARG, "orctm_set_wait_cycles: out of range");
+  launch_set_wait(h->S, cycles, h->stream);
+  ORCTM_CUDA_OK(cudaGetLastError());
+  return ORCTM_OK;
+}
 
 int orctm_set_tuning(orctm_handle* h, int col_variant, int spmv_variant) {
   if (!h || col_variant < -1 || col_variant >= 6 || spmv_variant < -1 || spmv_variant >= 9)

@@ -66,11 +66,13 @@ struct RbVectors {
 // Device-resident scalars of one Krylov solve.
 struct SolverState {
   double rho, beta, alpha, alpha_prev, pq, rz, rr, bb, tol, res_rr, res_bb;
-  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown, 4 a staged copy timed out
+  int converged;  // 0 running, 1 converged, 2 NaN, 3 breakdown, 4 a wait gave up
+  int gave_up;    // a wait gave up since the solve began
   int iter;
   int limit;      // iteration limit of the device-side loop (orctm handle's maxit)
   unsigned ticket;
   unsigned gbar;  // arrivals at the barriers of the one-kernel loop
+  long long wait;    // clock cycles after which a wait gives up
   int max_blocks;    // partial sums per quantity: the most tiles of a kernel
   double* partials;  // [4 * max_blocks]
 };
@@ -250,7 +252,10 @@ void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, doub
 // r = b - A x in double-double, and x := 0 on land rows (their solution)
 void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const double* b, double* x,
                   double* r, cudaStream_t st);
-void launch_solver_reset(SolverState* S, double tol, cudaStream_t st);
+// first: of a solve
+void launch_solver_reset(SolverState* S, double tol, bool first, cudaStream_t st);
+void launch_set_wait(SolverState* S, long long cycles, cudaStream_t st);
+long long solver_wait_cycles();  // a solver's as created, about one second
 // device-side PCG loop: the limit of iterations, and the kernel that ends a
 // while-node body (keep looping while not converged and a further chunk of
 // `chunk` iterations stays within the limit)

@@ -330,11 +330,11 @@ struct Scan {
 
 // v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d (dm: the
 // pivot above the thread's first level) and couplings a; returns v.M^-1 v =
-// sum y^2 / d of this thread's levels.  Two block barriers; between() runs
-// after the first, when every thread has its inputs in registers.
+// sum y^2 / d of this thread's levels.  Two block barriers; first() is the first
+// of them, and runs after it: every thread has its inputs in registers there.
 template <typename Ln, typename T, int LC, typename F>
 __device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC], const T (&d)[LC],
-                                          T dm, const T (&a)[LC + 1], F&& between) {
+                                          T dm, const T (&a)[LC + 1], F&& first) {
   constexpr int G = Ln::GROUPS;
   // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the thread's levels as one affine
   // map y_out = A y_in + B, applied in turn to what comes from above
@@ -347,8 +347,7 @@ __device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC],
   }
   sc.fa[t.g][t.c] = A;
   sc.fb[t.g][t.c] = B;
-  __syncthreads();
-  between();
+  first();
   T y = T(0);
 #pragma unroll
   for (int k = 0; k < G - 1; ++k)
@@ -419,6 +418,11 @@ struct Tiles {
   }
 };
 
+__device__ __forceinline__ void solve_gave_up(SolverState* S) {
+  atomicExch(&S->converged, 4);
+  atomicExch(&S->gave_up, 1);
+}
+
 // Staging.  A block's next tile is copied to shared memory while it computes
 // this one: one thread issues a bulk copy per array (a tile is consecutive
 // memory; down to the tile's deepest wet level), all wait on an mbarrier.  NA
@@ -439,8 +443,11 @@ struct Stage {
   D* piv;
   uint64_t* bar;
   uint32_t phase;
-  bool ok;
-  __device__ __forceinline__ Stage(unsigned char* dsm, uint64_t* b) : bar(b), phase(0), ok(true) {
+  long long limit;
+  bool ok;    // this thread's waits
+  bool stop;  // a thread of the block has given up (the same for all)
+  __device__ __forceinline__ Stage(unsigned char* dsm, uint64_t* b, const SolverState* S)
+      : bar(b), phase(0), limit(S->wait), ok(true), stop(false) {
     pairs = reinterpret_cast<double2*>(dsm);
     data = reinterpret_cast<T*>(dsm + 16 * 4 * W);
     piv = reinterpret_cast<D*>(dsm + 16 * 4 * W + sizeof(T) * N * NA);
@@ -489,8 +496,14 @@ struct Stage {
   }
   __device__ __forceinline__ void wait() {
     copies_wait();
-    if (ok) ok = mbar_wait(bar, phase);
+    ok = mbar_wait(bar, phase, limit);
     phase ^= 1;
+  }
+  // A barrier of the block after wait(): whether the tiles go on.  If a thread gave
+  // up, no further copy is issued, and the block ends after this tile.
+  __device__ __forceinline__ bool goes_on() {
+    stop = __syncthreads_or(!ok);
+    return !stop;
   }
   __device__ __forceinline__ T get(const Ln& t, int n, int q) const {
     return data[n * N + (t.K0 + q) * W + t.c];
@@ -524,9 +537,11 @@ struct Stage {
     for (int q = 0; q < Ln::L; ++q)
       d[q] = t.K0 + 1 + q <= kb ? (T)piv[(t.K0 + q) * W + t.c] : T(0);
   }
-  // a copy that never landed stops the solve
+  // A copy that did not land stops the solve; it is waited for once more, so that it
+  // does not write to the next block's shared memory.
   __device__ __forceinline__ void report(SolverState* S) const {
-    if (!ok && threadIdx.x == 0) atomicExch(&S->converged, 4);
+    if (!ok) mbar_wait(bar, phase ^ 1, kWaitCycles);
+    if (stop && threadIdx.x == 0) solve_gave_up(S);
   }
 };
 
@@ -561,7 +576,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_red(RbGeo R, SolverState* S,
   }
   const Ln t;
   const Tiles<Ln> tiles{R, R.col[0], t, ntiles, nt, true};
-  RedStage<Ln, MODE> st(dsm, &bar);
+  RedStage<Ln, MODE> st(dsm, &bar, S);
   load_tables<Ln>(R, szw, siz);
   if (MODE == kIter && cc) load_profiles<Ln>(R, sphi);
   __syncthreads();
@@ -646,7 +661,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_red(RbGeo R, SolverState* S,
     }
     couplings(t, szw, kb, kb ? zwa : T(0), cp);
     column_solve(t, scan, g, d, dm, cp, [&] {
-      if (tile + (int)gridDim.x < ntiles) {
+      if (st.goes_on() && tile + (int)gridDim.x < ntiles) {
         next = tiles.at(tile + gridDim.x, kn);
         issue(next);
         kn = tiles.kk(tile + 2 * gridDim.x);
@@ -663,6 +678,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_red(RbGeo R, SolverState* S,
         }
       }
     }
+    if (st.stop) break;
   }
   st.report(S);
   if (MODE == kBefore) {
@@ -694,7 +710,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
   const bool first = S->iter == 0;
   const Ln t;
   const Tiles<Ln> tiles{R, R.col[1], t, ntiles, nt, false};
-  BlackStage<Ln> st(dsm, &bar);
+  BlackStage<Ln> st(dsm, &bar, S);
   load_tables<Ln>(R, szw, siz);
   if (cc) load_profiles<Ln>(R, sphi);
   __syncthreads();
@@ -729,8 +745,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
     st.neighbour_sum(t, a, 0, we, ns, v);
     top[buf][t.g][t.c] = pl[0];
     bottom[buf][t.g][t.c] = pl[LC - 1];
-    __syncthreads();
-    if (tile + (int)gridDim.x < ntiles) {
+    if (st.goes_on() && tile + (int)gridDim.x < ntiles) {
       next = tiles.at(tile + gridDim.x, kn);
       issue(next);
       kn = tiles.kk(tile + 2 * gridDim.x);
@@ -772,6 +787,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
       pu = p0;
     }
     pq += (double)pqt;
+    if (st.stop) break;
   }
   st.report(S);
   double w[1] = {pq};
@@ -810,7 +826,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
   if (INIT && sizeof(T) == 4) scale = S->res_rr > 0.0 ? 1.0 / sqrt(S->res_rr) : 0.0;
   const Ln t;
   const Tiles<Ln> tiles{R, R.col[1], t, ntiles, nt, false};
-  ColStage<Ln, INIT> st(dsm, &bar);
+  ColStage<Ln, INIT> st(dsm, &bar, S);
   load_tables<Ln, T>(R, szw, nullptr);
   if (rho) load_profiles<Ln>(R, sphi);
   __syncthreads();
@@ -864,13 +880,14 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
       }
     }
     rz += (double)column_solve(t, scan, g, d, dm, cp, [&] {
+      const bool on = st.goes_on();
       if (rho && t.g < NM && kb) {
         T f = T(0);
 #pragma unroll
         for (int k = 0; k < Ln::GROUPS; ++k) f += part[t.g][k][t.c];
         rho[t.g * R.plane2 + a.m + R.P2 * a.j] = f;
       }
-      if (tile + (int)gridDim.x < ntiles) {
+      if (on && tile + (int)gridDim.x < ntiles) {
         next = tiles.at(tile + gridDim.x, kn);
         issue(next);
         kn = tiles.kk(tile + 2 * gridDim.x);
@@ -880,6 +897,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
 #pragma unroll
     for (int e = 0; e < LC; ++e)
       if (t.K0 + 1 + e <= kb) z[a.o0 + W * e] = g[e];
+    if (st.stop) break;
   }
   st.report(S);
   double v[INIT ? 3 : 2];
@@ -1136,7 +1154,7 @@ __device__ __forceinline__ void grid_all(double (&v)[NV ? NV : 1], GridSync& g, 
       unsigned n;
       asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(n) : "l"(&S->gbar) : "memory");
       there = (int)(n - g.target) >= 0;
-      if (!there && clock64() - t0 > kWaitCycles) break;
+      if (!there && clock64() - t0 >= S->wait) break;
     }
     up = there;
   }
@@ -1248,7 +1266,7 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
     }
     T dm = t.K0 > 0 ? ds[me - W] : T(0);
     couplings(t, szw, kba, zwa0, cp);
-    column_solve(t, scan, h, d, dm, cp, [] {});
+    column_solve(t, scan, h, d, dm, cp, [] { __syncthreads(); });
 #pragma unroll
     for (int q = 0; q < LC; ++q)
       if (t.K0 + 1 + q <= kba) {
@@ -1317,7 +1335,7 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
     }
     dm = t.K0 > 0 ? (T)db[me - W] : T(0);
     couplings(t, szw, kbk, zwa1, cp);
-    const T rz = column_solve(t, scan, h, d, dm, cp, [] {});
+    const T rz = column_solve(t, scan, h, d, dm, cp, [] { __syncthreads(); });
 #pragma unroll
     for (int e = 0; e < LC; ++e)
       if (t.K0 + 1 + e <= kbk) {
@@ -1350,7 +1368,7 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
     S->alpha_prev = alpha;
     if (conv != 4) S->converged = conv;
   }
-  if (conv == 4 && threadIdx.x == 0) atomicExch(&S->converged, 4);
+  if (conv == 4 && threadIdx.x == 0) solve_gave_up(S);
 }
 
 // The black correction: the x update that the last iteration left open (none
@@ -1473,7 +1491,8 @@ __global__ void k_pcg_continue(cudaGraphConditionalHandle hc, const SolverState*
   cudaGraphSetConditional(hc, (S->converged == 0 && S->iter + chunk <= S->limit) ? 1u : 0u);
 }
 
-__global__ void k_reset(SolverState* S, double tol) {
+__global__ void k_reset(SolverState* S, double tol, bool first) {
+  if (first) S->gave_up = 0;
   S->converged = 0;
   S->iter = 0;
   S->ticket = 0;
@@ -1483,6 +1502,8 @@ __global__ void k_reset(SolverState* S, double tol) {
   S->alpha_prev = 0.0;
   S->bb = 0.0;
 }
+
+__global__ void k_set_wait(SolverState* S, long long cycles) { S->wait = cycles; }
 
 struct Shape {
   int ntiles, nt, grid;
@@ -1720,10 +1741,17 @@ void launch_resid(const Geo& G, const PoissonGeo& P, SolverState* S, const doubl
   count_launch();
 }
 
-void launch_solver_reset(SolverState* S, double tol, cudaStream_t st) {
-  k_reset<<<1, 1, 0, st>>>(S, tol);
+void launch_solver_reset(SolverState* S, double tol, bool first, cudaStream_t st) {
+  k_reset<<<1, 1, 0, st>>>(S, tol, first);
   count_launch();
 }
+
+void launch_set_wait(SolverState* S, long long cycles, cudaStream_t st) {
+  k_set_wait<<<1, 1, 0, st>>>(S, cycles);
+  count_launch();
+}
+
+long long solver_wait_cycles() { return kWaitCycles; }
 
 void launch_set_limit(SolverState* S, int limit, cudaStream_t st) {
   k_set_limit<<<1, 1, 0, st>>>(S, limit);

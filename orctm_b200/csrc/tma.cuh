@@ -2,7 +2,7 @@
 //
 // Only plain loads from this GPU's own memory are issued (no cluster
 // multicast).  Every wait on an mbarrier is bounded by a clock budget, so a
-// copy that never lands makes the waiting thread give up and report it
+// copy that never lands makes the waiting block give up and report it
 // instead of spinning forever.
 #pragma once
 #include <cuda_runtime.h>
@@ -47,13 +47,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Waits for the phase of the given parity to complete; false when the clock
-// budget ran out first.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+// Waits for the phase of the given parity to complete; false when the budget of
+// `limit` cycles ran out first (0: at once).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit) {
+  if (limit <= 0) return false;
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity))
-    if (clock64() - t0 > kWaitCycles) return false;
+    if (clock64() - t0 > limit) return false;
   return true;
 }
 

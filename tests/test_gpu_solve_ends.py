@@ -4,6 +4,7 @@ profiling selects)."""
 import numpy as np
 import pytest
 
+from orctm_b200 import _lib
 from orctm_b200 import configs as C
 from orctm_b200 import grid
 from orctm_b200.api import Instance
@@ -33,3 +34,36 @@ def test_breakdown_keeps_the_last_full_step():
         gpu.close()
     assert np.isfinite(got[0]).all() and np.abs(got[0]).max() > 0
     assert np.array_equal(got[0], got[1])
+
+
+# (cycles, profiling): at once at the first staged copy, with a form's own
+# kernels after it; and one cycle, which a barrier of the one-kernel loop cannot keep
+@pytest.mark.parametrize("mode", ["fp64", "fp32_refined"])
+@pytest.mark.parametrize("nx,ny,nz", [(45, 21, 50), (34, 34, 105)])
+@pytest.mark.parametrize("cycles,prof", [(0, False), (0, True), (1, False)])
+def test_a_wait_that_gives_up_is_an_error_and_no_more(nx, ny, nz, cycles, prof, mode):
+    """A limit that waits cannot keep: the solve returns ORCTM_E_CUDA and leaves
+    the fields alone; with the usual limit the same handle then solves as another
+    does."""
+    if cycles and nz > 104:
+        pytest.skip("columns too long for the one-kernel loop")
+    inst = C.make_instance("c2", builder=grid.build_grid, nx=nx, ny=ny, nz=nz)
+    want, gpu = Instance(inst), Instance(inst)
+    for g in (want, gpu):
+        g.upload_state(C.copy_state(inst))
+        g.set_solver(mode, rtol=1e-12, maxit=20000)
+    gpu.set_profiling(prof)
+    before = {k: gpu.download(k) for k in ("uoo", "voe", "wno", "pnh")}
+    _lib.check(gpu.lib.orctm_set_wait_cycles(gpu.h, cycles), gpu.h)
+    with pytest.raises(_lib.OrctmError) as e:
+        gpu.ocvtot_nh()
+    assert e.value.status == _lib.ORCTM_E_CUDA and "timed out" in str(e.value)
+    for k, a in before.items():
+        assert np.array_equal(gpu.download(k), a), k
+    _lib.check(gpu.lib.orctm_set_wait_cycles(gpu.h, 2000000000), gpu.h)
+    assert gpu.ocvtot_nh()["converged"] == 1 and want.ocvtot_nh()["converged"] == 1
+    for k in before:
+        assert np.array_equal(gpu.download(k), want.download(k)), k
+    assert gpu.lib.orctm_set_wait_cycles(gpu.h, -1) == gpu.lib.orctm_set_wait_cycles(gpu.h, 1 << 40) == _lib.ORCTM_E_ARG
+    want.close()
+    gpu.close()
