@@ -938,7 +938,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   // pass maxit, with no host round trip in between; the iterations left before
   // maxit, and all of them while profiling, one by one
   int it = 0, conv = 0;
-  const bool small = !h->prof && launch_rb_small<T>(h->R, h->S, v, maxit, h->stream);
+  const bool small = !h->prof && launch_rb_small<T>(h->R, h->S, v, maxit, h->hS->wait, h->stream);
   if (small) {
     if ((st = read_state(h))) return st;
     it = h->hS->iter;
@@ -2597,6 +2597,7 @@ int orctm_set_wait_cycles(orctm_handle* h, long long cycles) {
   if (cycles < 0 || cycles > solver_wait_cycles())
     return h->fail(ORCTM_E_ARG, "orctm_set_wait_cycles: out of range");
   launch_set_wait(h->S, cycles, h->stream);
+  h->hS->wait = cycles;
   ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
 }

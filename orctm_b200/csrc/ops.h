@@ -246,7 +246,8 @@ void coarse_plan(RbCoarse& co, const float* mu);
 template <typename T>
 bool rb_small(const RbGeo& R);
 template <typename T>
-bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit, cudaStream_t st);
+bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit, long long limit,
+                     cudaStream_t st);
 template <typename T>
 void launch_rb_after(const RbGeo& R, SolverState* S, const RbVectors<T>& v, double* x, cudaStream_t st);
 // r = b - A x in double-double, and x := 0 on land rows (their solution)

@@ -1113,6 +1113,7 @@ __global__ void __launch_bounds__(kCoThreads, 2)
 // (converged = 4).
 struct GridSync {
   SolverState* S;
+  long long limit;  // the kernel's argument: a load in the polling loop costs 4 % of a slice's step
   unsigned target;
   bool ok;
 };
@@ -1154,7 +1155,7 @@ __device__ __forceinline__ void grid_all(double (&v)[NV ? NV : 1], GridSync& g, 
       unsigned n;
       asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(n) : "l"(&S->gbar) : "memory");
       there = (int)(n - g.target) >= 0;
-      if (!there && clock64() - t0 >= S->wait) break;
+      if (!there && clock64() - t0 >= g.limit) break;
     }
     up = there;
   }
@@ -1188,7 +1189,7 @@ constexpr size_t small_smem() {
 template <typename Ln, typename T = typename Ln::V>
 __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 : 3))
     k_rb_small(RbGeo R, SolverState* S, RbVectors<T> vec,
-                                                     int ntiles, int nt, int maxit) {
+                                                     int ntiles, int nt, int maxit, long long limit) {
   constexpr int W = Ln::W, LC = Ln::L, N = Ln::ROWS * W;
   extern __shared__ __align__(128) unsigned char dsm[];
   __shared__ T szw[Ln::ROWS + 1], siz[Ln::ROWS + 1];
@@ -1250,7 +1251,7 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
       if (t.K0 + 1 + e > kb) h[e] = T(0);
     }
   };
-  GridSync g{S, 0u, true};
+  GridSync g{S, limit, 0u, true};
   double rho = S->rho, rr = S->rr, alpha = 0.0, beta = 0.0;
   const double tol = S->tol, bb = S->bb;
   int iter = 0, conv = 0;
@@ -1695,7 +1696,7 @@ bool rb_small(const RbGeo& R) {
 
 template <typename T>
 bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int maxit,
-                     cudaStream_t st) {
+                     long long limit, cudaStream_t st) {
   bool done = false;
   with_split<T>(R.ke, [&](auto* l) {
     using L = ORCTM_LANE(l);
@@ -1706,7 +1707,7 @@ bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int 
       RbGeo r = R;
       RbVectors<T> vec = v;
       int ntiles = s.ntiles, nt = s.nt;
-      void* args[] = {&r, &S, &vec, &ntiles, &nt, &maxit};
+      void* args[] = {&r, &S, &vec, &ntiles, &nt, &maxit, &limit};
       done = cudaLaunchCooperativeKernel((const void*)&k_rb_small<L>, dim3(s.grid), dim3(L::NT), args,
                                          m, st) == cudaSuccess;
       if (done) count_launch();
@@ -1718,7 +1719,8 @@ bool launch_rb_small(const RbGeo& R, SolverState* S, const RbVectors<T>& v, int 
 
 #define ORCTM_RB(T)                                                                              \
   template bool rb_small<T>(const RbGeo&);                                                      \
-  template bool launch_rb_small<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, cudaStream_t); \
+  template bool launch_rb_small<T>(const RbGeo&, SolverState*, const RbVectors<T>&, int, long long, \
+                                  cudaStream_t);                                                \
   template void launch_rb_setup<T>(const Geo&, const PoissonGeo&, const RbGeo&, const RbVectors<T>&, \
                                    cudaStream_t);                                                \
   template void launch_rb_before<T>(const RbGeo&, SolverState*, const double*, const RbVectors<T>&, \
