@@ -328,13 +328,29 @@ struct Scan {
       bb[Ln::GROUPS][Ln::W];
 };
 
+// A thread's part of a dot product, one term per level u.  FP32 terms are added in FP32
+// four levels at a time, then in FP64.
+template <typename T>
+struct Dot {
+  T part = T(0);
+  double sum = 0.0;
+  __device__ __forceinline__ void add(int u, T a, T b) {
+    part = fma(a, b, part);
+    if (sizeof(T) == 4 && u % 4 == 3) {
+      sum += (double)part;
+      part = T(0);
+    }
+  }
+  __device__ __forceinline__ double total() const { return sum + (double)part; }
+};
+
 // v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d (dm: the
 // pivot above the thread's first level) and couplings a; returns v.M^-1 v =
 // sum y^2 / d of this thread's levels.  Two block barriers; first() is the first
 // of them, and runs after it: every thread has its inputs in registers there.
 template <typename Ln, typename T, int LC, typename F>
-__device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC], const T (&d)[LC],
-                                          T dm, const T (&a)[LC + 1], F&& first) {
+__device__ __forceinline__ double column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC], const T (&d)[LC],
+                                               T dm, const T (&a)[LC + 1], F&& first) {
   constexpr int G = Ln::GROUPS;
   // forward: y(K) = v(K) - a(K) d(K-1) y(K-1); the thread's levels as one affine
   // map y_out = A y_in + B, applied in turn to what comes from above
@@ -352,12 +368,12 @@ __device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC],
 #pragma unroll
   for (int k = 0; k < G - 1; ++k)
     if (k < t.g) y = fma(sc.fa[k][t.c], y, sc.fb[k][t.c]);
-  T rz = T(0);
+  Dot<T> rz;
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
     y = fma(-(a[u] * (u ? d[u - 1] : dm)), y, v[u]);
     v[u] = y * d[u];
-    rz = fma(y, v[u], rz);
+    rz.add(u, y, v[u]);
   }
   // backward: z(K) = y(K) d(K) - a(K+1) d(K) z(K+1)
   A = T(1);
@@ -380,7 +396,7 @@ __device__ __forceinline__ T column_solve(const Ln& t, Scan<Ln>& sc, T (&v)[LC],
     z = fma(-(a[u + 1] * d[u]), z, v[u]);
     v[u] = z;
   }
-  return rz;
+  return rz.total();
 }
 
 __device__ __forceinline__ int wet_levels(unsigned long long kk, int nb) {
@@ -762,7 +778,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
     const T cw = (T)we.x, ce = (T)we.y, cn = (T)ns.x, cs = (T)ns.y, zwa = (T)zw.x;
     const int kbw = wet_levels(a.kk, 1), kbe = wet_levels(a.kk, 2);
     const int kbn = wet_levels(a.kk, 3), kbs = wet_levels(a.kk, 4);
-    T pqt = T(0);
+    Dot<T> pqt;
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
       const int K = t.K0 + 1 + e;
@@ -782,11 +798,11 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_black(RbGeo R, SolverState* S,
       s = fma(-hs, h, s);
       if (K <= kb) {
         q[a.o0 + W * e] = s;
-        pqt = fma(p0, s, pqt);
       }
+      pqt.add(e, p0, K <= kb ? s : T(0));
       pu = p0;
     }
-    pq += (double)pqt;
+    pq += pqt.total();
     if (st.stop) break;
   }
   st.report(S);
@@ -842,7 +858,8 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
   for (; tile < ntiles; tile += gridDim.x) {
     const Tile a = next;
     const int kb = wet_levels(a.kk, 0);
-    T g[LC], d[LC], cp[LC + 1], dm, rrt = T(0);
+    T g[LC], d[LC], cp[LC + 1], dm;
+    Dot<T> rrt;
     st.wait();
     const T zwa = (T)st.pairs[t.c].x;
     st.pivots(t, kb, dm, d);
@@ -868,7 +885,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
       if (t.K0 + 1 + e <= kb) r[a.o0 + W * e] = g[e];
-      rrt = fma(g[e], g[e], rrt);
+      rrt.add(e, g[e], g[e]);
     }
     if (rho) {  // the column's products with the profiles
 #pragma unroll
@@ -879,7 +896,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
         part[q][t.g][t.c] = f;
       }
     }
-    rz += (double)column_solve(t, scan, g, d, dm, cp, [&] {
+    rz += column_solve(t, scan, g, d, dm, cp, [&] {
       const bool on = st.goes_on();
       if (rho && t.g < NM && kb) {
         T f = T(0);
@@ -893,7 +910,7 @@ __global__ void __launch_bounds__(Ln::NT) k_rb_col(RbGeo R, SolverState* S, T* _
         kn = tiles.kk(tile + 2 * gridDim.x);
       }
     });
-    rr += (double)rrt;
+    rr += rrt.total();
 #pragma unroll
     for (int e = 0; e < LC; ++e)
       if (t.K0 + 1 + e <= kb) z[a.o0 + W * e] = g[e];
@@ -1288,7 +1305,8 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
     if (!g.ok) break;
     // q = D p - C u
     neighbours(k, kbk, ut, vec.u, we1, ns1, h);
-    T qv[LC], pqt = T(0);
+    T qv[LC];
+    Dot<T> pqt;
     {
       const T cw = (T)we1.x, ce = (T)we1.y, cn = (T)ns1.x, cs = (T)ns1.y;
       const int kbw = wet_levels(k.kk, 1), kbe = wet_levels(k.kk, 2);
@@ -1312,11 +1330,11 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
         s = fma(zwn, pd - p0, s);
         s = fma(-hs, hh, s);
         qv[e] = K <= kbk ? s : T(0);
-        if (K <= kbk) pqt = fma(p0, s, pqt);
+        pqt.add(e, p0, qv[e]);
         pu = p0;
       }
     }
-    double w1[1] = {(double)pqt};
+    double w1[1] = {pqt.total()};
     grid_all<1, Ln::NT>(w1, g, 0);
     if (!g.ok) break;
     alpha = rho / w1[0];
@@ -1326,24 +1344,24 @@ __global__ void __launch_bounds__(Ln::NT, sizeof(T) == 4 ? 2 : (Ln::L <= 6 ? 4 :
       break;
     }
     // ---- column: r -= alpha q, z = D^-1 r
-    T rrt = T(0);
+    Dot<T> rrt;
 #pragma unroll
     for (int e = 0; e < LC; ++e) {
       h[e] = fma(-(T)alpha, qv[e], rs[me + W * e]);
       rs[me + W * e] = h[e];
-      rrt = fma(h[e], h[e], rrt);
+      rrt.add(e, h[e], h[e]);
       d[e] = (T)db[me + W * e];
     }
     dm = t.K0 > 0 ? (T)db[me - W] : T(0);
     couplings(t, szw, kbk, zwa1, cp);
-    const T rz = column_solve(t, scan, h, d, dm, cp, [] { __syncthreads(); });
+    const double rz = column_solve(t, scan, h, d, dm, cp, [] { __syncthreads(); });
 #pragma unroll
     for (int e = 0; e < LC; ++e)
       if (t.K0 + 1 + e <= kbk) {
         zt[me + W * e] = h[e];
         vec.z[k.o0 + W * e] = h[e];
       }
-    double w2[2] = {(double)rz, (double)rrt};
+    double w2[2] = {rz, rrt.total()};
     grid_all<2, Ln::NT>(w2, g, 1);
     if (!g.ok) break;
     beta = w2[0] / rho;

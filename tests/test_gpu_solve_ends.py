@@ -67,3 +67,23 @@ def test_a_wait_that_gives_up_is_an_error_and_no_more(nx, ny, nz, cycles, prof, 
     assert gpu.lib.orctm_set_wait_cycles(gpu.h, -1) == gpu.lib.orctm_set_wait_cycles(gpu.h, 1 << 40) == _lib.ORCTM_E_ARG
     want.close()
     gpu.close()
+
+
+@pytest.mark.parametrize("mode", ["fp64", "fp32_refined"])
+@pytest.mark.parametrize("nz", [40, 41, 64, 80, 81, 89, 104])
+def test_both_forms_of_the_loop_agree_for_every_split_of_a_column(nz, mode):
+    """5, 6, 8, 10, 11 and 13 levels a thread (and the most of each): the same
+    pressure bits and iterations from one kernel and from separate ones."""
+    inst = C.make_instance("c2", builder=grid.build_grid, nx=45, ny=21, nz=nz)
+    got = []
+    for prof in (False, True):
+        gpu = Instance(inst)
+        gpu.upload_state(C.copy_state(inst))
+        gpu.set_solver(mode, rtol=1e-12, maxit=20000)
+        gpu.set_profiling(prof)
+        stats = gpu.ocvtot_nh()
+        assert stats["converged"] == 1
+        got.append((stats["iterations"], stats["outer_iterations"], gpu.download("pnh")))
+        gpu.close()
+    assert got[0][:2] == got[1][:2]
+    assert np.array_equal(got[0][2], got[1][2])
