@@ -128,6 +128,18 @@ __device__ __forceinline__ double div_by(double a, double b, double r) {
   return q;
 }
 
+// by the exponent, on the integer pipe
+__device__ __forceinline__ bool finite(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
+}
+
+// The same with r = 1 / b by any means and any b, without the division: for |a| below 1e-290
+// it may be off by an ulp; by or of an infinity, or by 0, the product is the quotient.
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+  const double q0 = a * r, q = __fma_rn(__fma_rn(-b, q0, a), r, q0);
+  return finite(q) ? q : q0;
+}
+
 // Fortran MAX/MIN for non-NaN operands, evaluated exactly as the oracle does.
 __device__ __forceinline__ double fmx(double a, double b) { return a > b ? a : b; }
 __device__ __forceinline__ double fmn(double a, double b) { return b < a ? b : a; }

@@ -378,10 +378,6 @@ __global__ void __launch_bounds__(kHbN) k_tdiff_hbih(Geo G, TrPtrs tp, int ntr, 
 // passes do not load land cells unless the vertical solves, which write every level,
 // have met a value that is not finite: they note it at `bad` (element (0, 0) of SPEEDU,
 // no u-point, which k_visc_speed clears).
-__device__ __forceinline__ bool finite(double x) {
-  return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
-}
-
 // bottom speeds SPEEDU/SPEEDV (ocvisc.f90:53-104): evaluated at the single
 // level where the mask drops from 1 to 0 (or at KE when the column is full)
 __global__ void k_visc_speed(Geo G, const double* __restrict__ uoo, const double* __restrict__ voe,
@@ -549,8 +545,9 @@ __global__ void __launch_bounds__(kVertBlock) k_visc_uv_b(Geo G, const double* _
 
 // implicit vertical diffusion of w, levels 2..KE (ocvisc.f90:225-270); the
 // levels 1 and KEP are carried.  Row K of the solve is level K + 1.
+// (Up to 48 levels two blocks fit an SM: 64 registers a thread.)
 template <typename Ln>
-__global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restrict__ Wi,
+__global__ void __launch_bounds__(Ln::NT, Ln::LC <= 3 ? 2 : 1) k_visc_w(Geo G, const double* __restrict__ Wi,
                                                    const double* __restrict__ avo,
                                                    double* __restrict__ O, double* bad) {
   constexpr int LC = Ln::LC;
@@ -578,13 +575,11 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
   const int kb = interior ? G.gp.kb[ij] : 0;
   const double bot = interior ? G.gp.bot[ij] : 0.;
   auto thickness = [&](int K) { return K < kb ? G.dzw[K - 1] : (K == kb ? bot : 0.0); };
-  auto rden = [&](int K) {
-    return div_nr(1., 2.0 * G.almzer + thickness(K - 1) + thickness(K));
-  };
+  auto den = [&](int K) { return 2.0 * G.almzer + thickness(K - 1) + thickness(K); };
   // TRIDSY(K,3) from AVO of levels K and K + 1
-  auto lower = [&](int K, double a0, double a1, double rd) {
+  auto lower = [&](int K, double a0, double a1, double dn, double rd) {
     const double avlo = K < KE && K <= kb ? 0.5 * (a1 + a0) : 0.0;
-    return -2.0 * G.dt * avlo * G.di[K - 1] * rd;
+    return quotient(-2.0 * G.dt * avlo * G.di[K - 1], dn, rd);
   };
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
@@ -594,15 +589,15 @@ __global__ void __launch_bounds__(Ln::NT) k_visc_w(Geo G, const double* __restri
     c[u] = 0. * (av[u + 1] + av[u + 2]);
     b[u] = 1. - a[u] - c[u];
     if (K <= KE && K <= kb) {
-      const double rd = rden(K);
-      a[u] = -2.0 * G.dt * (0.5 * (av[u] + av[u + 1])) * G.di[K - 2] * rd;
-      c[u] = lower(K, av[u + 1], av[u + 2], rd);
+      const double dn = den(K), rd = div_nr(1., dn);
+      a[u] = quotient(-2.0 * G.dt * (0.5 * (av[u] + av[u + 1])) * G.di[K - 2], dn, rd);
+      c[u] = lower(K, av[u + 1], av[u + 2], dn, rd);
       b[u] = 1. - a[u] - c[u];
       if (K == 2) a[u] = 0.;
     }
   }
   const int Kp = t.K0 + 1;  // the level above the thread's first
-  const double cprev = Kp >= 2 && Kp < KE && Kp <= kb ? lower(Kp, av[0], av[1], rden(Kp)) : 0.;
+  const double cprev = Kp >= 2 && Kp < KE && Kp <= kb ? lower(Kp, av[0], av[1], den(Kp), div_nr(1., den(Kp))) : 0.;
   bool ok = true;
   if (valid && t.g == 0) ok = finite(Wi[G.L.at(i, j, 0)]);
   if (valid && !interior) {

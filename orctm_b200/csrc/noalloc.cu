@@ -93,9 +93,9 @@ __global__ void __launch_bounds__(Ln::NT) k_na_vert(NaArgs a, const double* __re
   const bool above = interior && t.K0 > 0 && t.K0 < KE;
   const double thp = above ? a.ddpo[base - pl] : 0.;
   const double zo = interior ? a.zo[p2(a, i, j)] : 0.;
-  auto rden = [&](int K, double dd) {
+  auto den = [&](int K, double dd) {
     const double zzsurf = K == 1 ? 1. : 0.;
-    return 1. / (dd + zzsurf * (zo) + a.almzer);
+    return dd + zzsurf * (zo) + a.almzer;
   };
 #pragma unroll
   for (int u = 0; u < LC; ++u) {
@@ -103,14 +103,14 @@ __global__ void __launch_bounds__(Ln::NT) k_na_vert(NaArgs a, const double* __re
     ta[u] = tc[u] = 0.;
     tb[u] = 1.;
     if (interior && K <= KE) {
-      const double rd = rden(K, th[u]);
-      ta[u] = -a.dt * d[u] * wt[u] * a.di[K - 1] * rd;
-      tc[u] = -a.dt * d[u + 1] * a.di[K] * rd;
+      const double dn = den(K, th[u]), rd = div_nr(1., dn);
+      ta[u] = quotient(-a.dt * d[u] * wt[u] * a.di[K - 1], dn, rd);
+      tc[u] = quotient(-a.dt * d[u + 1] * a.di[K], dn, rd);
       tb[u] = 1. - ta[u] - tc[u];
       if (K == 1) ta[u] = 0.;
     }
   }
-  const double cprev = above ? -a.dt * d[0] * a.di[t.K0] * rden(t.K0, thp) : 0.;
+  const double cprev = above ? -a.dt * d[0] * a.di[t.K0] / den(t.K0, thp) : 0.;
   if (valid && !interior) {
 #pragma unroll
     for (int u = 0; u < LC; ++u)
