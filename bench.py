@@ -35,14 +35,14 @@ FALLBACK_HBM_GBS = 6650.0
 # Algorithmic bytes per interior cell per launch of each launcher group
 # (each distinct array the math needs read once, each output written once;
 # thickness/mask geometry is compressed to 2D and counts 0 B).  The Poisson
-# iteration works on the black columns' vectors (half of the cells): "pcg_spmv" is
-# the black kernel (x, p, z, u in; x, p, q out), "pcg_col" the average over the red
-# kernel (z, u in; u out; pivots in doubles), the column kernel (r, q in; r, z out; pivots
-# in floats) and the coarse correction, which moves planes only.
+# iteration works on the vectors of one colour's columns (half of the cells): "pcg_red"
+# is the red kernel (z, u in; u out; pivots in doubles), "pcg_spmv" the black one
+# (x, p, z, u in; x, p, q out), "pcg_col" the column kernel (r, q in; r, z out; pivots in
+# floats); the coarse correction ("pcg_coarse") moves planes only.
 BYTES_PER_CELL_F64 = {
     "ocuad": 40, "ocvad": 40, "ocwad": 40, "ocadpo": 40,
     "ocvisc": 56, "nh_rhs": 56, "nh_post": 56,
-    "pcg_spmv": 28, "pcg_col": (16 + 18 + 0) / 3, "resid": 24,
+    "pcg_red": 16, "pcg_spmv": 28, "pcg_col": 18, "resid": 24,
 }
 
 
@@ -58,8 +58,8 @@ def workload_config(inst: dict) -> dict:
             "cells_per_gpu": cells, "tracers": inst["ntracers"],
             "l2": "inputs larger than L2 (each 3D field "
                   f"{8 * cells / 1e9:.2f} GB vs 126 MB L2)",
-            "solver": "FP64 PCG (line preconditioner, scaled operator) in "
-                      "double-double-residual refinement"}
+            "solver": "FP64 CG on the red-black reduced system (column preconditioner with a "
+                      "coarse space) in double-double-residual refinement"}
 
 
 def log(*a):

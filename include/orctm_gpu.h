@@ -442,8 +442,12 @@ int orctm_timer_stop(orctm_handle* h, double* ms);
 enum {
   ORCTM_PROF_OCUAD = 0, ORCTM_PROF_OCVAD, ORCTM_PROF_OCWAD, ORCTM_PROF_OCADPO,
   ORCTM_PROF_OCTDIFF, ORCTM_PROF_OCVISC, ORCTM_PROF_NH_RHS, ORCTM_PROF_PCG_SPMV,
-  ORCTM_PROF_PCG_COL, ORCTM_PROF_RESID, ORCTM_PROF_NH_POST, ORCTM_PROF_KINDS
+  ORCTM_PROF_PCG_COL, ORCTM_PROF_RESID, ORCTM_PROF_NH_POST, ORCTM_PROF_PCG_RED,
+  ORCTM_PROF_PCG_COARSE, ORCTM_PROF_PCG_ENDS, ORCTM_PROF_KINDS
 };
+/* The Poisson iteration's kernels: PCG_RED the red columns, PCG_SPMV the black ones'
+ * operator, PCG_COL the black columns' solve, PCG_COARSE the coarse correction (where
+ * the solver uses it); PCG_ENDS the two kernels before and the two after the iterations. */
 int orctm_set_profiling(orctm_handle* h, int on);
 int orctm_profile_get(orctm_handle* h, int kind, long long* launches, double* total_ms);
 

@@ -137,7 +137,7 @@ EXPORTS = (
 )
 
 PROF_KINDS = ("ocuad", "ocvad", "ocwad", "ocadpo", "octdiff", "ocvisc", "nh_rhs", "pcg_spmv",
-              "pcg_col", "resid", "nh_post")
+              "pcg_col", "resid", "nh_post", "pcg_red", "pcg_coarse", "pcg_ends")
 
 _lib = None
 

@@ -81,17 +81,17 @@ __device__ __forceinline__ double wet(const ColGeo& c, int ij, int K) {
 }
 __device__ __forceinline__ bool wetb(const ColGeo& c, int ij, int K) { return K <= c.kb[ij]; }
 
+// the division itself, out of line: for the rare operands that the forms below leave to it
+static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+
 // a / b by Newton-Raphson refinement of a hardware reciprocal estimate
 // (rcp.approx.ftz.f64), two iterations r <- r + r (1 - b r), then one
 // residual correction q <- q + r (a - b q) (the quotient refinement of
 // P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", IBM J. Res. Develop. 34 (1990) 111-119).  The
 // result is within 1 ulp of the correctly rounded quotient (checked against
-// IEEE division by orctm_check_division).  Denominators that are zero,
-// subnormal, infinite, NaN or near the ends of the range take the IEEE division.
-static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
-
-// the refinement alone, for denominators known to be no smaller than 1e-290
+// IEEE division by orctm_check_division).
+// This form is the refinement alone, for denominators known to be no smaller than 1e-290
 // (up to 1e300; an infinity or NaN gives NaN, as a quotient of infinities does)
 __device__ __forceinline__ double div_in_range(double a, double b) {
   double r;
@@ -104,6 +104,8 @@ __device__ __forceinline__ double div_in_range(double a, double b) {
   return __fma_rn(r, __fma_rn(-b, q, a), q);
 }
 
+// for any operands: denominators that are zero, subnormal, infinite, NaN or near the
+// ends of the range take the IEEE division
 __device__ __forceinline__ double div_nr(double a, double b) {
   // exponent between -991 and 992, by the integer pipe: the double-precision
   // comparisons cost as much as the refinement's steps
@@ -133,8 +135,9 @@ __device__ __forceinline__ bool finite(double x) {
   return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u;
 }
 
-// The same with r = 1 / b by any means and any b, without the division: for |a| below 1e-290
-// it may be off by an ulp; by or of an infinity, or by 0, the product is the quotient.
+// a / b as by div_by, with r = 1 / b by any means for any b and without the division: for
+// |a| below 1e-290 it may be off by an ulp; by or of an infinity, or by 0, the product is
+// the quotient.
 __device__ __forceinline__ double quotient(double a, double b, double r) {
   const double q0 = a * r, q = __fma_rn(__fma_rn(-b, q0, a), r, q0);
   return finite(q) ? q : q0;

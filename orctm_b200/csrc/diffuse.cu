@@ -452,7 +452,7 @@ __device__ __forceinline__ void visc_uv(const Geo& G, const double* __restrict__
   const double BOFRIC = 3.E-3, RAYFRIC = 3.E-3;
   const double sp = speed[ij];
   // TRIDSY(K,1) and TRIDSY(K,3) from AVO of levels K (a0, b0) and K+1 (a1, b1)
-  // of the two columns, as k_visc_uv's tri
+  // of the two columns
   auto tri = [&](int K, double a0, double b0, double a1, double b1, double& t1, double& t3) {
     const double am = wet(cg, ij, K), dd = thick(cg, G.dzw, ij, K);
     const double avup = 0.5 * (a0 + b0) * am;

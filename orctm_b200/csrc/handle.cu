@@ -865,10 +865,10 @@ RbVectors<float>& rb_vectors<float>(orctm_handle* h) { return h->v32; }
 template <typename T>
 void pcg_iteration(orctm_handle* h) {
   const RbVectors<T>& v = rb_vectors<T>(h);
-  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_red<T>(h->R, h->S, v, h->stream));
+  PROF(h, ORCTM_PROF_PCG_RED, launch_rb_red<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_SPMV, launch_rb_black<T>(h->R, h->S, v, h->stream));
   PROF(h, ORCTM_PROF_PCG_COL, launch_rb_col<T>(h->R, h->S, v, h->stream));
-  if (v.coarse) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
+  if (v.coarse) PROF(h, ORCTM_PROF_PCG_COARSE, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
 }
 
 template <typename T>
@@ -930,7 +930,7 @@ int check_waits(orctm_handle* h) {
 template <typename T>
 int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   const RbVectors<T>& v = rb_vectors<T>(h);
-  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_before<T>(h->R, h->S, h->r, v, h->stream));
+  PROF(h, ORCTM_PROF_PCG_ENDS, launch_rb_before<T>(h->R, h->S, h->r, v, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   int st;
   // the loop on the device: chunks of kPcgChunk iterations replayed by a
@@ -944,7 +944,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
     it = h->hS->iter;
     conv = h->hS->converged;
   } else {
-    if (v.coarse) PROF(h, ORCTM_PROF_PCG_COL, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
+    if (v.coarse) PROF(h, ORCTM_PROF_PCG_COARSE, launch_rb_coarse<T>(h->R, h->S, v, h->stream));
     ORCTM_CUDA_OK(cudaGetLastError());
   }
   if (!small && !h->prof && maxit >= kPcgChunk) {
@@ -969,7 +969,7 @@ int pcg_loop(orctm_handle* h, int maxit, int* iters) {
   }
   *iters = h->hS->iter;
   if ((st = check_waits(h))) return st;
-  PROF(h, ORCTM_PROF_PCG_COL, launch_rb_after<T>(h->R, h->S, v, h->xs, h->stream));
+  PROF(h, ORCTM_PROF_PCG_ENDS, launch_rb_after<T>(h->R, h->S, v, h->xs, h->stream));
   ORCTM_CUDA_OK(cudaGetLastError());
   return ORCTM_OK;
 }

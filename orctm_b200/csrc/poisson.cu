@@ -21,7 +21,8 @@
 // and conjugate gradients on S preconditioned with D_b take half the
 // iterations that they take on B preconditioned with D (the two have the same
 // spectrum up to lambda -> lambda (2 - lambda)), with vectors of half the
-// length.  One iteration is three kernels:
+// length.  One iteration is three kernels (and on planes a fourth, the coarse
+// correction of z, below):
 //     red     u = D_r^-1 C_rb z + beta u        (u = D_r^-1 C_rb p)
 //     black   x += alpha p ; p = z + beta p ; q = D_b p - C_br u ; p.q
 //     column  r -= alpha q ; z = D_b^-1 r ; r.z, r.r
@@ -35,7 +36,7 @@
 // the other: offset ((j NT + b) KE + l) W + c, b W + c = m - 1.  A tile is some 10 KB
 // of consecutive memory; in the padded layout of the model's fields its levels lie
 // megabytes apart on 1024 x 1024 x 80, where every block then touched some 80
-// pages per vector (stencil kernel 1.65 ms a launch; see below).  The in-row
+// pages per vector (the operator's kernel took 1.65 ms a launch so).  The in-row
 // neighbours of column (m, j) are (m - 1 + s, j) and (m + s, j) of the other
 // colour, s = 0 or 1 by the parity of the row; north and south are (m, j -+ 1).
 //

@@ -1,6 +1,6 @@
-"""How the conjugate-gradient loop of the pressure solve ends when it cannot go
-on, in its two forms (one kernel on small grids; separate kernels, which
-profiling selects)."""
+"""The conjugate-gradient loop of the pressure solve: its two forms (one kernel on
+small grids; separate kernels, which profiling selects) give the same values, and how
+it ends when it cannot go on."""
 import numpy as np
 import pytest
 
@@ -87,3 +87,21 @@ def test_both_forms_of_the_loop_agree_for_every_split_of_a_column(nz, mode):
         gpu.close()
     assert got[0][:2] == got[1][:2]
     assert np.array_equal(got[0][2], got[1][2])
+
+
+@pytest.mark.parametrize("nx,ny,nz,coarse", [(45, 21, 50, False), (34, 34, 105, True)])
+def test_profile_tells_the_kernels_of_an_iteration_apart(nx, ny, nz, coarse):
+    """Red, black and column kernel as often as each other, the coarse correction once
+    more where there is one, and one record before and one after each correction."""
+    inst = C.make_instance("c2", builder=grid.build_grid, nx=nx, ny=ny, nz=nz)
+    gpu = Instance(inst)
+    gpu.upload_state(C.copy_state(inst))
+    gpu.set_solver("fp64", rtol=1e-12, maxit=20000)
+    gpu.set_profiling(True)
+    stats = gpu.ocvtot_nh()
+    n = {k: v["launches"] for k, v in gpu.profile().items()}
+    gpu.close()
+    assert n["pcg_red"] == n["pcg_spmv"] == n["pcg_col"] >= stats["iterations"] > 0
+    assert n["pcg_coarse"] == (n["pcg_red"] + stats["outer_iterations"] if coarse else 0)
+    assert n["pcg_ends"] == 2 * stats["outer_iterations"]
+    assert n["resid"] == stats["outer_iterations"] + 1
