@@ -339,13 +339,16 @@ def run_whole_step(inst, cells, args, ws, rank, pg, local, hot_ms_per_step):
     barrier(pg)
     ms = max_over_ranks(pg, ms)
     # the hot path's share in this state (its solve takes more iterations than
-    # in the headline state): per-launcher device time of the hot-path
-    # kernels over a few more, untimed whole steps
+    # in the headline state): the timed steps' solves, and the device time of the
+    # other launchers over a few more, untimed whole steps (with per-launcher timing
+    # the solve's loop runs from the host, on small grids several times as long)
     nprof = min(args.steps, 3)
     gpu.set_profiling(True)
     for s in range(nprof):
         gpu.step_full(args.warmup + args.steps + s + 1, check_contra=False)
-    hot_in_whole = sum(v["ms"] for v in gpu.profile().values()) / nprof
+    hot_in_whole = sum(v["ms"] for k, v in gpu.profile().items()
+                       if not k.startswith("pcg_") and k != "resid") / nprof
+    hot_in_whole += statistics.mean(s["solve_ms"] for s in stats)
     gpu.set_profiling(False)
     hot_in_whole = max_over_ranks(pg, hot_in_whole)
     gpu.close()
@@ -354,9 +357,8 @@ def run_whole_step(inst, cells, args, ws, rank, pg, local, hot_ms_per_step):
             "ms_per_step": per, "hot_path_ms_per_step": hot_in_whole,
             "before_hot_path_ms_per_step": per - hot_in_whole,
             "headline_hot_path_ms_per_step": hot_ms_per_step,
-            "hot_path_basis": f"sum of the hot-path launchers' CUDA-event times over {nprof} more "
-                              "whole steps with per-launcher timing on (the solve's loop then "
-                              "runs from the host), so the split slightly favours the hot path",
+            "hot_path_basis": "the timed steps' solve times, plus the other hot-path launchers' "
+                              f"CUDA-event times over {nprof} more whole steps",
             "poisson_iterations": statistics.mean(s["iterations"] for s in stats),
             "contra_max": max(s["contra"] for s in stats),
             "steps_above_contra_limit": sum(bool(s["unstable"]) for s in stats),
@@ -477,7 +479,11 @@ def main():
     # ---- roofline of the dominant kernel --------------------------------
     hbm, peak_kind = peaks()
     top = max((k for k in prof if prof[k]["launches"] > 0), key=lambda k: prof[k]["ms"])
-    per_launch_ms = prof[top]["ms"] / prof[top]["launches"]
+    # the solver's kernels are launched four iterations at a time; those after the
+    # last iteration return at once, so theirs is the time of an iteration
+    its = sum(st["iterations"] for st in stats)
+    runs = its if top in ("pcg_red", "pcg_spmv", "pcg_col") else prof[top]["launches"]
+    per_launch_ms = prof[top]["ms"] / runs
     # algorithmic bytes per cell x the cells of a launch; the solver kernels
     # skip the land rows among them (decoupled, exact zeros), which the
     # measured traffic shows
