@@ -342,7 +342,9 @@ struct Dot {
       part = T(0);
     }
   }
-  __device__ __forceinline__ double total() const { return sum + (double)part; }
+  __device__ __forceinline__ double total() const {
+    return sizeof(T) == 4 ? sum + (double)part : (double)part;
+  }
 };
 
 // v <- M^-1 v for the column tridiagonal M = L D L^T with pivots 1/d (dm: the
